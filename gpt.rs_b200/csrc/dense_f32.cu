@@ -11,7 +11,7 @@
 // each load instruction of a warp is one contiguous 128-byte row segment and no alignment of
 // N is needed), warps split the K rows, partial sums meet in shared memory and, when K is
 // split across a thread-block cluster, through distributed shared memory.
-#include "matmul_common.cuh"
+#include "split_f32.cuh"
 
 namespace gptrs {
 namespace {
@@ -343,7 +343,11 @@ int launch_sgemm(SgemmParams p, int batch, cudaStream_t st) {
     return launch_kernel(kern, grid, dim3(kSgWarps * 32), smem, st, p.n_split, p);
 }
 
-int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st) {
+int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st, int32_t* status) {
+    if (p.norm_kind == 0) {
+        const SplitF32Params q = {p.x, p.w, p.bias, p.residual, p.y, p.M, p.N, p.K, p.act, p.dense, p.ldx, p.ldy, p.x_step, p.y_step, batch, status};
+        if (split_f32_takes(q)) return split_f32_matmul(q, st);
+    }
     if (p.M == 1) return launch_sgemm<1>(p, batch, st);
     if (p.M == 2) return launch_sgemm<2>(p, batch, st);
     if (p.M <= 4) return launch_sgemm<4>(p, batch, st);
@@ -351,6 +355,24 @@ int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st) {
 }
 
 }  // namespace
+
+// gptrs_cuda_norm_matmul_f32 with the status word of the caller (null: the library's)
+int norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps,
+                    const float* d_w, float* d_y, int64_t m, int64_t n, int64_t k, const float* d_bias,
+                    const float* d_residual, int gelu, int32_t* d_status, cudaStream_t st) {
+    GPTRS_REQUIRE(d_x && d_w && d_y, "null pointer");
+    GPTRS_REQUIRE(m >= 0 && n > 0 && k > 0 && n < (1ll << 31) && k < (1ll << 31) && m < (1ll << 31), "bad shape");
+    GPTRS_REQUIRE(norm_kind >= 0 && norm_kind <= 2 && (norm_kind == 0 || d_gamma), "norm_kind 0 (none), 1 (layer norm) or 2 (rms norm) with a gain");
+    GPTRS_REQUIRE(!(norm_kind != 0 && d_residual == d_x), "a normalised input cannot also be the in-place residual target");
+    if (m == 0) return GPTRS_OK;
+    SgemmParams p = {};
+    p.x = d_x; p.w = d_w; p.bias = d_bias; p.residual = d_residual; p.y = d_y;
+    p.M = (int)m; p.N = (int)n; p.K = (int)k; p.act = gelu ? 1 : 0;
+    p.norm_kind = norm_kind; p.norm_gamma = d_gamma; p.norm_beta = norm_kind == 1 ? d_beta : nullptr; p.norm_eps = eps;
+    p.ldx = k; p.ldy = n;
+    return run_sgemm(p, 1, st, d_status);
+}
+
 }  // namespace gptrs
 
 using namespace gptrs;
@@ -365,17 +387,7 @@ int gptrs_cuda_matmul_f32(const float* d_x, const float* d_w, float* d_y, int64_
 int gptrs_cuda_norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps,
                                const float* d_w, float* d_y, int64_t m, int64_t n, int64_t k, const float* d_bias,
                                const float* d_residual, int gelu, void* stream) {
-    GPTRS_REQUIRE(d_x && d_w && d_y, "null pointer");
-    GPTRS_REQUIRE(m >= 0 && n > 0 && k > 0 && n < (1ll << 31) && k < (1ll << 31) && m < (1ll << 31), "bad shape");
-    GPTRS_REQUIRE(norm_kind >= 0 && norm_kind <= 2 && (norm_kind == 0 || d_gamma), "norm_kind 0 (none), 1 (layer norm) or 2 (rms norm) with a gain");
-    GPTRS_REQUIRE(!(norm_kind != 0 && d_residual == d_x), "a normalised input cannot also be the in-place residual target");
-    if (m == 0) return GPTRS_OK;
-    SgemmParams p = {};
-    p.x = d_x; p.w = d_w; p.bias = d_bias; p.residual = d_residual; p.y = d_y;
-    p.M = (int)m; p.N = (int)n; p.K = (int)k; p.act = gelu ? 1 : 0;
-    p.norm_kind = norm_kind; p.norm_gamma = d_gamma; p.norm_beta = norm_kind == 1 ? d_beta : nullptr; p.norm_eps = eps;
-    p.ldx = k; p.ldy = n;
-    return run_sgemm(p, 1, as_stream(stream));
+    return norm_matmul_f32(d_x, norm_kind, d_gamma, d_beta, eps, d_w, d_y, m, n, k, d_bias, d_residual, gelu, nullptr, as_stream(stream));
 }
 
 int gptrs_cuda_dense_f32(const float* d_x, const float* d_w, float* d_y, int64_t m, int64_t n, int64_t k, const gptrs_dense_epilogue* ep, void* stream) {
@@ -397,7 +409,7 @@ int gptrs_cuda_dense_f32(const float* d_x, const float* d_w, float* d_y, int64_t
         p.x_step = p.y_step = 0;
         return launch_sgemm<8>(p, (int)ep->max_tiles, as_stream(stream));
     }
-    return run_sgemm(p, ep->batch > 1 ? (int)ep->batch : 1, as_stream(stream));
+    return run_sgemm(p, ep->batch > 1 ? (int)ep->batch : 1, as_stream(stream), ep->d_status);
 }
 
 int gptrs_cuda_kv_append_f32(const float* d_qkv, const int32_t* d_positions, const int32_t* d_slot, float* d_k_cache,

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "split_f32.cuh"
 
 namespace gptrs {
 
@@ -206,10 +207,10 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
            bool pick = false) {
     ++m.launches;
     if (m.f32()) {
-        return gptrs_cuda_norm_matmul_f32(static_cast<const float*>(x), fold ? fold->f32_norm : 0, fold ? fold->f32_gamma : nullptr,
+        return norm_matmul_f32(static_cast<const float*>(x), fold ? fold->f32_norm : 0, fold ? fold->f32_gamma : nullptr,
                                           fold ? fold->f32_beta : nullptr, m.cfg.norm_eps, static_cast<const float*>(w.f32->data),
                                           static_cast<float*>(y), rows, w.out, w.in,
-                                          w.bias ? static_cast<const float*>(w.bias->data) : nullptr, residual, gelu ? 1 : 0, st);
+                                          w.bias ? static_cast<const float*>(w.bias->data) : nullptr, residual, gelu ? 1 : 0, m.d_status.as<int32_t>(), st);
     }
     gptrs_matmul_epilogue ep = {};
     ep.out_dtype = out_f32 ? GPTRS_F32 : GPTRS_BF16;
@@ -314,7 +315,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     cudaStream_t st = m.stream;
     float* hidden = m.hidden.as<float>();
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
-    if (m.mega_on && T == 1 && n_rows == 1 && rows_identity && !prefill_groups) {
+    if (m.mega_on && T == 1 && n_rows == 1 && !prefill_groups) {
         // one sequence, one token: the whole step is one cooperative kernel (+ the memset of its barrier word)
         MegaParams P = m.mega;
         P.greedy = temperature <= 0.f ? 1 : 0;
@@ -367,7 +368,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         return f;
     };
     // f32 models on one rank: the norm before a projection is computed by the projection itself while it stages x
-    const bool fold32 = m.fold_norm && m.f32() && m.tp == 1;
+    const bool fold32 = m.fold_norm && m.f32() && m.tp == 1 && T < kSplitF32Rows;
     auto fold32_for = [&](Tensor* g, Tensor* b) {
         NormFold f;
         f.f32_norm = gpt ? 1 : 2;
@@ -467,6 +468,9 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         if (m.f32()) {
             float* kc = m.k_cache.as<float>() + (size_t)l * m.cache_layer_elems;
             float* vc = m.v_cache.as<float>() + (size_t)l * m.cache_layer_elems;
+            if (!rows_identity && attention_rows_f32_takes(ln.T, c.head_dim))   // rows of prompts share the keys of their sequence
+                return attention_rows_f32(reinterpret_cast<float*>(at(m.qkv, (size_t)m.QKV() * 4, ln)), kc, vc, ints(m.d_pos, ln), ints(m.d_slot, ln),
+                                          static_cast<float*>(out), ln.T, c.n_q_heads, c.n_kv_heads, c.head_dim, c.context_length, ln.st);
             auto attend = rows_identity ? gptrs_cuda_kv_append_attention_decode_f32
                                         : [](const float* q, float* k, float* v, const int32_t* pos, const int32_t* sl, float* o, int64_t t,
                                              int64_t hq, int64_t hkv, int64_t hd, int64_t cap, void* st) {

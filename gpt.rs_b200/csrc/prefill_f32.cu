@@ -1,0 +1,176 @@
+// Attention of prompt rows in f32 over the dense KV cache (attention_decode_cache, crates/gpt-rs/src/ops/functional/attention.rs:657-779,
+// for every row of a prompt): a CTA takes one query head of 32 neighbouring rows, so that a key is read once for up to 32 queries
+// instead of once for each.
+//
+// 128 threads, 32 x 64 scores per block of keys with a 4 x 4 tile per thread (operands in shared memory, 16-byte reads: 4 + 4 of them
+// feed 64 fused multiply-adds), online softmax in f32 over the 16 threads of a row, then 4 rows x HD / 16 columns of the output per
+// thread. 109 us for 937 rows of 12 heads of 64 (464 with a CTA per row and head), a chain of up to 15 blocks in the last rows' CTAs.
+// Rows of a tile that belong to different sequences are taken one sequence after another.
+#include "common.cuh"
+
+namespace gptrs {
+namespace {
+
+struct PrefillF32Params {
+    const float* qkv;   // [T][(Hq + 2 Hkv) * hd]; only the Q part is read
+    const float* k_cache;
+    const float* v_cache;
+    const int* positions;
+    const int* slot;
+    float* out;         // [T][Hq * hd]
+    int T, Hq, Hkv, capacity;
+    float scale;
+};
+
+constexpr int kPfRows = 32, kPfKeys = 64, kPfThreads = 4 * kPfRows;
+
+template <int HD>
+__global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const PrefillF32Params p) {
+    constexpr int LD = HD + 4, LP = kPfKeys + 4, OC = HD / 64;   // OC float4 columns of a thread
+    extern __shared__ __align__(16) float pf_smem[];
+    float* qs = pf_smem;                   // [32][LD]
+    float* ks = qs + kPfRows * LD;         // [64][LD]
+    float* vs = ks + kPfKeys * LD;         // [64][LD]
+    float* ps = vs + kPfKeys * LD;         // [32][LP]
+    __shared__ int pos_s[kPfRows], slot_s[kPfRows];
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * kPfRows;   // the last rows see the most keys: they start first
+    const int h = blockIdx.y, hk = h / (p.Hq / p.Hkv), rows = min(kPfRows, p.T - t0);
+    const int width = (p.Hq + 2 * p.Hkv) * HD;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (tid < kPfRows) {
+        slot_s[tid] = tid < rows ? p.slot[t0 + tid] : -1;
+        pos_s[tid] = tid < rows ? min(max(p.positions[t0 + tid], 0), p.capacity - 1) : -1;   // DynamicUpdateSlice clamps its start
+    }
+    for (int i = tid; i < kPfRows * (HD / 4); i += kPfThreads) {
+        const int r = i / (HD / 4), c = i % (HD / 4) * 4;
+        *reinterpret_cast<float4*>(qs + r * LD + c) =
+            r < rows ? *reinterpret_cast<const float4*>(p.qkv + (size_t)(t0 + r) * width + h * HD + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    float o[4][4 * OC], mx[4], sum[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        mx[r] = -INFINITY; sum[r] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4 * OC; ++c) o[r][c] = 0.f;
+    }
+    for (int seg = 0; seg < rows;) {   // runs of rows of one sequence
+        const int slot = slot_s[seg];
+        int end = seg, last = 0;
+        for (; end < rows && slot_s[end] == slot; ++end) last = max(last, pos_s[end]);
+        const float* kc = p.k_cache + ((size_t)slot * p.Hkv + hk) * p.capacity * HD;
+        const float* vc = p.v_cache + ((size_t)slot * p.Hkv + hk) * p.capacity * HD;
+        int limit[4];   // last visible key of this thread's rows in this run
+#pragma unroll
+        for (int r = 0; r < 4; ++r) limit[r] = 4 * ty + r >= seg && 4 * ty + r < end ? pos_s[4 * ty + r] : -1;
+        for (int j0 = 0; j0 <= last; j0 += kPfKeys) {
+            __syncthreads();   // the block before has been used
+            for (int i = tid; i < kPfKeys * (HD / 4); i += kPfThreads) {
+                const int j = i / (HD / 4), c = i % (HD / 4) * 4;
+                const bool in = j0 + j <= last;
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                *reinterpret_cast<float4*>(ks + j * LD + c) = in ? *reinterpret_cast<const float4*>(kc + (size_t)(j0 + j) * HD + c) : zero;
+                *reinterpret_cast<float4*>(vs + j * LD + c) = in ? *reinterpret_cast<const float4*>(vc + (size_t)(j0 + j) * HD + c) : zero;
+            }
+            __syncthreads();
+            float s[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[r][j] = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < HD; c += 4) {
+                float4 q[4], k[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) q[r] = *reinterpret_cast<const float4*>(qs + (4 * ty + r) * LD + c);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) k[j] = *reinterpret_cast<const float4*>(ks + (tx + 16 * j) * LD + c);
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        s[r][j] = fmaf(q[r].x, k[j].x, s[r][j]); s[r][j] = fmaf(q[r].y, k[j].y, s[r][j]);
+                        s[r][j] = fmaf(q[r].z, k[j].z, s[r][j]); s[r][j] = fmaf(q[r].w, k[j].w, s[r][j]);
+                    }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                float top = mx[r];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    s[r][j] = j0 + tx + 16 * j <= limit[r] ? s[r][j] * p.scale : -INFINITY;
+                    top = fmaxf(top, s[r][j]);
+                }
+#pragma unroll
+                for (int off = 8; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+                const float base = top == -INFINITY ? 0.f : top;   // nothing visible so far
+                const float keep = expf(mx[r] - base);
+                mx[r] = top;
+                float part = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float e = j0 + tx + 16 * j <= limit[r] ? expf(s[r][j] - base) : 0.f;
+                    ps[(4 * ty + r) * LP + tx + 16 * j] = e;
+                    part += e;
+                }
+#pragma unroll
+                for (int off = 8; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+                sum[r] = sum[r] * keep + part;
+#pragma unroll
+                for (int c = 0; c < 4 * OC; ++c) o[r][c] *= keep;
+            }
+            __syncwarp();   // the 16 threads of a row write and read its weights, and they are in one warp
+#pragma unroll 4
+            for (int j = 0; j < kPfKeys; j += 4) {
+                float4 e[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) e[r] = *reinterpret_cast<const float4*>(ps + (4 * ty + r) * LP + j);
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+                    for (int c = 0; c < OC; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(vs + (j + jj) * LD + 4 * tx + 64 * c);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const float w = jj == 0 ? e[r].x : jj == 1 ? e[r].y : jj == 2 ? e[r].z : e[r].w;
+                            o[r][4 * c] = fmaf(w, v.x, o[r][4 * c]); o[r][4 * c + 1] = fmaf(w, v.y, o[r][4 * c + 1]);
+                            o[r][4 * c + 2] = fmaf(w, v.z, o[r][4 * c + 2]); o[r][4 * c + 3] = fmaf(w, v.w, o[r][4 * c + 3]);
+                        }
+                    }
+            }
+        }
+        seg = end;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        if (4 * ty + r >= rows) continue;
+        const float inv = sum[r];
+#pragma unroll
+        for (int c = 0; c < OC; ++c)
+            *reinterpret_cast<float4*>(p.out + ((size_t)(t0 + 4 * ty + r) * p.Hq + h) * HD + 4 * tx + 64 * c) =
+                make_float4(o[r][4 * c] / inv, o[r][4 * c + 1] / inv, o[r][4 * c + 2] / inv, o[r][4 * c + 3] / inv);
+    }
+}
+
+template <int HD>
+int launch(const PrefillF32Params& p, cudaStream_t st) {
+    constexpr size_t smem = (size_t)((kPfRows + 2 * kPfKeys) * (HD + 4) + kPfRows * (kPfKeys + 4)) * sizeof(float);
+    static PerDeviceOnce attr_once;
+    if (attr_once.first_time()) GPTRS_CUDA_OK(cudaFuncSetAttribute(attention_rows_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return launch_kernel(attention_rows_f32_kernel<HD>, dim3((unsigned)ceil_div(p.T, kPfRows), (unsigned)p.Hq), dim3(kPfThreads), smem, st, 1, p);
+}
+
+}  // namespace
+
+bool attention_rows_f32_takes(int64_t n_tokens, int64_t head_dim) { return n_tokens >= 8 && (head_dim == 64 || head_dim == 128); }
+
+int attention_rows_f32(const float* qkv, const float* k_cache, const float* v_cache, const int32_t* positions, const int32_t* slot, float* out,
+                       int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st) {
+    const PrefillF32Params p = {qkv, k_cache, v_cache, positions, slot, out, (int)n_tokens, (int)n_q_heads, (int)n_kv_heads, (int)capacity,
+                                1.0f / sqrtf((float)head_dim)};
+    return head_dim == 64 ? launch<64>(p, st) : launch<128>(p, st);
+}
+
+}  // namespace gptrs

@@ -1,0 +1,27 @@
+// f32 matmul on the tcgen05 tensor cores (split_f32.cu), called by dense_f32.cu for more than a few rows.
+#pragma once
+#include "matmul_common.cuh"
+
+namespace gptrs {
+
+struct SplitF32Params {
+    const float* x;         // [M][K], rows ldx apart
+    const float* w;         // [K][N]
+    const float* bias;      // optional [N]
+    const float* residual;  // optional [M][N]
+    float* y;               // [M][N], rows ldy apart
+    int M, N, K;
+    int act;                // 1: gelu (erf)
+    DenseAct dense;
+    int64_t ldx, ldy, x_step, y_step;   // steps between the entries of a batch; their weights follow each other
+    int batch;
+    int* status;            // code 3: a bounded wait gave up
+    int m_tiles, n_split;   // set by the launcher
+};
+
+// Least rows, and whether it takes this shape (the rule stands at its definition).
+constexpr int kSplitF32Rows = 24;
+bool split_f32_takes(const SplitF32Params& p);
+int split_f32_matmul(SplitF32Params p, cudaStream_t st);
+
+}  // namespace gptrs

@@ -1,0 +1,96 @@
+"""f32 matmuls of many rows on the tensor cores (three bf16 terms per value) and the f32 attention of prompt rows, at the edges of their
+tiles, against float64."""
+import numpy as np
+import pytest
+import torch
+
+from gptrs_b200 import model as gm, ops
+from oracle import models_ref as mr
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(x, w, extra):
+    """A dropped term is below 2^-26 of a product, a sum of 64 products in f32 off by at most 64 ulps of 2^-24, the f32 sums of K / 64
+    such parts by K / 64 more; with K up to 3072 that is below 128 ulps of the sum of magnitudes, plus the ulps of the epilogue."""
+    return 128 * 2.0 ** -24 * (x.abs().double() @ w.abs().double()) + 4 * 2.0 ** -24 * extra
+
+
+@pytest.mark.parametrize("m,n,k,form", [
+    (24, 2304, 768, "bias"), (32, 3072, 32, ""), (33, 1700, 64, "residual"), (64, 900, 96, "bias"), (65, 768, 3072, "residual"), (128, 400, 160, "gelu"),
+    (129, 385, 768, "bias"), (250, 129, 1024, "gelu"), (40, 50257, 64, ""), (300, 130, 32, "residual")])
+def test_matmul_of_many_rows(cuda, m, n, k, form):
+    g = torch.Generator(cuda).manual_seed(m * 7 + n)
+    x, w = torch.randn(m, k, device=cuda, generator=g), torch.randn(k, n, device=cuda, generator=g)
+    b = torch.randn(n, device=cuda, generator=g) if form in ("bias", "gelu") else None
+    r = torch.randn(m, n, device=cuda, generator=g) if form == "residual" else None
+    out = ops.matmul_f32(x, w, bias=b, residual=r, gelu=form == "gelu")
+    want, extra = x.double() @ w.double(), 0.0
+    for t in (b, r):
+        if t is not None:
+            want, extra = want + t.double(), extra + t.abs().double()
+    bound = _bound(x, w, extra + want.abs())
+    if form == "gelu":   # its slope stays below 1.2
+        want, bound = torch.nn.functional.gelu(want), 1.2 * bound + 8 * 2.0 ** -24 * want.abs()
+    assert ((out.double() - want).abs() <= bound).all()
+    assert ops.matmul_status() == 0
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+def test_matmul_of_values_that_bf16_cannot_hold(cuda, value):
+    """A tile with such a value gives what plain f32 arithmetic gives; the other tiles are not touched by it."""
+    g = torch.Generator(cuda).manual_seed(5)
+    x, w = torch.randn(200, 256, device=cuda, generator=g), torch.randn(256, 520, device=cuda, generator=g) * 0.1
+    x[77, 130] = value
+    w[130] = w[130].sign() * 0.25   # exact in one bf16: the remainders of the products are zeros
+    out, want = ops.matmul_f32(x, w), x.double() @ w.double()
+    fine = torch.isfinite(want) & (want.abs() < 3.4e38)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want.float()))
+    assert ((out.double() - want).abs()[fine] <= _bound(x, w, want.abs())[fine]).all()
+
+
+@pytest.mark.parametrize("kind,hd,n_q,n_kv", [("gpt", 64, 3, 3), ("ministral", 128, 4, 2)])
+def test_prompt_rows_of_several_sequences(cuda, kind, hd, n_q, n_kv):
+    """Rows of three sequences in one pass, in portions that leave tiles with rows of two sequences, then one token each: logits of
+    the last rows against the oracle."""
+    cfg = mr.Cfg(kind, n_layers=2, d_model=64, n_q=n_q, n_kv=n_kv, hd=hd, d_mlp=128, vocab=96, ctx=256, rot=hd if kind == "ministral" else 0, theta=1e4)
+    params = mr.random_params(cfg, seed=11, std=0.2)
+    mc = gm.ModelConfig(gm.KIND_GPT if kind == "gpt" else gm.KIND_MINISTRAL, cfg.n_layers, cfg.d_model, n_q, n_kv, hd, cfg.d_mlp, cfg.vocab, cfg.ctx, cfg.eps,
+                        cfg.theta, cfg.rot, max_seqs=3, max_tokens=256, max_logit_rows=3)
+    m = gm.LoadedModel(mc, namespace=7100 + hd)
+    for name, w in params.items():
+        m.load_param(name, w)
+    m.finalize()
+    rng = np.random.default_rng(0)
+    refs, at = [mr.RefModel(cfg, params) for _ in range(3)], [0, 0, 0]
+    for lengths in ((70, 5, 33), (1, 96, 31), (1, 1, 1)):
+        tok, sl, pos, rows, want = [], [], [], [], []
+        for s, n in enumerate(lengths):
+            t = rng.integers(0, cfg.vocab, n)
+            want.append(refs[s].forward(t)[-1])
+            tok += t.tolist()
+            sl += [s] * n
+            pos += range(at[s], at[s] + n)
+            at[s] += n
+            rows.append(len(tok) - 1)
+        got, _ = m.forward_with_decode_cache(tok, sl, pos, rows)
+        assert np.abs(got - np.stack(want)).max() <= 1e-4 * max(1.0, np.abs(want).max())
+
+
+def test_one_token_with_logits_takes_the_whole_step_kernel(cuda):
+    """GPT-2's widths: a forward pass of one token and a generator step are the same kernel, and both follow the oracle."""
+    cfg = mr.Cfg("gpt", n_layers=2, d_model=768, n_q=12, n_kv=12, hd=64, d_mlp=3072, vocab=500, ctx=64)
+    params = mr.random_params(cfg, seed=2, std=0.05)
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 768, 12, 12, 64, 3072, 500, 64, cfg.eps, max_seqs=2, max_tokens=40, max_logit_rows=2), namespace=7001)
+    for name, w in params.items():
+        m.load_param(name, w)
+    m.finalize()
+    ref = mr.RefModel(cfg, params)
+    prompt = [(7 * i) % 500 for i in range(37)]
+    want = ref.forward(prompt)[-1]
+    got, _ = m.prefill(1, prompt, want_logits=True)
+    assert np.abs(got - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
+    for i, t in enumerate((3, 499, 0)):
+        want = ref.forward([t])[-1]
+        got, ids = m.forward_with_decode_cache([t], [1], [37 + i], [0])
+        assert np.abs(got[0] - want).max() <= 1e-4 * max(1.0, np.abs(want).max()) and ids[0] == int(np.argmax(want))
