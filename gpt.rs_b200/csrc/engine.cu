@@ -315,15 +315,16 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     cudaStream_t st = m.stream;
     float* hidden = m.hidden.as<float>();
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
-    if (m.mega_on && T == 1 && n_rows == 1 && !prefill_groups) {
-        // one sequence, one token: the whole step is one cooperative kernel (+ the memset of its barrier word)
+    if (T <= m.mega_rows && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
+        // a token each of a few sequences: the whole step is one cooperative kernel (+ the memset of its barrier word)
         MegaParams P = m.mega;
+        P.rows = T;
         P.greedy = temperature <= 0.f ? 1 : 0;
         m.launches += 1;
         int r = mega_launch(P, st);
         if (r || P.greedy) return r;
         ++m.launches;
-        return gptrs_cuda_sample_rows_top_k(m.logits.as<float>(), 1, c.vocab, temperature, m.top_k, m.sample_seed, m.d_sampled.as<int32_t>(), st);
+        return gptrs_cuda_sample_rows_top_k(m.logits.as<float>(), T, c.vocab, temperature, m.top_k, m.sample_seed, m.d_sampled.as<int32_t>(), st);
     }
     int rc = gptrs_cuda_embedding_lookup(m.tok_emb->data, GPTRS_F32, c.vocab, D, m.d_tokens.as<int32_t>(), T,
                                          m.pos_emb ? static_cast<const float*>(m.pos_emb->data) : nullptr,
@@ -622,7 +623,7 @@ int sync_page_table(Model& m) {
 }
 
 // Transposed copies of the projection weights and the scratch vectors of the single-kernel decode step (f32 GPT kind,
-// one sequence). GPTRS_GPT_MEGA=0 keeps the kernel-per-projection path.
+// a few sequences). GPTRS_GPT_MEGA=0 keeps the kernel-per-projection path.
 int setup_mega(Model& m) {
     const auto& c = m.cfg;
     if (const char* e = getenv("GPTRS_GPT_MEGA")) if (atoi(e) == 0) return GPTRS_OK;
@@ -654,32 +655,32 @@ int setup_mega(Model& m) {
     }
     const float* lm_t = nullptr;
     if ((rc = tr(m.lm_head, &lm_t))) return rc;
-    const size_t n_sm = (size_t)sm_count();
+    const size_t n_sm = (size_t)sm_count(), R = kMegaMaxRows;
     auto pad = [](size_t n) { return (n + 63) & ~(size_t)63; };   // every vector starts on a 256-byte boundary
     const size_t n_part = pad(n_sm * (c.head_dim + 2));
-    const size_t floats = pad(3 * D) + n_part + pad(D) + pad(MLP) + pad(4 * D) + 2 * pad(n_sm) + 64 + 512;
+    const size_t floats = pad(R * 3 * D) + n_part + pad(R * D) + pad(R * MLP) + pad(R * 4 * D) + 2 * pad(R * n_sm) + 64 + 512;
     if ((rc = m.mega_scratch.alloc(floats * 4, true))) return rc;
     float* s = m.mega_scratch.as<float>();
     MegaParams& P = m.mega;
     P.n_layers = c.n_layers;
     P.tok_emb = fp(m.tok_emb); P.pos_emb = fp(m.pos_emb); P.lnf_g = fp(m.final_g); P.lnf_b = fp(m.final_b); P.lm_head_t = lm_t;
     P.token = m.d_tokens.as<int>(); P.pos = m.d_pos.as<int>(); P.slot = m.d_slot.as<int>();
-    P.qkv = s; s += pad(3 * D);
+    P.qkv = s; s += pad(R * 3 * D);
     P.att_part = s; s += n_part;
-    P.pc = s; s += pad(D);
-    P.mh = s; s += pad(MLP);
-    P.pe = s; s += pad(4 * D);
-    P.cand_val = s; s += pad(n_sm);
-    P.cand_idx = reinterpret_cast<int*>(s); s += pad(n_sm);
+    P.pc = s; s += pad(R * D);
+    P.mh = s; s += pad(R * MLP);
+    P.pe = s; s += pad(R * 4 * D);
+    P.cand_val = s; s += pad(R * n_sm);
+    P.cand_idx = reinterpret_cast<int*>(s); s += pad(R * n_sm);
     P.barrier = reinterpret_cast<unsigned*>(s); s += 64;
     P.timing = nullptr;
     if (const char* e = getenv("GPTRS_MEGA_TIMING")) if (atoi(e)) P.timing = reinterpret_cast<unsigned long long*>(s);
     P.logits = m.logits.as<float>();
     P.sampled = m.d_sampled.as<int>();
     P.status = m.d_status.as<int32_t>();
-    P.D = (int)D; P.H = c.n_q_heads; P.hd = c.head_dim; P.MLP = (int)MLP; P.vocab = c.vocab; P.ctx_cap = c.context_length;
+    P.H = c.n_q_heads; P.hd = c.head_dim; P.vocab = c.vocab; P.ctx_cap = c.context_length;
     P.n_pos = c.context_length; P.eps = c.norm_eps; P.greedy = 1;
-    m.mega_on = true;
+    m.mega_rows = mega_max_rows(c.n_q_heads, c.head_dim, c.context_length);
     return GPTRS_OK;
 }
 
@@ -1297,7 +1298,7 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
         ++m.launches;
         return launch_kernel(advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s, 1, ap);
     };
-    if (use_graph && !(m.mega_on && B == 1)) {   // the single-kernel step needs no graph
+    if (use_graph && B > m.mega_rows) {   // the single-kernel step needs no graph
         GraphKey key{B, chunk, splits};
         auto it = m.graphs.find(key);
         if (it == m.graphs.end()) {
@@ -1344,7 +1345,7 @@ int gptrs_cuda_generator_sync(gptrs_model* h) {
 int gptrs_cuda_debug_mega_timing(gptrs_model* h, uint64_t* out, int n) {
     GPTRS_REQUIRE(h && out && n > 0 && n <= 256, "bad arguments");
     Model& m = *reinterpret_cast<Model*>(h);
-    GPTRS_REQUIRE(m.mega_on && m.mega.timing, "the single-kernel step is off or was built without GPTRS_MEGA_TIMING=1");
+    GPTRS_REQUIRE(m.mega_rows && m.mega.timing, "the single-kernel step is off or was built without GPTRS_MEGA_TIMING=1");
     GPTRS_CUDA_OK(cudaStreamSynchronize(m.stream));
     GPTRS_CUDA_OK(cudaMemcpy(out, m.mega.timing, (size_t)n * 8, cudaMemcpyDeviceToHost));
     return GPTRS_OK;

@@ -202,7 +202,7 @@ struct Model {
     DevBuf best_val, best_idx;
     bool fuse_pick = true;   // GPTRS_FUSE_PICK=0: logits + sampling kernel
     // f32 GPT kind, one sequence: the whole decode step as one cooperative kernel (gpt_decode_mega.cu)
-    bool mega_on = false;
+    int mega_rows = 0;   // most sequences of a step that is one kernel (0: none)
     DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
     MegaParams mega = {};
     int gen_batch = 0;  // slots 0..gen_batch-1 are driven by generator_step

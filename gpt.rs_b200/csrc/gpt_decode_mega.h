@@ -1,4 +1,4 @@
-// Single-kernel decode step of one sequence of a GPT-2-style f32 model (gpt_decode_mega.cu).
+// Single-kernel decode step of up to eight sequences of a GPT-2-style f32 model (gpt_decode_mega.cu).
 #pragma once
 
 #include "common.cuh"
@@ -10,26 +10,28 @@ struct MegaLayer {
     float *k_cache, *v_cache;   // [slot][head][capacity][head_dim] of this layer
 };
 
-constexpr int kMegaMaxLayers = 16;
+constexpr int kMegaMaxLayers = 16, kMegaMaxRows = 8;
 
 struct MegaParams {
     MegaLayer layers[kMegaMaxLayers];   // in the kernel parameters themselves (constant bank)
     int n_layers;
     const float *tok_emb, *pos_emb, *lnf_g, *lnf_b, *lm_head_t;
-    const int *token, *pos, *slot;   // device scalars of the one row
-    float *qkv, *att_part, *pc, *mh, *pe, *logits, *cand_val;
+    int rows;                        // sequences of the step
+    const int *token, *pos, *slot;   // [rows]; the slots are distinct
+    float *qkv, *att_part, *pc, *mh, *pe, *logits, *cand_val;   // vectors of kMegaMaxRows rows, partials per CTA, logits [rows][vocab]
     int *cand_idx, *sampled;
     unsigned* barrier;
     int* status;
     unsigned long long* timing;   // optional (GPTRS_MEGA_TIMING=1): globaltimer of CTA 0 at kernel start and around every barrier
-    int D, H, hd, MLP, vocab, ctx_cap, n_pos;
+    int H, hd, vocab, ctx_cap, n_pos;
+    int big_floats;                  // set by the launcher
     float eps;
     int greedy;
 };
 
 bool mega_supported(int D, int H, int hd, int MLP, int ctx_cap, int n_layers);
-size_t mega_smem_bytes(int D, int MLP, int hd);
+int mega_max_rows(int H, int hd, int ctx_cap);   // most sequences of a step
 int mega_transpose(const float* src_in_out, float* dst_out_in, int64_t in, int64_t out, cudaStream_t st);
-int mega_launch(const MegaParams& p, cudaStream_t st);
+int mega_launch(MegaParams p, cudaStream_t st);
 
 }  // namespace gptrs

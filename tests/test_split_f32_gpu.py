@@ -77,20 +77,28 @@ def test_prompt_rows_of_several_sequences(cuda, kind, hd, n_q, n_kv):
         assert np.abs(got - np.stack(want)).max() <= 1e-4 * max(1.0, np.abs(want).max())
 
 
-def test_one_token_with_logits_takes_the_whole_step_kernel(cuda):
-    """GPT-2's widths: a forward pass of one token and a generator step are the same kernel, and both follow the oracle."""
-    cfg = mr.Cfg("gpt", n_layers=2, d_model=768, n_q=12, n_kv=12, hd=64, d_mlp=3072, vocab=500, ctx=64)
+@pytest.mark.parametrize("batch,ctx", [(1, 64), (2, 300), (3, 64), (5, 64), (8, 128), (9, 64)])
+def test_steps_of_a_few_sequences(cuda, batch, ctx):
+    """GPT-2's widths, where a step of up to eight sequences is one kernel: prompts of unequal lengths packed into one pass, greedy steps,
+    and a single token with logits, against the oracle (nine sequences: the kernel-per-projection path)."""
+    cfg = mr.Cfg("gpt", n_layers=2, d_model=768, n_q=12, n_kv=12, hd=64, d_mlp=3072, vocab=500, ctx=ctx)
     params = mr.random_params(cfg, seed=2, std=0.05)
-    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 768, 12, 12, 64, 3072, 500, 64, cfg.eps, max_seqs=2, max_tokens=40, max_logit_rows=2), namespace=7001)
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 768, 12, 12, 64, 3072, 500, ctx, cfg.eps, max_seqs=batch, max_tokens=400, max_logit_rows=batch),
+                       namespace=7000 + batch * 1000 + ctx)
     for name, w in params.items():
         m.load_param(name, w)
     m.finalize()
-    ref = mr.RefModel(cfg, params)
-    prompt = [(7 * i) % 500 for i in range(37)]
-    want = ref.forward(prompt)[-1]
-    got, _ = m.prefill(1, prompt, want_logits=True)
-    assert np.abs(got - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
-    for i, t in enumerate((3, 499, 0)):
-        want = ref.forward([t])[-1]
-        got, ids = m.forward_with_decode_cache([t], [1], [37 + i], [0])
-        assert np.abs(got[0] - want).max() <= 1e-4 * max(1.0, np.abs(want).max()) and ids[0] == int(np.argmax(want))
+    rng = np.random.default_rng(batch)
+    prompts = [rng.integers(0, 500, ctx - 12 if s == 0 else int(rng.integers(1, ctx - 12))) for s in range(batch)]
+    refs = [mr.RefModel(cfg, params) for _ in prompts]
+    want = np.stack([r.forward(p)[-1] for r, p in zip(refs, prompts)])
+    first = m.prefill_many(list(range(batch)), prompts)
+    assert first == want.argmax(1).tolist()
+    gen, cur = gm.Generator(m, first), list(first)
+    for _ in range(5):
+        want = np.stack([r.forward([t])[-1] for r, t in zip(refs, cur)])
+        cur = gen.step().tolist()
+        assert cur == want.argmax(1).tolist()
+    want = refs[-1].forward([7])[-1]
+    got, ids = m.forward_with_decode_cache([7], [batch - 1], [m.sequence_length(batch - 1)], [0])
+    assert np.abs(got[0] - want).max() <= 1e-4 * max(1.0, np.abs(want).max()) and ids[0] == int(np.argmax(want))
