@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kSgWarps * 32) sgemm_smallm_kernel(const Sgemm
 #pragma unroll
     for (int j = 0; j < 4; ++j) cv[j] = col0 + 32 * j < p.N;
 
-    constexpr int U = 4;
+    constexpr int U = MT <= 2 ? 12 : 8;   // K 768 in eight parts is twelve rows of a warp: one round trip to memory
     int k = warp;
     for (; k + (U - 1) * kSgWarps < kn; k += U * kSgWarps) {
         float wv[U][4];

@@ -113,15 +113,40 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(const NormParams
     // input itself no longer holds the addend-free value), else recomputed
     auto again = [&](int i) { return (p.delta && hst) ? hst[i] : value(i); };
     float sum = 0.f;
+    if (!p.peer_on) {
+        // every load of a thread under way at once: with the store of an updated element between two of them each was a round trip of
+        // its own (one row of 3072: 14 us, now 4)
 #pragma unroll
-    for (int j = 0; j < kKeep; ++j) {
-        const int i = tid + j * kNormThreads;
-        keep[j] = 0.f;
-        if (i < p.D) {
-            keep[j] = load(i);
-            sum += p.layer_norm ? keep[j] : keep[j] * keep[j];
+        for (int j = 0; j < kKeep; ++j) {
+            const int i = tid + j * kNormThreads;
+            keep[j] = i < p.D ? hin[i] : 0.f;
         }
+        if (p.delta) {
+            float d[kKeep];
+#pragma unroll
+            for (int j = 0; j < kKeep; ++j) {
+                const int i = tid + j * kNormThreads;
+                d[j] = i >= p.D ? 0.f : p.delta_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.delta)[(size_t)row * p.D + i])
+                                                     : static_cast<const float*>(p.delta)[(size_t)row * p.D + i];
+            }
+            if (p.delta_bias) {
+#pragma unroll
+                for (int j = 0; j < kKeep; ++j)
+                    if (tid + j * kNormThreads < p.D) d[j] += p.delta_bias[tid + j * kNormThreads];
+            }
+#pragma unroll
+            for (int j = 0; j < kKeep; ++j) {
+                const int i = tid + j * kNormThreads;
+                keep[j] += d[j];
+                if (hst && i < p.D) hst[i] = keep[j];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kKeep; ++j) keep[j] = tid + j * kNormThreads < p.D ? load(tid + j * kNormThreads) : 0.f;
     }
+#pragma unroll
+    for (int j = 0; j < kKeep; ++j) sum += p.layer_norm ? keep[j] : keep[j] * keep[j];
     for (int i = kKeepSpan + tid; i < p.D; i += kNormThreads) {
         float v = load(i);
         sum += p.layer_norm ? v : v * v;
@@ -153,10 +178,22 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(const NormParams
         if (p.out_f32) static_cast<float*>(p.out)[(size_t)row * p.D + i] = y;
         else static_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.D + i] = __float2bfloat16_rn(y);
     };
+    float gain[kKeep];
+#pragma unroll
+    for (int j = 0; j < kKeep; ++j) gain[j] = tid + j * kNormThreads < p.D ? p.gamma[tid + j * kNormThreads] : 0.f;
+#pragma unroll
+    for (int j = 0; j < kKeep; ++j) keep[j] = (keep[j] - mean) * inv * gain[j];
+    if (p.beta) {
+#pragma unroll
+        for (int j = 0; j < kKeep; ++j)
+            if (tid + j * kNormThreads < p.D) keep[j] += p.beta[tid + j * kNormThreads];
+    }
 #pragma unroll
     for (int j = 0; j < kKeep; ++j) {
         const int i = tid + j * kNormThreads;
-        if (i < p.D) store(i, keep[j]);
+        if (i >= p.D) break;
+        if (p.out_f32) static_cast<float*>(p.out)[(size_t)row * p.D + i] = keep[j];
+        else static_cast<__nv_bfloat16*>(p.out)[(size_t)row * p.D + i] = __float2bfloat16_rn(keep[j]);
     }
     for (int i = kKeepSpan + tid; i < p.D; i += kNormThreads) store(i, again(i));
     if (p.peer_on) {
@@ -188,13 +225,22 @@ __global__ void __launch_bounds__(256) embedding_kernel(const EmbedParams p) {
         pok = pid >= 0 && pid < p.P;
     }
     if ((!ok || !pok) && threadIdx.x == 0) atomicExch(p.status, 2);
-    for (int i = threadIdx.x; i < p.D; i += blockDim.x) {
-        float v = 0.f;
-        if (ok)
-            v = p.weight_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.weight)[(size_t)id * p.D + i])
-                              : static_cast<const float*>(p.weight)[(size_t)id * p.D + i];
-        if (p.pos_weight && pok) v += p.pos_weight[(size_t)pid * p.D + i];
-        p.out[(size_t)row * p.D + i] = v;
+    for (int base = threadIdx.x; base < p.D; base += 4 * blockDim.x) {   // four elements of a thread under way at once
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = base + j * blockDim.x;
+            v[j] = !ok || i >= p.D ? 0.f : p.weight_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.weight)[(size_t)id * p.D + i])
+                                                         : static_cast<const float*>(p.weight)[(size_t)id * p.D + i];
+        }
+        if (p.pos_weight && pok) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (base + j * (int)blockDim.x < p.D) v[j] += p.pos_weight[(size_t)pid * p.D + base + j * blockDim.x];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (base + j * (int)blockDim.x < p.D) p.out[(size_t)row * p.D + base + j * blockDim.x] = v[j];
     }
 }
 
@@ -289,51 +335,76 @@ __device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
     return x;
 }
 
-__global__ void __launch_bounds__(1024) sample_kernel(const SampleParams p) {
-    __shared__ float sv[32];
-    __shared__ int si[32];
+// The cluster of up to eight CTAs (grid.y) shares a row: each finds the best of its slice with eight logits of a thread under way at
+// once, the CTA of rank 0 the best of the cluster. A row of 131072 took one CTA 62 us, load by load; now 6.
+constexpr int kSampleThreads = 1024, kSampleSlice = 8192;
+__device__ __forceinline__ void better(float& best, int& besti, float v, int i) {
+    if (v > best || (v == best && i < besti)) { best = v; besti = i; }
+}
+__global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleParams p) {
+    __shared__ float sv[32], cluster_v[8];
+    __shared__ int si[32], cluster_i[8];
     pdl_launch_dependents();  // dependents still wait for this whole grid before reading its results
     pdl_wait();
-    const int row = blockIdx.x;
+    const int row = blockIdx.x, S = gridDim.y, rank = S > 1 ? (int)cluster_ctarank() : 0;
     const float* x = p.logits + (size_t)row * p.vocab;
+    const int lo = (int)((int64_t)p.vocab * rank / S), hi = (int)((int64_t)p.vocab * (rank + 1) / S);
     float best = -INFINITY;
     int besti = 0x7fffffff;
-    for (int i = threadIdx.x; i < p.vocab; i += blockDim.x) {
-        float v = x[i];
-        if (p.temperature > 0.f) {
-            // Gumbel-max: argmax(logit / T + g), g = -log(-log(u)), u from a stateless hash
-            uint32_t hsh = hash_u32(p.seed ^ hash_u32((uint32_t)i + 0x9e3779b9u * (uint32_t)(row + 1)));
-            float u = ((float)(hsh >> 8) + 0.5f) * (1.f / 16777216.f);
-            v = v / p.temperature - logf(-logf(u));
-        }
-        if (v > best || (v == best && i < besti)) { best = v; besti = i; }
-    }
+    for (int base = lo + threadIdx.x; base < hi; base += 8 * kSampleThreads) {
+        float v[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, besti, o);
-        if (ov > best || (ov == best && oi < besti)) { best = ov; besti = oi; }
+        for (int j = 0; j < 8; ++j) v[j] = base + j * kSampleThreads < hi ? x[base + j * kSampleThreads] : -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int i = base + j * kSampleThreads;
+            if (i >= hi) break;
+            if (p.temperature > 0.f) {
+                // Gumbel-max: argmax(logit / T + g), g = -log(-log(u)), u from a stateless hash
+                uint32_t hsh = hash_u32(p.seed ^ hash_u32((uint32_t)i + 0x9e3779b9u * (uint32_t)(row + 1)));
+                float u = ((float)(hsh >> 8) + 0.5f) * (1.f / 16777216.f);
+                v[j] = v[j] / p.temperature - logf(-logf(u));
+            }
+            better(best, besti, v[j], i);
+        }
     }
+    auto warp_best = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
+            better(best, besti, ov, oi);
+        }
+    };
+    warp_best();
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     if (l == 0) { sv[w] = best; si[w] = besti; }
     __syncthreads();
     if (w == 0) {
-        const int nw = blockDim.x >> 5;
-        best = l < nw ? sv[l] : -INFINITY;
-        besti = l < nw ? si[l] : 0x7fffffff;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            int oi = __shfl_xor_sync(0xffffffffu, besti, o);
-            if (ov > best || (ov == best && oi < besti)) { best = ov; besti = oi; }
+        best = sv[l]; besti = si[l];
+        warp_best();
+    }
+    if (S > 1) {
+        cluster_sync_all();   // rank 0 has started: its slots may be written
+        if (threadIdx.x == 0) {
+            const uint32_t v = map_to_cta(smem_u32(cluster_v + rank), 0), i = map_to_cta(smem_u32(cluster_i + rank), 0);
+            asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(v), "f"(best) : "memory");
+            asm volatile("st.shared::cluster.u32 [%0], %1;\n" ::"r"(i), "r"(besti) : "memory");
         }
-        if (l == 0) {
-            p.tokens[row] = besti == 0x7fffffff ? 0 : besti;
-            if (p.values) p.values[row] = best;
-        }
+        cluster_sync_all();
+        if (rank == 0 && threadIdx.x == 0)
+            for (int r = 1; r < S; ++r) better(best, besti, cluster_v[r], cluster_i[r]);
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        p.tokens[row] = besti == 0x7fffffff ? 0 : besti;
+        if (p.values) p.values[row] = best;
     }
 }
-
+int launch_sample(const SampleParams& p, cudaStream_t st) {
+    int s = ceil_div(p.vocab, kSampleSlice);
+    s = s < 1 ? 1 : s > 8 ? 8 : s;
+    return launch_kernel(sample_kernel, dim3((unsigned)p.rows, (unsigned)s), dim3(kSampleThreads), 0, st, s, p);
+}
 
 // ---- top-k sampler ----------------------------------------------------------------------------
 // inference/sampler.rs:35-52 keeps every logit >= the k-th largest (ties at the threshold stay),
@@ -449,7 +520,7 @@ __global__ void __launch_bounds__(kTopKThreads) sample_top_k_kernel(const TopKPa
 // Greedy argmax per row that also reports the winning value (vocab-parallel heads exchange the pairs).
 int sample_rows_with_values(const float* d_logits, int64_t rows, int64_t vocab, int32_t* d_tokens, float* d_values, cudaStream_t st) {
     SampleParams p = {d_logits, d_values, d_tokens, (int)rows, (int)vocab, 0.f, 0u};
-    return launch_kernel(sample_kernel, dim3((unsigned)rows), dim3(1024), 0, st, 1, p);
+    return launch_sample(p, st);
 }
 
 }  // namespace gptrs
@@ -594,7 +665,7 @@ int gptrs_cuda_sample_rows(const float* d_logits, int64_t rows, int64_t vocab, f
     GPTRS_REQUIRE(rows >= 0 && vocab > 0 && vocab < (1ll << 31) && rows < (1ll << 31), "bad shape");
     if (rows == 0) return GPTRS_OK;
     SampleParams p = {d_logits, nullptr, d_tokens, (int)rows, (int)vocab, temperature, seed};
-    return launch_kernel(sample_kernel, dim3((unsigned)rows), dim3(1024), 0, as_stream(stream), 1, p);
+    return launch_sample(p, as_stream(stream));
 }
 
 int gptrs_cuda_sample_decode_token(const float* d_logits, int64_t rows, int64_t vocab, float temperature,
