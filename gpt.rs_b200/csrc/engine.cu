@@ -1168,7 +1168,13 @@ int gptrs_cuda_model_forward_with_decode_cache(gptrs_model* h, const int32_t* h_
         ++m.launches;
         if ((rc = launch_kernel(record_history_kernel, dim3((T + 127) / 128), dim3(128), 0, s, 1, hp))) return rc;
     }
+    // The kernels of a short pass may start while the one in front ends, as in the generator's graphs: they are as long as a launch. The
+    // persistent kernels of a long one take the SMs that the rest of the grid in front still needs (5855 rows of a layered model:
+    // 6.5 ms without, 6.9 with).
+    const int pdl_before = g_use_pdl;
+    if (c.use_pdl && T <= 256) g_use_pdl = 1;
     rc = enqueue_forward(m, T, max_ctx, chunk, rows, false, temperature, prefill_groups);
+    g_use_pdl = pdl_before;
     if (rc) return rc;
     if (m.layered()) for (size_t r = 0; r < m.lay->runs.size(); r += 2) m.lay->parity[h_slots[m.lay->runs[r]]] ^= 1;
     if (h_logits && n_logit_rows)
