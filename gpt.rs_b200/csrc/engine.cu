@@ -191,6 +191,7 @@ struct NormFold {
     bool produce = false, consume = false;
     int dim = 0;
     float eps = 0.f;
+    int tiles = 0;                 // consume: column tiles of the producer
     // RoPE + KV append folded into the qkv projection (positions non-null switches it on)
     const int32_t* rope_positions = nullptr;
     const int32_t* rope_slot = nullptr;
@@ -221,7 +222,7 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
     ep.peer_push = push;
     if (pick) { ep.d_best_val = m.best_val.as<float>(); ep.d_best_idx = m.best_idx.as<int32_t>(); ep.skip_store = 1; }
     if (fold && fold->produce) { ep.d_norm_gamma = fold->gamma; ep.d_norm_x = fold->x_next; ep.d_sumsq_out = fold->sumsq; }
-    if (fold && fold->consume) { ep.d_sumsq_in = fold->sumsq; ep.sumsq_tiles = fold->dim / 128; ep.norm_dim = fold->dim; ep.norm_eps = fold->eps; }
+    if (fold && fold->consume) { ep.d_sumsq_in = fold->sumsq; ep.sumsq_tiles = fold->tiles; ep.norm_dim = fold->dim; ep.norm_eps = fold->eps; }
     if (fold && fold->rope_positions) {
         ep.d_rope_positions = fold->rope_positions; ep.d_rope_slot = fold->rope_slot;
         ep.d_rope_page_table = m.d_page_table.as<int32_t>(); ep.rope_max_pages = m.cfg.max_pages_per_seq;
@@ -229,6 +230,7 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
         ep.d_rope_q_out = fold->rope_q_out; ep.d_rope_kv_pool = fold->rope_pool;
         ep.rope_q_heads = m.cfg.n_q_heads; ep.rope_kv_heads = m.cfg.n_kv_heads;
     }
+    if (rows <= 16) return quant_matmul_few_rows(m.cfg.weight_mode == kModeW4 ? 4 : 8, x, w.packed->data, y, rows, w.out, w.in, &ep, st);
     return m.cfg.weight_mode == kModeW4
                ? gptrs_cuda_quant_matmul_w4a16(x, w.packed->data, y, rows, w.out, w.in, &ep, st)
                : gptrs_cuda_quant_matmul_w8a16(x, w.packed->data, y, rows, w.out, w.in, &ep, st);
@@ -351,10 +353,10 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     // (tensor-parallel steps always run as one lane).
     const float* pending = nullptr;
     bool pending_peer = false;   // the pending tile still has to be summed over the ranks (by the norm kernel)
-    // RMSNorm folded into the projections: quantised Ministral, one rank, more than 16 rows (tensor-core matmuls),
-    // d_model a multiple of 128. The sums of squares of a lane live at a row offset of the shared buffer: a lane's
+    // RMSNorm folded into the projections: quantised Ministral, one rank, d_model a multiple of 128. The sums of squares of a lane live at a row offset of the shared buffer: a lane's
     // tile t is at sumsq + t * T_lane, so each lane gets a disjoint slab of [tiles][T_lane] floats.
-    const bool fold = m.fold_norm && !gpt && !m.f32() && m.tp == 1 && T > 16 && D % 128 == 0;
+    const bool fold = m.fold_norm && !gpt && !m.f32() && m.tp == 1 && D % 128 == 0;
+    int fold_tiles = 0;   // column tiles that the last producer's sums are over
     auto fold_for = [&](const Lane& ln, Tensor* next_gamma, bool produce) {
         NormFold f;
         f.sumsq = m.sumsq.as<float>() + (size_t)(D / 128) * ln.r0;
@@ -362,6 +364,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         f.eps = c.norm_eps;
         f.produce = produce;
         f.consume = !produce;
+        f.tiles = fold_tiles;
         if (produce) {
             f.gamma = static_cast<const float*>(next_gamma->data);
             f.x_next = at(m.xn, (size_t)D * act, ln);
@@ -380,8 +383,9 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     auto row_parallel = [&](const Lane& ln, const Weight& w, const void* x, Tensor* next_gamma = nullptr) -> int {
         float* h = reinterpret_cast<float*>(at(m.hidden, (size_t)D * 4, ln));
         if (m.tp == 1) {
-            if (fold && next_gamma && ln.T > 16) {
+            if (fold && next_gamma) {
                 const NormFold f = fold_for(ln, next_gamma, true);
+                fold_tiles = D / quant_tile_cols(c.weight_mode == kModeW4 ? 4 : 8, ln.T, w.out, w.in);
                 return linear(m, w, x, h, ln.T, true, h, false, false, ln.st, &f);
             }
             return linear(m, w, x, h, ln.T, true, h, false, false, ln.st);
@@ -420,11 +424,14 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
                    : gptrs_cuda_add_rms_norm(h, delta, GPTRS_F32, (const float*)g->data, c.norm_eps, xn, act_dt,
                                              nullptr, ln.T, D, ln.st);
     };
+    // A decode step of few rows leaves RoPE, KV append and the merge of the splits to the attention kernel.
+    const int step_splits = rows_identity && !m.f32() && !gpt && T <= 16 && !prefill_groups && c.rotary_dim == c.head_dim && c.head_dim == 128
+                                ? attention_step_splits(max_ctx, T, c.n_q_heads, c.n_kv_heads) : 0;
     // ---- the three parts of a decoder block ------------------------------------------------------
     auto pre_attention = [&](const Lane& ln, int l) -> int {
         Layer& L = m.layers[l];
         int r;
-        const bool folded = fold && ln.T > 16;
+        const bool folded = fold;
         // RoPE + KV append ride on the qkv projection's epilogue (tensor-core path, full rotary dimension)
         const bool rope_folded = m.fold_rope && !m.f32() && !gpt && ln.T > 16 && c.rotary_dim == c.head_dim && c.head_dim == 128;
         void* qkv = at(m.qkv, (size_t)m.QKV() * act, ln);
@@ -441,7 +448,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
             f.rope_pool = m.kv_pool.as<unsigned char>() + (size_t)l * m.pool_layer_bytes;
         }
         if (!fold32 && (r = linear(m, L.qkv, at(m.xn, (size_t)D * act, ln), qkv, ln.T, false, nullptr, false, false, ln.st, &f))) return r;
-        if (rope_folded) return GPTRS_OK;
+        if (rope_folded || step_splits) return GPTRS_OK;
         if (m.f32()) {
             if (!gpt && c.rotary_dim > 0) {
                 ++m.launches;
@@ -482,6 +489,10 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
                                                    c.n_q_heads, c.n_kv_heads, c.head_dim, c.context_length, ln.st);
         }
         unsigned char* pool = m.kv_pool.as<unsigned char>() + (size_t)l * m.pool_layer_bytes;
+        if (step_splits)
+            return attention_step(at(m.qkv, (size_t)m.QKV() * act, ln), m.cos_tab.as<float>(), m.sin_tab.as<float>(), pool, m.d_page_table.as<int32_t>(),
+                                  c.max_pages_per_seq, ints(m.d_slot, ln), ints(m.d_ctx, ln), out, m.d_status.as<int32_t>(), ln.T, c.n_q_heads, c.n_kv_heads,
+                                  max_ctx, step_splits, ln.st);
         if (prefill_groups == 3)   // tensor cores: one CTA per tile of rows and kv head, never split along the keys
             return gptrs_cuda_paged_attention_prefill_tc(at(m.q_rot, (size_t)m.QD() * 2, ln), pool, m.d_page_table.as<int32_t>(), c.max_pages_per_seq,
                                                          ints(m.d_slot, ln), ints(m.d_ctx, ln), out, m.d_status.as<int32_t>(), ln.T, c.n_q_heads,
@@ -501,7 +512,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     auto post_attention = [&](const Lane& ln, int l) -> int {
         Layer& L = m.layers[l];
         int r;
-        const bool folded = fold && ln.T > 16;
+        const bool folded = fold;
         if ((r = row_parallel(ln, L.attn_out, at(m.attn, (size_t)m.QD() * act, ln), folded ? L.ln2_g : nullptr))) return r;
         if (!folded && !fold32 && (r = norm(ln, L.ln2_g, L.ln2_b))) return r;
         void* xn = fold32 ? at(m.hidden, (size_t)D * 4, ln) : at(m.xn, (size_t)D * act, ln);
@@ -1001,7 +1012,8 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
     // activations
     const int T = c.max_tokens;
     const size_t act = m.f32() ? 4 : 2;
-    if (!m.f32() && (rc = m.sumsq.alloc((size_t)((D + 127) / 128) * T * 4, true))) return rc;
+    // sums of squares per row and column tile: 128 columns, or 16 with up to 16 rows
+    if (!m.f32() && (rc = m.sumsq.alloc((size_t)((D + 127) / 128) * std::max<size_t>(T, 8 * 16) * 4, true))) return rc;
     if ((rc = m.hidden.alloc((size_t)T * D * 4)) || (rc = m.xn.alloc((size_t)T * D * act)) || (rc = m.xn_rows.alloc((size_t)T * D * act)) ||
         (rc = m.qkv.alloc((size_t)T * QKV * act)) || (rc = m.attn.alloc((size_t)T * QD * act)) ||
         (rc = m.mlp_h.alloc((size_t)T * MLP * act))) return rc;

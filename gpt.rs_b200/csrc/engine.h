@@ -267,4 +267,15 @@ bool attention_rows_f32_takes(int64_t n_tokens, int64_t head_dim);
 int attention_rows_f32(const float* qkv, const float* k_cache, const float* v_cache, const int32_t* positions, const int32_t* slot, float* out,
                        int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st);
 
+// Quantised matmuls of 1..16 rows with the norms around them folded in (quant_matmul.cu): the sums of squares are per quant_tile_cols
+// columns of the producer.
+int quant_tile_cols(int bits, int64_t m, int64_t n, int64_t k);
+int quant_matmul_few_rows(int bits, const void* x, const void* packed, void* y, int64_t m, int64_t n, int64_t k, const gptrs_matmul_epilogue* ep, cudaStream_t st);
+
+// A decode step's RoPE, KV append and attention in one kernel (paged_attention.cu); splits from attention_step_splits, not 0.
+int attention_step_splits(int64_t max_ctx_len, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads);
+int attention_step(const void* qkv, const float* cos_table, const float* sin_table, void* pool, const int32_t* page_table, int64_t max_pages, const int32_t* slot,
+                   const int32_t* ctx_len, void* out, int32_t* status, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t max_ctx_len, int splits,
+                   cudaStream_t st);
+
 }  // namespace gptrs

@@ -172,15 +172,31 @@ struct SplitReduce {
     }
 };
 
-// Second half: barrier, local sum over the S slots, bias / residual / SwiGLU, store. All threads of the CTA.
+// 1 / rms of up to 16 rows from the sums that the producer of a folded RMSNorm left per column tile, a warp per row: a kernel of few rows
+// asks for them beside its activations instead of at its end. Barrier before the first use by the caller.
+__device__ __forceinline__ void few_row_scales(const MatmulParams& p, float* scale, int warp, int n_warps, int lane) {
+    if (!p.sumsq_in) return;
+    for (int m = warp; m < p.M; m += n_warps) {
+        float ss = 0.f;
+#pragma unroll 6
+        for (int t = lane; t < p.sumsq_tiles; t += 32) ss += p.sumsq_in[(size_t)t * p.M + m];
+        ss = warp_sum(ss);
+        if (lane == 0) scale[m] = rsqrtf(ss / (float)p.norm_dim + p.norm_eps);
+    }
+}
+
+// Second half: barrier, local sum over the S slots, bias / residual / SwiGLU, store. All threads of the CTA. `scales`: what
+// few_row_scales left, by row; null: computed here.
 template <int MPAD, bool kDense = false>
 __device__ __forceinline__ void split_reduce_finish(const MatmulParams& p, const SplitReduce& sr, const float* slots, int tid,
                                                     int n_threads, int m0, int n_cta0, int tile_cols = kCtaN,
-                                                    bool cluster_barrier = true) {
+                                                    bool cluster_barrier = true, const float* scales = nullptr) {
     const int S = sr.S, rank = sr.rank, rows_max = sr.rows_max;
     // consumer of a folded RMSNorm: 1 / rms of every row this CTA owns, from the producer's per-tile sums
     __shared__ float row_scale[MPAD];
-    if (p.sumsq_in) {
+    if (p.sumsq_in && scales) {
+        for (int lr = tid; rank + S * lr < MPAD; lr += n_threads) row_scale[lr] = m0 + rank + S * lr < p.M ? scales[m0 + rank + S * lr] : 0.f;
+    } else if (p.sumsq_in) {
         const int rows_mine = (MPAD - rank + S - 1) / S;
         for (int lr = tid; lr < rows_mine; lr += n_threads) {
             const int m = m0 + rank + S * lr;
@@ -251,10 +267,12 @@ __device__ __forceinline__ void split_reduce_finish(const MatmulParams& p, const
     if (!p.swiglu) {
         const int cols4 = tile_cols >> 2;  // float4 columns of the CTA tile (a power of two)
         const int sh4 = 31 - __clz(cols4);
-        for (int j = tid; j < rows_own * cols4; j += n_threads) {
+        // a row's lanes add up below: whole warps stay together then
+        const int items = rows_own * cols4, bound = p.sumsq_out || p.best_val ? (items + 31) & ~31 : items;
+        for (int j = tid; j < bound; j += n_threads) {
             const int lr = j >> sh4, c4 = j & (cols4 - 1);
             const int m = m0 + rank + S * lr, n = n_cta0 + c4 * 4;
-            const bool live = m < p.M && n < p.N;
+            const bool live = j < items && m < p.M && n < p.N;
             if (!live && !p.sumsq_out && !p.best_val) continue;
             float4 v = live ? gather(lr, c4 * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
             if (p.sumsq_in) { const float r = row_scale[lr]; v.x *= r; v.y *= r; v.z *= r; v.w *= r; }
@@ -311,16 +329,15 @@ __device__ __forceinline__ void split_reduce_finish(const MatmulParams& p, const
                 }
             }
             if (p.sumsq_out) {
-                // producer of a folded RMSNorm: the 32 lanes of a warp hold one row of the 128-column tile
+                // producer of a folded RMSNorm: tile_cols / 4 lanes hold one row of the tile
                 if (live) {
                     const float4 g4 = *reinterpret_cast<const float4*>(p.norm_gamma + n);
                     uint2 o = make_uint2(pack_bf16x2(v.x * g4.x, v.y * g4.y), pack_bf16x2(v.z * g4.z, v.w * g4.w));
                     *reinterpret_cast<uint2*>(p.norm_x + (size_t)m * p.N + n) = o;
                 }
                 float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-                if ((tid & 31) == 0 && m < p.M) p.sumsq_out[(size_t)(n_cta0 / kCtaN) * p.M + m] = ss;
+                for (int off = cols4 >> 1; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+                if (c4 == 0 && live) p.sumsq_out[(size_t)(n_cta0 / tile_cols) * p.M + m] = ss;
             }
         }
     } else {

@@ -47,6 +47,9 @@ struct AttnParams {
     int max_len;                  // lengths above min(launch bound, page-table row) are clamped to it and flagged
     int fixed_chunks;             // splits are chunk_pages long (prefill groups) instead of balanced per sequence
     float scale_log2;
+    // decode step in one kernel: the packed qkv rows (RoPE still to come) and the rotary tables [positions][64]
+    const __nv_bfloat16* qkv;
+    const float *cos_table, *sin_table;
 };
 
 // A visible length read from device memory, held to what the launch was sized for: a larger value would walk off the
@@ -76,12 +79,15 @@ __device__ __forceinline__ int swz(int tok, int chunk) { return tok * 256 + ((ch
 // 16-row MMA tile). kMulti = true: 16 / group consecutive rows of the token list per CTA, all of ONE sequence (a
 // prefill chunk): row r of the tile is query head r % group of token r / group, every row has its own visible
 // length, so the K/V pages are streamed once for 16 / group tokens instead of once per token.
-template <int kDepth, bool kMulti>
+// kStep (decode steps of few rows): the kernel also does what stands around it. Queries are rotated as they are loaded; the CTA with
+// the last page rotates the new key, stores key and value into the pool and into its copy of the page; the splits of a row and kv head
+// are a cluster (grid.y) that merges through distributed shared memory. Two launches less per layer, 3.7 and 4.8 us at one row.
+template <int kDepth, bool kMulti, bool kStep = false>
 __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_attention_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full_bar[kAttnWarps][kDepth];
 
-    const int split = blockIdx.x, h = blockIdx.y;
+    const int split = kStep ? blockIdx.y : blockIdx.x, h = kStep ? blockIdx.x : blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int group = p.Hq / p.Hkv;
@@ -102,8 +108,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
     else split_geometry(len, p.chunk_pages, &n_splits, &split_pages);  // rows of a prefill group keep one fixed grid
     const int chunk_tokens = split_pages * kPageTokens;
     const int first_tok = split * chunk_tokens;
-    if (first_tok >= len) return;  // whole CTA leaves together, before any barrier
-    const int n_tok = min(chunk_tokens, len - first_tok);
+    if (!kStep && first_tok >= len) return;  // whole CTA leaves together, before any barrier
+    const int n_tok = max(0, min(chunk_tokens, len - first_tok));
     const int n_pages = (n_tok + kPageTokens - 1) / kPageTokens;
     const int* pt = p.page_table + (size_t)p.slot[b] * p.max_pages + first_tok / kPageTokens;
 
@@ -130,16 +136,46 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
     };
     for (int j = 0; j < kDepth && j < n_my; ++j) issue(j);
 
+    // kStep: the new token's key and value, channels 2 lane, 2 lane + 1 and those 64 further (value: 4 lane ..), in the warp whose
+    // last page holds the token
+    const int pos = len - 1;
+    const bool appends = kStep && n_tok > 0 && first_tok + n_tok == len && warp == (n_pages - 1) % kAttnWarps;
+    uint32_t k_lo = 0, k_hi = 0;
+    uint2 v_new = make_uint2(0, 0);
+    auto rotate = [](uint32_t& lo, uint32_t& hi, float2 c, float2 s) {   // pairs (channel, channel + 64), f32, rounded once
+        const float a0 = bf16_lo(lo), a1 = bf16_hi(lo), b0 = bf16_lo(hi), b1 = bf16_hi(hi);
+        lo = pack_bf16x2(a0 * c.x - b0 * s.x, a1 * c.y - b1 * s.y);
+        hi = pack_bf16x2(b0 * c.x + a0 * s.x, b1 * c.y + a1 * s.y);
+    };
+    if (appends) {
+        const __nv_bfloat16* kr = p.qkv + ((size_t)b * (p.Hq + 2 * p.Hkv) + p.Hq + h) * kHD;
+        k_lo = *reinterpret_cast<const uint32_t*>(kr + 2 * lane);
+        k_hi = *reinterpret_cast<const uint32_t*>(kr + 64 + 2 * lane);
+        v_new = *reinterpret_cast<const uint2*>(kr + (size_t)p.Hkv * kHD + 4 * lane);
+        rotate(k_lo, k_hi, *reinterpret_cast<const float2*>(p.cos_table + (size_t)pos * 64 + 2 * lane),
+               *reinterpret_cast<const float2*>(p.sin_table + (size_t)pos * 64 + 2 * lane));
+    }
+
     // Q fragments: row g of the A tile = query head h*group + g (rows >= group are zero); with kMulti rows g
     // and g + 8 are (token, head) pairs as described above.
     uint32_t qf[8][kMulti ? 4 : 2];
     {
         const int head_lo = h * group + (kMulti ? g % group : (valid_lo ? g : 0));
-        const __nv_bfloat16* qrow = p.q + ((size_t)(valid_lo ? tok_lo : b) * p.Hq + head_lo) * kHD;
+        const __nv_bfloat16* qrow = kStep ? p.qkv + ((size_t)b * (p.Hq + 2 * p.Hkv) + head_lo) * kHD
+                                          : p.q + ((size_t)(valid_lo ? tok_lo : b) * p.Hq + head_lo) * kHD;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
             qf[ks][0] = valid_lo ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 2 * t) : 0u;
             qf[ks][1] = valid_lo ? *reinterpret_cast<const uint32_t*>(qrow + ks * 16 + 8 + 2 * t) : 0u;
+        }
+        if (kStep && pos >= 0) {
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const size_t at = (size_t)pos * 64 + ks * 16 + 8 * i + 2 * t;
+                    rotate(qf[ks][i], qf[ks + 4][i], *reinterpret_cast<const float2*>(p.cos_table + at), *reinterpret_cast<const float2*>(p.sin_table + at));
+                }
         }
         if (kMulti) {
             const __nv_bfloat16* qhi = p.q + ((size_t)(valid_hi ? tok_hi : b) * p.Hq + h * group + (g + 8) % group) * kHD;
@@ -171,6 +207,20 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
             break;
         }
         const uint32_t kb = ring_addr + st * kPageHeadBytes, vb = kb + kBlockBytes;
+        if (kStep) {
+            const int page = __shfl_sync(0xffffffffu, my_page, j);
+            if (appends && j == n_my - 1) {   // the page has arrived: nothing else reads or writes the new token's rows any more
+                unsigned char* const blk = const_cast<unsigned char*>(p.pool) + ((size_t)page * p.Hkv + h) * kPageHeadBytes;
+                unsigned char* const own = my_ring + st * kPageHeadBytes;
+                const int tok = pos & (kPageTokens - 1), c = lane >> 2, in = (lane & 3) * 4;
+                for (unsigned char* to : {own, blk}) {
+                    *reinterpret_cast<uint32_t*>(to + swz(tok, c) + in) = k_lo;
+                    *reinterpret_cast<uint32_t*>(to + swz(tok, c + 8) + in) = k_hi;
+                    *reinterpret_cast<uint2*>(to + kBlockBytes + swz(tok, lane >> 1) + (lane & 1) * 8) = v_new;
+                }
+            }
+            __syncwarp();
+        }
         float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
@@ -298,6 +348,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
     }
     __syncthreads();
     const int n_rows = kMulti ? 16 : group;
+    constexpr int kOwn = kHD + 4;                                     // kStep: a row's output, maximum and sum of this CTA
+    __shared__ __align__(16) float own_part[kStep ? 8 * kOwn : 4];
     for (int idx = tid; idx < n_rows * (kHD / 4); idx += kAttnWarps * 32) {
         const int r = idx / (kHD / 4), c4 = (idx % (kHD / 4)) * 4;
         const int tok = kMulti ? b + r / group : b;
@@ -317,12 +369,15 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
 #pragma unroll
         for (int w = 0; w < kAttnWarps; ++w) {
             const float mw = mml[(w * kRows + r) * 2];
-            const float f = (kMulti && mw == -INFINITY) ? 0.f : exp2f(mw - M);  // a warp whose pages the row cannot see
+            const float f = ((kMulti || kStep) && mw == -INFINITY) ? 0.f : exp2f(mw - M);  // a warp that has seen no page of the row
             L += mml[(w * kRows + r) * 2 + 1] * f;
             float4 v = *reinterpret_cast<const float4*>(mo + (w * kRows + r) * kHD + c4);
             acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
         }
-        if (row_splits == 1) {
+        if (kStep) {
+            *reinterpret_cast<float4*>(own_part + r * kOwn + c4) = acc;
+            if (c4 == 0) { own_part[r * kOwn + kHD] = M; own_part[r * kOwn + kHD + 1] = L; }
+        } else if (row_splits == 1) {
             const float inv = 1.f / L;
             uint2 ov = make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
             *reinterpret_cast<uint2*>(p.out + ((size_t)tok * p.Hq + hq) * kHD + c4) = ov;
@@ -334,6 +389,39 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
                 p.part_ml[pi * 2 + 1] = L;
             }
         }
+    }
+    if (kStep) {   // the cluster's parts in rank order, 4 columns of a row per thread, the work dealt over the ranks
+        const int S = gridDim.y, rank = S > 1 ? (int)cluster_ctarank() : 0;
+        if (S > 1) cluster_sync_all();
+        else __syncthreads();
+        const uint32_t base = smem_u32(own_part);
+        for (int idx = tid * S + rank; idx < n_rows * (kHD / 4); idx += kAttnWarps * 32 * S) {
+            const int r = idx / (kHD / 4), c4 = (idx % (kHD / 4)) * 4;
+            float M = -INFINITY, L = 0.f;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), v[8];
+            float2 ml[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                ml[q] = make_float2(-INFINITY, 0.f);
+                if (q < S) {
+                    const uint32_t at = S > 1 ? map_to_cta(base + (uint32_t)(r * kOwn) * 4, (uint32_t)q) : base + (uint32_t)(r * kOwn) * 4;
+                    v[q] = ld_dsmem_f4(at + c4 * 4);
+                    asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];\n" : "=f"(ml[q].x), "=f"(ml[q].y) : "r"(at + kHD * 4));
+                }
+                M = fmaxf(M, ml[q].x);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (q < S && ml[q].x != -INFINITY) {
+                    const float f = exp2f(ml[q].x - M);
+                    L += ml[q].y * f;
+                    acc.x += v[q].x * f; acc.y += v[q].y * f; acc.z += v[q].z * f; acc.w += v[q].w * f;
+                }
+            const float inv = 1.f / L;
+            *reinterpret_cast<uint2*>(p.out + ((size_t)b * p.Hq + h * group + r) * kHD + c4) =
+                make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+        }
+        if (S > 1) cluster_sync_all();   // nobody leaves while a part of it is still read
     }
 }
 
@@ -619,6 +707,40 @@ __global__ void kv_gather_kernel(const unsigned char* pool, const int* page_row,
 }
 
 }  // namespace
+
+// Splits per row and kv head (a cluster) of a decode step in one kernel, 0: the step is left to the separate kernels. Eight pages per
+// warp at most, beyond that more splits and their merge kernel are faster; two CTAs per SM are enough.
+int attention_step_splits(int64_t max_ctx_len, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads) {
+    if (n_tokens > 16 || n_q_heads % n_kv_heads || n_q_heads / n_kv_heads > 8) return 0;
+    const int64_t pages = (max_ctx_len + kPageTokens - 1) / kPageTokens;
+    int64_t splits = 2 * (int64_t)sm_count() / (n_tokens * n_kv_heads);
+    splits = splits < 1 ? 1 : splits > 8 ? 8 : splits;
+    if (splits * 4 > pages) splits = (pages + 3) / 4;   // a page per warp
+    return splits * 32 < pages ? 0 : (int)splits;
+}
+
+// RoPE + KV append + attention of rows of distinct sequences, whose positions are ctx_len - 1.
+int attention_step(const void* qkv, const float* cos_table, const float* sin_table, void* pool, const int32_t* page_table, int64_t max_pages, const int32_t* slot,
+                   const int32_t* ctx_len, void* out, int32_t* status, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t max_ctx_len, int splits,
+                   cudaStream_t st) {
+    AttnParams p = {};
+    p.qkv = static_cast<const __nv_bfloat16*>(qkv); p.cos_table = cos_table; p.sin_table = sin_table;
+    p.pool = static_cast<const unsigned char*>(pool);
+    p.page_table = page_table; p.slot = slot; p.ctx_len = ctx_len;
+    p.out = static_cast<__nv_bfloat16*>(out);
+    p.status = status;
+    p.T = (int)n_tokens; p.Hq = (int)n_q_heads; p.Hkv = (int)n_kv_heads; p.max_pages = (int)max_pages;
+    p.chunk_pages = ceil_div(ceil_div(max_ctx_len, kPageTokens), splits);
+    p.max_splits = splits;
+    p.max_len = (int)std::min<int64_t>((int64_t)splits * p.chunk_pages * kPageTokens, max_pages * kPageTokens);
+    p.scale_log2 = kLog2e / sqrtf((float)kHD);
+    constexpr size_t smem = (size_t)kAttnWarps * 2 * kPageHeadBytes;
+    static PerDeviceOnce attr_once;
+    if (attr_once.first_time())
+        GPTRS_CUDA_OK(cudaFuncSetAttribute(paged_attention_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return launch_kernel(paged_attention_kernel<2, false, true>, dim3((unsigned)n_kv_heads, (unsigned)splits, (unsigned)n_tokens), dim3(kAttnWarps * 32), smem, st,
+                         splits, p);
+}
 
 }  // namespace gptrs
 

@@ -156,6 +156,8 @@ __global__ void __launch_bounds__(kGvWarps * 32, (MT * TPW >= 4) ? 2 : 3) w4_gem
     pdl_launch_dependents();  // dependents still wait for this whole grid before reading its results
     pdl_wait();
     // ---- all activation rows of this CTA's K range -> shared memory, and -136 * (group sum) of every row ----------
+    __shared__ float row_scales[MPAD];
+    few_row_scales(p, row_scales, warp, kGvWarps, lane);
     unsigned char* zero_block = smem + L.zero_block;               // 256 bytes of zeros
     float* negoff = reinterpret_cast<float*>(smem + L.negoff);     // [G][MT][4 (t)][4]: {m = 2t, 2t + 1, 2t, 2t + 1} of 8-row half i
     auto store_off = [&](int grp, int m, float v) {
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(kGvWarps * 32, (MT * TPW >= 4) ? 2 : 3) w4_gem
         if (sr.S == 1) sr.push(0, m, c, v);
         else sr.push(m % sr.S, m / sr.S, c, v);
     }
-    split_reduce_finish<MPAD>(p, sr, slots, tid, NT, 0, blockIdx.x * tile_cols, tile_cols);
+    split_reduce_finish<MPAD>(p, sr, slots, tid, NT, 0, blockIdx.x * tile_cols, tile_cols, true, row_scales);
 }
 
 template <int MT, int TPW>
@@ -334,22 +336,24 @@ int env_or(const char* name, int fallback) {
 
 }  // namespace
 
-// Called by quant_matmul.cu for W4 weights and 1..16 rows. Chooses the cluster split (only as large as the
-// shared-memory budget of the activation rows demands), the tiles per warp (as many as still leave every SM a
-// CTA or two), the split among the warps of a CTA and the ring depth (what fits beside a second CTA on the SM).
-// Returns GPTRS_UNIMPLEMENTED when no split fits.
-int w4_gemv(MatmulParams p, cudaStream_t st) {
-    if (p.M > 16) return GPTRS_UNIMPLEMENTED;
-    const int mt = p.M <= 8 ? 1 : 2;
-    const int groups = p.K / 128;
-    const size_t block_bytes = (size_t)p.M * 256;  // the valid rows of one 128-k block
+namespace {
+
+// Chooses the cluster split (only as large as the shared-memory budget of the activation rows demands), the tiles per warp (as
+// many as still leave every SM a CTA or two), the split among the warps of a CTA and the ring depth (what fits beside a second
+// CTA on the SM).
+struct GvPlan { int mt, split, G, tpw, ks, stages; size_t smem; };
+bool gv_plan(int M, int N, int K, GvPlan* out) {
+    if (M > 16) return false;
+    const int mt = M <= 8 ? 1 : 2;
+    const int groups = K / 128;
+    const size_t block_bytes = (size_t)M * 256;  // the valid rows of one 128-k block
     int split = 0;
     for (int s : {1, 2, 3, 4, 6, 8}) {
         if (groups % s == 0 && (groups / s) * block_bytes <= 48 * 1024) { split = s; break; }
     }
-    if (!split) return GPTRS_UNIMPLEMENTED;
+    if (!split) return false;
     const int G = groups / split;
-    const int n_tiles = p.N >> 4;
+    const int n_tiles = N >> 4;
     static const int forced_tpw = env_or("GPTRS_GEMV_TPW", 0), forced_stages = env_or("GPTRS_GEMV_STAGES", 0),
                      forced_ks = env_or("GPTRS_GEMV_KS", 0), ctas_per_sm = env_or("GPTRS_GEMV_CTAS_PER_SM", 0);
     const int want = sm_count();
@@ -375,25 +379,43 @@ int w4_gemv(MatmulParams p, cudaStream_t st) {
     const int per_sm = ctas_per_sm > 0 ? (ctas_per_sm < bound ? ctas_per_sm : bound) : bound;
     const size_t budget = (size_t)(227 * 1024) / (size_t)per_sm - 1024;
     int stages = G / ks < kGvMaxStages ? G / ks : kGvMaxStages;
-    while (stages > 2 && gv_layout(p.M, mt, tpw, G, ks, stages).total > budget) --stages;
+    while (stages > 2 && gv_layout(M, mt, tpw, G, ks, stages).total > budget) --stages;
     if (forced_stages > 0 && forced_stages <= kGvMaxStages) stages = forced_stages < G / ks ? forced_stages : G / ks;
     if (stages < 1) stages = 1;
-    const GvLayout L = gv_layout(p.M, mt, tpw, G, ks, stages);
-    if (L.total > 226 * 1024) return GPTRS_UNIMPLEMENTED;
+    const GvLayout L = gv_layout(M, mt, tpw, G, ks, stages);
+    if (L.total > 226 * 1024) return false;
+    *out = {mt, split, G, tpw, ks, stages, L.total};
+    return true;
+}
+
+}  // namespace
+
+// Output columns of a CTA of the W4 kernel for 1..16 rows (0: no plan fits and another kernel takes the call): the width of the tiles
+// that a folded RMSNorm is summed over.
+int w4_gemv_tile_cols(int M, int N, int K) {
+    GvPlan g;
+    return gv_plan(M, N, K, &g) ? kGvWarps / g.ks * g.tpw * 16 : 0;
+}
+
+// Called by quant_matmul.cu for W4 weights and 1..16 rows. Returns GPTRS_UNIMPLEMENTED when no split fits.
+int w4_gemv(MatmulParams p, cudaStream_t st) {
+    GvPlan g;
+    if (!gv_plan(p.M, p.N, p.K, &g)) return GPTRS_UNIMPLEMENTED;
+    const int mt = g.mt, tpw = g.tpw;
     if (!p.status) p.status = matmul_status_word();
     if (!p.status) return fail(GPTRS_EXECUTION, "cannot find the status word of this device");
-    p.n_split = split;
-    p.groups_per_cta = G;
-    p.k_intra = ks;
-    p.gemv_stages = stages;
-    dim3 grid(ceil_div(ceil_div(n_tiles, tpw) * ks, kGvWarps), split, 1);
+    p.n_split = g.split;
+    p.groups_per_cta = g.G;
+    p.k_intra = g.ks;
+    p.gemv_stages = g.stages;
+    dim3 grid(ceil_div(ceil_div(p.N >> 4, tpw) * g.ks, kGvWarps), g.split, 1);
     if (mt == 1) {
-        if (tpw == 4) return launch_gemv<1, 4>(p, grid, L.total, st);
-        if (tpw == 2) return launch_gemv<1, 2>(p, grid, L.total, st);
-        return launch_gemv<1, 1>(p, grid, L.total, st);
+        if (tpw == 4) return launch_gemv<1, 4>(p, grid, g.smem, st);
+        if (tpw == 2) return launch_gemv<1, 2>(p, grid, g.smem, st);
+        return launch_gemv<1, 1>(p, grid, g.smem, st);
     }
-    if (tpw == 2) return launch_gemv<2, 2>(p, grid, L.total, st);
-    return launch_gemv<2, 1>(p, grid, L.total, st);
+    if (tpw == 2) return launch_gemv<2, 2>(p, grid, g.smem, st);
+    return launch_gemv<2, 1>(p, grid, g.smem, st);
 }
 
 }  // namespace gptrs

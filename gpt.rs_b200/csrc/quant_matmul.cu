@@ -27,6 +27,7 @@ int umma_w8a16_matmul(MatmulParams p, cudaStream_t st);  // umma_matmul.cu
 int umma_status(int* out);
 void umma_debug_fault(int starve, uint32_t spin_limit);
 int w4_gemv(MatmulParams p, cudaStream_t st);  // quant_gemv.cu
+int w4_gemv_tile_cols(int M, int N, int K);
 
 namespace {
 
@@ -135,6 +136,8 @@ quant_matmul_kernel(const MatmulParams p) {
     };
     pdl_launch_dependents();  // dependents still wait for this whole grid before reading its results
     pdl_wait();  // x (and the residual) come from the previous kernel in the stream
+    __shared__ float row_scales[MPAD <= 16 ? MPAD : 1];
+    if (MPAD <= 16) few_row_scales(p, row_scales, warp, kWarps, lane);
 #pragma unroll
     for (int s = 0; s < kXStages - 1; ++s) issue_x(s);
 
@@ -256,7 +259,7 @@ quant_matmul_kernel(const MatmulParams p) {
             sr.push(owner, lr, c + 8, acc[i][2 + h]);
         }
     }
-    split_reduce_finish<MPAD>(p, sr, slots, tid, kWarps * 32, m0, blockIdx.x * kCtaN);
+    split_reduce_finish<MPAD>(p, sr, slots, tid, kWarps * 32, m0, blockIdx.x * kCtaN, kCtaN, true, MPAD <= 16 ? row_scales : nullptr);
 }
 
 // ---- layout conversion kernels --------------------------------------------------------------
@@ -546,7 +549,7 @@ int pick_split(int n_blocks, int groups) {
 
 template <int BITS>
 int quant_matmul(const void* d_x, const void* d_packed, void* d_y, int64_t m, int64_t n, int64_t k,
-                 const gptrs_matmul_epilogue* ep, void* stream) {
+                 const gptrs_matmul_epilogue* ep, void* stream, bool fold_few_rows = false) {
     GPTRS_REQUIRE(d_x && d_packed && d_y, "null pointer");
     GPTRS_REQUIRE(m >= 0 && n > 0 && k > 0, "bad shape");
     GPTRS_REQUIRE(k % 128 == 0, "K must be a multiple of 128");
@@ -581,7 +584,7 @@ int quant_matmul(const void* d_x, const void* d_packed, void* d_y, int64_t m, in
         GPTRS_REQUIRE(!p.swiglu || n % 32 == 0, "swiglu needs N % 32 == 0");
         if (ep->d_sumsq_out || ep->d_norm_x || ep->d_norm_gamma) {
             GPTRS_REQUIRE(ep->d_sumsq_out && ep->d_norm_x && ep->d_norm_gamma, "folded norm: gamma, x and sumsq_out go together");
-            GPTRS_REQUIRE(m > 16 && n % 128 == 0 && !p.swiglu, "folded norm producer: more than 16 rows, N % 128 == 0, no swiglu");
+            GPTRS_REQUIRE((m > 16 || fold_few_rows) && n % 128 == 0 && !p.swiglu, "folded norm producer: more than 16 rows, N % 128 == 0, no swiglu");
             p.norm_gamma = ep->d_norm_gamma;
             p.norm_x = static_cast<__nv_bfloat16*>(ep->d_norm_x);
             p.sumsq_out = ep->d_sumsq_out;
@@ -615,7 +618,7 @@ int quant_matmul(const void* d_x, const void* d_packed, void* d_y, int64_t m, in
             p.peer = *pv;
         }
         if (ep->d_sumsq_in) {
-            GPTRS_REQUIRE(m > 16 && ep->sumsq_tiles > 0 && ep->norm_dim > 0, "folded norm consumer: more than 16 rows, tiles and norm_dim set");
+            GPTRS_REQUIRE((m > 16 || fold_few_rows) && ep->sumsq_tiles > 0 && ep->norm_dim > 0, "folded norm consumer: more than 16 rows, tiles and norm_dim set");
             p.sumsq_in = ep->d_sumsq_in;
             p.sumsq_tiles = ep->sumsq_tiles;
             p.norm_dim = ep->norm_dim;
@@ -624,7 +627,7 @@ int quant_matmul(const void* d_x, const void* d_packed, void* d_y, int64_t m, in
     }
     cudaStream_t st = as_stream(stream);
     if (m > 16 && umma_enabled()) return BITS == 4 ? umma_w4a16_matmul(p, st) : umma_w8a16_matmul(p, st);
-    GPTRS_REQUIRE(!p.sumsq_in && !p.sumsq_out && !p.rope_pos, "the folded norm / RoPE epilogues need the tensor-core matmul path");
+    GPTRS_REQUIRE((fold_few_rows && m <= 16) || (!p.sumsq_in && !p.sumsq_out && !p.rope_pos), "the folded norm / RoPE epilogues need the tensor-core matmul path");
     const int groups = (int)(k / 128);
     const int n_blocks = ceil_div(n, kCtaN);
     p.n_split = pick_split(n_blocks, groups);
@@ -646,6 +649,16 @@ int quant_matmul(const void* d_x, const void* d_packed, void* d_y, int64_t m, in
 }
 
 }  // namespace
+
+// The engine's form for 1..16 rows: the folded RMSNorm is summed over tiles of quant_tile_cols columns instead of 128.
+int quant_tile_cols(int bits, int64_t m, int64_t n, int64_t k) {
+    const int cols = bits == 4 && m <= 16 && gemv_enabled() ? w4_gemv_tile_cols((int)m, (int)n, (int)k) : 0;
+    return cols ? cols : kCtaN;
+}
+int quant_matmul_few_rows(int bits, const void* x, const void* packed, void* y, int64_t m, int64_t n, int64_t k, const gptrs_matmul_epilogue* ep, cudaStream_t st) {
+    return bits == 4 ? quant_matmul<4>(x, packed, y, m, n, k, ep, st, true) : quant_matmul<8>(x, packed, y, m, n, k, ep, st, true);
+}
+
 }  // namespace gptrs
 
 using namespace gptrs;
