@@ -43,10 +43,126 @@ struct RowsParams {
     int64_t ldy, y_step;
     const gptrs_row_tile* tiles; // grouped form
     const int* n_row_tiles;
+    MatmulParams q;              // ACT 5: the epilogues of a quantised projection (quant_rows_matmul)
 };
 
+// ACT 5: what stands around a projection of the quantised engine (split_reduce_finish in matmul_common.cuh), for a thread that holds 128
+// columns of a row: the folded RMSNorm of the input, RoPE + KV append (the columns are a head), SwiGLU, or residual + output with the
+// folded norm that follows.
+__device__ __forceinline__ void projection_epilogue(const MatmulParams& q, uint32_t acc, int m, int n0, float rs) {
+    const bool live = m < q.M;
+    float v[32], u[32];
+    if (q.rope_pos) {
+        const int head = n0 >> 7;
+        const bool is_q = head < q.rope_hq, is_v = head >= q.rope_hq + q.rope_hkv;
+        const int pos = live ? q.rope_pos[m] : 0;
+        auto rb = [](float t) { return __bfloat162float(__float2bfloat16_rn(t)); };
+        unsigned char* blk = nullptr;
+        if (live && !is_q) {
+            const int kvh = is_v ? head - q.rope_hq - q.rope_hkv : head - q.rope_hq;
+            const int page = q.rope_page_table[(size_t)q.rope_slot[m] * q.rope_max_pages + (pos >> 4)];
+            blk = q.rope_pool + ((size_t)page * q.rope_hkv + kvh) * 8192 + (is_v ? 4096 : 0) + (pos & 15) * 256;
+        }
+#pragma unroll 1
+        for (int c0 = 0; c0 < 64; c0 += 32) {   // channels c and c + 64
+            __syncwarp();
+            tmem_ld_32(acc + c0, v);
+            tmem_ld_32(acc + c0 + 64, u);
+            if (!live) continue;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) { v[i] = rb(v[i] * rs); u[i] = rb(u[i] * rs); }
+            if (!is_v) {
+                const float4* cp = reinterpret_cast<const float4*>(q.rope_cos + (size_t)pos * 64 + c0);
+                const float4* sp = reinterpret_cast<const float4*>(q.rope_sin + (size_t)pos * 64 + c0);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float4 c = __ldg(cp + i), s = __ldg(sp + i);
+                    const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float a = v[4 * i + j], b = u[4 * i + j];
+                        v[4 * i + j] = a * cs[j] - b * sn[j];
+                        u[4 * i + j] = b * cs[j] + a * sn[j];
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 lo = make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
+                                            pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
+                const uint4 hi = make_uint4(pack_bf16x2(u[8 * i], u[8 * i + 1]), pack_bf16x2(u[8 * i + 2], u[8 * i + 3]),
+                                            pack_bf16x2(u[8 * i + 4], u[8 * i + 5]), pack_bf16x2(u[8 * i + 6], u[8 * i + 7]));
+                const int chunk = (c0 >> 3) + i;
+                if (is_q) {
+                    uint4* dst = reinterpret_cast<uint4*>(q.rope_q_out + ((size_t)m * q.rope_hq + head) * 128);
+                    dst[chunk] = lo;
+                    dst[chunk + 8] = hi;
+                } else {
+                    *reinterpret_cast<uint4*>(blk + ((chunk ^ (pos & 7)) << 4)) = lo;
+                    *reinterpret_cast<uint4*>(blk + (((chunk + 8) ^ (pos & 7)) << 4)) = hi;
+                }
+            }
+        }
+        return;
+    }
+    float ss = 0.f;
+#pragma unroll 1
+    for (int c0 = 0; c0 < 128; c0 += 32) {
+        __syncwarp();
+        tmem_ld_32(acc + c0, v);
+        if (!live) continue;
+        const int n = n0 + c0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] *= rs;
+        if (q.swiglu) {   // 8 gates, then the 8 values they meet
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(q.y) + (size_t)m * (q.N >> 1) + (n >> 1));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float o[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = v[16 * h + i] / (1.f + expf(-v[16 * h + i])) * v[16 * h + 8 + i];
+                dst[h] = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+            }
+            continue;
+        }
+        if (q.residual) {
+            const float4* r = reinterpret_cast<const float4*>(q.residual + (size_t)m * q.N + n);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 t = r[i];
+                v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
+            }
+        }
+        if (q.out_f32) {
+            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(q.y) + (size_t)m * q.N + n);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        } else {
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(q.y) + (size_t)m * q.N + n);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                dst[i] = make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]), pack_bf16x2(v[8 * i + 4], v[8 * i + 5]),
+                                    pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
+        }
+        if (q.sumsq_out) {
+            uint4* dst = reinterpret_cast<uint4*>(q.norm_x + (size_t)m * q.N + n);
+            const float4* gp = reinterpret_cast<const float4*>(q.norm_gamma + n);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 a = __ldg(gp + 2 * i), b = __ldg(gp + 2 * i + 1);
+                dst[i] = make_uint4(pack_bf16x2(v[8 * i] * a.x, v[8 * i + 1] * a.y), pack_bf16x2(v[8 * i + 2] * a.z, v[8 * i + 3] * a.w),
+                                    pack_bf16x2(v[8 * i + 4] * b.x, v[8 * i + 5] * b.y), pack_bf16x2(v[8 * i + 6] * b.z, v[8 * i + 7] * b.w));
+            }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) ss = fmaf(v[i], v[i], ss);
+        }
+    }
+    if (q.sumsq_out && live) q.sumsq_out[(size_t)(n0 >> 7) * q.M + m] = ss;
+}
+
 constexpr int kRowsThreads = 384;    // warps 0-3 and 8-11 epilogue, 4 MMA + tensor memory, 5 loader
-// ACT: 0 none, 1 xIELU, 2 whatever p.act says (with a soft cap), 3 act(gate) partner (8 gates, then their 8 partners), 4 squared relu.
+// ACT: 0 none, 1 xIELU, 2 whatever p.act says (with a soft cap), 3 act(gate) partner (8 gates, then their 8 partners), 4 squared relu, 5 the
+// epilogues of a quantised projection (BN 256).
 // GROUPED: the row tiles come from a list in device memory, each with the weight matrix that it meets.
 template <int BN, int STAGES, int ACT, bool GROUPED = false>
 __global__ void __launch_bounds__(kRowsThreads, 1) dense_rows_kernel(const __grid_constant__ RowsParams p) {
@@ -137,9 +253,25 @@ __global__ void __launch_bounds__(kRowsThreads, 1) dense_rows_kernel(const __gri
             const int buf = n & 1;
             const Tile tl = tile_of(t);
             const int m0 = tl.m0, n0 = tl.n0;
+            const int m = m0 + quarter * 32 + lane;
+            if constexpr (ACT == 5) {
+                float rs = 1.f;
+                if (p.q.sumsq_in && m < p.M) {
+                    float ss = 0.f;
+#pragma unroll 8
+                    for (int i = 0; i < p.q.sumsq_tiles; ++i) ss += __ldg(p.q.sumsq_in + (size_t)i * p.M + m);
+                    rs = rsqrtf(ss / (float)p.q.norm_dim + p.q.norm_eps);
+                }
+                if (!wait(&acc_full[buf], (uint32_t)(n / 2) & 1u)) break;
+                tc_fence_after();
+                if (n0 + c_lo < p.N) projection_epilogue(p.q, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN + c_lo), m, n0 + c_lo, rs);
+                __syncwarp();
+                tc_fence_before();
+                mbar_arrive(&acc_empty[buf]);
+                continue;
+            }
             if (!wait(&acc_full[buf], (uint32_t)(n / 2) & 1u)) break;
             tc_fence_after();
-            const int m = m0 + quarter * 32 + lane;
             const int64_t row = (GROUPED ? 0 : tl.b * p.y_step) + (int64_t)m * p.ldy;
 #pragma unroll 1
             for (int c0 = c_lo; c0 < c_lo + BN / 2 && n0 + c0 < p.N; c0 += 32) {
@@ -419,6 +551,27 @@ int launch_channels(const Call& c, cudaStream_t st) {
 }
 
 }  // namespace
+
+// A projection of many rows of the quantised engine on weights that have been widened to bf16 [N][K]: the prompt kernel above with the
+// epilogues of p. N a multiple of 128.
+int quant_rows_matmul(const MatmulParams& q, const void* w, cudaStream_t st) {
+    RowsParams p = {};
+    int rc = encode(&p.x_map, q.x, q.K, q.M, q.K, kTileM);
+    if (!rc) rc = encode(&p.w_map, w, q.K, q.N, q.K, 256);
+    if (rc) return rc;
+    p.q = q;
+    p.status = q.status;
+    p.M = q.M; p.N = q.N; p.K = q.K; p.batch = 1;
+    p.m_tiles = ceil_div(q.M, kTileM); p.n_tiles = ceil_div(q.N, 256);
+    p.w_rows = q.N;
+    constexpr size_t smem = 4 * (size_t)(kATile + 256 * 128) + 1024;
+    void (*kern)(RowsParams) = dense_rows_kernel<256, 4, 5>;
+    static PerDeviceOnce attr_once;
+    if (attr_once.first_time()) GPTRS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+    return launch_kernel(kern, dim3((unsigned)(tiles < sm_count() ? tiles : sm_count())), dim3(kRowsThreads), smem, st, 1, p);
+}
+
 }  // namespace gptrs
 
 using namespace gptrs;

@@ -232,7 +232,7 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
     }
     if (rows <= 16) return quant_matmul_few_rows(m.cfg.weight_mode == kModeW4 ? 4 : 8, x, w.packed->data, y, rows, w.out, w.in, &ep, st);
     return m.cfg.weight_mode == kModeW4
-               ? gptrs_cuda_quant_matmul_w4a16(x, w.packed->data, y, rows, w.out, w.in, &ep, st)
+               ? quant_matmul_rows(x, w.packed->data, y, rows, w.out, w.in, &ep, m.wide.p, m.wide.n, st)
                : gptrs_cuda_quant_matmul_w8a16(x, w.packed->data, y, rows, w.out, w.in, &ep, st);
 }
 
@@ -1012,6 +1012,12 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
     // activations
     const int T = c.max_tokens;
     const size_t act = m.f32() ? 4 : 2;
+    if (c.weight_mode == kModeW4 && T >= quant_widen_rows()) {   // as large as the largest projection of a layer; the head has few rows
+        size_t most = 0;
+        for (const Layer& L : m.layers)
+            for (const Weight* w : {&L.qkv, &L.attn_out, &L.mlp_gate_up, &L.mlp_out}) most = std::max(most, (size_t)w->in * w->out * 2);
+        if (m.wide.alloc(most)) cudaGetLastError();   // without it the kernel that widens inside its tiles takes every row count
+    }
     // sums of squares per row and column tile: 128 columns, or 16 with up to 16 rows
     if (!m.f32() && (rc = m.sumsq.alloc((size_t)((D + 127) / 128) * std::max<size_t>(T, 8 * 16) * 4, true))) return rc;
     if ((rc = m.hidden.alloc((size_t)T * D * 4)) || (rc = m.xn.alloc((size_t)T * D * act)) || (rc = m.xn_rows.alloc((size_t)T * D * act)) ||

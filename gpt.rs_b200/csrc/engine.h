@@ -203,6 +203,7 @@ struct Model {
     bool fuse_pick = true;   // GPTRS_FUSE_PICK=0: logits + sampling kernel
     // f32 GPT kind, one sequence: the whole decode step as one cooperative kernel (gpt_decode_mega.cu)
     int mega_rows = 0;   // most sequences of a step that is one kernel (0: none)
+    DevBuf wide;                    // W4 prompts: the widened weights of one projection at a time
     DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
     MegaParams mega = {};
     int gen_batch = 0;  // slots 0..gen_batch-1 are driven by generator_step
@@ -271,6 +272,11 @@ int attention_rows_f32(const float* qkv, const float* k_cache, const float* v_ca
 // columns of the producer.
 int quant_tile_cols(int bits, int64_t m, int64_t n, int64_t k);
 int quant_matmul_few_rows(int bits, const void* x, const void* packed, void* y, int64_t m, int64_t n, int64_t k, const gptrs_matmul_epilogue* ep, cudaStream_t st);
+
+// W4 matmuls of a prompt's rows, from quant_widen_rows() on with the weights widened to bf16 first, in a buffer of the caller.
+int quant_matmul_rows(const void* x, const void* packed, void* y, int64_t m, int64_t n, int64_t k, const gptrs_matmul_epilogue* ep, void* wide, size_t wide_bytes,
+                      cudaStream_t st);
+int64_t quant_widen_rows();
 
 // A decode step's RoPE, KV append and attention in one kernel (paged_attention.cu); splits from attention_step_splits, not 0.
 int attention_step_splits(int64_t max_ctx_len, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads);
