@@ -66,6 +66,48 @@ __global__ void strided_copy_kernel(const CopyParams p) {
     static_cast<T*>(p.out)[oo] = static_cast<const T*>(p.in)[io];
 }
 
+// out = in with `upd` written over it at clamped device starts, in one launch instead of a copy and an update: four neighbouring elements
+// of the innermost axis per thread (rows of a multiple of four 32-bit elements).
+struct UpdateParams {
+    const uint4* in;
+    const uint32_t* upd;
+    uint4* out;
+    const int* starts;
+    int rank;
+    uint32_t n4, dims[kMaxRank], size[kMaxRank];   // of the operand, of the update
+};
+__global__ void __launch_bounds__(256) update_slice_kernel(const UpdateParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= p.n4) return;
+    uint32_t rem = i * 4, at = 0, stride = 1, first = 0, start_in = 0;
+    bool inside = true;
+#pragma unroll 1
+    for (int d = p.rank - 1; d >= 0; --d) {
+        const uint32_t c = rem % p.dims[d];
+        rem /= p.dims[d];
+        const int lim = (int)(p.dims[d] - p.size[d]);
+        const uint32_t s = (uint32_t)min(max(p.starts[d], 0), lim);
+        if (d == p.rank - 1) { first = c; start_in = s; }
+        else {
+            inside = inside && c >= s && c - s < p.size[d];
+            at += (c - s) * stride;
+        }
+        stride *= p.size[d];
+    }
+    uint4 v = p.in[i];
+    const uint32_t inner = p.size[p.rank - 1];
+    if (inside && first + 3 >= start_in && first < start_in + inner) {
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (first + j >= start_in && first + j - start_in < inner) w[j] = p.upd[at + first + j - start_in];
+        v = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    p.out[i] = v;
+}
+
 enum { U_NEG, U_ABS, U_EXP, U_LOG, U_TANH, U_ERF, U_RSQRT, U_RECIP };
 enum { B_ADD, B_SUB, B_MUL, B_DIV, B_MAX, B_MIN };
 enum { C_LT, C_LE, C_EQ, C_GE, C_GT, C_NE };
@@ -791,7 +833,44 @@ void rewrite(Plan& pl, bool in_process = true) {
 
 // True for operations whose result is (or may be) the storage of an operand: their source must live as long as they do.
 bool may_alias_operand(const Inst& in) {
-    return in.op == Op::Reshape || in.op == Op::Constant || in.op == Op::StopGradient || in.op == Op::Cast;
+    return in.op == Op::Reshape || in.op == Op::Constant || in.op == Op::StopGradient || in.op == Op::Cast || in.view;
+}
+
+// Element offset of a Slice whose result lies in one piece in its operand (one index on the axes in front of an axis, all of the axes
+// behind it), -1 otherwise.
+int64_t slice_offset(const Inst& in, const std::vector<int64_t>& dims) {
+    if (in.op != Op::Slice || dims.size() != in.out.dims.size() || in.a.size() != dims.size()) return -1;
+    int64_t off = 0, stride = 1;
+    bool whole = true;   // every axis behind this one is taken whole
+    for (size_t d = dims.size(); d-- > 0;) {
+        if (in.a[d] < 0 || in.a[d] + in.out.dims[d] > dims[d]) return -1;   // the copy reports it
+        if (!whole && in.out.dims[d] != 1) return -1;
+        off += in.a[d] * stride;
+        stride *= dims[d];
+        whole = whole && in.out.dims[d] == dims[d];
+    }
+    return off;
+}
+
+// Slices of values of the plan that can be views: in one piece, on a 256-byte boundary of a buffer (kernels load 16 bytes at a time), and
+// not handed out as a result, directly or through another alias (a result owns its storage).
+void mark_views(Plan& pl) {
+    auto& body = pl.fn.body;
+    std::vector<char> out(body.size(), 0);
+    auto idx_of = [&](uint32_t id) { auto it = pl.def.find(id); return it == pl.def.end() ? -1 : it->second; };
+    for (uint32_t r : pl.fn.result_ids) { const int i = idx_of(r); if (i >= 0) out[i] = 1; }
+    for (int i = (int)body.size() - 1; i >= 0; --i) {
+        Inst& in = body[i];
+        if (in.dead) continue;
+        if (in.op == Op::Slice && !out[i] && !in.operands.empty() && !in.operands[0].is_literal && idx_of(in.operands[0].id) >= 0) {
+            const TSpec* src = spec_of(pl, in.operands[0]);
+            const int64_t off = src ? slice_offset(in, src->dims) : -1;
+            in.view = off >= 0 && off * (int64_t)dtype_size(in.out.dtype) % 256 == 0;
+        }
+        if (out[i] && may_alias_operand(in))
+            for (const Operand& o : in.operands)
+                if (!o.is_literal && idx_of(o.id) >= 0) out[idx_of(o.id)] = 1;
+    }
 }
 
 // Assigns arena offsets (see Plan). Lifetimes are instruction indices; a value that an aliasing operation forwards
@@ -1014,6 +1093,17 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
             break;
         }
         case Op::Transpose: case Op::BroadcastTo: case Op::Slice: case Op::DynamicSlice: {
+            if (in.view) {
+                const int64_t off = slice_offset(in, ops[0]->dims);
+                if (off < 0) return spec("slice out of bounds");
+                Tensor* t = new Tensor();
+                t->dtype = ops[0]->dtype; t->dims = in.out.dims; t->bytes = (size_t)n_out * dtype_size(in.out.dtype);
+                t->data = static_cast<unsigned char*>(ops[0]->data) + off * (int64_t)dtype_size(in.out.dtype);
+                t->owns = false; t->base = ops[0];
+                tensor_retain(ops[0]);
+                *result = t;
+                return GPTRS_OK;
+            }
             if ((rc = alloc_out())) return rc;
             const auto& od = in.out.dims;
             std::vector<int64_t> istr = row_major_strides(ops[0]->dims), ostr = row_major_strides(od), use(od.size(), 0);
@@ -1045,6 +1135,24 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
         case Op::DynamicUpdateSlice: {
             if ((rc = alloc_out())) return rc;
             if (ops[0]->dims != in.out.dims || ops[1]->dims.size() != in.out.dims.size() || ops[2]->dtype != GPTRS_SI32) { tensor_release(out); return spec("operand mismatch"); }
+            {
+                const size_t rank = in.out.dims.size();
+                const int64_t n = in.out.numel();
+                bool fits = rank >= 1 && rank <= (size_t)kMaxRank && dtype_size(in.out.dtype) == 4 && ops[0]->dtype == in.out.dtype && ops[1]->dtype == in.out.dtype &&
+                            ops[2]->numel() == (int64_t)rank && n > 0 && n < (1ll << 32) && in.out.dims[rank - 1] % 4 == 0 && ops[1]->numel() > 0 &&
+                            ((reinterpret_cast<uintptr_t>(ops[0]->data) | reinterpret_cast<uintptr_t>(out->data)) & 15) == 0;
+                UpdateParams p = {static_cast<const uint4*>(ops[0]->data), static_cast<const uint32_t*>(ops[1]->data), static_cast<uint4*>(out->data),
+                                  static_cast<const int*>(ops[2]->data), (int)rank, (uint32_t)(n / 4)};
+                for (size_t d = 0; d < rank && fits; ++d) {
+                    fits = ops[1]->dims[d] <= in.out.dims[d];
+                    p.dims[d] = (uint32_t)in.out.dims[d]; p.size[d] = (uint32_t)ops[1]->dims[d];
+                }
+                if (fits) {
+                    ++ex.launches;
+                    rc = launch_kernel(update_slice_kernel, dim3((unsigned)ceil_div(p.n4, 256)), dim3(256), 0, ex.st, 1, p);
+                    break;
+                }
+            }
             GPTRS_CUDA_OK(cudaMemcpyAsync(out->data, ops[0]->data, out->bytes, cudaMemcpyDeviceToDevice, ex.st));
             ++ex.launches;
             std::vector<int64_t> ostr = row_major_strides(in.out.dims), ustr = row_major_strides(ops[1]->dims), lim(in.out.dims.size());
@@ -1337,6 +1445,7 @@ int plan_for(const char* program_json, size_t len, std::shared_ptr<Plan>* out) {
         if (int rc = upload_literals(*p)) return rc;
         p->device = device;
         count_uses(*p);
+        mark_views(*p);
         if (g_arena_enabled) plan_buffers(*p);
         std::lock_guard<std::mutex> lk(g_plan_mu);
         g_plans[key] = p;

@@ -66,6 +66,7 @@ struct Inst {
     std::vector<Operand> operands;
     TSpec out;
     bool dead = false;            // removed by a rewrite
+    bool view = false;            // Slice: its result is a part of the operand's storage (set when a plan is built)
     int src = -1;                 // index of the instruction in the function body it was read from
     // A fused residual-add + norm also produces the sum itself when other instructions read it: the value id and type
     // of that second result (0 = none). Only the in-process rewrite uses it; the CustomCall text form has one result.
