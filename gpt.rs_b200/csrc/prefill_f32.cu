@@ -2,9 +2,11 @@
 // for every row of a prompt): a CTA takes one query head of 32 neighbouring rows, so that a key is read once for up to 32 queries
 // instead of once for each.
 //
-// 128 threads, 32 x 64 scores per block of keys with a 4 x 4 tile per thread (operands in shared memory, 16-byte reads: 4 + 4 of them
-// feed 64 fused multiply-adds), online softmax in f32 over the 16 threads of a row, then 4 rows x HD / 16 columns of the output per
-// thread. 109 us for 937 rows of 12 heads of 64 (464 with a CTA per row and head), a chain of up to 15 blocks in the last rows' CTAs.
+// Two groups of 128 threads take the blocks of 64 keys in turn, each with its own online softmax, and merge at the end: the last rows'
+// CTAs are a chain of blocks (15 at 937 rows), and that chain is what the kernel takes. Per block a group has 32 x 64 scores with a 4 x 4
+// tile per thread (operands in shared memory, 16-byte reads: 4 + 4 of them feed 64 fused multiply-adds), the softmax in f32 over the 16
+// threads of a row, then 4 rows x HD / 16 columns of the output per thread. Heads are the fastest grid axis, so that the longest chains
+// start first. 937 rows of 12 heads of 64: 72 us; 109 with one group, 464 with a CTA per row and head.
 // Rows of a tile that belong to different sequences are taken one sequence after another.
 #include "common.cuh"
 
@@ -22,28 +24,29 @@ struct PrefillF32Params {
     float scale;
 };
 
-constexpr int kPfRows = 32, kPfKeys = 64, kPfThreads = 4 * kPfRows;
+constexpr int kPfRows = 32, kPfKeys = 64, kPfGroup = 4 * kPfRows, kPfThreads = 2 * kPfGroup;
 
 template <int HD>
 __global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const PrefillF32Params p) {
     constexpr int LD = HD + 4, LP = kPfKeys + 4, OC = HD / 64;   // OC float4 columns of a thread
     extern __shared__ __align__(16) float pf_smem[];
-    float* qs = pf_smem;                   // [32][LD]
-    float* ks = qs + kPfRows * LD;         // [64][LD]
-    float* vs = ks + kPfKeys * LD;         // [64][LD]
-    float* ps = vs + kPfKeys * LD;         // [32][LP]
+    const int group = threadIdx.x / kPfGroup, tid = threadIdx.x % kPfGroup, ty = tid >> 4, tx = tid & 15;
+    float* qs = pf_smem;                                             // [32][LD]
+    float* ks = qs + kPfRows * LD + group * (2 * kPfKeys * LD + kPfRows * LP);   // a group's [64][LD]
+    float* vs = ks + kPfKeys * LD;                                   // [64][LD]
+    float* ps = vs + kPfKeys * LD;                                   // [32][LP]
     __shared__ int pos_s[kPfRows], slot_s[kPfRows];
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * kPfRows;   // the last rows see the most keys: they start first
-    const int h = blockIdx.y, hk = h / (p.Hq / p.Hkv), rows = min(kPfRows, p.T - t0);
+    auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "n"(kPfGroup) : "memory"); };
+    const int t0 = (int)(gridDim.y - 1 - blockIdx.y) * kPfRows;      // the last rows see the most keys: they start first
+    const int h = blockIdx.x, hk = h / (p.Hq / p.Hkv), rows = min(kPfRows, p.T - t0);
     const int width = (p.Hq + 2 * p.Hkv) * HD;
     pdl_launch_dependents();
     pdl_wait();
-    if (tid < kPfRows) {
+    if (threadIdx.x < kPfRows) {
         slot_s[tid] = tid < rows ? p.slot[t0 + tid] : -1;
         pos_s[tid] = tid < rows ? min(max(p.positions[t0 + tid], 0), p.capacity - 1) : -1;   // DynamicUpdateSlice clamps its start
     }
-    for (int i = tid; i < kPfRows * (HD / 4); i += kPfThreads) {
+    for (int i = threadIdx.x; i < kPfRows * (HD / 4); i += kPfThreads) {
         const int r = i / (HD / 4), c = i % (HD / 4) * 4;
         *reinterpret_cast<float4*>(qs + r * LD + c) =
             r < rows ? *reinterpret_cast<const float4*>(p.qkv + (size_t)(t0 + r) * width + h * HD + c) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -65,16 +68,17 @@ __global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const Pr
         int limit[4];   // last visible key of this thread's rows in this run
 #pragma unroll
         for (int r = 0; r < 4; ++r) limit[r] = 4 * ty + r >= seg && 4 * ty + r < end ? pos_s[4 * ty + r] : -1;
-        for (int j0 = 0; j0 <= last; j0 += kPfKeys) {
-            __syncthreads();   // the block before has been used
-            for (int i = tid; i < kPfKeys * (HD / 4); i += kPfThreads) {
+        for (int j0 = group * kPfKeys; j0 <= last; j0 += 2 * kPfKeys) {
+            group_sync();   // the block before has been used
+#pragma unroll 8
+            for (int i = tid; i < kPfKeys * (HD / 4); i += kPfGroup) {
                 const int j = i / (HD / 4), c = i % (HD / 4) * 4;
                 const bool in = j0 + j <= last;
                 const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                 *reinterpret_cast<float4*>(ks + j * LD + c) = in ? *reinterpret_cast<const float4*>(kc + (size_t)(j0 + j) * HD + c) : zero;
                 *reinterpret_cast<float4*>(vs + j * LD + c) = in ? *reinterpret_cast<const float4*>(vc + (size_t)(j0 + j) * HD + c) : zero;
             }
-            __syncthreads();
+            group_sync();
             float s[4][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
@@ -143,23 +147,43 @@ __global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const Pr
         }
         seg = end;
     }
+    // group 1 hands its state over in its own buffers: [row][16 threads][4 OC], then maximum and sum
+    float* other = qs + kPfRows * LD + 2 * kPfKeys * LD + kPfRows * LP;
+    float* other_ml = other + kPfRows * HD;
+    if (group == 1) {
+        group_sync();   // its last block has been used
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int c = 0; c < OC; ++c)
+                *reinterpret_cast<float4*>(other + (4 * ty + r) * HD + 4 * tx + 64 * c) = make_float4(o[r][4 * c], o[r][4 * c + 1], o[r][4 * c + 2], o[r][4 * c + 3]);
+            if (tx == 0) { other_ml[2 * (4 * ty + r)] = mx[r]; other_ml[2 * (4 * ty + r) + 1] = sum[r]; }
+        }
+    }
+    __syncthreads();
+    if (group == 1) return;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         if (4 * ty + r >= rows) continue;
-        const float inv = sum[r];
+        // group 0 has seen position 0 of every row: its maximum is a number
+        const float m1 = other_ml[2 * (4 * ty + r)], top = fmaxf(mx[r], m1), f0 = expf(mx[r] - top), f1 = expf(m1 - top);
+        const float inv = sum[r] * f0 + other_ml[2 * (4 * ty + r) + 1] * f1;
 #pragma unroll
-        for (int c = 0; c < OC; ++c)
+        for (int c = 0; c < OC; ++c) {
+            const float4 u = *reinterpret_cast<const float4*>(other + (4 * ty + r) * HD + 4 * tx + 64 * c);
             *reinterpret_cast<float4*>(p.out + ((size_t)(t0 + 4 * ty + r) * p.Hq + h) * HD + 4 * tx + 64 * c) =
-                make_float4(o[r][4 * c] / inv, o[r][4 * c + 1] / inv, o[r][4 * c + 2] / inv, o[r][4 * c + 3] / inv);
+                make_float4((o[r][4 * c] * f0 + u.x * f1) / inv, (o[r][4 * c + 1] * f0 + u.y * f1) / inv, (o[r][4 * c + 2] * f0 + u.z * f1) / inv,
+                            (o[r][4 * c + 3] * f0 + u.w * f1) / inv);
+        }
     }
 }
 
 template <int HD>
 int launch(const PrefillF32Params& p, cudaStream_t st) {
-    constexpr size_t smem = (size_t)((kPfRows + 2 * kPfKeys) * (HD + 4) + kPfRows * (kPfKeys + 4)) * sizeof(float);
+    constexpr size_t smem = (size_t)(kPfRows * (HD + 4) + 2 * (2 * kPfKeys * (HD + 4) + kPfRows * (kPfKeys + 4))) * sizeof(float);
     static PerDeviceOnce attr_once;
     if (attr_once.first_time()) GPTRS_CUDA_OK(cudaFuncSetAttribute(attention_rows_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return launch_kernel(attention_rows_f32_kernel<HD>, dim3((unsigned)ceil_div(p.T, kPfRows), (unsigned)p.Hq), dim3(kPfThreads), smem, st, 1, p);
+    return launch_kernel(attention_rows_f32_kernel<HD>, dim3((unsigned)p.Hq, (unsigned)ceil_div(p.T, kPfRows)), dim3(kPfThreads), smem, st, 1, p);
 }
 
 }  // namespace
