@@ -14,7 +14,10 @@ namespace {
 struct Params { gptrs_norm_step s; };
 
 // A thread holds the elements (i * THREADS + tid) * VEC + e, i < N.
-template <int THREADS, int N, int VEC>
+// EARLY: gains, the stream's row and up to eight experts' rows are asked for at once, beside what the first sum needs. For launches of few
+// rows, which are as long as a chain of loads (48 rows of 2048 with 6 experts each: 8.6 -> 5.6 us); with many rows the registers cost more
+// (113 instead of about 40; 1389 rows: 14.8 -> 18.2 us).
+template <int THREADS, int N, int VEC, bool EARLY = false>
 __global__ void __launch_bounds__(THREADS) norm_step_kernel(const Params p) {
     __shared__ float sh[32];
     const gptrs_norm_step& a = p.s;
@@ -22,7 +25,7 @@ __global__ void __launch_bounds__(THREADS) norm_step_kernel(const Params p) {
     pdl_launch_dependents();
     pdl_wait();
     const int row = a.d_rows ? a.d_rows[blockIdx.x] : (int)blockIdx.x;
-    float x[N][VEC];
+    float x[N][VEC], g_out[EARLY ? N : 1][VEC], old[EARLY ? N : 1][VEC], g_in[EARLY ? N : 1][VEC];
     bool in[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) in[i] = (i * THREADS + tid) * VEC < D;
@@ -46,11 +49,45 @@ __global__ void __launch_bounds__(THREADS) norm_step_kernel(const Params p) {
     } else if (a.d_y) {
         const bool y_bf16 = a.y_dtype == GPTRS_BF16;
         float ss = 0.f;
+        // what does not depend on the sums travels beside them (short rows: the registers are there)
+        if constexpr (EARLY) {
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (in[i]) {
+                    const int c = (i * THREADS + tid) * VEC;
+                    load_act<VEC>(a.d_gamma_out, c, false, g_out[i]);
+                    load_act<VEC>(a.d_x, (size_t)row * D + c, false, old[i]);
+                    if (a.d_gamma_in) load_act<VEC>(a.d_gamma_in, c, false, g_in[i]);
+                }
+        }
+        constexpr int kTop = 8;   // experts whose rows are asked for at once
+        int pair[kTop];
+        float weight[kTop];
+        const bool few = EARLY && a.d_pair && a.top <= kTop;
+        if constexpr (EARLY) if (few) {
+#pragma unroll
+            for (int k = 0; k < kTop; ++k) {
+                pair[k] = k < (int)a.top ? __ldg(a.d_pair + (size_t)row * a.top + k) : 0;
+                weight[k] = k < (int)a.top ? __ldg(a.d_pair_weight + (size_t)row * a.top + k) : 0.f;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < N; ++i)
             if (in[i]) {
                 const int c = (i * THREADS + tid) * VEC;
-                if (a.d_pair) {
+                if (few) {
+                    float v[kTop][VEC];
+#pragma unroll
+                    for (int k = 0; k < kTop; ++k)
+                        if (k < (int)a.top) load_act<VEC>(a.d_y, (size_t)pair[k] * a.ldy + c, y_bf16, v[k]);
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) x[i][e] = 0.f;
+#pragma unroll
+                    for (int k = 0; k < kTop; ++k)
+                        if (k < (int)a.top)
+#pragma unroll
+                            for (int e = 0; e < VEC; ++e) x[i][e] = fmaf(weight[k], v[k][e], x[i][e]);
+                } else if (a.d_pair) {
 #pragma unroll
                     for (int e = 0; e < VEC; ++e) x[i][e] = 0.f;
                     for (int k = 0; k < (int)a.top; ++k) {
@@ -71,11 +108,12 @@ __global__ void __launch_bounds__(THREADS) norm_step_kernel(const Params p) {
         for (int i = 0; i < N; ++i)
             if (in[i]) {
                 const int c = (i * THREADS + tid) * VEC;
-                float g[VEC], o[VEC];
-                load_act<VEC>(a.d_gamma_out, c, false, g);
-                load_act<VEC>(a.d_x, (size_t)row * D + c, false, o);
+                if constexpr (!EARLY) {
+                    load_act<VEC>(a.d_gamma_out, c, false, g_out[0]);
+                    load_act<VEC>(a.d_x, (size_t)row * D + c, false, old[0]);
+                }
 #pragma unroll
-                for (int e = 0; e < VEC; ++e) x[i][e] = o[e] + x[i][e] * inv * g[e];
+                for (int e = 0; e < VEC; ++e) x[i][e] = old[EARLY ? i : 0][e] + x[i][e] * inv * g_out[EARLY ? i : 0][e];
                 if (!a.d_rows) store_act<VEC>(a.d_x, (size_t)row * D + c, false, x[i]);
             }
     } else {
@@ -97,7 +135,12 @@ __global__ void __launch_bounds__(THREADS) norm_step_kernel(const Params p) {
         if (in[i]) {
             const int c = (i * THREADS + tid) * VEC;
             float g[VEC];
-            load_act<VEC>(a.d_gamma_in, c, false, g);
+            if (EARLY && a.d_y && !a.d_embed) {
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) g[e] = g_in[EARLY ? i : 0][e];
+            } else {
+                load_act<VEC>(a.d_gamma_in, c, false, g);
+            }
 #pragma unroll
             for (int e = 0; e < VEC; ++e) g[e] *= x[i][e] * inv;
             store_act<VEC>(a.d_h, (size_t)blockIdx.x * a.ldh + c, h_bf16, g);
@@ -127,6 +170,12 @@ extern "C" int gptrs_cuda_norm_step(const gptrs_norm_step* step, void* stream) {
     const dim3 grid((unsigned)a.rows);
     cudaStream_t st = as_stream(stream);
     if (vec) {
+        if (a.rows <= 2 * sm_count()) {
+            if (a.dim <= 512) return launch_kernel(norm_step_kernel<128, 1, 4, true>, grid, dim3(128), 0, st, 1, p);
+            if (a.dim <= 1024) return launch_kernel(norm_step_kernel<256, 1, 4, true>, grid, dim3(256), 0, st, 1, p);
+            if (a.dim <= 2048) return launch_kernel(norm_step_kernel<256, 2, 4, true>, grid, dim3(256), 0, st, 1, p);
+            if (a.dim <= 4096) return launch_kernel(norm_step_kernel<256, 4, 4, true>, grid, dim3(256), 0, st, 1, p);
+        }
         if (a.dim <= 512) return launch_kernel(norm_step_kernel<128, 1, 4>, grid, dim3(128), 0, st, 1, p);
         if (a.dim <= 1024) return launch_kernel(norm_step_kernel<256, 1, 4>, grid, dim3(256), 0, st, 1, p);
         if (a.dim <= 2048) return launch_kernel(norm_step_kernel<256, 2, 4>, grid, dim3(256), 0, st, 1, p);
