@@ -463,7 +463,7 @@ class LoadedModel:
         align = max(16 // group, 1)
         # passes the engine gives to the tensor-core prefill attention (the rule of gptrs_cuda_model_forward: paged bf16
         # cache, heads of 128, at least two 256-row tiles) need no alignment: a tile may hold two sequences
-        if cfg.kind == KIND_LAYERED or cfg.weight_mode == MODE_F32:   # query tiles are cut at sequence boundaries; the f32 kernels take any rows
+        if cfg.kind in (KIND_LAYERED, KIND_GPT):   # query tiles are cut at sequence boundaries
             align = 1
         elif (cfg.weight_mode != MODE_F32 and cfg.head_dim == 128 and group in (1, 2, 4, 8) and chunk >= 2 * (256 // group)
                 and os.environ.get("GPTRS_PREFILL_TC", "1") != "0"):
