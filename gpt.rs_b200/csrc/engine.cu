@@ -232,7 +232,7 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
     }
     if (rows <= 16) return quant_matmul_few_rows(m.cfg.weight_mode == kModeW4 ? 4 : 8, x, w.packed->data, y, rows, w.out, w.in, &ep, st);
     return m.cfg.weight_mode == kModeW4
-               ? quant_matmul_rows(x, w.packed->data, y, rows, w.out, w.in, &ep, m.wide.p, m.wide.n, st)
+               ? quant_matmul_rows(x, w.packed->data, y, rows, w.out, w.in, &ep, m.wide ? m.wide->data : nullptr, m.wide ? m.wide->bytes : 0, st)
                : gptrs_cuda_quant_matmul_w8a16(x, w.packed->data, y, rows, w.out, w.in, &ep, st);
 }
 
@@ -317,7 +317,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     cudaStream_t st = m.stream;
     float* hidden = m.hidden.as<float>();
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
-    if (T <= m.mega_rows && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
+    if (T <= m.mega_rows && T <= m.max_rows() && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
         // a token each of a few sequences: the whole step is one cooperative kernel (+ the memset of its barrier word)
         MegaParams P = m.mega;
         P.rows = T;
@@ -1016,7 +1016,8 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
         size_t most = 0;
         for (const Layer& L : m.layers)
             for (const Weight* w : {&L.qkv, &L.attn_out, &L.mlp_gate_up, &L.mlp_out}) most = std::max(most, (size_t)w->in * w->out * 2);
-        if (m.wide.alloc(most)) cudaGetLastError();   // without it the kernel that widens inside its tiles takes every row count
+        const int64_t dims[1] = {(int64_t)most};
+        if (tensor_alloc(GPTRS_UI8, 1, dims, false, &m.wide)) { m.wide = nullptr; cudaGetLastError(); }   // without it the kernel that widens inside its tiles takes every row count
     }
     // sums of squares per row and column tile: 128 columns, or 16 with up to 16 rows
     if (!m.f32() && (rc = m.sumsq.alloc((size_t)((D + 127) / 128) * std::max<size_t>(T, 8 * 16) * 4, true))) return rc;
@@ -1322,7 +1323,7 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
         ++m.launches;
         return launch_kernel(advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s, 1, ap);
     };
-    if (use_graph && B > m.mega_rows) {   // the single-kernel step needs no graph
+    if (use_graph && !(B <= m.mega_rows && B <= m.max_rows())) {   // the single-kernel step needs no graph
         GraphKey key{B, chunk, splits};
         auto it = m.graphs.find(key);
         if (it == m.graphs.end()) {

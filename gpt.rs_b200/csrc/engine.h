@@ -203,7 +203,7 @@ struct Model {
     bool fuse_pick = true;   // GPTRS_FUSE_PICK=0: logits + sampling kernel
     // f32 GPT kind, one sequence: the whole decode step as one cooperative kernel (gpt_decode_mega.cu)
     int mega_rows = 0;   // most sequences of a step that is one kernel (0: none)
-    DevBuf wide;                    // W4 prompts: the widened weights of one projection at a time
+    Tensor* wide = nullptr;         // W4 prompts: the widened weights of one projection at a time (a block of the tensor pool: a dropped f32 leaf's)
     DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
     MegaParams mega = {};
     int gen_batch = 0;  // slots 0..gen_batch-1 are driven by generator_step
@@ -231,6 +231,7 @@ struct Model {
         for (Tensor* t : {tok_emb, pos_emb, final_g, final_b}) tensor_release(t);
         if (h_page_table) cudaFreeHost(h_page_table);
         if (h_stage) cudaFreeHost(h_stage);
+        tensor_release(wide);
         if (h_logits) cudaFreeHost(h_logits);
         for (void* p : peer_maps) if (p) cudaIpcCloseMemHandle(p);
         if (peer_region) cudaFree(peer_region);
