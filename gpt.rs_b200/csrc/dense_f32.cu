@@ -1,5 +1,5 @@
 // f32 kernels for the unquantised reference-shaped path (GPT-2 small, fp32 weights):
-// small-M matmul on `[in, out]` weights with fused bias / GELU / residual, and decode attention
+// small-M matmul on `[in, out]` weights with fused bias / GELU / residual (many rows: split_f32.cu), and decode attention
 // over a dense f32 KV cache.
 //
 //   functional::matmul + add_bias   crates/gpt-rs/src/ops/functional/linalg.rs:109-127,

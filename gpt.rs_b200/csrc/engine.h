@@ -201,7 +201,7 @@ struct Model {
     // greedy head of the quantised engine: per-tile (max, argmax) candidates from the lm_head epilogue
     DevBuf best_val, best_idx;
     bool fuse_pick = true;   // GPTRS_FUSE_PICK=0: logits + sampling kernel
-    // f32 GPT kind, one sequence: the whole decode step as one cooperative kernel (gpt_decode_mega.cu)
+    // f32 GPT kind, up to eight sequences: the whole decode step as one cooperative kernel (gpt_decode_mega.cu)
     int mega_rows = 0;   // most sequences of a step that is one kernel (0: none)
     Tensor* wide = nullptr;         // W4 prompts: the widened weights of one projection at a time (a block of the tensor pool: a dropped f32 leaf's)
     DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
