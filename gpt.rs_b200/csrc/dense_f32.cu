@@ -343,9 +343,9 @@ int launch_sgemm(SgemmParams p, int batch, cudaStream_t st) {
     return launch_kernel(kern, grid, dim3(kSgWarps * 32), smem, st, p.n_split, p);
 }
 
-int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st, int32_t* status) {
+int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st, int32_t* status, bool w_constant = false) {
     if (p.norm_kind == 0) {
-        const SplitF32Params q = {p.x, p.w, p.bias, p.residual, p.y, p.M, p.N, p.K, p.act, p.dense, p.ldx, p.ldy, p.x_step, p.y_step, batch, status};
+        const SplitF32Params q = {p.x, p.w, p.bias, p.residual, p.y, p.M, p.N, p.K, p.act, p.dense, p.ldx, p.ldy, p.x_step, p.y_step, batch, status, w_constant};
         if (split_f32_takes(q)) return split_f32_matmul(q, st);
     }
     if (p.M == 1) return launch_sgemm<1>(p, batch, st);
@@ -356,10 +356,10 @@ int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st, int32_t* status)
 
 }  // namespace
 
-// gptrs_cuda_norm_matmul_f32 with the status word of the caller (null: the library's)
+// gptrs_cuda_norm_matmul_f32 with the status word of the caller (null: the library's); w_constant: no kernel in front writes d_w
 int norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps,
                     const float* d_w, float* d_y, int64_t m, int64_t n, int64_t k, const float* d_bias,
-                    const float* d_residual, int gelu, int32_t* d_status, cudaStream_t st) {
+                    const float* d_residual, int gelu, int32_t* d_status, bool w_constant, cudaStream_t st) {
     GPTRS_REQUIRE(d_x && d_w && d_y, "null pointer");
     GPTRS_REQUIRE(m >= 0 && n > 0 && k > 0 && n < (1ll << 31) && k < (1ll << 31) && m < (1ll << 31), "bad shape");
     GPTRS_REQUIRE(norm_kind >= 0 && norm_kind <= 2 && (norm_kind == 0 || d_gamma), "norm_kind 0 (none), 1 (layer norm) or 2 (rms norm) with a gain");
@@ -370,7 +370,7 @@ int norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const
     p.M = (int)m; p.N = (int)n; p.K = (int)k; p.act = gelu ? 1 : 0;
     p.norm_kind = norm_kind; p.norm_gamma = d_gamma; p.norm_beta = norm_kind == 1 ? d_beta : nullptr; p.norm_eps = eps;
     p.ldx = k; p.ldy = n;
-    return run_sgemm(p, 1, st, d_status);
+    return run_sgemm(p, 1, st, d_status, w_constant);
 }
 
 }  // namespace gptrs
@@ -387,7 +387,7 @@ int gptrs_cuda_matmul_f32(const float* d_x, const float* d_w, float* d_y, int64_
 int gptrs_cuda_norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps,
                                const float* d_w, float* d_y, int64_t m, int64_t n, int64_t k, const float* d_bias,
                                const float* d_residual, int gelu, void* stream) {
-    return norm_matmul_f32(d_x, norm_kind, d_gamma, d_beta, eps, d_w, d_y, m, n, k, d_bias, d_residual, gelu, nullptr, as_stream(stream));
+    return norm_matmul_f32(d_x, norm_kind, d_gamma, d_beta, eps, d_w, d_y, m, n, k, d_bias, d_residual, gelu, nullptr, false, as_stream(stream));
 }
 
 int gptrs_cuda_dense_f32(const float* d_x, const float* d_w, float* d_y, int64_t m, int64_t n, int64_t k, const gptrs_dense_epilogue* ep, void* stream) {

@@ -211,7 +211,7 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
         return norm_matmul_f32(static_cast<const float*>(x), fold ? fold->f32_norm : 0, fold ? fold->f32_gamma : nullptr,
                                           fold ? fold->f32_beta : nullptr, m.cfg.norm_eps, static_cast<const float*>(w.f32->data),
                                           static_cast<float*>(y), rows, w.out, w.in,
-                                          w.bias ? static_cast<const float*>(w.bias->data) : nullptr, residual, gelu ? 1 : 0, m.d_status.as<int32_t>(), st);
+                                          w.bias ? static_cast<const float*>(w.bias->data) : nullptr, residual, gelu ? 1 : 0, m.d_status.as<int32_t>(), true, st);
     }
     gptrs_matmul_epilogue ep = {};
     ep.out_dtype = out_f32 ? GPTRS_F32 : GPTRS_BF16;

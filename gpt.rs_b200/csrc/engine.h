@@ -260,9 +260,10 @@ int layered_first_visible(const Model& m, int pos);
 int layered_graph_bucket(const Model& m, int bucket);
 int layered_forward(Model& m, int rows, int max_ctx, int n_rows, bool rows_identity, float temperature, bool skip_logits);
 
-// gptrs_cuda_norm_matmul_f32 that reports a wait that gave up through the model's status word (dense_f32.cu)
+// gptrs_cuda_norm_matmul_f32 that reports a wait that gave up through the model's status word (dense_f32.cu); w_constant: no kernel in
+// front of it in the stream writes d_w, as with a model's parameters
 int norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps, const float* d_w, float* d_y, int64_t m, int64_t n,
-                    int64_t k, const float* d_bias, const float* d_residual, int gelu, int32_t* d_status, cudaStream_t st);
+                    int64_t k, const float* d_bias, const float* d_residual, int gelu, int32_t* d_status, bool w_constant, cudaStream_t st);
 
 // Attention of prompt rows over the dense f32 cache (prefill_f32.cu); takes() says whether rows and head size are its kind.
 bool attention_rows_f32_takes(int64_t n_tokens, int64_t head_dim);

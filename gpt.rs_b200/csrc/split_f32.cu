@@ -117,9 +117,10 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
     const int quarter = warp & 3, c_lo = (warp >> 2) * 32;
     const bool sums = warp < BN / 8;   // four warps take the sums of 32 columns (rows of y)
     {
+        if (!p.w_constant) pdl_wait();   // else the weights travel while the kernel in front still runs
 #pragma unroll
         for (int i = 0; i < kSets; ++i)
-            if (i < n_k) load_w(raw[i]);   // weights are constants: they travel while the kernel in front still runs
+            if (i < n_k) load_w(raw[i]);
         pdl_wait();
 #pragma unroll
         for (int i = 0; i < kSets; ++i)

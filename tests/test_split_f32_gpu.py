@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 import torch
 
-from gptrs_b200 import model as gm, ops
+from gptrs_b200 import model as gm, ops, ptir
+from gptrs_b200.backend import CudaBackend
 from oracle import models_ref as mr
 
 pytestmark = pytest.mark.gpu
@@ -34,6 +35,39 @@ def test_matmul_of_many_rows(cuda, m, n, k, form):
         want, bound = torch.nn.functional.gelu(want), 1.2 * bound + 8 * 2.0 ** -24 * want.abs()
     assert ((out.double() - want).abs() <= bound).all()
     assert ops.matmul_status() == 0
+
+
+# right operands that the kernel in front has just written: a transpose, a product, an update
+@pytest.mark.parametrize("form", ["transpose", "product", "update"])
+def test_programs_whose_right_operand_is_computed(cuda, form):
+    """From the third execution on a program is a graph whose kernels may start while the one in front ends. 128 rows, K of several
+    stages, fresh inputs every time: what a matmul reads has to be this execution's, from its first weights on."""
+    be = CudaBackend()
+    m, k, n = 128, 512, 256
+    b = ptir.Builder()
+    a = b.parameter(ptir.F32, [m, k])
+    if form == "transpose":
+        w = b.parameter(ptir.F32, [n, k])
+        b.set_results([ptir.matmul(a, (w + w).transpose([1, 0]))])
+        inputs, want = ([m, k], [n, k]), lambda a, w: a @ (2 * w).T
+    elif form == "product":
+        u, v = b.parameter(ptir.F32, [k, 768]), b.parameter(ptir.F32, [768, n])
+        b.set_results([ptir.matmul(a, ptir.matmul(u, v))])
+        inputs, want = ([m, k], [k, 768], [768, n]), lambda a, u, v: a @ (u @ v)
+    else:
+        w, u = b.parameter(ptir.F32, [k, n]), b.parameter(ptir.F32, [40, n])
+        b.set_results([ptir.matmul(a, w.dynamic_update_slice(u, b.literal(ptir.SI32, [2], [0, 0]), [40, n]))])
+        inputs, want = ([m, k], [k, n], [40, n]), lambda a, w, u: a @ np.concatenate([u, w[40:]])
+    prog = be.prepare(b.to_json())
+    rng = np.random.default_rng(2)
+    handles = [be.materialize(np.zeros(d, np.float32)) for d in inputs]
+    for _ in range(8):
+        arrays = [rng.normal(size=d).astype(np.float32) for d in inputs]
+        ref = want(*(x.astype(np.float64) for x in arrays))
+        del handles   # the blocks are handed out again, so that the graph recorded before fits
+        handles = [be.materialize(x) for x in arrays]
+        got = be.to_literal(prog.run(handles)[0])
+        assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
