@@ -231,8 +231,10 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
         ep.rope_q_heads = m.cfg.n_q_heads; ep.rope_kv_heads = m.cfg.n_kv_heads;
     }
     if (rows <= 16) return quant_matmul_few_rows(m.cfg.weight_mode == kModeW4 ? 4 : 8, x, w.packed->data, y, rows, w.out, w.in, &ep, st);
+    const Tensor* wide = st == m.stream ? m.wide : nullptr;
     return m.cfg.weight_mode == kModeW4
-               ? quant_matmul_rows(x, w.packed->data, y, rows, w.out, w.in, &ep, m.wide ? m.wide->data : nullptr, m.wide ? m.wide->bytes : 0, st)
+               // one buffer for widened weights: the second lane of a step, on its own stream, goes without
+               ? quant_matmul_rows(x, w.packed->data, y, rows, w.out, w.in, &ep, wide ? wide->data : nullptr, wide ? wide->bytes : 0, st)
                : gptrs_cuda_quant_matmul_w8a16(x, w.packed->data, y, rows, w.out, w.in, &ep, st);
 }
 
@@ -306,6 +308,9 @@ __global__ void record_history_kernel(const HistoryParams p) {
 
 int attention_plan(const Model& m, int T, int max_ctx, size_t scratch_bytes, int* chunk_pages);
 
+// Most sums of squares that a producer of `rows` rows leaves: one per row and 128 columns, or 16 columns with up to 16 rows.
+size_t sumsq_floats(int d_model, int rows) { return (size_t)rows * (d_model / (rows <= 16 ? 16 : 128)); }
+
 // Enqueues one forward pass over T tokens whose ids / slots / positions / visible lengths are
 // already in the device arrays. `rows`: number of rows that get logits (row indices in d_rows,
 // or all T rows in order when rows_identity).
@@ -343,7 +348,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     }
     // A lane is a contiguous range of token rows with its own stream; every activation buffer is row-major,
     // so a lane works on a row offset of the shared buffers.
-    struct Lane { cudaStream_t st; int r0, T, chunk; unsigned char* scratch; size_t scratch_n; };
+    struct Lane { cudaStream_t st; int r0, T, chunk; unsigned char* scratch; size_t scratch_n; size_t sumsq0 = 0; };
     const size_t act = m.f32() ? 4 : 2;
     auto at = [](DevBuf& b, size_t row_bytes, const Lane& ln) { return static_cast<unsigned char*>(b.p) + (size_t)ln.r0 * row_bytes; };
     auto ints = [](DevBuf& b, const Lane& ln) { return b.as<int32_t>() + ln.r0; };
@@ -353,18 +358,18 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     // (tensor-parallel steps always run as one lane).
     const float* pending = nullptr;
     bool pending_peer = false;   // the pending tile still has to be summed over the ranks (by the norm kernel)
-    // RMSNorm folded into the projections: quantised Ministral, one rank, d_model a multiple of 128. The sums of squares of a lane live at a row offset of the shared buffer: a lane's
-    // tile t is at sumsq + t * T_lane, so each lane gets a disjoint slab of [tiles][T_lane] floats.
+    // RMSNorm folded into the projections: quantised Ministral, one rank, d_model a multiple of 128. A lane's sums of squares are a slab
+    // [tiles][T_lane] of its own in the shared buffer. How many columns a tile has depends on the lane's rows (quant_tile_cols).
     const bool fold = m.fold_norm && !gpt && !m.f32() && m.tp == 1 && D % 128 == 0;
-    int fold_tiles = 0;   // column tiles that the last producer's sums are over
-    auto fold_for = [&](const Lane& ln, Tensor* next_gamma, bool produce) {
+    auto fold_for = [&](const Lane& ln, const Weight& producer, Tensor* next_gamma = nullptr) {   // next_gamma: for the producer itself
+        const bool produce = next_gamma != nullptr;
         NormFold f;
-        f.sumsq = m.sumsq.as<float>() + (size_t)(D / 128) * ln.r0;
+        f.sumsq = m.sumsq.as<float>() + ln.sumsq0;
         f.dim = D;
         f.eps = c.norm_eps;
         f.produce = produce;
         f.consume = !produce;
-        f.tiles = fold_tiles;
+        f.tiles = D / quant_tile_cols(c.weight_mode == kModeW4 ? 4 : 8, ln.T, producer.out, producer.in);
         if (produce) {
             f.gamma = static_cast<const float*>(next_gamma->data);
             f.x_next = at(m.xn, (size_t)D * act, ln);
@@ -384,8 +389,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         float* h = reinterpret_cast<float*>(at(m.hidden, (size_t)D * 4, ln));
         if (m.tp == 1) {
             if (fold && next_gamma) {
-                const NormFold f = fold_for(ln, next_gamma, true);
-                fold_tiles = D / quant_tile_cols(c.weight_mode == kModeW4 ? 4 : 8, ln.T, w.out, w.in);
+                const NormFold f = fold_for(ln, w, next_gamma);
                 return linear(m, w, x, h, ln.T, true, h, false, false, ln.st, &f);
             }
             return linear(m, w, x, h, ln.T, true, h, false, false, ln.st);
@@ -439,7 +443,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         if (fold32) {
             f = fold32_for(L.ln1_g, L.ln1_b);
             if ((r = linear(m, L.qkv, at(m.hidden, (size_t)D * 4, ln), qkv, ln.T, false, nullptr, false, false, ln.st, &f))) return r;
-        } else if (folded && l > 0) f = fold_for(ln, nullptr, false);  // the previous block's last projection left bf16(hidden * gain) and the row sums
+        } else if (folded && l > 0) f = fold_for(ln, m.layers[l - 1].mlp_out);  // the previous block's last projection left bf16(hidden * gain) and the row sums
         else if ((r = norm(ln, L.ln1_g, L.ln1_b))) return r;
         if (rope_folded) {
             f.rope_positions = ints(m.d_pos, ln);
@@ -531,7 +535,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
             if ((r = gptrs_cuda_swiglu(static_cast<float*>(g), static_cast<float*>(u), static_cast<float*>(mlp_h),
                                        (int64_t)ln.T * c.d_mlp, ln.st))) return r;
         } else if (folded) {
-            const NormFold f = fold_for(ln, nullptr, false);
+            const NormFold f = fold_for(ln, L.attn_out);
             if ((r = linear(m, L.mlp_gate_up, xn, mlp_h, ln.T, false, nullptr, true, false, ln.st, &f))) return r;
         } else {
             if ((r = linear(m, L.mlp_gate_up, xn, mlp_h, ln.T, false, nullptr, true, false, ln.st))) return r;
@@ -551,7 +555,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         const int ta = (T + 1) / 2;
         const size_t half = (m.attn_scratch.n / 2) & ~(size_t)255;
         Lane a = {st, 0, ta, 1, m.attn_scratch.as<unsigned char>(), half};
-        Lane b = {m.stream2, ta, T - ta, 1, m.attn_scratch.as<unsigned char>() + half, half};
+        Lane b = {m.stream2, ta, T - ta, 1, m.attn_scratch.as<unsigned char>() + half, half, sumsq_floats(D, ta)};
         attention_plan(m, a.T, max_ctx, half, &a.chunk);
         attention_plan(m, b.T, max_ctx, half, &b.chunk);
         GPTRS_CUDA_OK(cudaEventRecord(m.ev_fork, st));
@@ -1019,8 +1023,8 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
         const int64_t dims[1] = {(int64_t)most};
         if (tensor_alloc(GPTRS_UI8, 1, dims, false, &m.wide)) { m.wide = nullptr; cudaGetLastError(); }   // without it the kernel that widens inside its tiles takes every row count
     }
-    // sums of squares per row and column tile: 128 columns, or 16 with up to 16 rows
-    if (!m.f32() && (rc = m.sumsq.alloc((size_t)((D + 127) / 128) * std::max<size_t>(T, 8 * 16) * 4, true))) return rc;
+    // sums of squares of two lanes of at most 16 rows, of 17 and 16, or of all rows
+    if (!m.f32() && (rc = m.sumsq.alloc(std::max(2 * sumsq_floats((int)D + 127, 16), sumsq_floats((int)D + 127, T)) * 4, true))) return rc;
     if ((rc = m.hidden.alloc((size_t)T * D * 4)) || (rc = m.xn.alloc((size_t)T * D * act)) || (rc = m.xn_rows.alloc((size_t)T * D * act)) ||
         (rc = m.qkv.alloc((size_t)T * QKV * act)) || (rc = m.attn.alloc((size_t)T * QD * act)) ||
         (rc = m.mlp_h.alloc((size_t)T * MLP * act))) return rc;

@@ -43,3 +43,38 @@ def test_steps_follow_the_oracle(cuda, mode, n_q, n_kv, d, batch, ctx):
     want = np.stack([r.forward([int(t)])[-1] for r, t in zip(refs, given[5])])
     got, _ = m.forward_with_decode_cache(given[5], list(range(batch)), [n + 5 for n in lengths], list(range(batch)))
     assert np.sqrt(np.mean((got - want) ** 2)) <= 2e-2 * np.sqrt(np.mean(want ** 2))   # bf16 activations through two layers
+
+
+def _model(mode, d, n_q, n_kv, layers, mlp, batch, ctx, max_tokens, namespace):
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_MINISTRAL, layers, d, n_q, n_kv, 128, mlp, 256, ctx, 1e-5, 1e4, 128,
+                                      weight_mode=gm.MODE_W4A16 if mode == "w4" else gm.MODE_W8A16, max_seqs=batch, max_tokens=max_tokens, max_logit_rows=batch,
+                                      kv_pages=batch * (ctx // 16) + 4, max_pages_per_seq=ctx // 16, use_pdl=1), namespace=namespace)
+    cfg = mr.Cfg("ministral", n_layers=layers, d_model=d, n_q=n_q, n_kv=n_kv, hd=128, d_mlp=mlp, vocab=256, ctx=ctx, rot=128, theta=1e4)
+    params = mr.random_params(cfg, seed=batch, std=0.5 * d ** -0.5)
+    params["tok_embeddings.weight"] = np.random.default_rng(0).normal(0, 1, (256, d)).astype(np.float32)
+    for name, w in params.items():
+        m.load_param(name, w)
+    m.finalize()
+    return m
+
+
+# lanes of 16 + 16, 17 + 16 and 17 + 17 rows, whose norms are summed over column tiles of unlike widths; lanes that both have the rows of
+# the widened weights
+@pytest.mark.parametrize("mode,d,batch", [("w4", 1024, 32), ("w4", 1024, 33), ("w4", 1024, 34), ("w8", 512, 33), ("w4", 128, 3072)])
+def test_two_lanes_give_what_one_gives(cuda, monkeypatch, mode, d, batch):
+    """A step in two halves on two streams leaves the cache that a step in one piece leaves: logits of a pass that reads it, to what bf16
+    keeps when sums are taken in another order."""
+    rng = np.random.default_rng(batch)
+    ids = rng.integers(0, 256, (8, batch))
+    got = []
+    for lanes in ("1", "2"):
+        monkeypatch.setenv("GPTRS_LANES", lanes)
+        m = _model(mode, d, 2, 1, 2, 256, batch, 16, max(batch, 64), 7800 + batch + int(lanes) * 10000)
+        rows = list(range(batch))
+        m.prefill_many(rows, [ids[0, s:s + 1] for s in rows])
+        gen = gm.Generator(m, ids[1])
+        for row in ids[1:7]:
+            gen.step(row)
+        got.append(m.forward_with_decode_cache(ids[7], rows, [7] * batch, rows)[0])
+    diff, scale = np.abs(got[0] - got[1]), np.sqrt(np.mean(got[0] ** 2, axis=1))
+    assert np.isfinite(got[1]).all() and (np.sqrt(np.mean(diff ** 2, axis=1)) <= 2e-2 * scale).all()
