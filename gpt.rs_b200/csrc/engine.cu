@@ -308,6 +308,13 @@ __global__ void record_history_kernel(const HistoryParams p) {
 
 int attention_plan(const Model& m, int T, int max_ctx, size_t scratch_bytes, int* chunk_pages);
 
+// Splits of a decode step of few rows that leaves RoPE, KV append and the merge of the splits to the attention kernel; 0: other steps.
+int decode_step_splits(const Model& m, int T, int max_ctx) {
+    const auto& c = m.cfg;
+    if (m.f32() || c.kind != kKindMinistral || T > 16 || c.rotary_dim != c.head_dim || c.head_dim != 128) return 0;
+    return attention_step_splits(max_ctx, T, c.n_q_heads, c.n_kv_heads);
+}
+
 // Most sums of squares that a producer of `rows` rows leaves: one per row and 128 columns, or 16 columns with up to 16 rows.
 size_t sumsq_floats(int d_model, int rows) { return (size_t)rows * (d_model / (rows <= 16 ? 16 : 128)); }
 
@@ -428,9 +435,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
                    : gptrs_cuda_add_rms_norm(h, delta, GPTRS_F32, (const float*)g->data, c.norm_eps, xn, act_dt,
                                              nullptr, ln.T, D, ln.st);
     };
-    // A decode step of few rows leaves RoPE, KV append and the merge of the splits to the attention kernel.
-    const int step_splits = rows_identity && !m.f32() && !gpt && T <= 16 && !prefill_groups && c.rotary_dim == c.head_dim && c.head_dim == 128
-                                ? attention_step_splits(max_ctx, T, c.n_q_heads, c.n_kv_heads) : 0;
+    const int step_splits = rows_identity && !prefill_groups ? decode_step_splits(m, T, max_ctx) : 0;
     // ---- the three parts of a decoder block ------------------------------------------------------
     auto pre_attention = [&](const Lane& ln, int l) -> int {
         Layer& L = m.layers[l];
@@ -1328,7 +1333,7 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
         return launch_kernel(advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s, 1, ap);
     };
     if (use_graph && !(B <= m.mega_rows && B <= m.max_rows())) {   // the single-kernel step needs no graph
-        GraphKey key{B, chunk, splits};
+        GraphKey key{B, chunk, splits, decode_step_splits(m, B, bucket) ? bucket : 0};
         auto it = m.graphs.find(key);
         if (it == m.graphs.end()) {
             const int64_t launches_before = m.launches;

@@ -51,10 +51,12 @@ struct Layer {
     Weight qkv, attn_out, mlp_in, mlp_gate, mlp_up, mlp_gate_up, mlp_out;
 };
 
+// Everything that a recorded step's launches depend on. step_ctx: the visible length that attention_step was sized for (its bound on
+// lengths and its splits come from it), 0 where attention is the separate kernels.
 struct GraphKey {
-    int batch, chunk_pages, splits;
+    int batch, chunk_pages, splits, step_ctx;
     bool operator<(const GraphKey& o) const {
-        return std::tie(batch, chunk_pages, splits) < std::tie(o.batch, o.chunk_pages, o.splits);
+        return std::tie(batch, chunk_pages, splits, step_ctx) < std::tie(o.batch, o.chunk_pages, o.splits, o.step_ctx);
     }
 };
 

@@ -78,3 +78,23 @@ def test_two_lanes_give_what_one_gives(cuda, monkeypatch, mode, d, batch):
         got.append(m.forward_with_decode_cache(ids[7], rows, [7] * batch, rows)[0])
     diff, scale = np.abs(got[0] - got[1]), np.sqrt(np.mean(got[0] ** 2, axis=1))
     assert np.isfinite(got[1]).all() and (np.sqrt(np.mean(diff ** 2, axis=1)) <= 2e-2 * scale).all()
+
+
+def test_recorded_steps_past_the_length_they_were_recorded_for(cuda):
+    """14 sequences of 64 kv heads: the separate attention kernels would launch alike for 512 and for 1024 visible tokens, the step's own kernel
+    would not. One sequence goes from 506 tokens past 512, key and value of every step where they belong."""
+    batch, d, ctx = 14, 128, 1024
+    m = _model("w4", d, 64, 64, 2, 256, batch, ctx, 1024, 7600)
+    rng = np.random.default_rng(1)
+    prompts = [rng.integers(0, 256, 506 if s == 5 else 3 + s) for s in range(batch)]
+    given = rng.integers(0, 256, (13, batch))
+    rows, got = list(range(batch)), []
+    for graphs in (False, True):
+        for s in rows:
+            m.reset_sequence(s)
+        m.prefill_many(rows, prompts)
+        gen = gm.Generator(m, given[0], use_graph=graphs)
+        ids = [gen.step(row).tolist() for row in given[:12]]
+        at = [m.sequence_length(s) for s in rows]
+        got.append((ids, m.forward_with_decode_cache(given[12], rows, at, rows)[0]))
+    assert got[0][0] == got[1][0] and np.array_equal(got[0][1], got[1][1])
