@@ -37,6 +37,12 @@ __global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const Pr
     float* ps = vs + kPfKeys * LD;                                   // [32][LP]
     __shared__ int pos_s[kPfRows], slot_s[kPfRows];
     auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "n"(kPfGroup) : "memory"); };
+    auto group_any = [&](bool mine) {   // a barrier that says whether it is so for a thread of the group
+        uint32_t any;
+        asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                     : "=r"(any) : "r"((uint32_t)mine), "r"(1 + group), "n"(kPfGroup) : "memory");
+        return any != 0;
+    };
     const int t0 = (int)(gridDim.y - 1 - blockIdx.y) * kPfRows;      // the last rows see the most keys: they start first
     const int h = blockIdx.x, hk = h / (p.Hq / p.Hkv), rows = min(kPfRows, p.T - t0);
     const int width = (p.Hq + 2 * p.Hkv) * HD;
@@ -70,15 +76,18 @@ __global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const Pr
         for (int r = 0; r < 4; ++r) limit[r] = 4 * ty + r >= seg && 4 * ty + r < end ? pos_s[4 * ty + r] : -1;
         for (int j0 = group * kPfKeys; j0 <= last; j0 += 2 * kPfKeys) {
             group_sync();   // the block before has been used
+            float probe = 0.f;   // NaN once a value of this block is not finite
 #pragma unroll 8
             for (int i = tid; i < kPfKeys * (HD / 4); i += kPfGroup) {
                 const int j = i / (HD / 4), c = i % (HD / 4) * 4;
                 const bool in = j0 + j <= last;
                 const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                 *reinterpret_cast<float4*>(ks + j * LD + c) = in ? *reinterpret_cast<const float4*>(kc + (size_t)(j0 + j) * HD + c) : zero;
-                *reinterpret_cast<float4*>(vs + j * LD + c) = in ? *reinterpret_cast<const float4*>(vc + (size_t)(j0 + j) * HD + c) : zero;
+                const float4 v = in ? *reinterpret_cast<const float4*>(vc + (size_t)(j0 + j) * HD + c) : zero;
+                *reinterpret_cast<float4*>(vs + j * LD + c) = v;
+                probe = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, probe))));
             }
-            group_sync();
+            const bool special = group_any(probe != probe);
             float s[4][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
@@ -126,6 +135,22 @@ __global__ void __launch_bounds__(kPfThreads) attention_rows_f32_kernel(const Pr
                 for (int c = 0; c < 4 * OC; ++c) o[r][c] *= keep;
             }
             __syncwarp();   // the 16 threads of a row write and read its weights, and they are in one warp
+            if (special) {   // the weight 0 of a key that a row does not see would not keep an infinity or NaN from it
+#pragma unroll 1
+                for (int j = 0; j < kPfKeys; ++j)
+#pragma unroll
+                    for (int c = 0; c < OC; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(vs + j * LD + 4 * tx + 64 * c);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            if (j0 + j > limit[r]) continue;
+                            const float w = ps[(4 * ty + r) * LP + j];
+                            o[r][4 * c] = fmaf(w, v.x, o[r][4 * c]); o[r][4 * c + 1] = fmaf(w, v.y, o[r][4 * c + 1]);
+                            o[r][4 * c + 2] = fmaf(w, v.z, o[r][4 * c + 2]); o[r][4 * c + 3] = fmaf(w, v.w, o[r][4 * c + 3]);
+                        }
+                    }
+                continue;
+            }
 #pragma unroll 4
             for (int j = 0; j < kPfKeys; j += 4) {
                 float4 e[4];

@@ -111,6 +111,31 @@ def test_prompt_rows_of_several_sequences(cuda, kind, hd, n_q, n_kv):
         assert np.abs(got - np.stack(want)).max() <= 1e-4 * max(1.0, np.abs(want).max())
 
 
+@pytest.mark.parametrize("kind,hd,n_q,n_kv", [("gpt", 64, 8, 8), ("ministral", 128, 8, 2)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_token_that_is_not_finite_reaches_only_rows_that_see_it(cuda, kind, hd, n_q, n_kv, value):
+    """Rows of other sequences in the same tile and earlier rows of its own keep their bits. (Widths that leave the matmuls to the f32 kernel,
+    whose rows do not meet.)"""
+    cfg = mr.Cfg(kind, n_layers=1, d_model=40, n_q=n_q, n_kv=n_kv, hd=hd, d_mlp=80, vocab=96, ctx=128, rot=hd if kind == "ministral" else 0, theta=1e4)
+    params = mr.random_params(cfg, seed=3, std=0.2)
+    params["tok_embeddings.weight"][95] = value
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT if kind == "gpt" else gm.KIND_MINISTRAL, 1, 40, n_q, n_kv, hd, 80, 96, 128, cfg.eps, cfg.theta, cfg.rot,
+                                      max_seqs=3, max_tokens=128, max_logit_rows=128), namespace=7200 + hd + (value != value) * 100)
+    for name, w in params.items():
+        m.load_param(name, w)
+    m.finalize()
+    rng = np.random.default_rng(4)
+    lengths = (21, 50, 40)
+    tok = rng.integers(0, 95, sum(lengths))
+    sl, pos = np.repeat(np.arange(3), lengths), np.concatenate([np.arange(n) for n in lengths])
+    rows, at = np.arange(len(tok)), 21 + 30   # in the second sequence
+    want, _ = m.forward_with_decode_cache(tok, sl, pos, rows)
+    tok[at] = 95
+    got, _ = m.forward_with_decode_cache(tok, sl, pos, rows)
+    hit = (sl == 1) & (rows >= at)
+    assert np.array_equal(got[~hit], want[~hit]) and np.isnan(got[hit]).all()
+
+
 @pytest.mark.parametrize("batch,ctx", [(1, 64), (2, 300), (3, 64), (5, 64), (8, 128), (9, 64)])
 def test_steps_of_a_few_sequences(cuda, batch, ctx):
     """GPT-2's widths, where a step of up to eight sequences is one kernel: prompts of unequal lengths packed into one pass, greedy steps,
