@@ -11,6 +11,7 @@
 // each load instruction of a warp is one contiguous 128-byte row segment and no alignment of
 // N is needed), warps split the K rows, partial sums meet in shared memory and, when K is
 // split across a thread-block cluster, through distributed shared memory.
+#include "engine.h"
 #include "split_f32.cuh"
 
 namespace gptrs {
@@ -237,6 +238,7 @@ struct AttnF32Params {
     float scale;
     float* append_k;  // non-null: the CTA first stores the token's K / V row of its kv head at `pos` (decode steps of
     float* append_v;  // distinct sequences only: no other token of the launch may read that row)
+    const int* rows;  // optional: the rows that the launch is for
 };
 
 // One CTA (128 threads) per (query head, token); scores live in dynamic shared memory.
@@ -245,9 +247,10 @@ __global__ void __launch_bounds__(128) attention_f32_kernel(const AttnF32Params 
     float* qs = at_smem;              // [hd]
     float* sc = at_smem + p.hd;       // [len]
     __shared__ float sh[32];
-    const int hq = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+    const int hq = blockIdx.x, tid = threadIdx.x;
     pdl_launch_dependents();  // dependents still wait for this whole grid before reading its results
     pdl_wait();
+    const int b = p.rows ? p.rows[blockIdx.y] : blockIdx.y;
     const int pos = min(max(p.positions[b], 0), p.capacity - 1);
     const int len = pos + 1;
     const int group = p.Hq / p.Hkv, hk = hq / group;
@@ -354,7 +357,28 @@ int run_sgemm(const SgemmParams& p, int batch, cudaStream_t st, int32_t* status,
     return launch_sgemm<8>(p, batch, st);
 }
 
+int attend_f32(AttnF32Params p, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st) {
+    GPTRS_REQUIRE(p.qkv && p.k_cache && p.v_cache && p.positions && p.slot && p.out, "null pointer");
+    GPTRS_REQUIRE(n_q_heads > 0 && n_kv_heads > 0 && n_q_heads % n_kv_heads == 0, "bad head counts");
+    GPTRS_REQUIRE(head_dim > 0 && head_dim <= 128, "head_dim must be 1..128");
+    GPTRS_REQUIRE(capacity > 0 && capacity <= 32768, "capacity out of range");
+    if (n_tokens == 0) return GPTRS_OK;
+    p.T = (int)n_tokens; p.Hq = (int)n_q_heads; p.Hkv = (int)n_kv_heads; p.hd = (int)head_dim; p.capacity = (int)capacity;
+    p.scale = 1.0f / sqrtf((float)head_dim);
+    const size_t smem = ((size_t)head_dim + (size_t)(capacity > 128 ? capacity : 128)) * sizeof(float);
+    GPTRS_CUDA_OK(cudaFuncSetAttribute(attention_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    return launch_kernel(attention_f32_kernel, dim3((unsigned)n_q_heads, (unsigned)n_tokens), dim3(128), smem, st, 1, p);
+}
+
 }  // namespace
+
+// The rows of a list, of passes whose other rows go to attention_tiles_f32
+int attention_listed_f32(const float* qkv, const float* k_cache, const float* v_cache, const int32_t* positions, const int32_t* slot, float* out,
+                         const int32_t* rows, int n_rows, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st) {
+    AttnF32Params p = {qkv, k_cache, v_cache, positions, slot, out};
+    p.rows = rows;
+    return attend_f32(p, n_rows, n_q_heads, n_kv_heads, head_dim, capacity, st);
+}
 
 // gptrs_cuda_norm_matmul_f32 with the status word of the caller (null: the library's); w_constant: no kernel in front writes d_w
 int norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps,
@@ -427,34 +451,17 @@ int gptrs_cuda_attention_decode_f32(const float* d_qkv, const float* d_k_cache, 
                                     const int32_t* d_positions, const int32_t* d_slot, float* d_out,
                                     int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim,
                                     int64_t capacity, void* stream) {
-    GPTRS_REQUIRE(d_qkv && d_k_cache && d_v_cache && d_positions && d_slot && d_out, "null pointer");
-    GPTRS_REQUIRE(n_q_heads > 0 && n_kv_heads > 0 && n_q_heads % n_kv_heads == 0, "bad head counts");
-    GPTRS_REQUIRE(head_dim > 0 && head_dim <= 128, "head_dim must be 1..128");
-    GPTRS_REQUIRE(capacity > 0 && capacity <= 32768, "capacity out of range");
-    if (n_tokens == 0) return GPTRS_OK;
-    AttnF32Params p = {d_qkv, d_k_cache, d_v_cache, d_positions, d_slot, d_out, (int)n_tokens, (int)n_q_heads,
-                       (int)n_kv_heads, (int)head_dim, (int)capacity, 1.0f / sqrtf((float)head_dim), nullptr, nullptr};
-    size_t smem = ((size_t)head_dim + (size_t)(capacity > 128 ? capacity : 128)) * sizeof(float);
-    GPTRS_CUDA_OK(cudaFuncSetAttribute(attention_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    return launch_kernel(attention_f32_kernel, dim3((unsigned)n_q_heads, (unsigned)n_tokens), dim3(128), smem,
-                         as_stream(stream), 1, p);
+    return attend_f32({d_qkv, d_k_cache, d_v_cache, d_positions, d_slot, d_out}, n_tokens, n_q_heads, n_kv_heads, head_dim, capacity, as_stream(stream));
 }
 
 int gptrs_cuda_kv_append_attention_decode_f32(const float* d_qkv, float* d_k_cache, float* d_v_cache,
                                               const int32_t* d_positions, const int32_t* d_slot, float* d_out,
                                               int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim,
                                               int64_t capacity, void* stream) {
-    GPTRS_REQUIRE(d_qkv && d_k_cache && d_v_cache && d_positions && d_slot && d_out, "null pointer");
-    GPTRS_REQUIRE(n_q_heads > 0 && n_kv_heads > 0 && n_q_heads % n_kv_heads == 0, "bad head counts");
-    GPTRS_REQUIRE(head_dim > 0 && head_dim <= 128, "head_dim must be 1..128");
-    GPTRS_REQUIRE(capacity > 0 && capacity <= 32768, "capacity out of range");
-    if (n_tokens == 0) return GPTRS_OK;
-    AttnF32Params p = {d_qkv, d_k_cache, d_v_cache, d_positions, d_slot, d_out, (int)n_tokens, (int)n_q_heads,
-                       (int)n_kv_heads, (int)head_dim, (int)capacity, 1.0f / sqrtf((float)head_dim), d_k_cache, d_v_cache};
-    size_t smem = ((size_t)head_dim + (size_t)(capacity > 128 ? capacity : 128)) * sizeof(float);
-    GPTRS_CUDA_OK(cudaFuncSetAttribute(attention_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    return launch_kernel(attention_f32_kernel, dim3((unsigned)n_q_heads, (unsigned)n_tokens), dim3(128), smem,
-                         as_stream(stream), 1, p);
+    AttnF32Params p = {d_qkv, d_k_cache, d_v_cache, d_positions, d_slot, d_out};
+    p.append_k = d_k_cache;
+    p.append_v = d_v_cache;
+    return attend_f32(p, n_tokens, n_q_heads, n_kv_heads, head_dim, capacity, as_stream(stream));
 }
 
 }  // extern "C"

@@ -485,9 +485,16 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         if (m.f32()) {
             float* kc = m.k_cache.as<float>() + (size_t)l * m.cache_layer_elems;
             float* vc = m.v_cache.as<float>() + (size_t)l * m.cache_layer_elems;
-            if (!rows_identity && attention_rows_f32_takes(ln.T, c.head_dim))   // rows of prompts share the keys of their sequence
-                return attention_rows_f32(reinterpret_cast<float*>(at(m.qkv, (size_t)m.QKV() * 4, ln)), kc, vc, ints(m.d_pos, ln), ints(m.d_slot, ln),
-                                          static_cast<float*>(out), ln.T, c.n_q_heads, c.n_kv_heads, c.head_dim, c.context_length, ln.st);
+            if (!rows_identity && m.attn_f32.tiles) {
+                const float* qkv = reinterpret_cast<float*>(at(m.qkv, (size_t)m.QKV() * 4, ln));
+                const int32_t* lists = m.d_attn_f32.as<int32_t>();
+                const int r = attention_tiles_f32(qkv, kc, vc, ints(m.d_pos, ln), ints(m.d_slot, ln), static_cast<float*>(out), lists, m.attn_f32.tiles,
+                                                  c.n_q_heads, c.n_kv_heads, c.head_dim, c.context_length, ln.st);
+                if (r || !m.attn_f32.rows) return r;
+                ++m.launches;
+                return attention_listed_f32(qkv, kc, vc, ints(m.d_pos, ln), ints(m.d_slot, ln), static_cast<float*>(out), lists + 2 * m.attn_f32.tiles,
+                                            m.attn_f32.rows, c.n_q_heads, c.n_kv_heads, c.head_dim, c.context_length, ln.st);
+            }
             auto attend = rows_identity ? gptrs_cuda_kv_append_attention_decode_f32
                                         : [](const float* q, float* k, float* v, const int32_t* pos, const int32_t* sl, float* o, int64_t t,
                                              int64_t hq, int64_t hkv, int64_t hd, int64_t cap, void* st) {
@@ -1045,7 +1052,8 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
     if (m.tp > 1 && ((rc = m.partial.alloc((size_t)T * D * 4)) || (rc = m.tp_vals.alloc((size_t)max_rows * 4)) || (rc = m.tp_idx.alloc((size_t)max_rows * 4)) ||
                      (rc = m.tp_gvals.alloc((size_t)m.tp * max_rows * 4)) || (rc = m.tp_gidx.alloc((size_t)m.tp * max_rows * 4)))) return rc;
     if (m.tp > 1 && (rc = setup_peer_allreduce(m, std::min(T, 256)))) return rc;
-    if ((rc = alloc_step_buffers(m, 6))) return rc;
+    if ((rc = alloc_step_buffers(m, m.f32() ? 8 : 6))) return rc;
+    if (m.f32() && (rc = m.d_attn_f32.alloc((size_t)2 * m.stage_stride() * 4))) return rc;
 
     // KV storage
     if (m.f32()) {
@@ -1153,6 +1161,11 @@ int gptrs_cuda_model_forward_with_decode_cache(gptrs_model* h, const int32_t* h_
     GPTRS_CUDA_OK(cudaMemcpyAsync(m.d_pos.p, st + 2 * stride, (size_t)T * 4, cudaMemcpyHostToDevice, s));
     GPTRS_CUDA_OK(cudaMemcpyAsync(m.d_ctx.p, st + 3 * stride, (size_t)T * 4, cudaMemcpyHostToDevice, s));
     if (n_logit_rows) GPTRS_CUDA_OK(cudaMemcpyAsync(m.d_rows.p, st + 4 * stride, (size_t)n_logit_rows * 4, cudaMemcpyHostToDevice, s));
+    if (m.f32() && !m.layered()) {
+        m.attn_f32 = attention_f32_plan(h_slots, T, c.n_q_heads, c.head_dim, c.context_length, st + 6 * stride);
+        if (m.attn_f32.tiles)
+            GPTRS_CUDA_OK(cudaMemcpyAsync(m.d_attn_f32.p, st + 6 * stride, (size_t)(2 * m.attn_f32.tiles + m.attn_f32.rows) * 4, cudaMemcpyHostToDevice, s));
+    }
     // Prefill chunks: when every aligned group of 16 / (query heads per kv head) rows belongs to one sequence,
     // the attention kernel streams the K/V pages once per group instead of once per row.
     // GPTRS_PREFILL_BLOCKS=1: when every aligned block of four such groups (16 tokens at a group of 4) is one sequence, a

@@ -144,6 +144,8 @@ struct Layered {
     }
 };
 
+struct AttentionF32Plan { int tiles = 0, rows = 0; };   // see attention_f32_plan
+
 struct Model {
     gptrs_model_config cfg;
     bool finalized = false;
@@ -175,7 +177,7 @@ struct Model {
     std::vector<int> seq_first_page;  // first page a slot still holds (pages that every layer's window has passed go back)
     std::unique_ptr<Layered> lay;     // kind kKindLayered
     // staging (pinned)
-    int32_t* h_stage = nullptr;  // 6 * max_tokens int32
+    int32_t* h_stage = nullptr;  // 6 * max_tokens int32 (f32 kinds: 8)
     float* h_logits = nullptr;
     cudaStream_t stream = nullptr;
     // Optional (GPTRS_LANES=2): decode steps of >= 32 sequences run as two half-batches ("lanes") on two
@@ -208,6 +210,8 @@ struct Model {
     Tensor* wide = nullptr;         // W4 prompts: the widened weights of one projection at a time (a block of the tensor pool: a dropped f32 leaf's)
     DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
     MegaParams mega = {};
+    AttentionF32Plan attn_f32;      // f32 kinds: the split of the pass under way, its lists in d_attn_f32
+    DevBuf d_attn_f32;
     int gen_batch = 0;  // slots 0..gen_batch-1 are driven by generator_step
     int64_t launches = 0;
     uint32_t sample_seed = 0;
@@ -267,10 +271,13 @@ int layered_forward(Model& m, int rows, int max_ctx, int n_rows, bool rows_ident
 int norm_matmul_f32(const float* d_x, int norm_kind, const float* d_gamma, const float* d_beta, float eps, const float* d_w, float* d_y, int64_t m, int64_t n,
                     int64_t k, const float* d_bias, const float* d_residual, int gelu, int32_t* d_status, bool w_constant, cudaStream_t st);
 
-// Attention of prompt rows over the dense f32 cache (prefill_f32.cu); takes() says whether rows and head size are its kind.
-bool attention_rows_f32_takes(int64_t n_tokens, int64_t head_dim);
-int attention_rows_f32(const float* qkv, const float* k_cache, const float* v_cache, const int32_t* positions, const int32_t* slot, float* out,
-                       int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st);
+// Attention over the dense f32 cache: runs of rows of one sequence in tiles that share its keys (prefill_f32.cu), single rows with a CTA
+// per row and head (dense_f32.cu). `lists`: room for two int32 per row.
+AttentionF32Plan attention_f32_plan(const int32_t* slots, int n_tokens, int n_q_heads, int head_dim, int capacity, int32_t* lists);
+int attention_tiles_f32(const float* qkv, const float* k_cache, const float* v_cache, const int32_t* positions, const int32_t* slot, float* out,
+                        const int32_t* tiles, int n_tiles, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st);
+int attention_listed_f32(const float* qkv, const float* k_cache, const float* v_cache, const int32_t* positions, const int32_t* slot, float* out,
+                         const int32_t* rows, int n_rows, int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim, int64_t capacity, cudaStream_t st);
 
 // Quantised matmuls of 1..16 rows with the norms around them folded in (quant_matmul.cu): the sums of squares are per quant_tile_cols
 // columns of the producer.

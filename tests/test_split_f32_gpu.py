@@ -111,6 +111,32 @@ def test_prompt_rows_of_several_sequences(cuda, kind, hd, n_q, n_kv):
         assert np.abs(got - np.stack(want)).max() <= 1e-4 * max(1.0, np.abs(want).max())
 
 
+def test_passes_of_many_sequences(cuda):
+    """Runs of eight rows and more go to tiles, the others to the kernel with a CTA per row and head: prompts of every length around
+    that line, a token each, and a pass of both kinds, against the oracle."""
+    n = 24
+    cfg = mr.Cfg("gpt", n_layers=2, d_model=64, n_q=12, n_kv=12, hd=64, d_mlp=128, vocab=96, ctx=128)
+    params = mr.random_params(cfg, seed=12, std=0.2)
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 64, 12, 12, 64, 128, 96, 128, cfg.eps, max_seqs=n, max_tokens=512, max_logit_rows=n), namespace=7150)
+    for name, w in params.items():
+        m.load_param(name, w)
+    m.finalize()
+    rng = np.random.default_rng(0)
+    refs, at = [mr.RefModel(cfg, params) for _ in range(n)], [0] * n
+    for lengths in ([(8, 7, 33, 1, 32, 9, 65, 2)[s % 8] for s in range(n)], [1] * n, [{3: 40, 9: 8, 10: 7}.get(s, 1) for s in range(n)]):
+        tok, sl, pos, rows, want = [], [], [], [], []
+        for s, k in enumerate(lengths):
+            t = rng.integers(0, 96, k)
+            want.append(refs[s].forward(t)[-1])
+            tok += t.tolist()
+            sl += [s] * k
+            pos += range(at[s], at[s] + k)
+            at[s] += k
+            rows.append(len(tok) - 1)
+        got, _ = m.forward_with_decode_cache(tok, sl, pos, rows)
+        assert np.abs(got - np.stack(want)).max() <= 1e-4 * max(1.0, np.abs(want).max())
+
+
 @pytest.mark.parametrize("kind,hd,n_q,n_kv", [("gpt", 64, 8, 8), ("ministral", 128, 8, 2)])
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_a_token_that_is_not_finite_reaches_only_rows_that_see_it(cuda, kind, hd, n_q, n_kv, value):
