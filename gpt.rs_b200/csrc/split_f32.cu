@@ -16,8 +16,10 @@
 //
 // Relative error against 64 bits (random operands, K 768 / 3072, N 768, 937 rows): 5.3e-8 / 9.6e-8, plain f32 fused multiply-adds 5.8e-8 / 1.15e-7.
 //
-// Inputs that a bf16 cannot hold (infinities, NaN, magnitudes from 3.39e38 on) would turn into NaN in the remainders: a CTA that meets
-// one computes its tile again with plain f32 fused multiply-adds.
+// Infinities, NaN and magnitudes from 3.39e38 on, which a bf16 cannot hold, become NaN in the remainders and so in every sum that they
+// enter, and a product past the f32 range can be an infinity of one sign in each accumulator: sums that are not finite are computed again
+// with plain f32 fused multiply-adds, the others keep what they have. Below 2^-110 the third term, then the second, falls under what a
+// bf16 holds: an operand is then off by up to 2^-134, which against the sum's other products counts only where all of them are as small.
 #include "split_f32.cuh"
 #include "umma_common.cuh"
 
@@ -28,8 +30,8 @@ namespace {
 constexpr int kSfBK = 32;
 constexpr int kSfTile = 128 * 128;   // bytes of 128 rows of 128
 
-// 8 consecutive k of a row -> three planes; `check` keeps a NaN once a value is not the sum of its parts
-__device__ __forceinline__ void split3(const float (&v)[8], uint4 (&o)[3], uint32_t& check) {
+// 8 consecutive k of a row -> three planes
+__device__ __forceinline__ void split3(const float (&v)[8], uint4 (&o)[3]) {
     uint32_t p[3][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -39,12 +41,10 @@ __device__ __forceinline__ void split3(const float (&v)[8], uint4 (&o)[3], uint3
         p[1][i] = pack_bf16x2(a, b);
         a -= bf16_lo(p[1][i]); b -= bf16_hi(p[1][i]);
         p[2][i] = pack_bf16x2(a, b);
-        asm("max.NaN.bf16x2 %0, %0, %1;\n" : "+r"(check) : "r"(p[2][i]));
     }
 #pragma unroll
     for (int j = 0; j < 3; ++j) o[j] = make_uint4(p[j][0], p[j][1], p[j][2], p[j][3]);
 }
-__device__ __forceinline__ bool split_failed(uint32_t check) { return bf16_lo(check) != bf16_lo(check) || bf16_hi(check) != bf16_hi(check); }
 
 template <int BN>
 struct SfShape {
@@ -113,7 +113,6 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
     };
     bool failed = false;
     float acc[32];
-    uint32_t check = 0;
     const int quarter = warp & 3, c_lo = (warp >> 2) * 32;
     const bool sums = warp < BN / 8;   // four warps take the sums of 32 columns (rows of y)
     {
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
 #pragma unroll
             for (int i = 0; i < kWItems; ++i) {
                 uint4 o[3];
-                split3(r.w[i], o, check);
+                split3(r.w[i], o);
                 const int c = wc + 2 * i;
                 *reinterpret_cast<uint4*>(w_out + st + ((c ^ w_sw) << 4)) = o[0];
                 *reinterpret_cast<uint4*>(w_out + st + (((c + 4) ^ w_sw) << 4)) = o[1];
@@ -179,7 +178,7 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
             if (s + kSets < n_k) load_w(r);
             if (x_has) {
                 uint4 o[3];
-                split3(r.x, o, check);
+                split3(r.x, o);
                 *reinterpret_cast<uint4*>(x_out + st + ((xc ^ x_sw) << 4)) = o[0];
                 *reinterpret_cast<uint4*>(x_out + st + (((xc + 4) ^ x_sw) << 4)) = o[1];
                 *reinterpret_cast<uint4*>(x_out + st + kXTile + ((xc ^ x_sw) << 4)) = o[2];
@@ -213,7 +212,7 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
     }
     if (failed && lane == 0) atomicExch(p.status, 3);
     tc_fence_before();
-    const bool redo = __syncthreads_or(split_failed(check));
+    __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols) : "memory");
     // Row r of the tile belongs to rank r % S of the cluster; its receive slots [rank][row / S][128] lie over the stages, so nobody
     // pushes before everybody's MMAs have read theirs.
@@ -226,21 +225,20 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
     };
     const int col = quarter * 32 + lane;
     if (sums) {
-        if (!redo) {
+        uint32_t special = 0;   // rows whose sum is not finite
 #pragma unroll
-            for (int i = 0; i < 32; ++i) push(c_lo + i, col, acc[i]);
-        } else {
-            const int k_hi = (kt0 + n_k) * kSfBK;
+        for (int i = 0; i < 32; ++i) {
+            push(c_lo + i, col, acc[i]);
+            special |= fabsf(acc[i]) < INFINITY ? 0u : 1u << i;
+        }
+        const int n = n0 + col, k_hi = (kt0 + n_k) * kSfBK;
+        for (; special; special &= special - 1) {
+            const int r = c_lo + __ffs(special) - 1, m = m0 + r;
+            if (m >= p.M || n >= p.N) continue;
+            float sum = 0.f;
 #pragma unroll 1
-            for (int i = 0; i < 32; ++i) {
-                float sum = 0.f;
-                const int r = c_lo + i, m = m0 + r, n = n0 + col;
-                if (m < p.M && n < p.N) {
-#pragma unroll 1
-                    for (int k = kt0 * kSfBK; k < k_hi; ++k) sum = fmaf(x[(size_t)m * p.ldx + k], w[(size_t)k * p.N + n], sum);
-                }
-                push(r, col, sum);
-            }
+            for (int k = kt0 * kSfBK; k < k_hi; ++k) sum = fmaf(x[(size_t)m * p.ldx + k], w[(size_t)k * p.N + n], sum);
+            push(r, col, sum);
         }
     }
     if (S > 1) cluster_sync_all();

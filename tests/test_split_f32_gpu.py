@@ -72,15 +72,45 @@ def test_programs_whose_right_operand_is_computed(cuda, form):
 
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
 def test_matmul_of_values_that_bf16_cannot_hold(cuda, value):
-    """A tile with such a value gives what plain f32 arithmetic gives; the other tiles are not touched by it."""
+    """Sums that such a value enters are what plain f32 arithmetic gives; the others keep their bits."""
     g = torch.Generator(cuda).manual_seed(5)
     x, w = torch.randn(200, 256, device=cuda, generator=g), torch.randn(256, 520, device=cuda, generator=g) * 0.1
-    x[77, 130] = value
     w[130] = w[130].sign() * 0.25   # exact in one bf16: the remainders of the products are zeros
+    before = ops.matmul_f32(x, w)
+    x[77, 130] = value
     out, want = ops.matmul_f32(x, w), x.double() @ w.double()
     fine = torch.isfinite(want) & (want.abs() < 3.4e38)
     assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want.float()))
     assert ((out.double() - want).abs()[fine] <= _bound(x, w, want.abs())[fine]).all()
+    rest = torch.arange(200, device=cuda) != 77
+    assert torch.equal(out[rest], before[rest])
+
+
+def test_matmul_of_products_past_the_range(cuda):
+    """One product of a sum is an infinity, its second and third terms are infinities of either sign: the sum is the infinity that plain
+    f32 arithmetic gives, not NaN. Sums that leave the range and come back are its business too."""
+    g = torch.Generator(cuda).manual_seed(6)
+    x, w = torch.randn(64, 256, device=cuda, generator=g), torch.randn(256, 1024, device=cuda, generator=g)
+    before = ops.matmul_f32(x, w)
+    x[9, 40], x[30] = 3.1e30, 0.0
+    x[30, :2] = 1.7e38
+    w[40] = w[40].sign() * (1e9 + 1e6 * torch.rand(1024, device=cuda, generator=g))
+    w[:2, 500] = torch.tensor([1.5, -1.5], device=cuda)
+    out = ops.matmul_f32(x, w)
+    assert torch.equal(out[9], w[40].sign() * float("inf"))
+    plain = torch.zeros((), device=cuda)
+    for k in range(2):
+        plain = plain + x[30, k] * w[k, 500]
+    assert out[30, 500] == plain == 0
+    untouched = x[:, 40].abs() > 1e30   # rows whose own operands changed
+    untouched[30] = True
+    columns = torch.arange(1024, device=cuda) == 500
+    keep = ~untouched
+    assert torch.isfinite(out[keep]).all()
+    x0 = x.clone()
+    x0[9], x0[30] = 0, 0
+    want = x0.double() @ w.double()
+    assert ((out.double() - want).abs()[keep] <= _bound(x0, w, want.abs())[keep]).all() and before.shape == out.shape and columns.any()
 
 
 @pytest.mark.parametrize("kind,hd,n_q,n_kv", [("gpt", 64, 3, 3), ("ministral", 128, 4, 2)])
