@@ -55,7 +55,8 @@ struct SfShape {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
 };
 
-template <int BN>
+// EARLY: the weights were there before the kernel in front began
+template <int BN, bool EARLY>
 __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) split_f32_kernel(const SplitF32Params p) {
     using Shape = SfShape<BN>;
     constexpr int kWarps = Shape::kWarps, kSplitters = 32 * kWarps, STAGES = Shape::kStages, kXTile = BN * 128, kStage = Shape::kStageBytes;
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
     const int quarter = warp & 3, c_lo = (warp >> 2) * 32;
     const bool sums = warp < BN / 8;   // four warps take the sums of 32 columns (rows of y)
     {
-        if (!p.w_constant) pdl_wait();   // else the weights travel while the kernel in front still runs
+        if constexpr (!EARLY) pdl_wait();   // else the weights travel while the kernel in front still runs
 #pragma unroll
         for (int i = 0; i < kSets; ++i)
             if (i < n_k) load_w(raw[i]);
@@ -278,7 +279,7 @@ int64_t slots_of(int cluster) {
             cfg.attrs = &attr;
             cfg.numAttrs = 1;
             int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, split_f32_kernel<BN>, &cfg) != cudaSuccess) { cudaGetLastError(); clusters = 0; }
+            if (cudaOccupancyMaxActiveClusters(&clusters, split_f32_kernel<BN, true>, &cfg) != cudaSuccess) { cudaGetLastError(); clusters = 0; }
             n = clusters > 0 ? clusters * cluster : 1;
         }
         slot.store(n, std::memory_order_relaxed);
@@ -302,11 +303,13 @@ template <int BN>
 int launch(SplitF32Params p, cudaStream_t st) {
     using Shape = SfShape<BN>;
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time()) GPTRS_CUDA_OK(cudaFuncSetAttribute(split_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::kSmem));
+    if (attr_once.first_time())
+        for (auto k : {split_f32_kernel<BN, true>, split_f32_kernel<BN, false>})
+            GPTRS_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::kSmem));
     plan<BN>(p);
     const int64_t z = (int64_t)p.m_tiles * p.batch;
     if (z > 65535) return fail(GPTRS_UNIMPLEMENTED, "f32 matmul: too many rows in one launch");
-    return launch_kernel(split_f32_kernel<BN>, dim3((unsigned)ceil_div(p.N, 128), (unsigned)p.n_split, (unsigned)z), dim3(Shape::kThreads), Shape::kSmem, st,
+    return launch_kernel(p.w_constant ? split_f32_kernel<BN, true> : split_f32_kernel<BN, false>, dim3((unsigned)ceil_div(p.N, 128), (unsigned)p.n_split, (unsigned)z), dim3(Shape::kThreads), Shape::kSmem, st,
                          p.n_split, p);
 }
 

@@ -16,7 +16,7 @@ struct SplitF32Params {
     int64_t ldx, ldy, x_step, y_step;   // steps between the entries of a batch; their weights follow each other
     int batch;
     int* status;            // code 3: a bounded wait gave up
-    bool w_constant;        // no kernel in front writes w: its first stages may be read before that kernel has ended
+    bool w_constant;        // no kernel in front writes w: its first stages may be read before that kernel has ended (a template: a branch cost 2 %)
     int m_tiles, n_split;   // set by the launcher
 };
 
