@@ -43,7 +43,8 @@ struct SgemmParams {
     const int* n_row_tiles;
 };
 
-template <int MT>
+// U: weight rows of a warp under way at once
+template <int MT, int U>
 __global__ void __launch_bounds__(kSgWarps * 32) sgemm_smallm_kernel(const SgemmParams pp) {
     SgemmParams p = pp;
     extern __shared__ __align__(16) float sg_smem[];
@@ -126,7 +127,6 @@ __global__ void __launch_bounds__(kSgWarps * 32) sgemm_smallm_kernel(const Sgemm
 #pragma unroll
     for (int j = 0; j < 4; ++j) cv[j] = col0 + 32 * j < p.N;
 
-    constexpr int U = MT <= 2 ? 12 : 8;   // K 768 in eight parts is twelve rows of a warp: one round trip to memory
     int k = warp;
     for (; k + (U - 1) * kSgWarps < kn; k += U * kSgWarps) {
         float wv[U][4];
@@ -337,10 +337,15 @@ int launch_sgemm(SgemmParams p, int batch, cudaStream_t st) {
     p.k_per_cta = p.K / p.n_split;
     size_t smem = ((size_t)MT * p.k_per_cta + (size_t)kSgWarps * MT * kSgCols) * sizeof(float);
     if (smem > 200 * 1024) return fail(GPTRS_UNIMPLEMENTED, "f32 matmul: K too large for the shared-memory x tile");
-    void (*kern)(SgemmParams) = sgemm_smallm_kernel<MT>;
-    GPTRS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     p.m_tiles = ceil_div(p.M, MT);
     const int64_t z = p.tiles ? batch : (int64_t)p.m_tiles * batch;   // grouped form: `batch` is the most tiles there can be
+    // K 768 in eight parts is twelve weight rows of a warp: with one or two rows of x they are asked for at once, one round trip to memory.
+    // With eight rows of x, eight weight rows leave room for two CTAs on an SM, six for three: those are faster once two per SM are not
+    // enough (us, eight / six; K 768, N 768, 64 rows 17.6 / 11.7; N 3072, 12 rows 15.8 / 10.6; K 3072, N 768, 16 rows, 96 CTAs, 12.1 / 12.6).
+    void (*kern)(SgemmParams);
+    if constexpr (MT == 8) kern = (int64_t)n_blocks * p.n_split * z * 8 <= 14 * (int64_t)sm_count() ? sgemm_smallm_kernel<MT, 8> : sgemm_smallm_kernel<MT, 6>;
+    else kern = sgemm_smallm_kernel<MT, (MT <= 2 ? 12 : 8)>;
+    GPTRS_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     if (z > 65535) return fail(GPTRS_UNIMPLEMENTED, "f32 matmul: too many rows in one launch");
     dim3 grid(n_blocks, p.n_split, (unsigned)z);
     return launch_kernel(kern, grid, dim3(kSgWarps * 32), smem, st, p.n_split, p);

@@ -37,6 +37,17 @@ def test_matmul_of_many_rows(cuda, m, n, k, form):
     assert ops.matmul_status() == 0
 
 
+# shares of a warp with every remainder of the loads under way at once, one and two CTAs of eight rows per SM and more
+@pytest.mark.parametrize("m,n,k", [(1, 300, 72), (1, 128, 1000), (2, 130, 776), (3, 256, 100), (4, 129, 864), (8, 129, 104), (8, 2304, 768), (12, 2304, 768),
+                                   (20, 3072, 100), (23, 2050, 808), (64, 768, 352), (64, 640, 1000)])
+def test_matmul_of_few_rows(cuda, m, n, k):
+    """Sums of K fused multiply-adds: off by at most K ulps of the sum of magnitudes."""
+    g = torch.Generator(cuda).manual_seed(m + k)
+    x, w = torch.randn(m, k, device=cuda, generator=g), torch.randn(k, n, device=cuda, generator=g)
+    out, mag = ops.matmul_f32(x, w), x.abs().double() @ w.abs().double()
+    assert ((out.double() - x.double() @ w.double()).abs() <= k * 2.0 ** -24 * mag).all()
+
+
 # right operands that the kernel in front has just written: a transpose, a product, an update
 @pytest.mark.parametrize("form", ["transpose", "product", "update"])
 def test_programs_whose_right_operand_is_computed(cuda, form):
