@@ -43,6 +43,28 @@ struct SgemmParams {
     const int* n_row_tiles;
 };
 
+// A warp's weight rows from its k-th on, U under way at once, as long as so many are left
+template <int U, int MT>
+__device__ __forceinline__ void take_rows(int& k, int kn, const float* w, int N, const bool (&cv)[4], const float* xs, int ldx, float (&acc)[MT][4]) {
+    for (; k + (U - 1) * kSgWarps < kn; k += U * kSgWarps) {
+        float wv[U][4];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float* wr = w + (size_t)(k + u * kSgWarps) * N;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) wv[u][j] = cv[j] ? __ldg(wr + 32 * j) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float xv = xs[m * ldx + k + u * kSgWarps];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[m][j] = fmaf(xv, wv[u][j], acc[m][j]);
+            }
+    }
+}
+
 // U: weight rows of a warp under way at once
 template <int MT, int U>
 __global__ void __launch_bounds__(kSgWarps * 32) sgemm_smallm_kernel(const SgemmParams pp) {
@@ -128,34 +150,41 @@ __global__ void __launch_bounds__(kSgWarps * 32) sgemm_smallm_kernel(const Sgemm
     for (int j = 0; j < 4; ++j) cv[j] = col0 + 32 * j < p.N;
 
     int k = warp;
-    for (; k + (U - 1) * kSgWarps < kn; k += U * kSgWarps) {
-        float wv[U][4];
+    if constexpr (MT <= 2) {   // written out: through take_rows K 3072, N 768, 2 rows take 7.2 us instead of 6.7
+        for (; k + (U - 1) * kSgWarps < kn; k += U * kSgWarps) {
+            float wv[U][4];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const float* wr = pw + (size_t)(kb + k + u * kSgWarps) * p.N + col0;
+            for (int u = 0; u < U; ++u) {
+                const float* wr = pw + (size_t)(kb + k + u * kSgWarps) * p.N + col0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) wv[u][j] = cv[j] ? __ldg(wr + 32 * j) : 0.f;
+                for (int j = 0; j < 4; ++j) wv[u][j] = cv[j] ? __ldg(wr + 32 * j) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const float xv = xs[m * p.k_per_cta + k + u * kSgWarps];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[m][j] = fmaf(xv, wv[u][j], acc[m][j]);
+                }
         }
+        for (; k < kn; k += kSgWarps) {
+            const float* wr = pw + (size_t)(kb + k) * p.N + col0;
+            float wv[4];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+            for (int j = 0; j < 4; ++j) wv[j] = cv[j] ? __ldg(wr + 32 * j) : 0.f;
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const float xv = xs[m * p.k_per_cta + k + u * kSgWarps];
+                const float xv = xs[m * p.k_per_cta + k];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[m][j] = fmaf(xv, wv[u][j], acc[m][j]);
+                for (int j = 0; j < 4; ++j) acc[m][j] = fmaf(xv, wv[j], acc[m][j]);
             }
-    }
-    for (; k < kn; k += kSgWarps) {
-        const float* wr = pw + (size_t)(kb + k) * p.N + col0;
-        float wv[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) wv[j] = cv[j] ? __ldg(wr + 32 * j) : 0.f;
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            const float xv = xs[m * p.k_per_cta + k];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[m][j] = fmaf(xv, wv[j], acc[m][j]);
         }
+    } else {
+        const float* w = pw + (size_t)kb * p.N + col0;
+        take_rows<U>(k, kn, w, p.N, cv, xs, p.k_per_cta, acc);
+        take_rows<4>(k, kn, w, p.N, cv, xs, p.k_per_cta, acc);
+        take_rows<1>(k, kn, w, p.N, cv, xs, p.k_per_cta, acc);
     }
 #pragma unroll
     for (int m = 0; m < MT; ++m)
