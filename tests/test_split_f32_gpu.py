@@ -19,7 +19,8 @@ def _bound(x, w, extra):
 
 @pytest.mark.parametrize("m,n,k,form", [
     (24, 2304, 768, "bias"), (32, 3072, 32, ""), (33, 1700, 64, "residual"), (64, 900, 96, "bias"), (65, 768, 3072, "residual"), (128, 400, 160, "gelu"),
-    (129, 385, 768, "bias"), (250, 129, 1024, "gelu"), (40, 50257, 64, ""), (300, 130, 32, "residual")])
+    (129, 385, 768, "bias"), (250, 129, 1024, "gelu"), (40, 50257, 64, ""), (300, 130, 32, "residual"),
+    (33, 20000, 32, ""), (64, 12900, 96, "bias"), (300, 4100, 32, "residual"), (129, 9000, 64, "gelu")])   # small K: enough columns for this kernel
 def test_matmul_of_many_rows(cuda, m, n, k, form):
     g = torch.Generator(cuda).manual_seed(m * 7 + n)
     x, w = torch.randn(m, k, device=cuda, generator=g), torch.randn(k, n, device=cuda, generator=g)
