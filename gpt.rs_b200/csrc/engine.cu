@@ -1213,10 +1213,11 @@ int gptrs_cuda_model_forward_with_decode_cache(gptrs_model* h, const int32_t* h_
         if ((rc = launch_kernel(record_history_kernel, dim3((T + 127) / 128), dim3(128), 0, s, 1, hp))) return rc;
     }
     // The kernels of a short pass may start while the one in front ends, as in the generator's graphs: they are as long as a launch. The
-    // persistent kernels of a long one take the SMs that the rest of the grid in front still needs (5855 rows of a layered model:
-    // 6.5 ms without, 6.9 with).
+    // persistent kernels of a long one take the SMs that the rest of the grid in front still needs. Without / with, us: four layers of a
+    // hybrid of width 2048, 64 rows 941 / 857, 128 rows 1090 / 1046, 160 rows 1104 / 1100, 200 rows 1130 / 1206, 5855 rows 6500 / 6900; W4
+    // of width 3072, 64 rows 420 / 356, 256 rows 791 / 729; W8 of width 2048, 256 rows 552 / 501; GPT-2, 256 rows 1766 / 1692.
     const int pdl_before = g_use_pdl;
-    if (c.use_pdl && T <= 256) g_use_pdl = 1;
+    if (c.use_pdl && T <= (m.layered() ? 128 : 256)) g_use_pdl = 1;
     rc = enqueue_forward(m, T, max_ctx, chunk, rows, false, temperature, prefill_groups);
     g_use_pdl = pdl_before;
     if (rc) return rc;
