@@ -14,6 +14,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "engine.h"
 #include "ptir_json.h"
 #include "tensor.h"
 
@@ -1027,6 +1028,10 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
         }
         return tensor_alloc(in.out.dtype, (int)in.out.dims.size(), in.out.dims.data(), false, &out);
     };
+    // the right operand may be what the instruction in front computes; a wait that gives up is the program's error
+    auto matmul = [&](const float* x, const float* w, float* y, int64_t m, int64_t n, int64_t k, const float* bias, int gelu) {
+        return norm_matmul_f32(x, 0, nullptr, nullptr, 0.f, w, y, m, n, k, bias, nullptr, gelu, status_word(), false, ex.st);
+    };
     const int64_t n_out = in.out.numel();
     int rc = GPTRS_OK;
     switch (in.op) {
@@ -1260,7 +1265,7 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
             p.n = fb.empty() ? 1 : B->dims[fb[0]]; p.b_sn = fb.empty() ? 0 : bs[fb[0]];
             ++ex.launches;
             if (p.nb == 1 && p.a_sk == 1 && p.a_sm == p.k && p.b_sn == 1 && p.b_sk == p.n)
-                rc = gptrs_cuda_matmul_f32(p.a, p.b, p.out, p.m, p.n, p.k, nullptr, nullptr, 0, ex.st);  // [M,K].[K,N]
+                rc = matmul(p.a, p.b, p.out, p.m, p.n, p.k, nullptr, 0);  // [M,K].[K,N]
             else
                 rc = launch_flat(dot_kernel, p.nb * p.m * p.n, p, ex.st);
             break;
@@ -1293,9 +1298,8 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
         case Op::FusedMatmulBias: {   // in.axis = 1: GELU on the sum
             if ((rc = alloc_out())) return rc;
             ++ex.launches;
-            rc = gptrs_cuda_matmul_f32(static_cast<const float*>(ops[0]->data), static_cast<const float*>(ops[1]->data), static_cast<float*>(out->data),
-                                       ops[0]->dims[0], ops[1]->dims[1], ops[0]->dims[1], static_cast<const float*>(ops[2]->data), nullptr,
-                                       in.axis == 1 ? 1 : 0, ex.st);
+            rc = matmul(static_cast<const float*>(ops[0]->data), static_cast<const float*>(ops[1]->data), static_cast<float*>(out->data),
+                        ops[0]->dims[0], ops[1]->dims[1], ops[0]->dims[1], static_cast<const float*>(ops[2]->data), in.axis == 1 ? 1 : 0);
             break;
         }
         case Op::FusedAttentionDecode: {
@@ -1370,6 +1374,7 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
             if (!rc) {
                 gptrs_matmul_epilogue ep = {};
                 ep.out_dtype = GPTRS_F32;
+                ep.d_status = status_word();
                 rc = w8 ? gptrs_cuda_quant_matmul_w8a16(xb->data, packed->data, out->data, M, N, K, &ep, ex.st)
                         : gptrs_cuda_quant_matmul_w4a16(xb->data, packed->data, out->data, M, N, K, &ep, ex.st);
             }
@@ -1656,7 +1661,7 @@ int execute_plan(const std::shared_ptr<Plan>& plan, gptrs_tensor* const* inputs,
     *n_outputs = fn.result_ids.size();
     g_last_launches = ex.launches;
     g_last_fused = plan->fused;
-    // report a device-side index error (take / gather) the way ref-cpu reports it: as an error
+    // report a device-side index error (take / gather) the way ref-cpu reports it, as an error, and so a wait of a matmul that gave up
     int* sw = status_word();
     if (sw) {
         int hs = 0;
@@ -1666,7 +1671,7 @@ int execute_plan(const std::shared_ptr<Plan>& plan, gptrs_tensor* const* inputs,
             cudaMemsetAsync(sw, 0, 4, ex_st);
             for (size_t i = 0; i < fn.result_ids.size(); ++i) tensor_release(reinterpret_cast<Tensor*>(outputs[i]));
             *n_outputs = 0;
-            return fail(GPTRS_EXECUTION, "index out of range in take/gather");
+            return fail(GPTRS_EXECUTION, hs == 2 ? "index out of range in take/gather" : "a bounded wait inside a tensor-core matmul gave up");
         }
     }
     return GPTRS_OK;

@@ -24,7 +24,9 @@
 #include "umma_common.cuh"
 
 namespace gptrs {
-int* matmul_status_word();  // umma_matmul.cu: the library's per-device status word
+// umma_matmul.cu: the library's per-device status word, and the polls of a wait and the test switch of gptrs_cuda_debug_matmul_fault
+int* matmul_status_word();
+void matmul_wait_limits(uint32_t* spin_limit, int* starve);
 namespace {
 
 constexpr int kSfBK = 32;
@@ -55,10 +57,12 @@ struct SfShape {
     static constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024;
 };
 
-// EARLY: the weights were there before the kernel in front began
-template <int BN, bool EARLY>
+// EARLY: the weights were there before the kernel in front began. DEBUG: the wait limits and the test switch of the call (as reads of the
+// parameters they cost the others 3 %)
+template <int BN, bool EARLY, bool DEBUG = false>
 __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) split_f32_kernel(const SplitF32Params p) {
     using Shape = SfShape<BN>;
+    const uint32_t limit = DEBUG ? p.spin_limit : kSpinLimit;
     constexpr int kWarps = Shape::kWarps, kSplitters = 32 * kWarps, STAGES = Shape::kStages, kXTile = BN * 128, kStage = Shape::kStageBytes;
     constexpr uint32_t kCols = BN == 128 ? 512 : BN == 64 ? 256 : 128;
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (8u << 24);
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
         };
         auto step = [&](int s, Raw& r) {
             if (s >= STAGES) {   // the MMAs of stage s - STAGES are complete
-                if (!failed && !mbar_wait_relaxed(&empty[buf], parity)) failed = true;
+                if (!failed && !mbar_wait_relaxed(&empty[buf], parity, limit)) failed = true;
                 tc_fence_after();
             }
             if (!(s & 1) && s >= 4) {
@@ -189,9 +193,9 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
             tc_fence_before();
             mbar_arrive(&full[buf]);
             if (warp == kWarps - 1) {
-                if (!failed && !mbar_wait_relaxed(&full[buf], parity ^ 1)) failed = true;
+                if (!failed && !mbar_wait_relaxed(&full[buf], parity ^ 1, limit)) failed = true;
                 tc_fence_after();
-                if (lane == 0 && !failed) issue(s, smem_u32(smem) + (uint32_t)st);
+                if (lane == 0 && !failed && !(DEBUG && p.debug_starve && s == 0)) issue(s, smem_u32(smem) + (uint32_t)st);
                 __syncwarp();
             }
             if (++buf == STAGES) { buf = 0; parity ^= 1; }
@@ -203,7 +207,7 @@ __global__ void __launch_bounds__(SfShape<BN>::kThreads, BN == 128 ? 1 : 2) spli
                 if (s + 1 < n_k) step(s + 1, raw[kSets - 1]);
         }
         for (int s = max(n_k - STAGES, 0); s < n_k; ++s)
-            if (!failed && !mbar_wait_relaxed(&empty[s % STAGES], (uint32_t)(s / STAGES) & 1u)) failed = true;
+            if (!failed && !mbar_wait_relaxed(&empty[s % STAGES], (uint32_t)(s / STAGES) & 1u, limit)) failed = true;
         tc_fence_after();
         if (sums) {
 #pragma unroll 1
@@ -304,13 +308,13 @@ int launch(SplitF32Params p, cudaStream_t st) {
     using Shape = SfShape<BN>;
     static PerDeviceOnce attr_once;
     if (attr_once.first_time())
-        for (auto k : {split_f32_kernel<BN, true>, split_f32_kernel<BN, false>})
+        for (auto k : {split_f32_kernel<BN, true>, split_f32_kernel<BN, false>, split_f32_kernel<BN, false, true>})
             GPTRS_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape::kSmem));
     plan<BN>(p);
     const int64_t z = (int64_t)p.m_tiles * p.batch;
     if (z > 65535) return fail(GPTRS_UNIMPLEMENTED, "f32 matmul: too many rows in one launch");
-    return launch_kernel(p.w_constant ? split_f32_kernel<BN, true> : split_f32_kernel<BN, false>, dim3((unsigned)ceil_div(p.N, 128), (unsigned)p.n_split, (unsigned)z), dim3(Shape::kThreads), Shape::kSmem, st,
-                         p.n_split, p);
+    auto kern = p.debug_starve || p.spin_limit != kSpinLimit ? split_f32_kernel<BN, false, true> : p.w_constant ? split_f32_kernel<BN, true> : split_f32_kernel<BN, false>;
+    return launch_kernel(kern, dim3((unsigned)ceil_div(p.N, 128), (unsigned)p.n_split, (unsigned)z), dim3(Shape::kThreads), Shape::kSmem, st, p.n_split, p);
 }
 
 }  // namespace
@@ -330,6 +334,7 @@ bool split_f32_takes(const SplitF32Params& p) {
 int split_f32_matmul(SplitF32Params p, cudaStream_t st) {
     if (!p.status) p.status = matmul_status_word();
     if (!p.status) return fail(GPTRS_EXECUTION, "no status word");
+    matmul_wait_limits(&p.spin_limit, &p.debug_starve);
     if (p.M <= 32) return launch<32>(p, st);
     if (p.M <= 64) return launch<64>(p, st);
     return launch<128>(p, st);

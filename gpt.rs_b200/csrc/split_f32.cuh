@@ -18,6 +18,8 @@ struct SplitF32Params {
     int* status;            // code 3: a bounded wait gave up
     bool w_constant;        // no kernel in front writes w: its first stages may be read before that kernel has ended (a template: a branch cost 2 %)
     int m_tiles, n_split;   // set by the launcher
+    uint32_t spin_limit;
+    int debug_starve;       // test switch: the first stage's products are never begun
 };
 
 // Least rows, and whether it takes this shape (the rule stands at its definition).

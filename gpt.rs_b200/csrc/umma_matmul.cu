@@ -677,14 +677,19 @@ int encode_x_map(const MatmulParams& p, int bn, CUtensorMap* map) {
     return GPTRS_OK;
 }
 
-int fill_wait_params(MatmulParams& p) {
-
-    if (!p.status) p.status = umma_status_word();
-    if (!p.status) return fail(GPTRS_EXECUTION, "cannot find the status word of this device");
+}  // namespace
+void matmul_wait_limits(uint32_t* spin_limit, int* starve) {
     static const uint32_t env_limit = [] { const char* e = getenv("GPTRS_SPIN_LIMIT"); return e ? (uint32_t)atoll(e) : 0u; }();
     const uint32_t lim = g_debug_spin_limit.load(std::memory_order_relaxed);
-    p.spin_limit = lim ? lim : (env_limit ? env_limit : kSpinLimit);
-    p.debug_starve = g_debug_starve.load(std::memory_order_relaxed);
+    *spin_limit = lim ? lim : (env_limit ? env_limit : kSpinLimit);
+    *starve = g_debug_starve.load(std::memory_order_relaxed);
+}
+namespace {
+
+int fill_wait_params(MatmulParams& p) {
+    if (!p.status) p.status = umma_status_word();
+    if (!p.status) return fail(GPTRS_EXECUTION, "cannot find the status word of this device");
+    matmul_wait_limits(&p.spin_limit, &p.debug_starve);
     static const int rotate = [] { const char* e = getenv("GPTRS_STAGE_ROTATION"); return e ? atoi(e) : 1; }();
     p.stage_rotation = rotate;
     return GPTRS_OK;

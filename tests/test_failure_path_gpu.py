@@ -6,8 +6,9 @@ import numpy as np
 import pytest
 import torch
 
-from gptrs_b200 import BackendError, check, lib, ops
+from gptrs_b200 import BackendError, check, lib, ops, ptir
 from gptrs_b200 import model as gm
+from gptrs_b200.backend import CudaBackend
 from oracle import models_ref as mr
 from oracle import quant_ref as qr
 
@@ -43,6 +44,52 @@ def test_matmul_wait_runs_out_sets_status_and_recovers(cuda, starved):
     assert ops.matmul_status() == 0
     assert np.abs(ops.quant_matmul_w4a16(xd, packed, m, n, k, out_f32=True).cpu().numpy() - want).max() <= tol
     assert ops.matmul_status() == 0
+
+
+def test_f32_matmul_wait_runs_out_sets_status_and_recovers(cuda, starved):
+    """The tensor-core f32 matmul with the products of its first stage withheld, K of more stages than its ring holds."""
+    g = torch.Generator(cuda).manual_seed(2)
+    for m in (32, 64, 200):   # each of its row tiles
+        x, w = torch.randn(m, 768, device=cuda, generator=g), torch.randn(768, 2304, device=cuda, generator=g)
+        good = ops.matmul_f32(x, w)
+        assert ops.matmul_status() == 0
+        starved()
+        ops.matmul_f32(x, w)   # returns; the result is unspecified
+        torch.cuda.synchronize()
+        assert ops.matmul_status() == 3
+        check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
+        assert torch.equal(ops.matmul_f32(x, w), good) and ops.matmul_status() == 0
+
+
+@pytest.mark.parametrize("form", ["plain", "bias", "quantised"])
+def test_program_reports_a_matmul_wait_that_ran_out(cuda, starved, form):
+    be = CudaBackend()
+    b = ptir.Builder()
+    rng = np.random.default_rng(3)
+    x = b.parameter(ptir.F32, [64, 512])
+    inputs = [rng.normal(size=(64, 512)).astype(np.float32)]
+    if form == "quantised":
+        q, s = b.parameter(ptir.SI8, [1024, 512]), b.parameter(ptir.F16, [1024])
+        b.set_results([ptir.matmul(x, q.dequantize(s).transpose([1, 0]))])
+        inputs += [rng.integers(-100, 100, (1024, 512)).astype(np.int8), np.full(1024, 0.01, np.float16)]
+    else:
+        w = b.parameter(ptir.F32, [512, 1024])
+        inputs.append(rng.normal(size=(512, 1024)).astype(np.float32))
+        y = ptir.matmul(x, w)
+        if form == "bias":
+            y = ptir.add_bias(y, b.parameter(ptir.F32, [1024]))
+            inputs.append(rng.normal(size=1024).astype(np.float32))
+        b.set_results([y])
+    prog = be.prepare(b.to_json())
+    handles = [be.materialize(a) for a in inputs]
+    good = be.to_literal(prog.run(handles)[0])
+    starved()
+    with pytest.raises(BackendError) as e:
+        prog.run(handles)
+    assert e.value.kind == "Execution" and "matmul" in str(e.value)
+    check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
+    for _ in range(3):
+        assert np.array_equal(be.to_literal(prog.run(handles)[0]), good)
 
 
 def test_engine_reports_a_matmul_wait_that_ran_out(cuda, starved):
