@@ -68,7 +68,8 @@ __global__ void strided_copy_kernel(const CopyParams p) {
 }
 
 // out = in with `upd` written over it at clamped device starts, in one launch instead of a copy and an update: four neighbouring elements
-// of the innermost axis per thread (rows of a multiple of four 32-bit elements).
+// of the innermost axis per thread (rows of a multiple of four 32-bit elements, less than 2^31 in all: the
+// starts are int).
 struct UpdateParams {
     const uint4* in;
     const uint32_t* upd;
@@ -1144,7 +1145,7 @@ int exec_inst(Exec& ex, const Inst& in, std::vector<Tensor*>& ops, Tensor** resu
                 const size_t rank = in.out.dims.size();
                 const int64_t n = in.out.numel();
                 bool fits = rank >= 1 && rank <= (size_t)kMaxRank && dtype_size(in.out.dtype) == 4 && ops[0]->dtype == in.out.dtype && ops[1]->dtype == in.out.dtype &&
-                            ops[2]->numel() == (int64_t)rank && n > 0 && n < (1ll << 32) && in.out.dims[rank - 1] % 4 == 0 && ops[1]->numel() > 0 &&
+                            ops[2]->numel() == (int64_t)rank && n > 0 && n < (1ll << 31) && in.out.dims[rank - 1] % 4 == 0 && ops[1]->numel() > 0 &&
                             ((reinterpret_cast<uintptr_t>(ops[0]->data) | reinterpret_cast<uintptr_t>(out->data)) & 15) == 0;
                 UpdateParams p = {static_cast<const uint4*>(ops[0]->data), static_cast<const uint32_t*>(ops[1]->data), static_cast<uint4*>(out->data),
                                   static_cast<const int*>(ops[2]->data), (int)rank, (uint32_t)(n / 4)};

@@ -64,3 +64,13 @@ def test_updates(be, dims, sizes, starts, dtype):
     b.set_results([x.dynamic_update_slice(u, s, sizes)])
     kind = np.float32 if dtype == F32 else np.int32
     _run(be, b, [rng.integers(-99, 99, dims).astype(kind), rng.integers(100, 999, sizes).astype(kind), np.array(starts, np.int32)])
+
+
+def test_update_of_an_axis_longer_than_int(be):
+    n = 2 ** 31 + 8
+    b = ptir.Builder()
+    u, at = b.parameter(SI32, [4]), b.parameter(SI32, [1])
+    y = b.iota([n], 0).dynamic_update_slice(u, at, [4])
+    b.set_results([y.slice([996], [12])])
+    got, = be.run_program(b.to_json(), [be.materialize(np.array([-1, -2, -3, -4], np.int32)), be.materialize(np.array([1000], np.int32))])
+    assert be.to_literal(got).tolist() == [996, 997, 998, 999, -1, -2, -3, -4, 1004, 1005, 1006, 1007]
