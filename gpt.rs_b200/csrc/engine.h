@@ -284,7 +284,8 @@ int attention_listed_f32(const float* qkv, const float* k_cache, const float* v_
 int quant_tile_cols(int bits, int64_t m, int64_t n, int64_t k);
 int quant_matmul_few_rows(int bits, const void* x, const void* packed, void* y, int64_t m, int64_t n, int64_t k, const gptrs_matmul_epilogue* ep, cudaStream_t st);
 
-// W4 matmuls of a prompt's rows, from quant_widen_rows() on with the weights widened to bf16 first, in a buffer of the caller.
+// W4 matmuls of a prompt's rows, from quant_widen_rows() on and where the projection is large enough with the weights widened to bf16
+// first, in a buffer of the caller.
 int quant_matmul_rows(const void* x, const void* packed, void* y, int64_t m, int64_t n, int64_t k, const gptrs_matmul_epilogue* ep, void* wide, size_t wide_bytes,
                       cudaStream_t st);
 int64_t quant_widen_rows();

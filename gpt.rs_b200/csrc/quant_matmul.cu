@@ -567,8 +567,12 @@ __global__ void __launch_bounds__(256) w4_widen_kernel(const WidenParams p) {
 }
 
 // Rows from which a projection is faster on widened weights: widening costs 2 bytes per weight and call, the matmul on bf16 weights runs
-// at 0.75-0.8 of the measured peak where the kernel that widens inside every row tile runs at 0.53-0.57.
+// at 0.75-0.8 of the measured peak where the kernel that widens inside every row tile runs at 0.53-0.57. Two launches instead of one cost
+// about 10 us, which a small projection wins back only with more rows: over four layers (us, inside the tiles / widened) width 512 with
+// 1540 rows 602 / 692, 2100 rows 690 / 757, 4000 rows 1014 / 991; width 1024 with 1536 rows 746 / 790, 1700 rows 847 / 846, 4000 rows
+// 1470 / 1234; width 2048 with 1536 rows 1214 / 1160. With the line below, per projection: 592, 677, 956; 694, 811, 1232; 1154.
 constexpr int kWidenRows = 1536;
+bool widen_pays(int64_t m, int64_t n, int64_t k) { return m >= kWidenRows && (m - 1000) * n * k >= 2000000000; }
 
 int pick_split(int n_blocks, int groups) {
     // Smallest power-of-two K split that puts about 1.2 CTAs on every SM (each CTA should keep a
@@ -662,7 +666,7 @@ int quant_matmul(const void* d_x, const void* d_packed, void* d_y, int64_t m, in
         }
     }
     cudaStream_t st = as_stream(stream);
-    if (BITS == 4 && wide && m >= kWidenRows && n % kCtaN == 0 && umma_enabled() && !p.bias && !p.best_val && !p.peer_on) {
+    if (BITS == 4 && wide && widen_pays(m, n, k) && n % kCtaN == 0 && umma_enabled() && !p.bias && !p.best_val && !p.peer_on) {
         if (!p.status) p.status = matmul_status_word();
         if (!p.status) return fail(GPTRS_EXECUTION, "cannot find the status word of this device");
         const WidenParams wp = {p.wq_rows, p.scales_rows, static_cast<__nv_bfloat16*>(wide), n / kCtaN * (k / 64) * 256, (int)(k / 64)};
