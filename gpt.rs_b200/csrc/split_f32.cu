@@ -1,7 +1,7 @@
 // f32 matmul on the tcgen05 tensor cores: y[M][N] = act(x[M][K] . w[K][N] + bias) + residual for many rows
 // (functional::matmul, crates/gpt-rs/src/ops/functional/linalg.rs:109-127; Linear::forward, nn/layers/linear.rs:50-71).
 //
-// Every f32 value is the sum of three bf16 values (8 significant bits each, the remainders exact in f32): v = v1 + v2 + v3. The product
+// An f32 value of 2^-110 and more is the sum of three bf16 values (8 significant bits each, the remainders exact in f32): v = v1 + v2 + v3. The product
 // keeps the six terms of at least 2^-18 of it, w1x1 + (w1x2 + w2x1 + w2x2 + w1x3 + w3x1); what is left out is below 2^-26, less than
 // the rounding of one f32 product. Products of bf16 values are exact; what the tensor core loses is in the order of its sums, so the
 // leading term w1x1 is summed in tensor memory over 64 k only and then added to f32 registers, and the five small terms, 2^-8 of the
@@ -15,6 +15,9 @@
 // of the CTA that owns the row and are added in the order of the ranks.
 //
 // Relative error against 64 bits (random operands, K 768 / 3072, N 768, 937 rows): 5.3e-8 / 9.6e-8, plain f32 fused multiply-adds 5.8e-8 / 1.15e-7.
+// Operands of one sign do worse, because the tensor core cuts its sums where f32 arithmetic rounds them (magnitudes of random operands,
+// N 2304, K 768 / 3072: 64 rows 8.9e-8 / 8.9e-8, 937 rows, whose K is not split, 9.5e-8 / 1.23e-7; the kernel for few rows 4.7e-8 / 4.5e-8,
+// a library's f32 matmul 3.7e-7 / 1.5e-7 to 7.4e-7). Sums taken after 32 k instead of 64 would halve the cut and double the additions.
 //
 // Infinities, NaN and magnitudes from 3.39e38 on, which a bf16 cannot hold, become NaN in the remainders and so in every sum that they
 // enter, and a product past the f32 range can be an infinity of one sign in each accumulator: sums that are not finite are computed again

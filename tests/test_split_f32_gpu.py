@@ -38,6 +38,36 @@ def test_matmul_of_many_rows(cuda, m, n, k, form):
     assert ops.matmul_status() == 0
 
 
+def _three_terms(shape, g):
+    """Positive values whose second and third bf16 terms are positive too, near the largest that such terms can be."""
+    term = lambda low, high, unit: torch.randint(low, high, shape, device=g.device, generator=g).float() * unit  # noqa: E731
+    return 1 + term(0, 128, 2.0 ** -7) + term(64, 127, 2.0 ** -15) + term(64, 127, 2.0 ** -23)
+
+
+@pytest.mark.parametrize("m,n,k", [(129, 4100, 64), (40, 2304, 768), (300, 768, 3072)])
+def test_no_term_of_the_product_is_missing(cuda, m, n, k):
+    """Root of the mean square of the errors over that of the sums of magnitudes. Operands of either sign: not above what eight rows at a time
+    leave (plain f32 arithmetic; half as much again allowed, the orders of the sums differ). Operands of one sign whose terms all are
+    too: without one of the six products of terms every sum lacks 2^-18 of itself or more (3.7e-6); the tensor core's sums, cut and not
+    rounded, lose up to an ulp of 2^-24 at each of the four steps of 64 k, and K / 64 additions in f32 half an ulp each, at random:
+    below 2^-21."""
+    g = torch.Generator(cuda).manual_seed(k)
+    x, w = torch.randn(m, k, device=cuda, generator=g), torch.randn(k, n, device=cuda, generator=g)
+    rms = lambda y, x, w: float((y.double() - x.double() @ w.double()).norm() / (x.abs().double() @ w.abs().double()).norm())  # noqa: E731
+    plain = torch.cat([ops.matmul_f32(r.contiguous(), w) for r in x.split(8)])
+    assert rms(ops.matmul_f32(x, w), x, w) <= 1.5 * rms(plain, x, w)
+    for a, b in ((x.abs(), w.abs()), (_three_terms((m, k), g), _three_terms((k, n), g))):
+        assert rms(ops.matmul_f32(a, b), a, b) <= 2.0 ** -21
+
+
+def test_matmul_of_operands_whose_lower_terms_underflow(cuda):
+    """Weights around 2^-118 against inputs around 2^100: a weight is off by what lies below the subnormals of a bf16, 2^-134 at most."""
+    g = torch.Generator(cuda).manual_seed(8)
+    x, w = torch.randn(64, 256, device=cuda, generator=g) * 2.0 ** 100, torch.randn(256, 2304, device=cuda, generator=g) * 2.0 ** -118
+    out, want = ops.matmul_f32(x, w), x.double() @ w.double()
+    assert ((out.double() - want).abs() <= _bound(x, w, want.abs()) + 2.0 ** -134 * x.abs().double().sum(1, keepdim=True)).all()
+
+
 # shares of a warp with every remainder of the loads under way at once, one and two CTAs of eight rows per SM and more
 @pytest.mark.parametrize("m,n,k", [(1, 300, 72), (1, 128, 1000), (2, 130, 776), (3, 256, 100), (4, 129, 864), (8, 129, 104), (8, 2304, 768), (12, 2304, 768),
                                    (20, 3072, 100), (23, 2050, 808), (64, 768, 352), (64, 640, 1000)])
