@@ -330,9 +330,10 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     float* hidden = m.hidden.as<float>();
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
     if (T <= m.mega_rows && T <= m.max_rows() && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
-        // a token each of a few sequences: the whole step is one cooperative kernel (+ the memset of its barrier word)
+        // a token each of a few sequences: the whole step is one cooperative kernel
         MegaParams P = m.mega;
         P.rows = T;
+        m.mega.epoch += (uint32_t)c.n_layers + 1u;   // every word of this step carries a flag that no other step's does
         P.greedy = temperature <= 0.f ? 1 : 0;
         m.launches += 1;
         int r = mega_launch(P, st);
@@ -686,23 +687,23 @@ int setup_mega(Model& m) {
     const float* lm_t = nullptr;
     if ((rc = tr(m.lm_head, &lm_t))) return rc;
     const size_t n_sm = (size_t)sm_count(), R = kMegaMaxRows;
-    auto pad = [](size_t n) { return (n + 63) & ~(size_t)63; };   // every vector starts on a 256-byte boundary
-    const size_t n_part = pad(n_sm * (c.head_dim + 2));
-    const size_t floats = pad(R * 3 * D) + n_part + pad(R * D) + pad(R * MLP) + pad(R * 4 * D) + 2 * pad(R * n_sm) + 64 + 512;
-    if ((rc = m.mega_scratch.alloc(floats * 4, true))) return rc;
-    float* s = m.mega_scratch.as<float>();
+    auto pad = [](size_t n) { return (n + 31) & ~(size_t)31; };   // words; every vector starts on a 256-byte boundary
+    const size_t n_part = pad(n_sm * (c.head_dim + 4));
+    const size_t words = pad(R * 3 * D) + n_part + 2 * pad(R * D) + pad(R * MLP) + pad(R * 4 * D) + pad(R * n_sm * 2) + 512;
+    if ((rc = m.mega_scratch.alloc(words * 8, true))) return rc;
+    unsigned char* s = m.mega_scratch.as<unsigned char>();
+    auto take = [&](size_t n) { unsigned char* at = s; s += n * 8; return at; };
     MegaParams& P = m.mega;
     P.n_layers = c.n_layers;
     P.tok_emb = fp(m.tok_emb); P.pos_emb = fp(m.pos_emb); P.lnf_g = fp(m.final_g); P.lnf_b = fp(m.final_b); P.lm_head_t = lm_t;
     P.token = m.d_tokens.as<int>(); P.pos = m.d_pos.as<int>(); P.slot = m.d_slot.as<int>();
-    P.qkv = s; s += pad(R * 3 * D);
-    P.att_part = s; s += n_part;
-    P.pc = s; s += pad(R * D);
-    P.mh = s; s += pad(R * MLP);
-    P.pe = s; s += pad(R * 4 * D);
-    P.cand_val = s; s += pad(R * n_sm);
-    P.cand_idx = reinterpret_cast<int*>(s); s += pad(R * n_sm);
-    P.barrier = reinterpret_cast<unsigned*>(s); s += 64;
+    P.qkv = take(pad(R * 3 * D));
+    P.att_part = take(n_part);
+    P.att = take(pad(R * D));
+    P.pc = take(pad(R * D));
+    P.mh = take(pad(R * MLP));
+    P.pe = take(pad(R * 4 * D));
+    P.cand = take(pad(R * n_sm * 2));
     P.timing = nullptr;
     if (const char* e = getenv("GPTRS_MEGA_TIMING")) if (atoi(e)) P.timing = reinterpret_cast<unsigned long long*>(s);
     P.logits = m.logits.as<float>();
@@ -779,6 +780,7 @@ int check_status(Model& m) {
         return fail(GPTRS_EXECUTION, st == 2   ? "token or position id out of range"
                                      : st == 3 ? "a bounded wait inside a tensor-core kernel (matmul or attention) gave up"
                                      : st == 4 ? "a tensor-parallel peer did not deliver its partial sums in time"
+                             : st == 5 ? "a bounded wait of a single-kernel step gave up"
                                                : "a bounded wait inside the attention kernel gave up");
     }
     return GPTRS_OK;

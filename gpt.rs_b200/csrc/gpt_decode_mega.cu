@@ -5,8 +5,8 @@
 //
 // Why one kernel: at one row every projection is a 2-9 MB weight stream that takes about a microsecond of HBM time and
 // 6-9 us as a launch of its own (launch, first DRAM round trip, barrier, reduction); 64 launches per token left the step
-// at 0.13 of its weight-stream roofline. Here the launch boundary becomes a grid-wide barrier (one CTA per SM, all
-// co-resident: the launch is cooperative), and what crosses a barrier is a short vector in global memory:
+// at 0.13 of its weight-stream roofline. Here the CTAs stay (one per SM, all co-resident: the launch is cooperative), and what crosses from
+// phase to phase are short vectors of {value, flag} words in global memory (flag_words.cuh):
 //   * every CTA keeps the residual stream (d_model floats per sequence) in its own shared memory and updates it redundantly, so
 //     the LayerNorms need no exchange at all,
 //   * a projection is a set of items (output row, K chunk of 768) dealt round-robin to all warps of the grid;
@@ -16,18 +16,24 @@
 //     a multiple of the four chunks, so a CTA meets one chunk of the MLP hidden only,
 //   * attention: CTA (sequence, head, context chunk) computes scores, a local softmax and a partial (max, sum, context) over its
 //     slice of the cache; the CTA whose slice holds the new position takes K/V of the token from the qkv vector and stores
-//     them into the cache; every CTA merges the partials of all heads when it stages the input of the out projection.
-// 5 barriers per layer + 1. Every barrier wait is bounded (a CTA that gives up records status 5 and goes on).
+//     them into the cache; the CTA of the first chunk adds the others' parts,
+//   * a context is cut into chunks of 64 keys and more: a short one leaves nothing to merge,
+//   * every phase of every layer goes through one copy of the code: with a copy per projection (103 KB at one row, 201 KB at eight) the phases
+//     ran from a cold instruction cache.
+// A buffer is written again a layer later: a CTA that gets that far has consumed outputs of all CTAs (every phase's vector has items of every
+// CTA), and these were computed after their readings. With grid barriers in place of the words, partials of 12 chunks merged by every CTA and a
+// copy of the code per projection a token took 326 us (one sequence), 517 (six sequences); now 262 and 374: a phase's exchange is 2.5 to 3.7 us, of
+// which the round trips alone are 1.3, its projection 0.7 to 1.4, the head 20. Every wait is bounded (a thread that gives up records status 5 and goes on).
+#include <algorithm>
+
+#include "flag_words.cuh"
 #include "gpt_decode_mega.h"
 
 namespace gptrs {
 namespace {
 
 constexpr int kMegaThreads = 256, kMegaWarps = kMegaThreads / 32;
-constexpr uint32_t kMegaSpin = 1u << 24;
 constexpr int kD = 768, kMlp = 3072;   // the widths it is built for (mega_supported)
-
-struct BarrierState { unsigned* ctr; unsigned target; unsigned step; int* status; unsigned long long* timing; int n; };
 
 __device__ __forceinline__ float4 ldg_stream_f4(const float4* p) {
     float4 v;
@@ -40,35 +46,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
     return t;
 }
-// A grid barrier in two halves, so that the loads of the next projection's weights can be issued BETWEEN them: issued
-// before the arrival they would sit in front of its fence (a fence waits for the thread's outstanding loads too: the
-// prefetch would delay every arrival by a DRAM round trip), issued after the wait they would hide nothing.
-__device__ __forceinline__ void grid_arrive(BarrierState& b) {
-    b.target += b.step;
-    __syncthreads();
-    if (b.timing && blockIdx.x == 0 && threadIdx.x == 0) b.timing[b.n++] = global_ns();   // arrival of CTA 0
-    if (threadIdx.x == 0) {
-        __threadfence();
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(b.ctr) : "memory");
-    }
-}
-__device__ __forceinline__ void grid_wait(BarrierState& b) {
-    if (threadIdx.x == 0) {
-        unsigned v = 0;
-        uint32_t it = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(b.ctr) : "memory");
-        } while (v < b.target && ++it < kMegaSpin);
-        if (v < b.target) atomicExch(b.status, 5);
-        if (b.timing && blockIdx.x == 0) b.timing[b.n++] = global_ns();   // release of CTA 0
-    }
-    __syncthreads();
-}
-__device__ __forceinline__ void grid_barrier(BarrierState& b) {
-    grid_arrive(b);
-    grid_wait(b);
-}
-
 __device__ __forceinline__ float block_sum(float v, float* red) {
     v = warp_sum(v);
     __syncthreads();   // red may still be read from the previous use
@@ -80,33 +57,60 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return t;
 }
 
-// h += bias + the PARTS partial sums per element that other CTAs left (PARTS 0: h is complete), xn = LayerNorm(h) * gamma + beta, for R
+// h += bias + the PARTS partial sums per element that other CTAs left (part null: h is complete), xn = LayerNorm(h) * gamma + beta, for R
 // rows at once: 8 / R warps per row, the row in registers between the two sums.
 template <int R, int PARTS>
-__device__ __forceinline__ void residual_norm(float* h, float* xn, const float* part, const float* __restrict__ bias, const float* __restrict__ gamma,
-                                              const float* __restrict__ beta, float eps, float* red) {
+__device__ __forceinline__ void residual_norm(float* h, float* xn, const unsigned char* part, uint32_t flag, FlagWaiter& wait, int rows,
+                                              const float* __restrict__ bias, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
+                                              float* red) {
     constexpr int W = kMegaWarps / R, N = kD / (32 * W);
     const int warp = threadIdx.x >> 5, row = warp / W, first = threadIdx.x - row * W * 32;
-    constexpr int G = N < 6 ? N : 6;   // loads under way at once: the next projection's weights already hold 96 registers
+    constexpr int G = N < 12 / PARTS * 2 ? N : 12 / PARTS * 2;   // elements under way at once: the next projection's weights already hold 96 registers
+    static_assert(N % G == 0, "whole groups");
     float v[N];
+    const unsigned char* const own = part + (size_t)(row * kD + first) * (8 * PARTS);
+    const bool adds = part && row < rows;
+    if (R > 1 && adds) {   // (one row: a warp's whole request is three of these)
+        if ((threadIdx.x & 31) == 0) wait.wait_word(own, flag);
+        __syncwarp();
+    }
 #pragma unroll
     for (int j0 = 0; j0 < N; j0 += G) {
+#pragma unroll
+        for (int j = 0; j < G; ++j) v[j0 + j] = 0.f;
+        if (!adds) continue;
+        bool found;
         if constexpr (PARTS == 4) {
-            float4 p4[G];
+            FlagWords p[G][2];
+#pragma unroll 1
+            do {
+                found = true;
 #pragma unroll
-            for (int j = 0; j < G; ++j) p4[j] = __ldcg(reinterpret_cast<const float4*>(part) + row * kD + first + (j0 + j) * W * 32);
+                for (int j = 0; j < G; ++j) { p[j][0] = peek_words(own + (j0 + j) * W * 1024); p[j][1] = peek_words(own + (j0 + j) * W * 1024 + 16); }
 #pragma unroll
-            for (int j = 0; j < G; ++j) v[j0 + j] = (p4[j].x + p4[j].y) + (p4[j].z + p4[j].w);
-        } else if constexpr (PARTS == 1) {
+                for (int j = 0; j < G; ++j) found = found && has_flag(p[j][0], flag) && has_flag(p[j][1], flag);
+            } while (!found && wait.again());
 #pragma unroll
-            for (int j = 0; j < G; ++j) v[j0 + j] = __ldcg(part + row * kD + first + (j0 + j) * W * 32);
+            for (int j = 0; j < G; ++j) v[j0 + j] = (word_f32(p[j][0].a) + word_f32(p[j][0].b)) + (word_f32(p[j][1].a) + word_f32(p[j][1].b));
+        } else {
+            uint64_t p[G];
+#pragma unroll 1
+            do {
+                found = true;
+#pragma unroll
+                for (int j = 0; j < G; ++j) p[j] = peek_word(own + (j0 + j) * W * 256);
+#pragma unroll
+                for (int j = 0; j < G; ++j) found = found && has_flag(p[j], flag);
+            } while (!found && wait.again());
+#pragma unroll
+            for (int j = 0; j < G; ++j) v[j0 + j] = word_f32(p[j]);
         }
     }
     float s = 0.f;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
         const int i = first + j * W * 32;
-        v[j] = PARTS ? h[row * kD + i] + (bias[i] + v[j]) : h[row * kD + i];
+        v[j] = part ? h[row * kD + i] + (bias[i] + v[j]) : h[row * kD + i];
         s += v[j];
     }
     auto row_sum = [&](float t, float* at) {
@@ -158,9 +162,9 @@ __device__ __forceinline__ float row_sums(float (&v)[R], int lane) {
 }
 
 // Items (row, chunk of 768) of y = Wt . x dealt to the warps of the whole grid, U at a time per warp. The raw dot products
-// of sequence s go to out[s][row * n_chunks + chunk]; biases are applied by whoever reads them (kGelu: bias and GELU here). The loads of a warp's FIRST
-// round are a call of their own (gemv_prefetch), made BEFORE the grid barrier in front of the phase: the weights do not
-// depend on what the barrier waits for, so their DRAM latency hides behind it. With kBest, the lanes that store also keep the largest
+// of sequence s go to word out[s][row * n_chunks + chunk], or to the logits; biases are applied by whoever reads them (gelu_bias: bias and GELU here). The loads of a
+// warp's FIRST round are a call of their own (gemv_prefetch), made BEFORE the waits of the phase: the weights do not
+// depend on what those wait for, so their DRAM latency hides behind them. With logits, the lanes that store also keep the largest
 // value of their sequence that they have produced (ties: the smaller row).
 constexpr int kF4 = 6;   // float4 per lane per item
 constexpr int kU = 4;    // items in flight per warp
@@ -175,14 +179,13 @@ __device__ __forceinline__ void gemv_load(Round& r, const float* __restrict__ Wt
         for (int j = 0; j < kF4; ++j) r.w[u][j] = ldg_stream_f4(src + 32 * j);
     }
 }
-__device__ __forceinline__ void gemv_prefetch(Round& r, const float* __restrict__ Wt, int n_rows, int K) {
+__device__ __forceinline__ void gemv_prefetch(Round& r, const float* __restrict__ Wt, int n_items) {
     const int total = gridDim.x * kMegaWarps, gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const int n_items = n_rows * (K / (kF4 * 128));
     if (gw < n_items) gemv_load(r, Wt, n_items, gw, total, threadIdx.x & 31);
 }
-template <int R, bool kBest, bool kGelu = false>
-__device__ __forceinline__ void gemv_items(Round& r, const float* __restrict__ Wt, int n_items, const float* xs, float* __restrict__ out, int rows,
-                                           float& best, int& best_i, const float* __restrict__ bias = nullptr) {
+template <int R>
+__device__ __forceinline__ void gemv_items(Round& r, const float* __restrict__ Wt, int n_items, const float* xs, unsigned char* __restrict__ out, uint32_t flag,
+                                           float* __restrict__ logits, int rows, float& best, int& best_i, const float* __restrict__ gelu_bias) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int total = gridDim.x * kMegaWarps, gw = warp * gridDim.x + blockIdx.x;
     const int seq = lane / (32 / R);
@@ -206,36 +209,26 @@ __device__ __forceinline__ void gemv_items(Round& r, const float* __restrict__ W
                 }
             }
         }
+        float sum[kU];
 #pragma unroll
+        for (int u = 0; u < kU; ++u) sum[u] = row_sums<R>(acc[u], lane);
+#pragma unroll 1
         for (int u = 0; u < kU; ++u) {
             const int item = item0 + u * total;
-            float v = row_sums<R>(acc[u], lane);
+            float v = u == 0 ? sum[0] : u == 1 ? sum[1] : u == 2 ? sum[2] : sum[3];
             if (stores && item < n_items) {
-                if constexpr (kGelu) {
-                    v += bias[item];
+                if (gelu_bias) {
+                    v += gelu_bias[item];
                     v = (0.5f * v) * (1.f + erff(v / 1.4142135f));
                 }
-                out[(size_t)seq * n_items + item] = v;
-                if (kBest && (v > best || (v == best && item < best_i))) { best = v; best_i = item; }
+                if (!logits) {
+                    put_word(out + ((size_t)seq * n_items + item) * 8, __float_as_uint(v), flag);
+                } else {
+                    logits[(size_t)seq * n_items + item] = v;
+                    if (v > best || (v == best && item < best_i)) { best = v; best_i = item; }
+                }
             }
         }
-    }
-}
-
-// n4 float4 written by other CTAs -> shared memory, read past L1, with every load of a thread in flight at once (a loop the
-// compiler unrolls by four waits for DRAM / L2 once per four elements: nine round trips for the attention partials).
-template <int kPer>
-__device__ __forceinline__ void stage_f4(float* dst, const float* src, int n4) {
-    float4 v[kPer];
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        const int i = threadIdx.x + j * kMegaThreads;
-        if (i < n4) v[j] = __ldcg(reinterpret_cast<const float4*>(src) + i);
-    }
-#pragma unroll
-    for (int j = 0; j < kPer; ++j) {
-        const int i = threadIdx.x + j * kMegaThreads;
-        if (i < n4) reinterpret_cast<float4*>(dst)[i] = v[j];
     }
 }
 
@@ -249,6 +242,9 @@ __host__ __device__ inline int mega_scores(int grid, int rows, int heads, int ct
     return (ctx_cap + n - 1) / n;
 }
 
+// Chunks that the context of a sequence of `len` is cut into: 64 keys are one pass of a CTA, so a short context leaves few partial results to merge.
+__device__ __forceinline__ int mega_live_chunks(int len, int n_chunks) { return max(1, min(n_chunks, (len + 63) >> 6)); }
+
 // R: rows that the arithmetic is laid out for; p.rows of them are sequences.
 template <int R>
 __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const MegaParams p) {
@@ -259,12 +255,15 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
     float* red = big + p.big_floats;   // [64]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rows = p.rows;
     const int H = p.H, hd = p.hd;
-    BarrierState bar = {p.barrier, 0u, gridDim.x, p.status, p.timing, 0};
-    if (p.timing && blockIdx.x == 0 && threadIdx.x == 0) p.timing[bar.n++] = global_ns();
+    FlagWaiter wait = {kFlagPolls, p.status};
+    int n_time = 0;
+    auto stamp = [&]() { if (p.timing && blockIdx.x == 0 && tid == 0) p.timing[n_time++] = global_ns(); };
+    stamp();
     float best = -INFINITY;   // lm_head: the largest logit this lane has produced
     int best_i = 0x7fffffff;
     Round rnd;                // the weights of this warp's first items of the next projection
-    gemv_prefetch(rnd, p.layers[0].w_qkv_t, 3 * kD, kD);
+    gemv_prefetch(rnd, p.layers[0].w_qkv_t, 3 * kD);
+    uint32_t flag = p.epoch;   // of the layer; every phase's vector has a buffer of its own
 
     for (int s = 0; s < R; ++s) {
         const int token = s < rows ? p.token[s] : 0;
@@ -280,152 +279,176 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
     const bool attends = (int)blockIdx.x < n_tasks;
     const int seq = attends ? blockIdx.x / (H * n_chunks) : 0, head = (blockIdx.x / n_chunks) % H, ck = blockIdx.x % n_chunks;
     const int pos = min(max(p.pos[seq], 0), p.ctx_cap - 1), len = pos + 1;
-    const int chunk_len = (len + n_chunks - 1) / n_chunks, j0 = ck * chunk_len, j1 = min(len, j0 + chunk_len);
+    const int live = mega_live_chunks(len, n_chunks);
+    const int chunk_len = (len + live - 1) / live, j0 = min(len, ck * chunk_len), j1 = min(len, j0 + chunk_len);
     const size_t cache_at = ((size_t)p.slot[seq] * H + head) * p.ctx_cap * hd;
     const float scale = 1.0f / sqrtf((float)hd);
-    const int part_stride = hd + 2;
+    const int part_stride = (hd + 4) * 8;   // context, maximum, sum
 
 #pragma unroll 1
-    for (int l = 0; l < p.n_layers; ++l) {
-        const MegaLayer& L = p.layers[l];   // the table is part of the kernel parameters: no pointer chase through memory
-        // ---- residual update from the previous block's MLP (four partial sums), ln_1, qkv --------------------------
-        if (l > 0) residual_norm<R, 4>(h, xn, p.pe, p.layers[l - 1].b_mlp_out, L.ln1_g, L.ln1_b, p.eps, red);
-        else residual_norm<R, 0>(h, xn, nullptr, nullptr, L.ln1_g, L.ln1_b, p.eps, red);
-        gemv_items<R, false>(rnd, L.w_qkv_t, 3 * kD, xn, p.qkv, rows, best, best_i);
-        grid_arrive(bar);
-        gemv_prefetch(rnd, L.w_out_t, kD, kD);   // kept across the attention phase
-        grid_wait(bar);
-        // ---- attention: CTA = (sequence, head, context chunk) ---------------------------------------------------------
-        if (attends) {
-            float* kc = L.k_cache + cache_at;
-            float* vc = L.v_cache + cache_at;
-            // q, and K / V of the new token, from the qkv vector the other CTAs wrote (read past L1)
-            float* qs = xn;            // [hd]
-            float* k_new = xn + hd;    // [hd]
-            float* v_new = xn + 2 * hd;
-            const float* qkv = p.qkv + (size_t)seq * 3 * kD + head * hd;
-            for (int c = tid; c < 3 * hd; c += kMegaThreads) {
-                const int which = c / hd, e = c - which * hd;
-                xn[c] = __ldcg(qkv + which * kD + e) + L.b_qkv[which * kD + head * hd + e];
-            }
-            __syncthreads();
-            float* sc = big;   // scores of this slice
-            if (j0 <= pos && pos < j1)   // the new token's row goes into the cache for the steps to come
-                for (int c = tid; c < hd; c += kMegaThreads) { kc[(size_t)pos * hd + c] = k_new[c]; vc[(size_t)pos * hd + c] = v_new[c]; }
-            // scores: hd / 4 lanes per key, four times 128 / hd keys of a warp under way at once
-            {
-                const int lanes = hd >> 2, per = 32 / lanes, sub = lane / lanes, c4 = (lane - sub * lanes) * 4;
-                const float4 q4 = *reinterpret_cast<const float4*>(qs + c4);
-                for (int base = j0 + warp * per; base < j1; base += 4 * kMegaWarps * per) {
-                    float4 k4[4];
+    for (int phase = 0;; ++phase) {
+        // phases of a layer: qkv, out projection (attention in front of it), MLP in, MLP out; after the last layer the head
+        const int l = phase >> 2, kind = phase & 3;
+        const bool at_head = l == p.n_layers;
+        const MegaLayer& L = p.layers[at_head ? l - 1 : l];   // the table is part of the kernel parameters: no pointer chase through memory
+        const float* xs = xn;
+        if (kind == 0) ++flag;
+        if (kind == 0) {
+            // residual update from the previous block's MLP (four partial sums), ln_1 or the final LayerNorm
+            residual_norm<R, 4>(h, xn, l > 0 ? p.pe : nullptr, flag - 1, wait, rows, l > 0 ? p.layers[l - 1].b_mlp_out : nullptr, at_head ? p.lnf_g : L.ln1_g, at_head ? p.lnf_b : L.ln1_b,
+                                p.eps, red);
+        } else if (kind == 1) {
+            // ---- attention: CTA = (sequence, head, context chunk) ---------------------------------------------------------
+            if (attends && ck < live) {
+                float* kc = L.k_cache + cache_at;
+                float* vc = L.v_cache + cache_at;
+                // q, and K / V of the new token, from the qkv vector the other CTAs write
+                float* qs = xn;            // [hd]
+                float* k_new = xn + hd;    // [hd]
+                float* v_new = xn + 2 * hd;
+                const unsigned char* qkv = p.qkv + (size_t)(seq * 3 * kD + head * hd) * 8;
+#pragma unroll 1
+                for (int c = tid; c < 3 * hd; c += kMegaThreads) {
+                    const int which = c / hd, e = c - which * hd;
+                    const float bias = L.b_qkv[which * kD + head * hd + e];
+                    xn[c] = __uint_as_float(wait.wait_word(qkv + (which * kD + e) * 8, flag)) + bias;
+                }
+                __syncthreads();
+                float* sc = big;   // scores of this slice
+                if (j0 <= pos && pos < j1)   // the new token's row goes into the cache for the steps to come
+                    for (int c = tid; c < hd; c += kMegaThreads) { kc[(size_t)pos * hd + c] = k_new[c]; vc[(size_t)pos * hd + c] = v_new[c]; }
+                // scores: hd / 4 lanes per key, four times 128 / hd keys of a warp under way at once
+                {
+                    const int lanes = hd >> 2, per = 32 / lanes, sub = lane / lanes, c4 = (lane - sub * lanes) * 4;
+                    const float4 q4 = *reinterpret_cast<const float4*>(qs + c4);
+#pragma unroll 1
+                    for (int base = j0 + warp * per; base < j1; base += 4 * kMegaWarps * per) {
+                        float4 k4[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int j = base + u * kMegaWarps * per + sub;
-                        k4[u] = j >= j1 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>((j == pos ? k_new : kc + (size_t)j * hd) + c4);
-                    }
+                        for (int u = 0; u < 4; ++u) {
+                            const int j = base + u * kMegaWarps * per + sub;
+                            k4[u] = j >= j1 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>((j == pos ? k_new : kc + (size_t)j * hd) + c4);
+                        }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int j = base + u * kMegaWarps * per + sub;
-                        float t = fmaf(q4.w, k4[u].w, fmaf(q4.z, k4[u].z, fmaf(q4.y, k4[u].y, q4.x * k4[u].x)));
-                        for (int o = lanes >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-                        if (c4 == 0 && j < j1) sc[j - j0] = t * scale;
+                        for (int u = 0; u < 4; ++u) {
+                            const int j = base + u * kMegaWarps * per + sub;
+                            float t = fmaf(q4.w, k4[u].w, fmaf(q4.z, k4[u].z, fmaf(q4.y, k4[u].y, q4.x * k4[u].x)));
+#pragma unroll 1
+                            for (int o = lanes >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                            if (c4 == 0 && j < j1) sc[j - j0] = t * scale;
+                        }
                     }
                 }
-            }
-            __syncthreads();
-            float mx = -INFINITY;
-            for (int j = tid; j < j1 - j0; j += kMegaThreads) mx = fmaxf(mx, sc[j]);
-            mx = warp_max(mx);
-            if (lane == 0) red[32 + warp] = mx;
-            __syncthreads();
-            mx = red[32];
+                __syncthreads();
+                float mx = -INFINITY;
+#pragma unroll 1
+                for (int j = tid; j < j1 - j0; j += kMegaThreads) mx = fmaxf(mx, sc[j]);
+                mx = warp_max(mx);
+                if (lane == 0) red[32 + warp] = mx;
+                __syncthreads();
+                mx = red[32];
 #pragma unroll
-            for (int w = 1; w < kMegaWarps; ++w) mx = fmaxf(mx, red[32 + w]);
-            float sum = 0.f;
-            for (int j = tid; j < j1 - j0; j += kMegaThreads) {
-                const float e = expf(sc[j] - mx);
-                sc[j] = e;
-                sum += e;
-            }
-            sum = block_sum(sum, red);
-            // context: thread (part, c) walks positions part, part + parts, ...
-            const int parts = kMegaThreads / hd;
-            const int c = tid % hd, part = tid / hd;
-            float acc = 0.f;
+                for (int w = 1; w < kMegaWarps; ++w) mx = fmaxf(mx, red[32 + w]);
+                float sum = 0.f;
+#pragma unroll 1
+                for (int j = tid; j < j1 - j0; j += kMegaThreads) {
+                    const float e = expf(sc[j] - mx);
+                    sc[j] = e;
+                    sum += e;
+                }
+                sum = block_sum(sum, red);
+                // context: thread (part, c) walks positions part, part + parts, ...
+                const int parts = kMegaThreads / hd;
+                const int c = tid % hd, part = tid / hd;
+                float acc = 0.f;
 #pragma unroll 8
-            for (int j = j0 + part; j < j1; j += parts) acc = fmaf(sc[j - j0], (j == pos ? v_new : vc + (size_t)j * hd)[c], acc);
-            float* comb = red + 64;   // [parts][hd], where the partials of all heads are staged later
-            comb[part * hd + c] = acc;
-            __syncthreads();
-            float* out = p.att_part + (size_t)blockIdx.x * part_stride;
-            if (tid < hd) {
-                float v = 0.f;
-                for (int q2 = 0; q2 < parts; ++q2) v += comb[q2 * hd + tid];
-                out[2 + tid] = v;
-            }
-            if (tid == 0) { out[0] = j1 > j0 ? mx : -INFINITY; out[1] = j1 > j0 ? sum : 0.f; }
-        }
-        grid_barrier(bar);
-        // ---- merge the attention partials (every CTA, all heads), out projection --------------------------------------
-        {
-            // all partials -> shared memory with independent loads (a dependent chain of L2 round trips per element cost
-            // 7 us here), then the merge from shared memory
-            float* parts_s = red + 64;   // [rows * H * n_chunks][hd + 2]
-            const int n_part = n_tasks * part_stride;
-            for (int base = 0; base < n_part / 4; base += 12 * kMegaThreads)   // one pass for GPT-2's 12 x 12 x 66 floats
-                stage_f4<12>(parts_s + 4 * base, p.att_part + 4 * base, n_part / 4 - base);
-            for (int i = (n_part / 4) * 4 + tid; i < n_part; i += kMegaThreads) parts_s[i] = __ldcg(p.att_part + i);
-            __syncthreads();
-            for (int i = tid; i < rows * kD; i += kMegaThreads) {
-                const int unit = i / hd, c = i - unit * hd;   // sequence * H + head
-                const float* part = parts_s + unit * n_chunks * part_stride;
-                float M = -INFINITY;
-                for (int k = 0; k < n_chunks; ++k) M = fmaxf(M, part[k * part_stride]);
-                float Ls = 0.f, O = 0.f;
-                for (int k = 0; k < n_chunks; ++k) {
-                    const float m_k = part[k * part_stride];
-                    if (m_k == -INFINITY) continue;
-                    const float wgt = expf(m_k - M);
-                    Ls = fmaf(part[k * part_stride + 1], wgt, Ls);
-                    O = fmaf(part[k * part_stride + 2 + c], wgt, O);
-                }
-                xn[i] = O / Ls;
-            }
-            __syncthreads();
-        }
-        gemv_items<R, false>(rnd, L.w_out_t, kD, xn, p.pc, rows, best, best_i);
-        grid_arrive(bar);
-        gemv_prefetch(rnd, L.w_mlp_in_t, kMlp, kD);
-        grid_wait(bar);
-        // ---- residual update, ln_2, MLP in + GELU ---------------------------------------------------------------------
-        residual_norm<R, 1>(h, xn, p.pc, L.b_out, L.ln2_g, L.ln2_b, p.eps, red);
-        gemv_items<R, false, true>(rnd, L.w_mlp_in_t, kMlp, xn, p.mh, rows, best, best_i, L.b_mlp_in);
-        grid_arrive(bar);
-        gemv_prefetch(rnd, L.w_mlp_out_t, kD, kMlp);
-        grid_wait(bar);
-        // ---- MLP out: partial sums per 768-k chunk; a CTA's items all lie in chunk blockIdx % 4 --------------------------
-        {
-            constexpr int N = (R * kD / 4 + kMegaThreads - 1) / kMegaThreads;
-            float4 v[N];
+                for (int j = j0 + part; j < j1; j += parts) acc = fmaf(sc[j - j0], (j == pos ? v_new : vc + (size_t)j * hd)[c], acc);
+                float* comb = red + 64;   // [parts][hd]
+                comb[part * hd + c] = acc;
+                __syncthreads();
+                float m_all = j1 > j0 ? mx : -INFINITY, l_all = j1 > j0 ? sum : 0.f;
+                unsigned char* out = p.att_part + (size_t)blockIdx.x * part_stride;
+                if (tid < hd) {
+                    float v = 0.f;
+#pragma unroll 2
+                    for (int q2 = 0; q2 < parts; ++q2) v += comb[q2 * hd + tid];
+                    if (ck > 0) {
+                        put_word(out + tid * 8, __float_as_uint(v), flag);
+                        if (tid == 0) put_words(out + hd * 8, __float_as_uint(m_all), __float_as_uint(l_all), flag);
+                    } else {   // the first chunk's CTA adds the others' parts, in order
+#pragma unroll 1
+                        for (int k0 = 1; k0 < live; k0 += 4) {
+                            uint64_t o[4];
+                            FlagWords ms[4];
+                            bool found;
+#pragma unroll 1
+                            do {
+                                found = true;
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
-                const int i = tid + j * kMegaThreads, s = i / (kD / 4), e = i - s * (kD / 4);
-                if (i < R * kD / 4) v[j] = __ldcg(reinterpret_cast<const float4*>(p.mh + (size_t)s * kMlp + (blockIdx.x & 3) * kD) + e);
+                                for (int k = 0; k < 4; ++k) {   // past the end: the last one once more
+                                    const unsigned char* from = out + (size_t)min(k0 + k, live - 1) * part_stride;
+                                    o[k] = peek_word(from + tid * 8);
+                                    ms[k] = peek_words(from + hd * 8);
+                                }
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) found = found && has_flag(o[k], flag) && has_flag(ms[k], flag);
+                            } while (!found && wait.again());
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                const float mk = word_f32(ms[k].a);
+                                if (k0 + k >= live || mk == -INFINITY) continue;
+                                const float top = fmaxf(m_all, mk), fa = m_all == -INFINITY ? 0.f : expf(m_all - top), fb = expf(mk - top);
+                                l_all = fmaf(word_f32(ms[k].b), fb, l_all * fa);
+                                v = fmaf(word_f32(o[k]), fb, v * fa);
+                                m_all = top;
+                            }
+                        }
+                        put_word(p.att + (size_t)(seq * kD + head * hd + tid) * 8, __float_as_uint(v / l_all), flag);
+                    }
+                }
+                __syncthreads();   // scores, comb and the token's vectors have been read
             }
+            stamp();
+        } else if (kind == 2) {
+            residual_norm<R, 1>(h, xn, p.pc, flag, wait, rows, L.b_out, L.ln2_g, L.ln2_b, p.eps, red);
+        }
+        if (kind & 1) {   // the attention output, or the 768 values of the MLP hidden that this CTA's items of the last projection need
+            constexpr int N = (R * kD / 2 + kMegaThreads - 1) / kMegaThreads;
+            const int n2 = rows * (kD / 2);   // pairs of words
+            auto word_at = [&](int i) {
+                const int s2 = i / (kD / 2), e = i - s2 * (kD / 2);
+                return kind == 1 ? p.att + (size_t)i * 16 : p.mh + ((size_t)s2 * kMlp + (blockIdx.x & 3) * kD) * 8 + e * 16;
+            };
+            if (lane == 0 && tid < n2) wait.wait_word(word_at(tid), flag);
+            __syncwarp();
+            FlagWords v[N];
+            bool found;
+#pragma unroll 1
+            do {   // past the end: the last pair once more
+                found = true;
+#pragma unroll
+                for (int j = 0; j < N; ++j) v[j] = peek_words(word_at(min(tid + j * kMegaThreads, n2 - 1)));
+#pragma unroll
+                for (int j = 0; j < N; ++j) found = found && has_flag(v[j], flag);
+            } while (!found && wait.again());
 #pragma unroll
             for (int j = 0; j < N; ++j)
-                if (tid + j * kMegaThreads < R * kD / 4) reinterpret_cast<float4*>(big)[tid + j * kMegaThreads] = v[j];
+                if (tid + j * kMegaThreads < n2) reinterpret_cast<float2*>(big)[tid + j * kMegaThreads] = make_float2(word_f32(v[j].a), word_f32(v[j].b));
             __syncthreads();
+            xs = big;
         }
-        gemv_items<R, false>(rnd, L.w_mlp_out_t, kMlp, big, p.pe, rows, best, best_i);
-        grid_arrive(bar);
-        if (l + 1 < p.n_layers) gemv_prefetch(rnd, p.layers[l + 1].w_qkv_t, 3 * kD, kD);
-        else gemv_prefetch(rnd, p.lm_head_t, p.vocab, kD);
-        grid_wait(bar);
+        const float* w = at_head ? p.lm_head_t : kind == 0 ? L.w_qkv_t : kind == 1 ? L.w_out_t : kind == 2 ? L.w_mlp_in_t : L.w_mlp_out_t;
+        const int n_items = at_head ? p.vocab : kind == 0 ? 3 * kD : kind == 1 ? kD : kMlp;   // MLP out: four chunks of 768 rows
+        stamp();
+        gemv_items<R>(rnd, w, n_items, xs, kind == 0 ? p.qkv : kind == 1 ? p.pc : kind == 2 ? p.mh : p.pe, flag, at_head ? p.logits : nullptr, rows, best, best_i,
+                      kind == 2 ? L.b_mlp_in : nullptr);
+        stamp();
+        if (at_head) break;
+        __syncthreads();   // xn and big have been read
+        const float* next = kind == 0 ? L.w_out_t : kind == 1 ? L.w_mlp_in_t : kind == 2 ? L.w_mlp_out_t : l + 1 < p.n_layers ? p.layers[l + 1].w_qkv_t : p.lm_head_t;
+        gemv_prefetch(rnd, next, kind == 0 ? kD : kind < 3 ? kMlp : l + 1 < p.n_layers ? 3 * kD : p.vocab);   // of the out projection: kept across attention
     }
-    // ---- last residual update, final LayerNorm, lm_head, greedy pick ----------------------------------------------------
-    residual_norm<R, 4>(h, xn, p.pe, p.layers[p.n_layers - 1].b_mlp_out, p.lnf_g, p.lnf_b, p.eps, red);
-    gemv_items<R, true>(rnd, p.lm_head_t, p.vocab, xn, p.logits, rows, best, best_i);
+    // ---- the greedy pick ------------------------------------------------------------------------------------------------
     // the storing lanes hold their warp's best of a sequence; CTA best -> cand[sequence][blockIdx.x]
     float* bv = big;                                        // [warp][R]
     int* bi = reinterpret_cast<int*>(big + kMegaWarps * R);
@@ -435,16 +458,16 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
     if (tid < rows) {
         for (int w = 1; w < kMegaWarps; ++w)
             if (bv[w * R + tid] > bv[tid] || (bv[w * R + tid] == bv[tid] && bi[w * R + tid] < bi[tid])) { bv[tid] = bv[w * R + tid]; bi[tid] = bi[w * R + tid]; }
-        p.cand_val[tid * gridDim.x + blockIdx.x] = bv[tid];
-        p.cand_idx[tid * gridDim.x + blockIdx.x] = bi[tid];
+        put_words(p.cand + (size_t)(tid * gridDim.x + blockIdx.x) * 16, __float_as_uint(bv[tid]), (uint32_t)bi[tid], flag);
     }
-    grid_barrier(bar);
     if (blockIdx.x == 0 && warp < rows) {
         float v = -INFINITY;
         int ix = 0x7fffffff;
+#pragma unroll 1
         for (int k = lane; k < (int)gridDim.x; k += 32) {
-            const float cv = __ldcg(p.cand_val + warp * gridDim.x + k);
-            const int ci = __ldcg(p.cand_idx + warp * gridDim.x + k);
+            const FlagWords w = wait.wait_words(p.cand + (size_t)(warp * gridDim.x + k) * 16, flag);
+            const float cv = word_f32(w.a);
+            const int ci = (int)(uint32_t)w.b;
             if (cv > v || (cv == v && ci < ix)) { v = cv; ix = ci; }
         }
 #pragma unroll
@@ -494,7 +517,8 @@ size_t mega_big_floats(int layout, int rows, int H, int ctx_cap) {
     return scores > hidden ? scores : hidden;
 }
 size_t mega_smem_bytes(int layout, int rows, int H, int hd, int ctx_cap) {
-    return (2 * (size_t)layout * kD + mega_big_floats(layout, rows, H, ctx_cap) + 64 + (size_t)sm_count() * (hd + 2) + 64) * sizeof(float);
+    (void)hd;
+    return (2 * (size_t)layout * kD + mega_big_floats(layout, rows, H, ctx_cap) + 64 + std::max(kMegaThreads, 2 * sm_count()) + 64) * sizeof(float);
 }
 int mega_layout(int rows) { return rows <= 1 ? 1 : rows <= 2 ? 2 : rows <= 4 ? 4 : 8; }
 constexpr size_t kMegaSmem = 227 * 1024;
@@ -511,7 +535,6 @@ int mega_launch(MegaParams p, cudaStream_t st) {
     static PerDeviceOnce attr_once;
     if (attr_once.first_time())
         for (auto k : kerns) GPTRS_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMegaSmem));
-    GPTRS_CUDA_OK(cudaMemsetAsync(p.barrier, 0, sizeof(unsigned), st));
     const int layout = mega_layout(p.rows);
     p.big_floats = (int)mega_big_floats(layout, p.rows, p.H, p.ctx_cap);
     cudaLaunchConfig_t cfg = {};
@@ -520,7 +543,7 @@ int mega_launch(MegaParams p, cudaStream_t st) {
     cfg.dynamicSmemBytes = mega_smem_bytes(layout, p.rows, p.H, p.hd, p.ctx_cap);
     cfg.stream = st;
     cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeCooperative;   // all CTAs co-resident: they meet at grid-wide barriers
+    attr.id = cudaLaunchAttributeCooperative;   // all CTAs co-resident: they wait for each other's words
     attr.val.cooperative = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;

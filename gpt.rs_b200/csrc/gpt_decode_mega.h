@@ -18,11 +18,12 @@ struct MegaParams {
     const float *tok_emb, *pos_emb, *lnf_g, *lnf_b, *lm_head_t;
     int rows;                        // sequences of the step
     const int *token, *pos, *slot;   // [rows]; the slots are distinct
-    float *qkv, *att_part, *pc, *mh, *pe, *logits, *cand_val;   // vectors of kMegaMaxRows rows, partials per CTA, logits [rows][vocab]
-    int *cand_idx, *sampled;
-    unsigned* barrier;
+    unsigned char *qkv, *att_part, *att, *pc, *mh, *pe, *cand;   // {value, flag} words: vectors of kMegaMaxRows rows, partials and candidates per CTA
+    uint32_t epoch;                  // flags of this step are epoch + 1 ... epoch + n_layers + 1
+    float* logits;                   // [rows][vocab]
+    int* sampled;
     int* status;
-    unsigned long long* timing;   // optional (GPTRS_MEGA_TIMING=1): globaltimer of CTA 0 at kernel start and around every barrier
+    unsigned long long* timing;   // optional (GPTRS_MEGA_TIMING=1): globaltimer of CTA 0 at kernel start, where its part in attention has ended, and around every projection
     int H, hd, vocab, ctx_cap, n_pos;
     int big_floats;                  // set by the launcher
     float eps;
