@@ -82,12 +82,13 @@ __device__ __forceinline__ int swz(int tok, int chunk) { return tok * 256 + ((ch
 // kStep (decode steps of few rows): the kernel also does what stands around it. Queries are rotated as they are loaded; the CTA with
 // the last page rotates the new key, stores key and value into the pool and into its copy of the page; the splits of a row and kv head
 // are a cluster (grid.y) that merges through distributed shared memory. Two launches less per layer, 3.7 and 4.8 us at one row.
-template <int kDepth, bool kMulti, bool kStep = false>
+// kMerge alone: rotated queries and a complete cache, the splits merged by their cluster (one launch and no scratch instead of two with it).
+template <int kDepth, bool kMulti, bool kStep = false, bool kMerge = kStep>
 __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_attention_kernel(const AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full_bar[kAttnWarps][kDepth];
 
-    const int split = kStep ? blockIdx.y : blockIdx.x, h = kStep ? blockIdx.x : blockIdx.y;
+    const int split = kMerge ? blockIdx.y : blockIdx.x, h = kMerge ? blockIdx.x : blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int group = p.Hq / p.Hkv;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
     else split_geometry(len, p.chunk_pages, &n_splits, &split_pages);  // rows of a prefill group keep one fixed grid
     const int chunk_tokens = split_pages * kPageTokens;
     const int first_tok = split * chunk_tokens;
-    if (!kStep && first_tok >= len) return;  // whole CTA leaves together, before any barrier
+    if (!kMerge && first_tok >= len) return;  // whole CTA leaves together, before any barrier
     const int n_tok = max(0, min(chunk_tokens, len - first_tok));
     const int n_pages = (n_tok + kPageTokens - 1) / kPageTokens;
     const int* pt = p.page_table + (size_t)p.slot[b] * p.max_pages + first_tok / kPageTokens;
@@ -348,8 +349,8 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
     }
     __syncthreads();
     const int n_rows = kMulti ? 16 : group;
-    constexpr int kOwn = kHD + 4;                                     // kStep: a row's output, maximum and sum of this CTA
-    __shared__ __align__(16) float own_part[kStep ? 8 * kOwn : 4];
+    constexpr int kOwn = kHD + 4;                                     // kMerge: a row's output, maximum and sum of this CTA
+    __shared__ __align__(16) float own_part[kMerge ? 8 * kOwn : 4];
     for (int idx = tid; idx < n_rows * (kHD / 4); idx += kAttnWarps * 32) {
         const int r = idx / (kHD / 4), c4 = (idx % (kHD / 4)) * 4;
         const int tok = kMulti ? b + r / group : b;
@@ -369,12 +370,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
 #pragma unroll
         for (int w = 0; w < kAttnWarps; ++w) {
             const float mw = mml[(w * kRows + r) * 2];
-            const float f = ((kMulti || kStep) && mw == -INFINITY) ? 0.f : exp2f(mw - M);  // a warp that has seen no page of the row
+            const float f = ((kMulti || kMerge) && mw == -INFINITY) ? 0.f : exp2f(mw - M);  // a warp that has seen no page of the row
             L += mml[(w * kRows + r) * 2 + 1] * f;
             float4 v = *reinterpret_cast<const float4*>(mo + (w * kRows + r) * kHD + c4);
             acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
         }
-        if (kStep) {
+        if (kMerge) {
             *reinterpret_cast<float4*>(own_part + r * kOwn + c4) = acc;
             if (c4 == 0) { own_part[r * kOwn + kHD] = M; own_part[r * kOwn + kHD + 1] = L; }
         } else if (row_splits == 1) {
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
             }
         }
     }
-    if (kStep) {   // the cluster's parts in rank order, 4 columns of a row per thread, the work dealt over the ranks
+    if (kMerge) {   // the cluster's parts in rank order, 4 columns of a row per thread, the work dealt over the ranks
         const int S = gridDim.y, rank = S > 1 ? (int)cluster_ctarank() : 0;
         if (S > 1) cluster_sync_all();
         else __syncthreads();
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32, (kDepth <= 2) ? 3 : 2) paged_
                     L += ml[q].y * f;
                     acc.x += v[q].x * f; acc.y += v[q].y * f; acc.z += v[q].z * f; acc.w += v[q].w * f;
                 }
-            const float inv = 1.f / L;
+            const float inv = kStep || L > 0.f ? 1.f / L : 0.f;   // a row that sees nothing
             *reinterpret_cast<uint2*>(p.out + ((size_t)b * p.Hq + h * group + r) * kHD + c4) =
                 make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
         }
@@ -706,6 +707,8 @@ __global__ void kv_gather_kernel(const unsigned char* pool, const int* page_row,
     v_out[o] = *reinterpret_cast<const __nv_bfloat16*>(blk + kBlockBytes + swz(tk, c >> 3) + (c & 7) * 2);
 }
 
+__global__ void clear_word_kernel(int* word) { if (threadIdx.x == 0) *word = 0; }
+
 }  // namespace
 
 // Splits per row and kv head (a cluster) of a decode step in one kernel, 0: the step is left to the separate kernels. Eight pages per
@@ -875,6 +878,48 @@ static int paged_attention_launch(int multi, const void* d_q, const void* d_kv_p
         }
     }
     return GPTRS_OK;
+}
+
+int64_t gptrs_cuda_attention_few_rows_splits(int64_t max_ctx_len, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads) {
+    if (max_ctx_len < 1 || n_tokens < 1 || n_kv_heads < 1 || n_q_heads < 1) return 0;
+    return attention_step_splits(max_ctx_len, n_tokens, n_q_heads, n_kv_heads);
+}
+
+int gptrs_cuda_paged_attention_decode_few_rows(const void* d_q, const void* d_kv_pool, const int32_t* d_page_table, int64_t max_pages, const int32_t* d_slot,
+                                               const int32_t* d_ctx_len, void* d_out, int32_t* d_status, int clear_status, int64_t n_tokens, int64_t n_q_heads,
+                                               int64_t n_kv_heads, int64_t head_dim, int64_t max_ctx_len, void* stream) {
+    GPTRS_REQUIRE(d_q && d_kv_pool && d_page_table && d_slot && d_ctx_len && d_out && d_status, "null pointer");
+    GPTRS_REQUIRE(head_dim == kHD, "paged bf16 attention supports head_dim 128 only");
+    GPTRS_REQUIRE(n_q_heads > 0 && n_kv_heads > 0 && n_q_heads % n_kv_heads == 0, "bad head counts");
+    GPTRS_REQUIRE(n_q_heads / n_kv_heads <= 8, "GQA group size above 8 is not supported");
+    GPTRS_REQUIRE(max_ctx_len >= 1 && max_ctx_len <= max_pages * kPageTokens, "max_ctx_len exceeds the page table");
+    const int splits = n_tokens > 0 ? attention_step_splits(max_ctx_len, n_tokens, n_q_heads, n_kv_heads) : 0;
+    if (splits == 0) return fail(GPTRS_UNIMPLEMENTED, "attention of few rows: more rows or longer contexts than a cluster takes");
+    cudaStream_t st = as_stream(stream);
+    if (clear_status) {   // a memset is 2 us less work for the host than a launch; as a node of a graph it takes 3 us longer than a kernel
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        GPTRS_CUDA_OK(cudaStreamIsCapturing(st, &capture));
+        if (capture == cudaStreamCaptureStatusNone) GPTRS_CUDA_OK(cudaMemsetAsync(d_status, 0, 4, st));
+        else clear_word_kernel<<<1, 32, 0, st>>>(d_status);
+        GPTRS_CUDA_OK(cudaGetLastError());
+    }
+    AttnParams p = {};
+    p.q = static_cast<const __nv_bfloat16*>(d_q);
+    p.pool = static_cast<const unsigned char*>(d_kv_pool);
+    p.page_table = d_page_table; p.slot = d_slot; p.ctx_len = d_ctx_len;
+    p.out = static_cast<__nv_bfloat16*>(d_out);
+    p.status = d_status;
+    p.T = (int)n_tokens; p.Hq = (int)n_q_heads; p.Hkv = (int)n_kv_heads; p.max_pages = (int)max_pages;
+    p.chunk_pages = ceil_div(ceil_div(max_ctx_len, kPageTokens), splits);
+    p.max_splits = splits;
+    p.max_len = (int)std::min<int64_t>((int64_t)splits * p.chunk_pages * kPageTokens, max_pages * kPageTokens);
+    p.scale_log2 = kLog2e / sqrtf((float)kHD);
+    constexpr size_t smem = (size_t)kAttnWarps * 2 * kPageHeadBytes;
+    static PerDeviceOnce attr_once;
+    if (attr_once.first_time())
+        GPTRS_CUDA_OK(cudaFuncSetAttribute(paged_attention_kernel<2, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return launch_kernel(paged_attention_kernel<2, false, false, true>, dim3((unsigned)n_kv_heads, (unsigned)splits, (unsigned)n_tokens), dim3(kAttnWarps * 32), smem, st,
+                         splits, p);
 }
 
 int gptrs_cuda_paged_attention_decode(const void* d_q, const void* d_kv_pool, const int32_t* d_page_table,

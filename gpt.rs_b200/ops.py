@@ -5,6 +5,7 @@ torch kernel runs on behalf of these functions except output allocation.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -21,7 +22,7 @@ def _ptr(t: torch.Tensor | None):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())   # the handle without a Stream object around it
 
 
 # ---- quantised weights --------------------------------------------------------------------------
@@ -178,6 +179,11 @@ def rope_kv_append(qkv, positions, slot, page_table, cos, sin, rotary_dim, kv_po
     return q_out
 
 
+@functools.lru_cache(maxsize=1024)
+def _few_rows_splits(max_ctx_len, t, n_q, n_kv, device):
+    return lib().gptrs_cuda_attention_few_rows_splits(max_ctx_len, t, n_q, n_kv) if n_kv > 0 and n_q % n_kv == 0 else 0
+
+
 def paged_attention_decode(q, kv_pool, page_table, slot, ctx_len, n_q, n_kv, max_ctx_len, head_dim=128,
                            chunk_pages=None, status=None, prefill=False):
     """q bf16 [T][Hq][hd] -> out bf16 [T][Hq*hd]. prefill=True uses the prefill-chunk entry point (aligned groups
@@ -190,6 +196,14 @@ def paged_attention_decode(q, kv_pool, page_table, slot, ctx_len, n_q, n_kv, max
         out = torch.empty((t, n_q * head_dim), dtype=torch.bfloat16, device=q.device)
         check(lib().gptrs_cuda_paged_attention_prefill_tc(_ptr(q), _ptr(kv_pool), _ptr(page_table), page_table.shape[1], _ptr(slot),
                                                           _ptr(ctx_len), _ptr(out), _ptr(status), t, n_q, n_kv, head_dim, _stream()))
+        return out, status
+    if chunk_pages is None and not prefill and t and _few_rows_splits(max_ctx_len, t, n_q, n_kv, q.device.index):
+        out = torch.empty((t, n_q * head_dim), dtype=torch.bfloat16, device=q.device)
+        clear = status is None
+        if clear:
+            status = torch.empty(1, dtype=torch.int32, device=q.device)
+        check(lib().gptrs_cuda_paged_attention_decode_few_rows(_ptr(q), _ptr(kv_pool), _ptr(page_table), page_table.shape[1], _ptr(slot), _ptr(ctx_len), _ptr(out),
+                                                               _ptr(status), clear, t, n_q, n_kv, head_dim, max_ctx_len, _stream()))
         return out, status
     if chunk_pages is None:
         chunk_pages = lib().gptrs_cuda_attention_chunk_pages(max_ctx_len, t, n_kv)

@@ -609,6 +609,15 @@ int gptrs_cuda_paged_attention_decode(const void* d_q, const void* d_kv_pool, co
                                       int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads,
                                       int64_t head_dim, int64_t max_ctx_len, int64_t chunk_pages,
                                       void* stream);
+/* The same for up to 16 rows, whose splits a cluster merges: one launch, no scratch. gptrs_cuda_attention_few_rows_splits says how many
+ * splits a row and kv head get (at most eight pages per warp), 0: the call is for gptrs_cuda_paged_attention_decode
+ * (GPTRS_UNIMPLEMENTED here). clear_status != 0: the status word is set to 0 in front. */
+int64_t gptrs_cuda_attention_few_rows_splits(int64_t max_ctx_len, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads);
+int gptrs_cuda_paged_attention_decode_few_rows(const void* d_q, const void* d_kv_pool, const int32_t* d_page_table,
+                                               int64_t max_pages, const int32_t* d_slot, const int32_t* d_ctx_len,
+                                               void* d_out, int32_t* d_status, int clear_status, int64_t n_tokens,
+                                               int64_t n_q_heads, int64_t n_kv_heads, int64_t head_dim,
+                                               int64_t max_ctx_len, void* stream);
 /* The same attention for a PREFILL CHUNK: the rows are tokens of which every aligned group of
  * 16 / (n_q_heads / n_kv_heads) consecutive rows belongs to ONE sequence (same d_slot value; a chunk of
  * one prompt satisfies this trivially). The K/V pages are then streamed once per group instead of once per

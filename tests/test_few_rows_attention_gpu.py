@@ -1,0 +1,48 @@
+"""Decode attention of up to 16 rows in one launch (the splits merged by their cluster) against the kernel with scratch and a merge of its own:
+page edges, one split and eight, rows without tokens in some splits, a row that sees nothing, lengths above the launch bound."""
+import pytest
+import torch
+
+from gptrs_b200 import BackendError, lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _cache(lengths, n_kv, longest, cuda, seed):
+    g = torch.Generator(device=cuda).manual_seed(seed)
+    per = (longest + 15) // 16
+    pool = ops.new_kv_pool(len(lengths) * per, n_kv, cuda)
+    pool.view(torch.bfloat16).normal_(generator=g)
+    table = torch.randperm(len(lengths) * per, device=cuda, generator=g).int().view(len(lengths), per)
+    return g, pool, table
+
+
+@pytest.mark.parametrize("lengths,n_q,n_kv", [([1], 8, 2), ([16], 8, 8), ([17], 4, 4), ([1500], 32, 8), ([4096], 32, 8), ([65, 64, 63], 8, 1), ([0, 40], 8, 2),
+                                              ([300, 1, 128, 129, 15], 16, 4), (list(range(1, 1024, 64)), 32, 8)])
+def test_one_launch_equals_two(cuda, lengths, n_q, n_kv):
+    longest = max(lengths)
+    g, pool, table = _cache(lengths, n_kv, longest, cuda, longest + n_q)
+    assert lib().gptrs_cuda_attention_few_rows_splits(longest, len(lengths), n_q, n_kv) > 0
+    q = torch.randn((len(lengths), n_q, 128), device=cuda, generator=g).bfloat16()
+    slot, ctx = torch.arange(len(lengths), dtype=torch.int32, device=cuda), torch.tensor(lengths, dtype=torch.int32, device=cuda)
+    out, status = ops.paged_attention_decode(q, pool, table, slot, ctx, n_q, n_kv, longest)
+    ref, _ = ops.paged_attention_decode(q, pool, table, slot, ctx, n_q, n_kv, longest, chunk_pages=4)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for row, n in enumerate(lengths):
+        if n == 0:
+            assert not out[row].any()
+        else:   # one rounding to bf16 each (2^-9), f32 sums in another order, probabilities rounded to bf16 against another maximum
+            assert (out[row].float() - ref[row].float()).norm() <= 2 ** -7 * ref[row].float().norm()
+
+
+def test_lengths_and_shapes_that_do_not_fit(cuda):
+    g, pool, table = _cache([100, 100], 2, 100, cuda, 1)
+    q = torch.randn((2, 8, 128), device=cuda, generator=g).bfloat16()
+    slot = torch.arange(2, dtype=torch.int32, device=cuda)
+    own = torch.zeros(1, dtype=torch.int32, device=cuda)
+    out, status = ops.paged_attention_decode(q, pool, table, slot, torch.tensor([100, 5000], dtype=torch.int32, device=cuda), 8, 2, 100, status=own)
+    assert status is own and int(status.item()) == 2 and torch.isfinite(out.float()).all()
+    assert lib().gptrs_cuda_attention_few_rows_splits(100000, 16, 32, 8) == 0 and lib().gptrs_cuda_attention_few_rows_splits(100, 17, 8, 2) == 0
+    with pytest.raises(BackendError):
+        ops.paged_attention_decode(q, pool, table, slot, slot, 8, 2, 200)   # more than the page table holds
