@@ -22,8 +22,8 @@
 //     ran from a cold instruction cache.
 // A buffer is written again a layer later: a CTA that gets that far has consumed outputs of all CTAs (every phase's vector has items of every
 // CTA), and these were computed after their readings. With grid barriers in place of the words, partials of 12 chunks merged by every CTA and a
-// copy of the code per projection a token took 326 us (one sequence), 517 (six sequences); now 262 and 374: a phase's exchange is 2.5 to 3.7 us, of
-// which the round trips alone are 1.3, its projection 0.7 to 1.4, the head 20. Every wait is bounded (a thread that gives up records status 5 and goes on).
+// copy of the code per projection a token took 326 us (one sequence), 517 (six sequences); now 240 and 369: a phase's exchange is 2.5 to 3.2 us, of
+// which the round trips alone are 1.3, its projection 0.7 to 1.0, attention 4.4, the head 20. Every wait is bounded (a thread that gives up records status 5 and goes on).
 #include <algorithm>
 
 #include "flag_words.cuh"
@@ -34,6 +34,7 @@ namespace {
 
 constexpr int kMegaThreads = 256, kMegaWarps = kMegaThreads / 32;
 constexpr int kD = 768, kMlp = 3072;   // the widths it is built for (mega_supported)
+constexpr int kEarlyV = 16;            // values of a thread that attention asks for early: 64 keys of heads of 64
 
 __device__ __forceinline__ float4 ldg_stream_f4(const float4* p) {
     float4 v;
@@ -65,11 +66,20 @@ __device__ __forceinline__ void residual_norm(float* h, float* xn, const unsigne
                                               float* red) {
     constexpr int W = kMegaWarps / R, N = kD / (32 * W);
     const int warp = threadIdx.x >> 5, row = warp / W, first = threadIdx.x - row * W * 32;
-    constexpr int G = N < 12 / PARTS * 2 ? N : 12 / PARTS * 2;   // elements under way at once: the next projection's weights already hold 96 registers
+    constexpr int G = PARTS == 4 ? (N < 6 ? N : N % 8 ? 6 : 8) : N;   // elements under way at once: the next projection's weights already hold 96 registers
     static_assert(N % G == 0, "whole groups");
     float v[N];
     const unsigned char* const own = part + (size_t)(row * kD + first) * (8 * PARTS);
     const bool adds = part && row < rows;
+    // what does not depend on the other CTAs is asked for first (of eight rows a thread has 24 elements: their gains come later)
+    constexpr bool kEarly = R < 8;
+    float b_in[N], g_in[kEarly ? N : 1], s_in[kEarly ? N : 1];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        const int i = first + j * W * 32;
+        b_in[j] = part ? __ldg(bias + i) : 0.f;
+        if (kEarly) { g_in[j] = __ldg(gamma + i); s_in[j] = __ldg(beta + i); }
+    }
     if (R > 1 && adds) {   // (one row: a warp's whole request is three of these)
         if ((threadIdx.x & 31) == 0) wait.wait_word(own, flag);
         __syncwarp();
@@ -110,7 +120,7 @@ __device__ __forceinline__ void residual_norm(float* h, float* xn, const unsigne
 #pragma unroll
     for (int j = 0; j < N; ++j) {
         const int i = first + j * W * 32;
-        v[j] = part ? h[row * kD + i] + (bias[i] + v[j]) : h[row * kD + i];
+        v[j] = part ? h[row * kD + i] + (b_in[j] + v[j]) : h[row * kD + i];
         s += v[j];
     }
     auto row_sum = [&](float t, float* at) {
@@ -132,7 +142,7 @@ __device__ __forceinline__ void residual_norm(float* h, float* xn, const unsigne
     for (int j = 0; j < N; ++j) {
         const int e = first + j * W * 32;
         h[row * kD + e] = v[j];
-        xn[row * kD + e] = (v[j] - mean) * inv * gamma[e] + beta[e];
+        xn[row * kD + e] = (v[j] - mean) * inv * (kEarly ? g_in[kEarly ? j : 0] : gamma[e]) + (kEarly ? s_in[kEarly ? j : 0] : beta[e]);
     }
     __syncthreads();
 }
@@ -168,7 +178,7 @@ __device__ __forceinline__ float row_sums(float (&v)[R], int lane) {
 // value of their sequence that they have produced (ties: the smaller row).
 constexpr int kF4 = 6;   // float4 per lane per item
 constexpr int kU = 4;    // items in flight per warp
-struct Round { float4 w[kU][kF4]; };
+struct Round { float4 w[kU][kF4]; float bias[kU]; };   // bias: of the items, where GELU follows
 
 __device__ __forceinline__ void gemv_load(Round& r, const float* __restrict__ Wt, int n_items, int item0, int total, int lane) {
 #pragma unroll
@@ -179,9 +189,14 @@ __device__ __forceinline__ void gemv_load(Round& r, const float* __restrict__ Wt
         for (int j = 0; j < kF4; ++j) r.w[u][j] = ldg_stream_f4(src + 32 * j);
     }
 }
-__device__ __forceinline__ void gemv_prefetch(Round& r, const float* __restrict__ Wt, int n_items) {
+__device__ __forceinline__ void load_bias(Round& r, const float* __restrict__ bias, int n_items, int item0, int total) {
+#pragma unroll
+    for (int u = 0; u < kU; ++u) r.bias[u] = __ldg(bias + min(item0 + u * total, n_items - 1));
+}
+__device__ __forceinline__ void gemv_prefetch(Round& r, const float* __restrict__ Wt, int n_items, const float* __restrict__ gelu_bias) {
     const int total = gridDim.x * kMegaWarps, gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     if (gw < n_items) gemv_load(r, Wt, n_items, gw, total, threadIdx.x & 31);
+    if (gw < n_items && gelu_bias) load_bias(r, gelu_bias, n_items, gw, total);
 }
 template <int R>
 __device__ __forceinline__ void gemv_items(Round& r, const float* __restrict__ Wt, int n_items, const float* xs, unsigned char* __restrict__ out, uint32_t flag,
@@ -192,7 +207,10 @@ __device__ __forceinline__ void gemv_items(Round& r, const float* __restrict__ W
     const bool stores = lane % (32 / R) == 0 && seq < rows;
 #pragma unroll 1
     for (int item0 = gw; item0 < n_items; item0 += kU * total) {
-        if (item0 != gw) gemv_load(r, Wt, n_items, item0, total, lane);   // the first round is already on its way
+        if (item0 != gw) {   // the first round is already on its way
+            gemv_load(r, Wt, n_items, item0, total, lane);
+            if (gelu_bias) load_bias(r, gelu_bias, n_items, item0, total);
+        }
         float acc[kU][R];
 #pragma unroll
         for (int s = 0; s < R; ++s) {   // a sequence's values are read once for the four items
@@ -218,7 +236,7 @@ __device__ __forceinline__ void gemv_items(Round& r, const float* __restrict__ W
             float v = u == 0 ? sum[0] : u == 1 ? sum[1] : u == 2 ? sum[2] : sum[3];
             if (stores && item < n_items) {
                 if (gelu_bias) {
-                    v += gelu_bias[item];
+                    v += u == 0 ? r.bias[0] : u == 1 ? r.bias[1] : u == 2 ? r.bias[2] : r.bias[3];
                     v = (0.5f * v) * (1.f + erff(v / 1.4142135f));
                 }
                 if (!logits) {
@@ -262,7 +280,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
     float best = -INFINITY;   // lm_head: the largest logit this lane has produced
     int best_i = 0x7fffffff;
     Round rnd;                // the weights of this warp's first items of the next projection
-    gemv_prefetch(rnd, p.layers[0].w_qkv_t, 3 * kD);
+    gemv_prefetch(rnd, p.layers[0].w_qkv_t, 3 * kD, nullptr);
     uint32_t flag = p.epoch;   // of the layer; every phase's vector has a buffer of its own
 
     for (int s = 0; s < R; ++s) {
@@ -306,33 +324,46 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
                 float* qs = xn;            // [hd]
                 float* k_new = xn + hd;    // [hd]
                 float* v_new = xn + 2 * hd;
+                // the first 64 keys and values of the slice are asked for before the token's vectors have arrived
+                const int lanes = hd >> 2, per = 32 / lanes, sub = lane / lanes, c4 = (lane - sub * lanes) * 4;
+                const int parts = kMegaThreads / hd, c = tid % hd, part = tid / hd;
+                float4 k4[4];
+                float v_in[kEarlyV];
+                auto load_keys = [&](int base) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int j = base + u * kMegaWarps * per + sub;
+                        k4[u] = j >= j1 || j == pos ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(kc + (size_t)j * hd + c4);
+                    }
+                };
+                load_keys(j0 + warp * per);
+#pragma unroll
+                for (int u = 0; u < kEarlyV; ++u) {
+                    const int j = j0 + part + u * parts;
+                    v_in[u] = j < j1 && j != pos ? vc[(size_t)j * hd + c] : 0.f;
+                }
                 const unsigned char* qkv = p.qkv + (size_t)(seq * 3 * kD + head * hd) * 8;
 #pragma unroll 1
-                for (int c = tid; c < 3 * hd; c += kMegaThreads) {
-                    const int which = c / hd, e = c - which * hd;
+                for (int i = tid; i < 3 * hd; i += kMegaThreads) {
+                    const int which = i / hd, e = i - which * hd;
                     const float bias = L.b_qkv[which * kD + head * hd + e];
-                    xn[c] = __uint_as_float(wait.wait_word(qkv + (which * kD + e) * 8, flag)) + bias;
+                    xn[i] = __uint_as_float(wait.wait_word(qkv + (which * kD + e) * 8, flag)) + bias;
                 }
                 __syncthreads();
                 float* sc = big;   // scores of this slice
                 if (j0 <= pos && pos < j1)   // the new token's row goes into the cache for the steps to come
-                    for (int c = tid; c < hd; c += kMegaThreads) { kc[(size_t)pos * hd + c] = k_new[c]; vc[(size_t)pos * hd + c] = v_new[c]; }
+                    for (int i = tid; i < hd; i += kMegaThreads) { kc[(size_t)pos * hd + i] = k_new[i]; vc[(size_t)pos * hd + i] = v_new[i]; }
                 // scores: hd / 4 lanes per key, four times 128 / hd keys of a warp under way at once
                 {
-                    const int lanes = hd >> 2, per = 32 / lanes, sub = lane / lanes, c4 = (lane - sub * lanes) * 4;
-                    const float4 q4 = *reinterpret_cast<const float4*>(qs + c4);
+                    const float4 q4 = *reinterpret_cast<const float4*>(qs + c4), own = *reinterpret_cast<const float4*>(k_new + c4);
 #pragma unroll 1
                     for (int base = j0 + warp * per; base < j1; base += 4 * kMegaWarps * per) {
-                        float4 k4[4];
+                        if (base != j0 + warp * per) load_keys(base);
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             const int j = base + u * kMegaWarps * per + sub;
-                            k4[u] = j >= j1 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>((j == pos ? k_new : kc + (size_t)j * hd) + c4);
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int j = base + u * kMegaWarps * per + sub;
-                            float t = fmaf(q4.w, k4[u].w, fmaf(q4.z, k4[u].z, fmaf(q4.y, k4[u].y, q4.x * k4[u].x)));
+                            const float4 k = j == pos ? own : k4[u];
+                            float t = fmaf(q4.w, k.w, fmaf(q4.z, k.z, fmaf(q4.y, k.y, q4.x * k.x)));
 #pragma unroll 1
                             for (int o = lanes >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
                             if (c4 == 0 && j < j1) sc[j - j0] = t * scale;
@@ -358,11 +389,14 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
                 }
                 sum = block_sum(sum, red);
                 // context: thread (part, c) walks positions part, part + parts, ...
-                const int parts = kMegaThreads / hd;
-                const int c = tid % hd, part = tid / hd;
                 float acc = 0.f;
-#pragma unroll 8
-                for (int j = j0 + part; j < j1; j += parts) acc = fmaf(sc[j - j0], (j == pos ? v_new : vc + (size_t)j * hd)[c], acc);
+#pragma unroll
+                for (int u = 0; u < kEarlyV; ++u) {
+                    const int j = j0 + part + u * parts;
+                    if (j < j1) acc = fmaf(sc[j - j0], j == pos ? v_new[c] : v_in[u], acc);
+                }
+#pragma unroll 4
+                for (int j = j0 + part + kEarlyV * parts; j < j1; j += parts) acc = fmaf(sc[j - j0], (j == pos ? v_new : vc + (size_t)j * hd)[c], acc);
                 float* comb = red + 64;   // [parts][hd]
                 comb[part * hd + c] = acc;
                 __syncthreads();
@@ -446,7 +480,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
         if (at_head) break;
         __syncthreads();   // xn and big have been read
         const float* next = kind == 0 ? L.w_out_t : kind == 1 ? L.w_mlp_in_t : kind == 2 ? L.w_mlp_out_t : l + 1 < p.n_layers ? p.layers[l + 1].w_qkv_t : p.lm_head_t;
-        gemv_prefetch(rnd, next, kind == 0 ? kD : kind < 3 ? kMlp : l + 1 < p.n_layers ? 3 * kD : p.vocab);   // of the out projection: kept across attention
+        gemv_prefetch(rnd, next, kind == 0 ? kD : kind < 3 ? kMlp : l + 1 < p.n_layers ? 3 * kD : p.vocab, kind == 1 ? L.b_mlp_in : nullptr);   // of the out projection: kept across attention
     }
     // ---- the greedy pick ------------------------------------------------------------------------------------------------
     // the storing lanes hold their warp's best of a sequence; CTA best -> cand[sequence][blockIdx.x]
