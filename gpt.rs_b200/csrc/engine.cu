@@ -58,7 +58,9 @@ int alloc_step_buffers(Model& m, int stage_arrays) {
     if ((rc = m.history.alloc((size_t)c.max_seqs * c.context_length * 4, true))) return rc;
     for (DevBuf* b : {&m.d_tokens, &m.d_slot, &m.d_pos, &m.d_ctx, &m.d_rows, &m.d_sampled})
         if ((rc = b->alloc((size_t)m.stage_stride() * 4, true))) return rc;
-    if ((rc = m.d_status.alloc(4, true))) return rc;
+    const size_t words = (size_t)1 + c.max_seqs;
+    GPTRS_CUDA_OK(cudaMallocHost(&m.d_status.p, words * 4));
+    memset(m.d_status.p, 0, words * 4);
     GPTRS_CUDA_OK(cudaMallocHost(&m.h_stage, (size_t)stage_arrays * m.stage_stride() * 4));
     GPTRS_CUDA_OK(cudaMallocHost(&m.h_logits, (size_t)m.max_rows() * m.vocab_l * 4));
     m.seq_pages.assign(c.max_seqs, 0);
@@ -281,8 +283,8 @@ __global__ void tp_pick_kernel(const TpPickParams p) {
 }
 
 // End of a generator step: the token a slot consumed goes into its history at the position it had, the sampled id
-// becomes the slot's next input, position and visible length advance.
-struct AdvanceParams { int* tokens; const int* sampled; int* pos; int* ctx; int* history; int n, context_length; int* parity; };
+// becomes the slot's next input and goes to the host, position and visible length advance.
+struct AdvanceParams { int* tokens; const int* sampled; int* pos; int* ctx; int* history; int n, context_length; int* parity; int* out; };
 __global__ void advance_kernel(const AdvanceParams p) {
     pdl_launch_dependents();  // dependents still wait for this whole grid before reading its results
     pdl_wait();
@@ -290,7 +292,9 @@ __global__ void advance_kernel(const AdvanceParams p) {
     if (i < p.n) {
         const int at = p.pos[i];
         if (at >= 0 && at < p.context_length) p.history[(size_t)i * p.context_length + at] = p.tokens[i];
-        p.tokens[i] = p.sampled[i];
+        const int id = p.sampled[i];
+        p.tokens[i] = id;
+        p.out[i] = id;
         p.pos[i] = at + 1;
         p.ctx[i] += 1;
         if (p.parity) p.parity[i] ^= 1;   // the half of the convolution state that the next step reads
@@ -329,12 +333,15 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     cudaStream_t st = m.stream;
     float* hidden = m.hidden.as<float>();
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
-    if (T <= m.mega_rows && T <= m.max_rows() && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
+    if (m.one_kernel_step(T) && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
         // a token each of a few sequences: the whole step is one cooperative kernel
         MegaParams P = m.mega;
         P.rows = T;
         m.mega.epoch += (uint32_t)c.n_layers + 1u;   // every word of this step carries a flag that no other step's does
         P.greedy = temperature <= 0.f ? 1 : 0;
+        P.advance = m.step_advance ? 1 : 0;
+        P.given = m.step_tokens ? 1 : 0;
+        if (m.step_tokens) memcpy(P.token_in, m.step_tokens, (size_t)T * 4);
         m.launches += 1;
         int r = mega_launch(P, st);
         if (r || P.greedy) return r;
@@ -696,7 +703,8 @@ int setup_mega(Model& m) {
     MegaParams& P = m.mega;
     P.n_layers = c.n_layers;
     P.tok_emb = fp(m.tok_emb); P.pos_emb = fp(m.pos_emb); P.lnf_g = fp(m.final_g); P.lnf_b = fp(m.final_b); P.lm_head_t = lm_t;
-    P.token = m.d_tokens.as<int>(); P.pos = m.d_pos.as<int>(); P.slot = m.d_slot.as<int>();
+    P.token = m.d_tokens.as<int>(); P.pos = m.d_pos.as<int>(); P.slot = m.d_slot.as<int>(); P.ctx = m.d_ctx.as<int>();
+    P.history = m.history.as<int>(); P.out = m.step_out();
     P.qkv = take(pad(R * 3 * D));
     P.att_part = take(n_part);
     P.att = take(pad(R * D));
@@ -772,11 +780,10 @@ int setup_peer_allreduce(Model& m, int max_rows_peer) {
 }
 
 int check_status(Model& m) {
-    int32_t st = 0;
-    GPTRS_CUDA_OK(cudaMemcpyAsync(&st, m.d_status.p, 4, cudaMemcpyDeviceToHost, m.stream));
     GPTRS_CUDA_OK(cudaStreamSynchronize(m.stream));
+    const int32_t st = *static_cast<volatile int32_t*>(m.d_status.p);
     if (st != 0) {
-        cudaMemsetAsync(m.d_status.p, 0, 4, m.stream);
+        *m.d_status.p = 0;
         return fail(GPTRS_EXECUTION, st == 2   ? "token or position id out of range"
                                      : st == 3 ? "a bounded wait inside a tensor-core kernel (matmul or attention) gave up"
                                      : st == 4 ? "a tensor-parallel peer did not deliver its partial sums in time"
@@ -1329,7 +1336,8 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
     int rc = sync_page_table(m);
     if (rc) return rc;
     cudaStream_t s = m.stream;
-    if (h_tokens_in) {
+    const bool own_step = m.f32() && m.one_kernel_step(B);   // takes the ids as parameters and advances its sequences itself
+    if (h_tokens_in && !own_step) {
         GPTRS_CUDA_OK(cudaStreamSynchronize(s));  // the staging buffer may still feed an earlier copy
         memcpy(m.h_stage, h_tokens_in, (size_t)B * 4);
         GPTRS_CUDA_OK(cudaMemcpyAsync(m.d_tokens.p, m.h_stage, (size_t)B * 4, cudaMemcpyHostToDevice, s));
@@ -1347,11 +1355,18 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
         if (r) return r;
         // next step: the consumed ids go into the history, the sampled ids become the inputs, positions advance
         AdvanceParams ap = {m.d_tokens.as<int>(), m.d_sampled.as<int>(), m.d_pos.as<int>(), m.d_ctx.as<int>(), m.history.as<int>(), B,
-                            c.context_length, m.layered() ? m.lay->d_parity.as<int>() : nullptr};
+                            c.context_length, m.layered() ? m.lay->d_parity.as<int>() : nullptr, m.step_out()};
         ++m.launches;
         return launch_kernel(advance_kernel, dim3((B + 127) / 128), dim3(128), 0, s, 1, ap);
     };
-    if (use_graph && !(B <= m.mega_rows && B <= m.max_rows())) {   // the single-kernel step needs no graph
+    if (own_step) {   // one launch, which needs no graph
+        m.step_tokens = h_tokens_in;
+        m.step_advance = true;
+        const int r = enqueue_forward(m, B, bucket, chunk, B, true, 0.f, false, true);
+        m.step_tokens = nullptr;
+        m.step_advance = false;
+        if (r) return r;
+    } else if (use_graph) {
         GraphKey key{B, chunk, splits, decode_step_splits(m, B, bucket) ? bucket : 0};
         auto it = m.graphs.find(key);
         if (it == m.graphs.end()) {
@@ -1382,10 +1397,9 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
     for (int b = 0; b < B; ++b) ++m.seq_len[b];
     if (m.layered()) for (int b = 0; b < B; ++b) m.lay->parity[b] ^= 1;
     if (h_tokens_out) {
-        GPTRS_CUDA_OK(cudaMemcpyAsync(m.h_stage + B, m.d_sampled.p, (size_t)B * 4, cudaMemcpyDeviceToHost, s));
-        rc = check_status(m);
+        rc = check_status(m);   // the ids are in pinned memory by then
         if (rc) return rc;
-        memcpy(h_tokens_out, m.h_stage + B, (size_t)B * 4);
+        memcpy(h_tokens_out, m.step_out(), (size_t)B * 4);
     }
     return GPTRS_OK;
 }

@@ -158,7 +158,14 @@ struct Model {
 
     // activations
     DevBuf hidden, xn, qkv, q_rot, attn, mlp_h, mlp_g, mlp_u, logits, xn_rows;
-    DevBuf d_tokens, d_slot, d_pos, d_ctx, d_rows, d_sampled, d_status, attn_scratch;
+    DevBuf d_tokens, d_slot, d_pos, d_ctx, d_rows, d_sampled, attn_scratch;
+    // What every step hands to the host, written by its kernels into pinned memory (two copies of a few bytes less per step): the status word
+    // (0 unless a kernel reports an error), and the sampled ids of the generator's rows.
+    struct HostWords {
+        int32_t* p = nullptr;
+        template <typename T> T* as() const { return reinterpret_cast<T*>(p); }
+    } d_status;
+    int32_t* step_out() const { return d_status.p + 1; }
     DevBuf sumsq;  // [d_model / 128][max_tokens] row sums of squares of the folded RMSNorm
     DevBuf history;  // [max_seqs][context_length] token ids by position (the generator re-windows from it)
     bool fold_norm = true, fold_rope = true;
@@ -212,6 +219,9 @@ struct Model {
     MegaParams mega = {};
     AttentionF32Plan attn_f32;      // f32 kinds: the split of the pass under way, its lists in d_attn_f32
     DevBuf d_attn_f32;
+    // single-kernel f32 steps: the ids that the generator gives (null: those on the device), and whether the kernel advances its sequences
+    const int32_t* step_tokens = nullptr;
+    bool step_advance = false;
     int gen_batch = 0;  // slots 0..gen_batch-1 are driven by generator_step
     int64_t launches = 0;
     uint32_t sample_seed = 0;
@@ -222,6 +232,7 @@ struct Model {
     bool f32() const { return cfg.weight_mode == kModeF32; }
     bool layered() const { return cfg.kind == kKindLayered; }
     bool paged() const { return !f32() || layered(); }
+    bool one_kernel_step(int rows) const { return rows <= mega_rows && rows <= max_rows(); }
     int max_rows() const { return cfg.max_logit_rows > 0 ? cfg.max_logit_rows : cfg.max_seqs; }
     int stage_stride() const { return std::max(cfg.max_tokens, max_rows()); }
 
@@ -237,6 +248,7 @@ struct Model {
         for (Tensor* t : {tok_emb, pos_emb, final_g, final_b}) tensor_release(t);
         if (h_page_table) cudaFreeHost(h_page_table);
         if (h_stage) cudaFreeHost(h_stage);
+        if (d_status.p) cudaFreeHost(d_status.p);
         tensor_release(wide);
         if (h_logits) cudaFreeHost(h_logits);
         for (void* p : peer_maps) if (p) cudaIpcCloseMemHandle(p);

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
     uint32_t flag = p.epoch;   // of the layer; every phase's vector has a buffer of its own
 
     for (int s = 0; s < R; ++s) {
-        const int token = s < rows ? p.token[s] : 0;
+        const int token = s < rows ? (p.given ? p.token_in[s] : p.token[s]) : 0;
         const bool ok = s < rows && token >= 0 && token < p.vocab;
         if (s < rows && !ok && tid == 0 && blockIdx.x == 0) atomicExch(p.status, 2);
         const int pos = ok ? min(max(p.pos[s], 0), p.n_pos - 1) : 0;
@@ -510,7 +510,17 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
             const int oi = __shfl_xor_sync(0xffffffffu, ix, o);
             if (ov > v || (ov == v && oi < ix)) { v = ov; ix = oi; }
         }
-        if (lane == 0 && p.greedy) p.sampled[warp] = ix;
+        if (lane == 0 && p.greedy) {
+            p.sampled[warp] = ix;
+            if (p.advance) {   // every CTA has read its token and position by now: its candidate came behind
+                const int at = p.pos[warp];
+                if (at >= 0 && at < p.n_pos) p.history[(size_t)warp * p.n_pos + at] = p.given ? p.token_in[warp] : p.token[warp];
+                p.token[warp] = ix;
+                p.pos[warp] = at + 1;
+                p.ctx[warp] += 1;
+                p.out[warp] = ix;
+            }
+        }
     }
 }
 

@@ -17,7 +17,11 @@ struct MegaParams {
     int n_layers;
     const float *tok_emb, *pos_emb, *lnf_g, *lnf_b, *lm_head_t;
     int rows;                        // sequences of the step
-    const int *token, *pos, *slot;   // [rows]; the slots are distinct
+    int *token, *pos, *ctx;          // [rows]
+    const int* slot;                 // [rows], distinct
+    int given, advance;              // given: the ids are token_in. advance: as the kernel of that name does for the other steps (the slots are 0 ... rows - 1)
+    int token_in[kMegaMaxRows];
+    int *history, *out;              // [slots][n_pos]; [rows] in pinned memory
     unsigned char *qkv, *att_part, *att, *pc, *mh, *pe, *cand;   // {value, flag} words: vectors of kMegaMaxRows rows, partials and candidates per CTA
     uint32_t epoch;                  // flags of this step are epoch + 1 ... epoch + n_layers + 1
     float* logits;                   // [rows][vocab]
