@@ -335,16 +335,28 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
     if (m.one_kernel_step(T) && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
         // a token each of a few sequences: the whole step is one cooperative kernel
-        MegaParams P = m.mega;
-        P.rows = T;
-        m.mega.epoch += (uint32_t)c.n_layers + 1u;   // every word of this step carries a flag that no other step's does
-        P.greedy = temperature <= 0.f ? 1 : 0;
-        P.advance = m.step_advance ? 1 : 0;
-        P.given = m.step_tokens ? 1 : 0;
-        if (m.step_tokens) memcpy(P.token_in, m.step_tokens, (size_t)T * 4);
+        auto call = [&](auto& P) {
+            P.rows = T;
+            P.advance = m.step_advance ? 1 : 0;
+            P.given = m.step_tokens ? 1 : 0;
+            if (m.step_tokens) memcpy(P.token_in, m.step_tokens, (size_t)T * 4);
+        };
+        int r;
         m.launches += 1;
-        int r = mega_launch(P, st);
-        if (r || P.greedy) return r;
+        // every word of this step carries a flag that no other step's does
+        if (m.f32()) {
+            MegaParams P = m.mega;
+            call(P);
+            P.greedy = temperature <= 0.f ? 1 : 0;
+            m.mega.epoch += (uint32_t)c.n_layers + 1u;
+            r = mega_launch(P, st);
+        } else {
+            QuantStepParams P = m.qstep;
+            call(P);
+            m.qstep.epoch += (uint32_t)c.n_layers + 1u;
+            r = quant_step_launch(c.weight_mode == kModeW4 ? 4 : 8, P, max_ctx, st);
+        }
+        if (r || temperature <= 0.f) return r;
         ++m.launches;
         return gptrs_cuda_sample_rows_top_k(m.logits.as<float>(), T, c.vocab, temperature, m.top_k, m.sample_seed, m.d_sampled.as<int32_t>(), st);
     }
@@ -723,6 +735,43 @@ int setup_mega(Model& m) {
     return GPTRS_OK;
 }
 
+// The single-kernel decode step of the quantised Ministral kind. GPTRS_QUANT_STEP=0 keeps the kernel-per-projection path.
+int setup_quant_step(Model& m) {
+    const auto& c = m.cfg;
+    if (const char* e = getenv("GPTRS_QUANT_STEP")) if (atoi(e) == 0) return GPTRS_OK;
+    if (m.f32() || c.kind != kKindMinistral || m.tp != 1 || !m.fold_norm || c.head_dim != 128 || c.rotary_dim != 128) return GPTRS_OK;
+    const int bits = c.weight_mode == kModeW4 ? 4 : 8;
+    const int rows = quant_step_max_rows(bits, c.n_layers, c.d_model, c.d_mlp, c.n_q_heads, c.n_kv_heads, c.vocab);
+    if (!rows) return GPTRS_OK;
+    int rc = m.qstep_exchange.alloc(quant_step_exchange_bytes(c.d_model, c.d_mlp, c.n_q_heads, c.n_kv_heads), true);
+    if (rc) return rc;
+    QuantStepParams& P = m.qstep;
+    auto packed = [](const Weight& w) { return static_cast<const unsigned char*>(w.packed->data); };
+    auto gain = [](Tensor* t) { return static_cast<const float*>(t->data); };
+    for (int l = 0; l < c.n_layers; ++l) {
+        const Layer& L = m.layers[l];
+        P.layers[l] = {packed(L.qkv), packed(L.attn_out), packed(L.mlp_gate_up), packed(L.mlp_out), gain(L.ln1_g), gain(L.ln2_g)};
+    }
+    P.n_layers = c.n_layers;
+    P.D = c.d_model; P.FF = c.d_mlp; P.Hq = c.n_q_heads; P.Hkv = c.n_kv_heads; P.vocab = c.vocab;
+    P.tok_emb = gain(m.tok_emb); P.final_gain = gain(m.final_g); P.cos_table = m.cos_tab.as<float>(); P.sin_table = m.sin_tab.as<float>();
+    P.w_head = packed(m.lm_head);
+    P.token = m.d_tokens.as<int>(); P.pos = m.d_pos.as<int>(); P.slot = m.d_slot.as<int>(); P.ctx = m.d_ctx.as<int>(); P.page_table = m.d_page_table.as<int>();
+    P.history = m.history.as<int>(); P.out = m.step_out(); P.context_length = c.context_length;
+    P.max_pages = c.max_pages_per_seq;
+    P.max_len = std::min((int)c.max_pages_per_seq * kPage, (int)c.context_length);
+    P.pool = m.kv_pool.as<unsigned char>();
+    P.pool_layer_bytes = m.pool_layer_bytes;
+    P.exchange = m.qstep_exchange.as<unsigned char>();
+    P.logits = m.logits.as<float>();
+    P.sampled = m.d_sampled.as<int>();
+    P.status = m.d_status.as<int32_t>();
+    P.eps = c.norm_eps;
+    P.scale_log2 = 1.4426950408889634f / sqrtf(128.f);
+    m.qstep_rows = rows;
+    return GPTRS_OK;
+}
+
 // Maps every peer's receive region into this process (CUDA IPC) so that the row-parallel partial sums of a decode
 // step travel as plain stores over NVLink. The 64-byte handles are exchanged with the communicator that already
 // exists; if any rank cannot map any peer, every rank stays on ncclAllReduce (the ranks agree through one more
@@ -1086,7 +1135,7 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
         worst = std::min<size_t>(worst, (size_t)1 << 30);
         if ((rc = m.attn_scratch.alloc(worst))) return rc;
     }
-    if ((rc = setup_mega(m))) return rc;
+    if ((rc = setup_mega(m)) || (rc = setup_quant_step(m))) return rc;
     GPTRS_CUDA_OK(cudaStreamSynchronize(m.stream));
     m.finalized = true;
     return GPTRS_OK;
@@ -1336,7 +1385,7 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
     int rc = sync_page_table(m);
     if (rc) return rc;
     cudaStream_t s = m.stream;
-    const bool own_step = m.f32() && m.one_kernel_step(B);   // takes the ids as parameters and advances its sequences itself
+    const bool own_step = m.one_kernel_step(B);   // takes the ids as parameters and advances its sequences itself
     if (h_tokens_in && !own_step) {
         GPTRS_CUDA_OK(cudaStreamSynchronize(s));  // the staging buffer may still feed an earlier copy
         memcpy(m.h_stage, h_tokens_in, (size_t)B * 4);

@@ -14,6 +14,7 @@
 #include "nccl_dl.h"
 #include "peer_allreduce.h"
 #include "gpt_decode_mega.h"
+#include "quant_step.h"
 #include "tensor.h"
 
 namespace gptrs {
@@ -217,9 +218,13 @@ struct Model {
     Tensor* wide = nullptr;         // W4 prompts: the widened weights of one projection at a time (a block of the tensor pool: a dropped f32 leaf's)
     DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
     MegaParams mega = {};
+    // quantised Ministral kind, a few sequences: the same (quant_step.cu)
+    int qstep_rows = 0;
+    QuantStepParams qstep = {};
+    DevBuf qstep_exchange;
     AttentionF32Plan attn_f32;      // f32 kinds: the split of the pass under way, its lists in d_attn_f32
     DevBuf d_attn_f32;
-    // single-kernel f32 steps: the ids that the generator gives (null: those on the device), and whether the kernel advances its sequences
+    // single-kernel steps: the ids that the generator gives (null: those on the device), and whether the kernel advances its sequences
     const int32_t* step_tokens = nullptr;
     bool step_advance = false;
     int gen_batch = 0;  // slots 0..gen_batch-1 are driven by generator_step
@@ -232,7 +237,7 @@ struct Model {
     bool f32() const { return cfg.weight_mode == kModeF32; }
     bool layered() const { return cfg.kind == kKindLayered; }
     bool paged() const { return !f32() || layered(); }
-    bool one_kernel_step(int rows) const { return rows <= mega_rows && rows <= max_rows(); }
+    bool one_kernel_step(int rows) const { return rows <= std::max(mega_rows, qstep_rows) && rows <= max_rows(); }
     int max_rows() const { return cfg.max_logit_rows > 0 ? cfg.max_logit_rows : cfg.max_seqs; }
     int stage_stride() const { return std::max(cfg.max_tokens, max_rows()); }
 

@@ -1,0 +1,80 @@
+"""The single-kernel decode step of quantised models: fewer tiles than CTAs and warps without a unit, tiles over several warps, group sizes, contexts
+around the edges of pages and slices of attention, ids from the device and given, against the oracle and the kernel-per-projection path."""
+import numpy as np
+import pytest
+
+from gptrs_b200 import model as gm
+from oracle import models_ref as mr
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(mode, n_q, n_kv, d, mlp, vocab, batch, ctx, params, namespace):
+    pages = (ctx + 15) // 16
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_MINISTRAL, 2, d, n_q, n_kv, 128, mlp, vocab, ctx, 1e-5, 1e4, 128,
+                                      weight_mode=gm.MODE_W4A16 if mode == "w4" else gm.MODE_W8A16, max_seqs=batch, max_tokens=1024, max_logit_rows=batch,
+                                      kv_pages=batch * pages + 4, max_pages_per_seq=pages, use_pdl=1), namespace=namespace)
+    for name, w in params.items():
+        m.load_param(name, w)
+    m.finalize()
+    return m
+
+
+@pytest.mark.parametrize("mode,n_q,n_kv,d,mlp,vocab,lengths", [
+    ("w4", 1, 1, 128, 128, 64, [1]),                       # one group of 128 k, eight tiles: most CTAs and warps have nothing
+    ("w8", 2, 1, 128, 256, 32, [15, 16, 17]),
+    ("w4", 8, 1, 384, 640, 1616, [223]), ("w4", 8, 1, 384, 640, 1616, [224]), ("w8", 8, 1, 384, 640, 1616, [225, 111]),   # one slice, two slices of pages
+    ("w4", 32, 8, 3072, 1152, 256, [40, 350]),             # odd numbers of units per stage; two tiles of the residual stream in some CTAs
+    ("w8", 16, 4, 2048, 4864, 256, [100, 7, 64, 65, 31, 1, 200, 90]),
+    ("w4", 6, 2, 256, 5120, 512, [129, 128, 127, 30, 2]),  # groups of three query heads
+    ("w4", 4, 4, 512, 512, 256, [600, 17, 33, 500, 18, 1, 300, 16])])
+def test_steps_follow_the_oracle(cuda, mode, n_q, n_kv, d, mlp, vocab, lengths):
+    batch, ctx = len(lengths), (max(lengths) + 24 + 15) // 16 * 16
+    cfg = mr.Cfg("ministral", n_layers=2, d_model=d, n_q=n_q, n_kv=n_kv, hd=128, d_mlp=mlp, vocab=vocab, ctx=ctx, rot=128, theta=1e4)
+    params = mr.random_params(cfg, seed=batch + d, std=0.5 * d ** -0.5)
+    params["tok_embeddings.weight"] = np.random.default_rng(0).normal(0, 1, (vocab, d)).astype(np.float32)
+    params["lm_head"] = (np.roll(params["tok_embeddings.weight"], 1, 0).T * d ** -0.5).astype(np.float32)   # no close calls
+    q = mr.quantised_params(cfg, params, mode)
+    m = _model(mode, n_q, n_kv, d, mlp, vocab, batch, ctx, params, 7900 + d + batch + lengths[0] * 7)
+    rng = np.random.default_rng(batch)
+    prompts = [rng.integers(0, vocab, n) for n in lengths]
+    refs = [mr.RefModel(cfg, q) for _ in prompts]
+    for r, p in zip(refs, prompts):
+        r.forward(p)
+    m.prefill_many(list(range(batch)), prompts)
+    launches = m.stats()["kernel_launches"]
+    given = rng.integers(0, vocab, (4, batch))
+    gen = gm.Generator(m, given[0])
+    for row in given[:3]:
+        want = np.stack([r.forward([int(t)])[-1] for r, t in zip(refs, row)])
+        got = gen.step(row)
+        assert got.tolist() == want.argmax(1).tolist()
+    assert m.stats()["kernel_launches"] == launches + 3   # one each
+    # the ids of the last step, from the device; then a pass that sees what the steps left in the cache
+    want = np.stack([r.forward([int(t)])[-1] for r, t in zip(refs, got)])
+    assert gen.step().tolist() == want.argmax(1).tolist()
+    want = np.stack([r.forward([int(t)])[-1] for r, t in zip(refs, given[3])])
+    logits, _ = m.forward_with_decode_cache(given[3], list(range(batch)), [n + 4 for n in lengths], list(range(batch)))   # one row: the kernel itself
+    assert np.sqrt(np.mean((logits - want) ** 2)) <= 2e-2 * np.sqrt(np.mean(want ** 2))   # bf16 activations through two layers
+
+
+@pytest.mark.parametrize("mode", ["w4", "w8"])
+def test_window_slide_and_sampling(cuda, mode, monkeypatch):
+    """Steps across the end of the context window, and a temperature draw of one row, as the kernel-per-projection path does them."""
+    d, vocab, ctx = 256, 512, 64
+    cfg = mr.Cfg("ministral", n_layers=2, d_model=d, n_q=4, n_kv=2, hd=128, d_mlp=512, vocab=vocab, ctx=ctx, rot=128, theta=1e4)
+    params = mr.random_params(cfg, seed=3, std=0.05)
+    params["tok_embeddings.weight"] = np.random.default_rng(0).normal(0, 1, (vocab, d)).astype(np.float32)
+    params["lm_head"] = (np.roll(params["tok_embeddings.weight"], 1, 0).T * d ** -0.5).astype(np.float32)
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("GPTRS_QUANT_STEP", on)
+        m = _model(mode, 4, 2, d, 512, vocab, 2, ctx, params, 7700 + (mode == "w8"))
+        m.prefill_many([0, 1], [np.arange(60) % vocab, np.arange(50) % vocab])
+        gen = gm.Generator(m, [5, 6])
+        ids = [gen.step().tolist() for _ in range(20)]
+        m.reset_sequence(0)
+        m.prefill(0, list(range(30)))
+        _, drawn = m.forward_with_decode_cache([7], [0], [30], [0], temperature=0.8, seed=11)
+        out.append((ids, drawn.tolist()))
+    assert out[0] == out[1]
