@@ -439,13 +439,13 @@ class LoadedModel:
         (optional) and greedy id of the LAST prompt row (the generator's first sampled token)."""
         chunk = chunk or self.config.max_tokens
         start = self.sequence_length(slot)
-        tokens = list(tokens)
+        tokens = np.ascontiguousarray(tokens if isinstance(tokens, np.ndarray) else list(tokens), dtype=np.int32)
         logits, sampled = None, None
         for o in range(0, len(tokens), chunk):
             part = tokens[o:o + chunk]
             last = o + len(part) == len(tokens)
             lg, sm = self.forward_with_decode_cache(
-                part, [slot] * len(part), list(range(start + o, start + o + len(part))),
+                part, np.full(len(part), slot, dtype=np.int32), np.arange(start + o, start + o + len(part), dtype=np.int32),
                 [len(part) - 1] if last else [], want_logits=want_logits and last)
             if last:
                 logits, sampled = lg, sm
@@ -470,30 +470,34 @@ class LoadedModel:
             align = 1
         max_rows = cfg.max_logit_rows if cfg.max_logit_rows > 0 else cfg.max_seqs
         first = [None] * len(prompts)
-        tok, sl, pos, rows, owners = [], [], [], [], []
+        tok, sl, pos, rows, owners = [], [], [], [], []   # pieces of the pass that is being packed; its logit rows and whose they are
+        packed = 0
 
         def flush():
-            if not tok:
+            nonlocal packed
+            if not packed:
                 return
-            _, sampled = self.forward_with_decode_cache(tok, sl, pos, rows, want_logits=False)
+            _, sampled = self.forward_with_decode_cache(np.concatenate(tok), np.concatenate(sl), np.concatenate(pos), rows, want_logits=False)
             for r, o in enumerate(owners):
                 first[o] = int(sampled[r])
             tok.clear(), sl.clear(), pos.clear(), rows.clear(), owners.clear()
+            packed = 0
 
         for i, (slot, prompt) in enumerate(zip(slots, prompts)):
             prompt = np.asarray(prompt, dtype=np.int32)
             start = self.sequence_length(slot)
             done = 0
             while done < len(prompt):
-                n = min(len(prompt) - done, chunk - len(tok))
-                tok.extend(prompt[done:done + n].tolist())
-                sl.extend([slot] * n)
-                pos.extend(range(start + done, start + done + n))
+                n = min(len(prompt) - done, chunk - packed)
+                tok.append(prompt[done:done + n])
+                sl.append(np.full(n, slot, dtype=np.int32))
+                pos.append(np.arange(start + done, start + done + n, dtype=np.int32))
+                packed += n
                 done += n
                 if done == len(prompt):
-                    rows.append(len(tok) - 1)
+                    rows.append(packed - 1)
                     owners.append(i)
-                if len(tok) == chunk or (done == len(prompt) and (len(tok) % align != 0 or len(rows) == max_rows)):
+                if packed == chunk or (done == len(prompt) and (packed % align != 0 or len(rows) == max_rows)):
                     flush()
         flush()
         return first
