@@ -23,6 +23,7 @@
 
 #include "engine.h"
 #include "split_f32.cuh"
+#include "split_planes.cuh"
 
 namespace gptrs {
 
@@ -209,6 +210,24 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
            bool swiglu, bool gelu, cudaStream_t st, const NormFold* fold = nullptr, const PeerView* push = nullptr,
            bool pick = false) {
     ++m.launches;
+    // Planes that the kernel in front has left serve the projection right behind it and no other: whatever it is, they are forgotten here.
+    const bool ready = m.planes.of == x && m.planes.rows == rows && m.planes.k == w.in;
+    m.planes.of = nullptr;
+    // f32 rows against weights whose planes lie ready (GPT-2 small, a pass in us, this side / split_f32_kernel: 24 rows 838 / 1075, 64 rows
+    // 900 / 1304, 128 rows 1062 / 1285, 300 rows 1361 / 2002, 937 rows 2753 / 4347); fewer rows stay with the tiled FMA kernels.
+    if (m.f32() && w.planes && rows >= kSplitF32Rows && st == m.stream && !(fold && fold->f32_norm)) {
+        const float* xf = static_cast<const float*>(x);
+        if (!ready) {
+            ++m.launches;
+            m.planes.turn ^= 1;
+            if (int rc = split_row_planes(xf, m.planes_at(), rows, w.in, st)) return rc;
+        }
+        void* const own = m.planes_at();
+        const bool leave = gelu && w.out % 64 == 0;   // the projection behind this one reads its rows
+        if (leave) m.planes.leave(y, rows, w.out);
+        return planes_matmul({w.planes, own, xf, static_cast<const float*>(w.f32->data), w.bias ? static_cast<const float*>(w.bias->data) : nullptr, residual,
+                              static_cast<float*>(y), leave ? m.planes_at() : nullptr, (int)rows, (int)w.out, (int)w.in, gelu ? 1 : 0, m.d_status.as<int32_t>()}, st);
+    }
     if (m.f32()) {
         return norm_matmul_f32(static_cast<const float*>(x), fold ? fold->f32_norm : 0, fold ? fold->f32_gamma : nullptr,
                                           fold ? fold->f32_beta : nullptr, m.cfg.norm_eps, static_cast<const float*>(w.f32->data),
@@ -328,6 +347,7 @@ size_t sumsq_floats(int d_model, int rows) { return (size_t)rows * (d_model / (r
 int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, bool rows_identity, float temperature,
                     int prefill_groups = 0, bool skip_logits = false) {
     if (m.layered()) return layered_forward(m, T, max_ctx, n_rows, rows_identity, temperature, skip_logits);
+    m.planes.of = nullptr;
     const auto& c = m.cfg;
     const int D = c.d_model;
     cudaStream_t st = m.stream;
@@ -449,6 +469,10 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
             pending_peer = false;
             return add_norm_peer(h, delta, m.peer, m.d_status.as<int32_t>(), kPeerSpinLimit, (const float*)g->data,
                                  gpt ? (const float*)b->data : nullptr, c.norm_eps, xn, act_dt, ln.T, D, gpt, ln.st);
+        }
+        if (m.x_planes.p && !delta && ln.T >= kSplitF32Rows && ln.st == m.stream && norm_planes_takes(D)) {   // split for the projection behind it
+            m.planes.leave(xn, ln.T, D);
+            return norm_planes(h, (const float*)g->data, gpt && b ? (const float*)b->data : nullptr, c.norm_eps, gpt, static_cast<float*>(xn), m.planes_at(), ln.T, D, ln.st);
         }
         return gpt ? gptrs_cuda_add_layer_norm(h, delta, GPTRS_F32, nullptr, (const float*)g->data, (const float*)b->data,
                                                c.norm_eps, xn, act_dt, nullptr, nullptr, ln.T, D, ln.st)
@@ -732,6 +756,36 @@ int setup_mega(Model& m) {
     P.H = c.n_q_heads; P.hd = c.head_dim; P.vocab = c.vocab; P.ctx_cap = c.context_length;
     P.n_pos = c.context_length; P.eps = c.norm_eps; P.greedy = 1;
     m.mega_rows = mega_max_rows(c.n_q_heads, c.head_dim, c.context_length);
+    return GPTRS_OK;
+}
+
+// bf16 planes of the layers' f32 weights, for passes of many rows: six bytes more per weight, so only for models whose planes take 2 GiB at
+// most and where the memory is there; other models split inside their tiles.
+int setup_planes(Model& m) {
+    const auto& c = m.cfg;
+    if (!m.f32() || c.max_tokens < kSplitF32Rows) return GPTRS_OK;
+    std::vector<Weight*> all;
+    for (Layer& L : m.layers)
+        for (Weight* w : {&L.qkv, &L.attn_out, &L.mlp_in, &L.mlp_gate, &L.mlp_up, &L.mlp_out})
+            if (w->f32 && w->in % 64 == 0 && w->out % 4 == 0) all.push_back(w);
+    size_t total = 0;
+    int64_t widest = 0;
+    for (const Weight* w : all) { total += plane_bytes(w->out, w->in); widest = std::max(widest, w->in); }
+    if (!total || total > ((size_t)2 << 30)) return GPTRS_OK;
+    int rc;
+    m.planes.half = (plane_bytes(c.max_tokens, widest) + 255) & ~(size_t)255;
+    if (m.w_planes.alloc(total) || m.x_planes.alloc(2 * m.planes.half)) {
+        cudaGetLastError();
+        m.w_planes.release();
+        m.x_planes.release();
+        return GPTRS_OK;
+    }
+    unsigned char* at = m.w_planes.as<unsigned char>();
+    for (Weight* w : all) {
+        if ((rc = split_weight_planes(static_cast<const float*>(w->f32->data), at, w->in, w->out, m.stream))) return rc;
+        w->planes = at;
+        at += plane_bytes(w->out, w->in);
+    }
     return GPTRS_OK;
 }
 
@@ -1135,7 +1189,7 @@ int gptrs_cuda_model_finalize(gptrs_model* h, int drop_f32_leaves) {
         worst = std::min<size_t>(worst, (size_t)1 << 30);
         if ((rc = m.attn_scratch.alloc(worst))) return rc;
     }
-    if ((rc = setup_mega(m)) || (rc = setup_quant_step(m))) return rc;
+    if ((rc = setup_mega(m)) || (rc = setup_quant_step(m)) || (rc = setup_planes(m))) return rc;
     GPTRS_CUDA_OK(cudaStreamSynchronize(m.stream));
     m.finalized = true;
     return GPTRS_OK;
@@ -1275,7 +1329,9 @@ int gptrs_cuda_model_forward_with_decode_cache(gptrs_model* h, const int32_t* h_
     // hybrid of width 2048, 64 rows 941 / 857, 128 rows 1090 / 1046, 160 rows 1104 / 1100, 200 rows 1130 / 1206, 5855 rows 6500 / 6900; W4
     // of width 3072, 64 rows 420 / 356, 256 rows 791 / 729; W8 of width 2048, 256 rows 552 / 501; GPT-2, 256 rows 1766 / 1692.
     const int pdl_before = g_use_pdl;
-    if (c.use_pdl && T <= (m.layered() ? 128 : 256)) g_use_pdl = 1;
+    // With the weights' planes, whose first tiles travel while the kernel in front ends, early launches pay at every size: GPT-2 without /
+    // with, 300 rows 1602 / 1361, 512 rows 1858 / 1660, 937 rows 3000 / 2753.
+    if (c.use_pdl && (m.w_planes.p || T <= (m.layered() ? 128 : 256))) g_use_pdl = 1;
     rc = enqueue_forward(m, T, max_ctx, chunk, rows, false, temperature, prefill_groups);
     g_use_pdl = pdl_before;
     if (rc) return rc;

@@ -44,6 +44,7 @@ struct Weight {        // one Linear
     Tensor* f32 = nullptr;     // [in][out] (f32 mode)
     Tensor* packed = nullptr;  // quantised + repacked (W4/W8 modes)
     Tensor* bias = nullptr;    // optional [out]
+    void* planes = nullptr;    // f32 mode: the transpose as bf16 planes (split_planes.cuh), in Model::w_planes
     int64_t in = 0, out = 0;
 };
 
@@ -222,6 +223,15 @@ struct Model {
     int qstep_rows = 0;
     QuantStepParams qstep = {};
     DevBuf qstep_exchange;
+    DevBuf w_planes, x_planes;      // f32 kinds: planes of the layers' weights; of the rows of the projection under way (in halves, by turns)
+    struct {                        // while a pass is enqueued: whose planes lie in the half of x_planes whose turn it is
+        const void* of = nullptr;
+        int64_t rows = 0, k = 0;
+        size_t half = 0;
+        int turn = 0;
+        void leave(const void* y, int64_t r, int64_t n) { of = y; rows = r; k = n; turn ^= 1; }
+    } planes;
+    void* planes_at() const { return x_planes.as<unsigned char>() + planes.turn * planes.half; }
     AttentionF32Plan attn_f32;      // f32 kinds: the split of the pass under way, its lists in d_attn_f32
     DevBuf d_attn_f32;
     // single-kernel steps: the ids that the generator gives (null: those on the device), and whether the kernel advances its sequences
