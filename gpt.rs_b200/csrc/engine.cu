@@ -213,8 +213,8 @@ int linear(Model& m, const Weight& w, const void* x, void* y, int64_t rows, bool
     // Planes that the kernel in front has left serve the projection right behind it and no other: whatever it is, they are forgotten here.
     const bool ready = m.planes.of == x && m.planes.rows == rows && m.planes.k == w.in;
     m.planes.of = nullptr;
-    // f32 rows against weights whose planes lie ready (GPT-2 small, a pass in us, this side / split_f32_kernel: 24 rows 838 / 1075, 64 rows
-    // 900 / 1304, 128 rows 1062 / 1285, 300 rows 1361 / 2002, 937 rows 2753 / 4347); fewer rows stay with the tiled FMA kernels.
+    // f32 rows against weights whose planes lie ready (GPT-2 small, a pass in us, this side / split_f32_kernel: 24 rows 823 / 1075, 64 rows
+    // 893 / 1304, 128 rows 998 / 1285, 300 rows 1350 / 2002, 937 rows 2432 / 4347); fewer rows stay with the tiled FMA kernels.
     if (m.f32() && w.planes && rows >= kSplitF32Rows && st == m.stream && !(fold && fold->f32_norm)) {
         const float* xf = static_cast<const float*>(x);
         if (!ready) {

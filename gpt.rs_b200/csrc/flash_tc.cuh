@@ -135,12 +135,6 @@ __device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr, uint32_t group_
     d |= (uint64_t)2 << 61;
     return d;
 }
-// true in one lane of a converged warp; unlike a test of the lane number it leaves the branch known to be warp-uniform
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ float ex2f(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));

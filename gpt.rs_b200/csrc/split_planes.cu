@@ -6,11 +6,13 @@
 // split_f32_kernel splits inside its tiles: 512 threads load, split, store and fence every 32 k, 2900 cycles a stage, of which the MMAs are 770.
 // Here a loader warp requests the planes by TMA, one warp issues the MMAs and eight warps add up the leading sums beside them. CTA: 128 output
 // channels (M side of the MMA) x BN rows, stages of 64 k in the 128-byte swizzle (two blocks of planes 1 and 2 of 32 k each, one block of plane
-// 3). What bounds it: the planes from L2, 96 KB per 64 k and CTA of 128 rows, beside 1536 cycles of MMA. The weights' first stages are under
-// way before the kernel in front has ended, and the norms and the GELU leave the planes of their rows themselves.
+// 3). What bounds it: the MMAs, 24 x BN / 2 cycles a stage (0.95 us with 128 rows), and what a CTA does once, 7 to 10 us. The weights' first
+// stages are under way before the kernel in front has ended, and the norms and the GELU leave the planes of their rows themselves.
 // K is split over a cluster where the output tiles do not fill the SMs, the parts meet in the shared memory of the CTA that owns the row; the
 // epilogue then takes four neighbouring channels per thread (a channel per thread and scalar residuals took 10 to 17 us more at 937 rows).
-// GPT-2 small at 937 rows, us, split_f32_kernel / this: qkv 47 / 25, attention output 33 / 20, MLP in 96 / 55, MLP out 83 / 43.
+// Pieces of a third of a stage, in rings of 6 to 11, bring nothing: what the loads take is hidden with two stages.
+// GPT-2 small, us, split_f32_kernel / this: at 937 rows qkv 47 / 20, attention output 33 / 16, MLP in 96 / 32, MLP out 83 / 32; at 64 rows
+// qkv 11 / 7.5, MLP out 16 / 10.
 #include "matmul_common.cuh"
 #include "split_planes.cuh"
 #include "umma_common.cuh"
@@ -76,18 +78,29 @@ struct KernelParams {
     int n_split;
 };
 
+// 32 lanes x 16 columns of this warp's quarter of the tensor memory
+__device__ __forceinline__ void tmem_ld_16(uint32_t at, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(at));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 constexpr int kThreads = 320;   // warps 0-7 sums and epilogue, 8 loader, 9 MMA + tensor memory
-template <int BN> constexpr int kStages = BN == 128 ? 2 : 3;
+template <int BN> constexpr int kStages = BN >= 128 ? 2 : 3;   // of 64 k, and as many accumulators of leading sums
 template <int BN> constexpr int kStageBytes = 3 * kBlock + 3 * BN * 128;
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid_constant__ KernelParams kp) {
     constexpr int S = kStages<BN>, kStage = kStageBytes<BN>, kX = BN * 128, kSumCols = BN >= 64 ? BN / 2 : 32;   // columns of a summing thread
     constexpr int kSumWarps = 4 * (BN / kSumCols);
-    constexpr uint32_t kCols = BN == 128 ? 512 : BN == 64 ? 256 : 128;
+    constexpr uint32_t kCols = BN >= 128 ? 512 : BN == 64 ? 256 : 128;
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (8u << 24);
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full[S], empty[S], lead_full[2], lead_empty[2];
+    __shared__ __align__(8) uint64_t full[S], done[S], lead_empty[S];
     __shared__ uint32_t tmem_holder;
     unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const PlanesMatmul& p = kp.q;
@@ -96,8 +109,7 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
     const int k_tiles = p.K / 64;
     const int kt0 = k_tiles * (int)blockIdx.y / kp.n_split, n_k = k_tiles * ((int)blockIdx.y + 1) / kp.n_split - kt0;
     if (tid == 0) {
-        for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&lead_full[i], 1); mbar_init(&lead_empty[i], 32 * kSumWarps); }
+        for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&done[s], 1); mbar_init(&lead_empty[s], 32 * kSumWarps); }
         mbar_fence_init();
     }
     if (warp == 9) {
@@ -143,21 +155,24 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
         __syncwarp();
         int last = min(S, n_k);
         for (int it = S; it < n_k; ++it) {
-            if (!wait(&empty[it % S], (uint32_t)(it / S - 1) & 1u)) break;
+            if (!wait(&done[it % S], (uint32_t)(it / S - 1) & 1u)) break;
             if (lane == 0) load(it, true, true);
             __syncwarp();
             last = it + 1;
         }
         for (int i = max(last - S, 0); i < last; ++i) mbar_wait_relaxed(&full[i % S], (uint32_t)(i / S) & 1u);   // what is in flight writes this CTA's shared memory
     } else if (warp == 9) {
-        for (int it = 0; it < n_k; ++it) {
-            const int s = it % S, b = it & 1;
-            if (it >= 2 && !wait(&lead_empty[b], (uint32_t)(it / 2 - 1) & 1u)) break;
-            if (!wait(&full[s], (uint32_t)(it / S) & 1u)) break;
-            tc_fence_after();
-            if (lane == 0) {
+        // One elected thread waits and issues for the whole loop: with the warp voting at every wait, lane 0 issuing and a commit per consumer, a
+        // stage of 128 rows took 1.45 us instead of 0.95, one of 32 rows 1.25 instead of 0.68.
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            for (int it = 0; it < n_k; ++it) {
+                if (it >= S && !mbar_wait_relaxed(&lead_empty[s], phase ^ 1u)) { failed = true; break; }
+                if (!mbar_wait_relaxed(&full[s], phase)) { failed = true; break; }
+                tc_fence_after();
                 const uint32_t at = smem_u32(smem) + (uint32_t)(s * kStage);
-                const uint32_t lead = tmem + (uint32_t)(b * BN), rest = tmem + 2u * BN;
+                const uint32_t lead = tmem + (uint32_t)(s * BN), rest = tmem + (uint32_t)(S * BN);
                 const uint64_t w3 = make_smem_desc(at + 2 * kBlock), x3 = make_smem_desc(at + 3 * kBlock + 2 * kX);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {   // K steps of 16 are 2 descriptor units apart; plane 2 lies 4 units behind plane 1
@@ -169,38 +184,45 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
                     umma_bf16(rest, w + 4, x, kIdesc, 1u);
                     umma_bf16(rest, w, x + 4, kIdesc, 1u);
                 }
-                umma_commit(&empty[s]);
-                umma_commit(&lead_full[b]);
+                umma_commit(&done[s]);
+                if (++s == S) { s = 0; phase ^= 1u; }
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else if (sums) {
 #pragma unroll
         for (int i = 0; i < kSumCols; ++i) acc[i] = 0.f;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c_lo;
         auto add = [&](uint32_t at) {
 #pragma unroll
-            for (int h = 0; h < kSumCols; h += 32) {
+            for (int h = 0; h < kSumCols / 32 * 32; h += 32) {
                 float v[32];
                 tmem_ld_32(lane_base + at + (uint32_t)h, v);
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[h + i] += v[i];
             }
+            if constexpr (kSumCols % 32) {
+                constexpr int h = kSumCols / 32 * 32;
+                float v[16];
+                tmem_ld_16(lane_base + at + (uint32_t)h, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[h + i] += v[i];
+            }
         };
 #pragma unroll 1
         for (int it = 0; it < n_k; ++it) {
-            const int b = it & 1;
-            if (!wait(&lead_full[b], (uint32_t)(it / 2) & 1u)) break;
+            const int b = it % S;
+            if (!wait(&done[b], (uint32_t)(it / S) & 1u)) break;
             tc_fence_after();
             add((uint32_t)(b * BN));
             tc_fence_before();
             mbar_arrive(&lead_empty[b]);
         }
         tc_fence_after();
-        add(2u * BN);   // complete with the last stage's leading sums
+        add((uint32_t)(S * BN));   // complete with the last stage's leading sums
         pdl_wait();     // what the epilogue reads (residual, x of a repeated sum)
     }
-    if (failed && lane == 0) atomicExch(p.status, 3);
+    if (failed) atomicExch(p.status, 3);
     tc_fence_before();
     __syncthreads();
     if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kCols) : "memory");
@@ -209,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
     // Row r of the tile belongs to rank r % parts of the cluster; its slots [rank][row / parts][128] lie over the stages, so nobody pushes before
     // everybody's MMAs have read theirs.
     if (parts > 1) cluster_sync_all();
-    const uint32_t inv = (65536u + (uint32_t)parts - 1u) / (uint32_t)parts;   // r / parts == (r * inv) >> 16 for r < 128
+    const uint32_t inv = (65536u + (uint32_t)parts - 1u) / (uint32_t)parts;   // r / parts == (r * inv) >> 16 for r < 160
     auto push = [&](int r, int col, float v) {
         const int local = (int)(((uint32_t)r * inv) >> 16);
         const uint32_t at = smem_u32(smem) + (uint32_t)(((rank * rows_max + local) * 128 + col) * 4);
@@ -218,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
     };
     if (sums) {
         const int col = quarter * 32 + lane, n = n0 + col, k_lo = kt0 * 64, k_hi = (kt0 + n_k) * 64;
-        uint64_t special = 0;   // rows whose sum is not finite: once more, in f32
+        uint64_t special = 0, behind = 0;   // rows whose sum is not finite (behind: from the 64th on): once more, in f32
         if (parts == 1) {
             float* at = reinterpret_cast<float*>(smem) + c_lo * 128 + col;
 #pragma unroll
@@ -228,10 +250,12 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
             for (int i = 0; i < kSumCols; ++i) push(c_lo + i, col, acc[i]);
         }
 #pragma unroll
-        for (int i = 0; i < kSumCols; ++i) special |= fabsf(acc[i]) < INFINITY ? 0ull : 1ull << i;
+        for (int i = 0; i < kSumCols; ++i) (i < 64 ? special : behind) |= fabsf(acc[i]) < INFINITY ? 0ull : 1ull << (i & 63);
 #pragma unroll 1
-        for (; special; special &= special - 1) {
-            const int r = c_lo + __ffsll((long long)special) - 1, m = m0 + r;
+        while (special | behind) {
+            const int r = c_lo + (special ? __ffsll((long long)special) - 1 : __ffsll((long long)behind) + 63), m = m0 + r;
+            if (special) special &= special - 1;
+            else behind &= behind - 1;
             if (m >= p.M || n >= p.N) continue;
             float sum = 0.f;
 #pragma unroll 1
@@ -327,6 +351,15 @@ int make_map(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, 
     return GPTRS_OK;
 }
 
+template <int BN> constexpr size_t kSmem = (size_t)kStages<BN> * kStageBytes<BN> + 1024;
+template <int BN>
+int allow_smem() {
+    static PerDeviceOnce once;
+    if (once.first_time())
+        GPTRS_CUDA_OK(cudaFuncSetAttribute(planes_matmul_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem<BN>));
+    return GPTRS_OK;
+}
+
 // How many CTAs of a cluster size run at one time, asked once per device.
 template <int BN>
 int64_t slots_of(int cluster) {
@@ -336,10 +369,11 @@ int64_t slots_of(int cluster) {
     if (n == 0) {
         n = sm_count();
         if (cluster > 1) {
+            allow_smem<BN>();
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(1, (unsigned)cluster, 1);
             cfg.blockDim = dim3(kThreads);
-            cfg.dynamicSmemBytes = (size_t)kStages<BN> * kStageBytes<BN> + 1024;
+            cfg.dynamicSmemBytes = kSmem<BN>;
             cudaLaunchAttribute attr;
             attr.id = cudaLaunchAttributeClusterDimension;
             attr.val.clusterDim.x = 1; attr.val.clusterDim.y = (unsigned)cluster; attr.val.clusterDim.z = 1;
@@ -355,25 +389,30 @@ int64_t slots_of(int cluster) {
 }
 
 template <int BN>
-int launch(const PlanesMatmul& q, cudaStream_t st) {
-    constexpr size_t smem = (size_t)kStages<BN> * kStageBytes<BN> + 1024;
-    static PerDeviceOnce attr_once;
-    if (attr_once.first_time())
-        GPTRS_CUDA_OK(cudaFuncSetAttribute(planes_matmul_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+int launch(const PlanesMatmul& q, int split, cudaStream_t st) {
+    if (int rc = allow_smem<BN>()) return rc;
     KernelParams p;
     p.q = q;
     const __nv_bfloat16 *w = static_cast<const __nv_bfloat16*>(q.w_planes), *x = static_cast<const __nv_bfloat16*>(q.x_planes);
     int rc;
     if ((rc = make_map(&p.w12, w, 2 * (uint64_t)q.K, (uint64_t)q.N, 128)) || (rc = make_map(&p.w3, w + (size_t)q.N * 2 * q.K, (uint64_t)q.K, (uint64_t)q.N, 128)) ||
         (rc = make_map(&p.x12, x, 2 * (uint64_t)q.K, (uint64_t)q.M, BN)) || (rc = make_map(&p.x3, x + (size_t)q.M * 2 * q.K, (uint64_t)q.K, (uint64_t)q.M, BN))) return rc;
-    // K parts: as many as make the last CTA end soonest, with the set-up, the reduction and the epilogue of a CTA as so many stages
+    p.n_split = split;
+    return launch_kernel(planes_matmul_kernel<BN>, dim3((unsigned)ceil_div(q.N, 128), (unsigned)p.n_split, (unsigned)ceil_div(q.M, BN)), dim3(kThreads), kSmem<BN>, st, p.n_split, p);
+}
+
+// The rows of a tile and the parts of K that make the last CTA end soonest, in hundredths of a microsecond as measured on GPT-2's projections
+// at 32 to 937 rows: a stage of 64 k takes 0.68 / 0.80 / 0.95 / 1.08 us with 32 / 64 / 128 / 160 rows, a CTA's beginning and end 6.4 / 7 / 9 / 10,
+// the exchange of the parts 1.5.
+struct Tiling { int rows = 0, split = 1; int64_t time = 1ll << 60; };
+template <int BN>
+void consider(const PlanesMatmul& q, Tiling& best) {
+    constexpr int64_t stage = BN == 32 ? 68 : BN == 64 ? 80 : BN == 128 ? 95 : 108, fixed = BN == 32 ? 640 : BN == 64 ? 700 : BN == 128 ? 900 : 1000;
     const int64_t ctas = (int64_t)ceil_div(q.N, 128) * ceil_div(q.M, BN), k_tiles = q.K / 64;
-    int64_t best = 1ll << 60;
     for (int s = 1; s <= 8 && s <= k_tiles; ++s) {
-        const int64_t slots = slots_of<BN>(s), t = ((ctas * s + slots - 1) / slots) * ((k_tiles + s - 1) / s + 4 + 2 * (s > 1));
-        if (t < best) { best = t; p.n_split = s; }
+        const int64_t slots = slots_of<BN>(s), t = ((ctas * s + slots - 1) / slots) * ((k_tiles + s - 1) / s * stage + fixed + (s > 1 ? 150 : 0));
+        if (t < best.time) best = {BN, s, t};
     }
-    return launch_kernel(planes_matmul_kernel<BN>, dim3((unsigned)ceil_div(q.N, 128), (unsigned)p.n_split, (unsigned)ceil_div(q.M, BN)), dim3(kThreads), smem, st, p.n_split, p);
 }
 
 }  // namespace
@@ -403,9 +442,14 @@ int planes_matmul(const PlanesMatmul& q, cudaStream_t st) {
     PlanesMatmul p = q;
     if (!p.status) p.status = matmul_status_word();
     if (!p.status) return fail(GPTRS_EXECUTION, "no status word");
-    if (p.M <= 32) return launch<32>(p, st);
-    if (p.M <= 64) return launch<64>(p, st);
-    return launch<128>(p, st);
+    Tiling t;
+    consider<32>(p, t); consider<64>(p, t); consider<128>(p, t); consider<160>(p, t);
+    switch (t.rows) {
+        case 32: return launch<32>(p, t.split, st);
+        case 64: return launch<64>(p, t.split, st);
+        case 128: return launch<128>(p, t.split, st);
+        default: return launch<160>(p, t.split, st);
+    }
 }
 
 }  // namespace gptrs

@@ -27,7 +27,7 @@ def run(d, heads, d_mlp, rows, edit=lambda p: None, layers=2, vocab=96):
     assert np.sqrt(np.mean((got - want) ** 2, axis=1)).max() <= 3e-6 * np.sqrt(np.mean(want ** 2))
 
 
-@pytest.mark.parametrize("rows", [23, 24, 32, 33, 64, 65, 128, 129, 160, 161, 300])
+@pytest.mark.parametrize("rows", [23, 24, 32, 33, 64, 65, 128, 129, 160, 161, 300, 480, 481])
 def test_rows_around_the_tiles(cuda, rows):
     run(256, 4, 1024, rows)
 
@@ -37,6 +37,11 @@ def test_rows_around_the_tiles(cuda, rows):
 @pytest.mark.parametrize("rows", [40, 140])
 def test_widths(cuda, d, heads, d_mlp, rows):
     run(d, heads, d_mlp, rows)
+
+
+@pytest.mark.parametrize("rows", [299, 320, 937])
+def test_tiles_of_160_rows(cuda, rows):
+    run(768, 12, 3072, rows)
 
 
 @pytest.mark.parametrize("rows", [30, 64, 200])
