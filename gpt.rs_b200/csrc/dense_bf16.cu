@@ -207,45 +207,46 @@ __global__ void __launch_bounds__(kRowsThreads, 1) dense_rows_kernel(const __gri
         return !failed;
     };
     if (warp == 5) {
-        int it = 0, last_it = 0;
-        for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
-            const Tile tl = tile_of(t);
-            const int m0 = tl.m0, n0 = tl.n0, b = tl.b;
-            for (int k = 0; k < n_k; ++k, ++it) {
-                const int s = it % STAGES;
-                if (it >= STAGES && !wait(&empty[s], (uint32_t)(it / STAGES - 1) & 1u)) break;
-                if (lane == 0) {
+        if (elect_one()) {   // one thread waits and requests, in warp 4 waits and issues: no votes of the warp between the stages
+            int it = 0, s = 0;
+            uint32_t phase = 1;
+            for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
+                const Tile tl = tile_of(t);
+                const int m0 = tl.m0, n0 = tl.n0, b = tl.b;
+                for (int k = 0; k < n_k; ++k, ++it) {
+                    if (it >= STAGES && !mbar_wait_relaxed(&empty[s], phase)) { failed = true; break; }
                     const uint32_t bar = smem_u32(&full[s]);
                     mbar_expect_tx_addr(bar, kStageBytes);
                     tma_load_2d(smem + s * kStageBytes, &p.x_map, (GROUPED ? 0 : b * p.x_step) + k * kBK, m0, bar);
                     tma_load_2d(smem + s * kStageBytes + kATile, &p.w_map, k * kBK, b * p.w_rows + n0, bar);
+                    if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-                __syncwarp();
-                last_it = it + 1;
             }
+            // stages in flight write this CTA's shared memory (only after a timeout are there any left unread)
+            for (int i = max(it - STAGES, 0); i < it; ++i) mbar_wait_relaxed(&full[i % STAGES], (uint32_t)(i / STAGES) & 1u);
         }
-        // stages in flight write this CTA's shared memory (only after a timeout are there any left unread)
-        for (int i = max(last_it - STAGES, 0); i < last_it; ++i) mbar_wait_relaxed(&full[i % STAGES], (uint32_t)(i / STAGES) & 1u);
+        __syncwarp();
     } else if (warp == 4) {
-        int it = 0, n = 0;
-        for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x, ++n) {
-            const int buf = n & 1;
-            if (n >= 2 && !wait(&acc_empty[buf], (uint32_t)(n / 2 - 1) & 1u)) break;
-            tc_fence_after();
-            for (int k = 0; k < n_k; ++k, ++it) {
-                const int s = it % STAGES;
-                if (!wait(&full[s], (uint32_t)(it / STAGES) & 1u)) break;
+        if (elect_one()) {
+            int s = 0, n = 0;
+            uint32_t phase = 0;
+            for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x, ++n) {
+                const int buf = n & 1;
+                if (n >= 2 && !mbar_wait_relaxed(&acc_empty[buf], (uint32_t)(n / 2 - 1) & 1u)) { failed = true; break; }
                 tc_fence_after();
-                if (lane == 0) {
+                for (int k = 0; k < n_k; ++k) {
+                    if (!mbar_wait_relaxed(&full[s], phase)) { failed = true; break; }
+                    tc_fence_after();
                     const uint64_t ad = make_smem_desc(smem_u32(smem + s * kStageBytes)), bd = make_smem_desc(smem_u32(smem + s * kStageBytes + kATile));
 #pragma unroll
                     for (int k4 = 0; k4 < 4; ++k4) umma_bf16(tmem + (uint32_t)(buf * BN), ad + 2 * k4, bd + 2 * k4, kIdesc, (k > 0 || k4 > 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
                     if (k == n_k - 1) umma_commit(&acc_full[buf]);
+                    if (++s == STAGES) { s = 0; phase ^= 1u; }
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (warp < 4 || warp >= 8) {
         const int quarter = warp & 3, c_lo = warp < 4 ? 0 : BN / 2;   // lane quarter and half of the columns
         int n = 0;
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) dense_rows_kernel(const __gri
             mbar_arrive(&acc_empty[buf]);
         }
     }
-    if (failed && lane == 0) atomicExch(p.status, 3);
+    if (failed) atomicExch(p.status, 3);
     tc_fence_before();
     __syncthreads();
     if (warp == 4) tmem_free(tmem, kCols);
@@ -401,36 +402,40 @@ __global__ void __launch_bounds__(kChThreads, BN <= 64 ? 2 : 1) dense_channels_k
     if constexpr (!GROUPED) pdl_wait();
     bool failed = false;
     if (warp == 8) {
-        for (int it = 0; it < n_k; ++it) {
-            const int s = it % STAGES;
-            if (it >= STAGES && !mbar_wait_relaxed(&empty[s], (uint32_t)(it / STAGES - 1) & 1u)) { failed = true; break; }
-            if (lane == 0) {
+        if (elect_one()) {   // one thread waits and requests, in warp 9 waits and issues
+            int s = 0;
+            uint32_t phase = 1;
+            for (int it = 0; it < n_k; ++it) {
+                if (it >= STAGES && !mbar_wait_relaxed(&empty[s], phase)) { failed = true; break; }
                 const uint32_t bar = smem_u32(&full[s]);
                 if (it >= STAGES) {
                     mbar_expect_tx_addr(bar, kStageBytes);
                     tma_load_2d(smem + s * kStageBytes, &cp.w_map, (k0 + it) * kBK, b * cp.w_rows + n0, bar);
                 }
                 tma_load_2d(smem + s * kStageBytes + kATile, &cp.x_map, (GROUPED ? 0 : b * cp.x_step) + (k0 + it) * kBK, m0, bar);
+                if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
-            __syncwarp();
         }
+        __syncwarp();
+        failed = __any_sync(0xffffffffu, failed);
         // copies in flight write this CTA's stages (only after a timeout are there any left unread)
         if (!failed)
             for (int it = max(n_k - STAGES, 0); it < n_k; ++it) mbar_wait_relaxed(&full[it % STAGES], (uint32_t)(it / STAGES) & 1u);
     } else if (warp == 9) {
-        for (int it = 0; it < n_k; ++it) {
-            const int s = it % STAGES;
-            if (!mbar_wait_relaxed(&full[s], (uint32_t)(it / STAGES) & 1u)) { failed = true; break; }
-            tc_fence_after();
-            if (lane == 0) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            for (int it = 0; it < n_k; ++it) {
+                if (!mbar_wait_relaxed(&full[s], phase)) { failed = true; break; }
+                tc_fence_after();
                 const uint64_t ad = make_smem_desc(smem_u32(smem + s * kStageBytes)), bd = make_smem_desc(smem_u32(smem + s * kStageBytes + kATile));
 #pragma unroll
                 for (int k4 = 0; k4 < 4; ++k4) umma_bf16(tmem, ad + 2 * k4, bd + 2 * k4, kIdesc, (it > 0 || k4 > 0) ? 1u : 0u);
                 umma_commit(&empty[s]);
+                if (++s == STAGES) { s = 0; phase ^= 1u; }
             }
-            __syncwarp();
+            if (!failed) umma_commit(&done);
         }
-        if (lane == 0 && !failed) umma_commit(&done);
         __syncwarp();
     }
     // every thread sees the MMAs of its own CTA complete before the cluster may write into the stage buffers
@@ -457,7 +462,7 @@ __global__ void __launch_bounds__(kChThreads, BN <= 64 ? 2 : 1) dense_channels_k
             }
         }
     }
-    if (failed && lane == 0) atomicExch(p.status, 3);
+    if (failed) atomicExch(p.status, 3);
     tc_fence_before();
     __syncthreads();
     if (warp == 9) tmem_free(tmem, kCols);

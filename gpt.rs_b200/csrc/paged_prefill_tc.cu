@@ -232,8 +232,9 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(const __g
         if (failed && lane == 0) atomicExch(p.status, 3);
     } else if (warp == kMmaWarp) {
         // ================= warp 8: MMA issue ==================================================================================
+        const bool one = elect_one();
         auto issue_s = [&](int i, int kb) {   // S_i = Q_i . K^T over the 8 sixteen-column steps of the head
-            if (lane == 0) {
+            if (one) {
                 const uint64_t a_desc = make_smem_desc(sQ + i * kTileBytes), b_desc = make_smem_desc(sK + (kb & 1) * kTileBytes);
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(const __g
             if (wait(&k_full[0], 0)) {
                 tc_fence_after();
                 for (int i = 0; i < kTiles; ++i) if (nb_t[i] > 0) issue_s(i, 0);
-                if (lane == 0) umma_commit(&k_empty[0]);
+                if (one) umma_commit(&k_empty[0]);
                 __syncwarp();
             }
         }
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(const __g
                         }
                     }
                     tc_fence_after();
-                    if (lane == 0) {
+                    if (one) {
                         const uint64_t b_desc = make_smem_desc_mn(sV + st * kTileBytes);
 #pragma unroll
                         for (int ks = 0; ks < 8; ++ks)
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(kThreads, 1) paged_prefill_tc_kernel(const __g
                 }
             }
             if (failed) break;
-            if (lane == 0) {
+            if (one) {
                 umma_commit(&v_empty[st]);
                 if (kb + 1 < n_blocks) umma_commit(&k_empty[st ^ 1]);
             }

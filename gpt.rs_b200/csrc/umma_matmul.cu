@@ -291,11 +291,12 @@ umma_w4a16_kernel(const MatmulParams p, const __grid_constant__ CUtensorMap x_ma
     } else {
         // ---------------- MMA issuer ---------------------------------------------------------------
         pdl_wait();  // this warp later reads the residual in the epilogue
+        const bool one = elect_one();
         for (int it = 0; it < n_it; ++it) {
             const int s = it % kStages;
             if (!mbar_wait_relaxed(&full_bar[s], (it / kStages) & 1, limit)) { failed = true; break; }
             tc_fence_after();
-            if (lane == 0) {
+            if (one) {
                 const uint64_t a_desc = make_smem_desc(smem_u32(sA + s * kABytes));
                 const uint64_t b_desc = make_smem_desc(smem_u32(sB + s * kBBytes));
 #pragma unroll
@@ -305,7 +306,7 @@ umma_w4a16_kernel(const MatmulParams p, const __grid_constant__ CUtensorMap x_ma
             }
             __syncwarp();
         }
-        if (lane == 0 && !failed) umma_commit(&done_bar);
+        if (one && !failed) umma_commit(&done_bar);
         __syncwarp();
     }
     // ---------------- epilogue: TMEM -> registers -> pushed to the owner CTA of each output row ----
@@ -557,7 +558,7 @@ umma_stream_kernel(const MatmulParams p, const __grid_constant__ CUtensorMap x_m
         // ---------------- MMA issuers: warp w takes the iterations it = w, w + 2, ...; iteration (j, c) adds A stage x
         // ---------------- activation stage j to accumulator c (CH = 1: to accumulator w) ------------------------------
         const int w = warp - (kProducerWarps + 2);
-        if (lane == 0) {
+        if (elect_one()) {   // one thread waits and issues for the whole loop
             int s = w, it = w;
             uint32_t ph = 0;
             bool first_round = true;
@@ -630,7 +631,7 @@ umma_stream_kernel(const MatmulParams p, const __grid_constant__ CUtensorMap x_m
             }
         }
     }
-    if (failed && lane == 0) atomicExch(p.status, 3);
+    if (failed) atomicExch(p.status, 3);
     tc_fence_before();
     __syncthreads();
     if (warp == kProducerWarps) {
