@@ -32,7 +32,11 @@ struct DevBuf {
         cudaError_t e = cudaMalloc(&p, bytes);
         if (e != cudaSuccess) return fail(GPTRS_EXECUTION, std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
         n = bytes;
-        if (zero) cudaMemset(p, 0, bytes);
+        if (zero) {   // ordered before the model's own stream, which does not wait for the default one
+            e = cudaMemset(p, 0, bytes);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+            if (e != cudaSuccess) return fail(GPTRS_EXECUTION, std::string("cudaMemset: ") + cudaGetErrorString(e));
+        }
         return GPTRS_OK;
     }
     void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
