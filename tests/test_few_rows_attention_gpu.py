@@ -36,6 +36,22 @@ def test_one_launch_equals_two(cuda, lengths, n_q, n_kv):
             assert (out[row].float() - ref[row].float()).norm() <= 2 ** -7 * ref[row].float().norm()
 
 
+@pytest.mark.parametrize("rows,length", [(1, 60), (1, 1500), (1, 4000), (8, 1500), (16, 1000)])
+def test_error_is_the_rounding_of_the_output(cuda, rows, length):
+    """Probabilities keep 16 bits and sums are f32, so the error against 64 bits is what rounding the exact result to bf16 leaves, and 2^-14 (a few
+    f32 ulps of a score in the exponent, 2^-17 of a probability). With probabilities rounded to bf16 it is 17 to 25 % more."""
+    g, pool, table = _cache([length] * rows, 8, length, cuda, rows + length)
+    q = torch.randn((rows, 32, 128), device=cuda, generator=g).bfloat16()
+    slot, ctx = torch.arange(rows, dtype=torch.int32, device=cuda), torch.full((rows,), length, dtype=torch.int32, device=cuda)
+    out, status = ops.paged_attention_decode(q, pool, table, slot, ctx, 32, 8, length)
+    for row in range(rows):
+        k, v = (t.double() for t in ops.kv_gather(pool, table[row], length, 8))
+        p = (torch.einsum("hgd,thd->hgt", q[row].double().view(8, 4, 128), k) * 128 ** -0.5).softmax(-1)
+        want = torch.einsum("hgt,thd->hgd", p, v).flatten()
+        assert (out[row].double() - want).norm() <= (want.bfloat16().double() - want).norm() + 2.0 ** -14 * want.norm()
+    assert int(status.item()) == 0
+
+
 def test_lengths_and_shapes_that_do_not_fit(cuda):
     g, pool, table = _cache([100, 100], 2, 100, cuda, 1)
     q = torch.randn((2, 8, 128), device=cuda, generator=g).bfloat16()
