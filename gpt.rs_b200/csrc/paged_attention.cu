@@ -921,7 +921,9 @@ int gptrs_cuda_paged_attention_decode_few_rows(const void* d_q, const void* d_kv
     p.out = static_cast<__nv_bfloat16*>(d_out);
     p.status = d_status;
     p.T = (int)n_tokens; p.Hq = (int)n_q_heads; p.Hkv = (int)n_kv_heads; p.max_pages = (int)max_pages;
-    p.chunk_pages = ceil_div(ceil_div(max_ctx_len, kPageTokens), splits);
+    // as many pages as the form with scratch covers: a launch may meet rows longer than the max_ctx_len it was planned with
+    const int64_t round = gptrs_cuda_attention_chunk_pages(max_ctx_len, n_tokens, n_kv_heads), covered = (ceil_div(max_ctx_len, kPageTokens) + round - 1) / round * round;
+    p.chunk_pages = ceil_div(covered, splits);
     p.max_splits = splits;
     p.max_len = (int)std::min<int64_t>((int64_t)splits * p.chunk_pages * kPageTokens, max_pages * kPageTokens);
     p.scale_log2 = kLog2e / sqrtf((float)kHD);

@@ -52,6 +52,21 @@ def test_error_is_the_rounding_of_the_output(cuda, rows, length):
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("planned,length,rows,n_kv", [(144, 192, 1, 8), (16, 64, 2, 2), (100, 128, 3, 8), (600, 640, 16, 8), (1500, 1536, 1, 8), (4000, 4032, 2, 8),
+                                                      (1000, 1024, 16, 8)])
+def test_rows_longer_than_planned(cuda, planned, length, rows, n_kv):
+    """A recorded launch is replayed for lengths up to the end of the last chunk that the form with scratch would have, here the planned length
+    rounded up to its chunks."""
+    assert lib().gptrs_cuda_attention_few_rows_splits(planned, rows, 4 * n_kv, n_kv) > 0
+    g, pool, table = _cache([length] * rows, n_kv, length, cuda, planned)
+    q = torch.randn((rows, 4 * n_kv, 128), device=cuda, generator=g).bfloat16()
+    slot, ctx = torch.arange(rows, dtype=torch.int32, device=cuda), torch.full((rows,), length, dtype=torch.int32, device=cuda)
+    out, status = ops.paged_attention_decode(q, pool, table, slot, ctx, 4 * n_kv, n_kv, planned)
+    ref, _ = ops.paged_attention_decode(q, pool, table, slot, ctx, 4 * n_kv, n_kv, length)
+    assert int(status.item()) == 0
+    assert (out.float() - ref.float()).norm() <= 2 ** -7 * ref.float().norm()   # one rounding to bf16 each
+
+
 def test_lengths_and_shapes_that_do_not_fit(cuda):
     g, pool, table = _cache([100, 100], 2, 100, cuda, 1)
     q = torch.randn((2, 8, 128), device=cuda, generator=g).bfloat16()
