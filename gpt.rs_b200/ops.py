@@ -5,13 +5,13 @@ torch kernel runs on behalf of these functions except output allocation.
 from __future__ import annotations
 
 import ctypes
-import functools
 
 import torch
 
 from . import _abi, check, lib
 
 F32, F16, BF16, SI32, I1, SI8, UI8 = range(7)
+UNIMPLEMENTED = 2   # gptrs_status
 
 
 def _ptr(t: torch.Tensor | None):
@@ -179,11 +179,6 @@ def rope_kv_append(qkv, positions, slot, page_table, cos, sin, rotary_dim, kv_po
     return q_out
 
 
-@functools.lru_cache(maxsize=1024)
-def _few_rows_splits(max_ctx_len, t, n_q, n_kv, device):
-    return lib().gptrs_cuda_attention_few_rows_splits(max_ctx_len, t, n_q, n_kv) if n_kv > 0 and n_q % n_kv == 0 else 0
-
-
 def paged_attention_decode(q, kv_pool, page_table, slot, ctx_len, n_q, n_kv, max_ctx_len, head_dim=128,
                            chunk_pages=None, status=None, prefill=False):
     """q bf16 [T][Hq][hd] -> out bf16 [T][Hq*hd]. prefill=True uses the prefill-chunk entry point (aligned groups
@@ -197,14 +192,14 @@ def paged_attention_decode(q, kv_pool, page_table, slot, ctx_len, n_q, n_kv, max
         check(lib().gptrs_cuda_paged_attention_prefill_tc(_ptr(q), _ptr(kv_pool), _ptr(page_table), page_table.shape[1], _ptr(slot),
                                                           _ptr(ctx_len), _ptr(out), _ptr(status), t, n_q, n_kv, head_dim, _stream()))
         return out, status
-    if chunk_pages is None and not prefill and t and _few_rows_splits(max_ctx_len, t, n_q, n_kv, q.device.index):
+    if chunk_pages is None and not prefill and 0 < t <= 16:   # up to 16 rows: one launch, where their contexts fit it
         out = torch.empty((t, n_q * head_dim), dtype=torch.bfloat16, device=q.device)
-        clear = status is None
-        if clear:
-            status = torch.empty(1, dtype=torch.int32, device=q.device)
-        check(lib().gptrs_cuda_paged_attention_decode_few_rows(_ptr(q), _ptr(kv_pool), _ptr(page_table), page_table.shape[1], _ptr(slot), _ptr(ctx_len), _ptr(out),
-                                                               _ptr(status), clear, t, n_q, n_kv, head_dim, max_ctx_len, _stream()))
-        return out, status
+        word = torch.empty(1, dtype=torch.int32, device=q.device) if status is None else status
+        rc = lib().gptrs_cuda_paged_attention_decode_few_rows(_ptr(q), _ptr(kv_pool), _ptr(page_table), page_table.shape[1], _ptr(slot), _ptr(ctx_len), _ptr(out),
+                                                              _ptr(word), status is None, t, n_q, n_kv, head_dim, max_ctx_len, _stream())
+        if rc != UNIMPLEMENTED:
+            check(rc)
+            return out, word
     if chunk_pages is None:
         chunk_pages = lib().gptrs_cuda_attention_chunk_pages(max_ctx_len, t, n_kv)
     nbytes = lib().gptrs_cuda_attention_scratch_bytes(t, n_q, max_ctx_len, chunk_pages)

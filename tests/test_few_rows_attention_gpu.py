@@ -77,3 +77,20 @@ def test_lengths_and_shapes_that_do_not_fit(cuda):
     assert lib().gptrs_cuda_attention_few_rows_splits(100000, 16, 32, 8) == 0 and lib().gptrs_cuda_attention_few_rows_splits(100, 17, 8, 2) == 0
     with pytest.raises(BackendError):
         ops.paged_attention_decode(q, pool, table, slot, slot, 8, 2, 200)   # more than the page table holds
+
+
+def test_one_library_call_whatever_the_length(cuda, monkeypatch):
+    """A chat's length is another one with every token: no size is asked for first, or remembered from an earlier call."""
+    g, pool, table = _cache([400], 2, 400, cuda, 1)
+    q = torch.randn((1, 8, 128), device=cuda, generator=g).bfloat16()
+    slot, called = torch.zeros(1, dtype=torch.int32, device=cuda), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            called.append(name)
+            return getattr(lib(), name)
+
+    monkeypatch.setattr(ops, "lib", Recorder)
+    for n in (300, 301, 301):
+        ops.paged_attention_decode(q, pool, table, slot, torch.full((1,), n, dtype=torch.int32, device=cuda), 8, 2, n)
+    assert called == ["gptrs_cuda_paged_attention_decode_few_rows"] * 3
