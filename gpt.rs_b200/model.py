@@ -326,6 +326,14 @@ def param_key(namespace: int, base_id: int) -> int:
     return int.from_bytes(h.digest()[:16], "little")
 
 
+def _token_ids(tokens) -> np.ndarray:
+    """Ids of any iterable as int32; ids that int32 does not hold are an OverflowError, not other ids."""
+    if isinstance(tokens, np.ndarray) and tokens.ndim and (np.can_cast(tokens.dtype, np.int32) or (tokens.dtype.kind in "iu" and tokens.size and
+                                                           -2 ** 31 <= tokens.min() and tokens.max() < 2 ** 31)):
+        return np.ascontiguousarray(tokens, dtype=np.int32)
+    return np.ascontiguousarray(list(tokens), dtype=np.int32)
+
+
 class LoadedModel:
     """A model resident on the current CUDA device."""
 
@@ -439,7 +447,7 @@ class LoadedModel:
         (optional) and greedy id of the LAST prompt row (the generator's first sampled token)."""
         chunk = chunk or self.config.max_tokens
         start = self.sequence_length(slot)
-        tokens = np.ascontiguousarray(tokens if isinstance(tokens, np.ndarray) else list(tokens), dtype=np.int32)
+        tokens = _token_ids(tokens)
         logits, sampled = None, None
         for o in range(0, len(tokens), chunk):
             part = tokens[o:o + chunk]

@@ -89,3 +89,19 @@ def test_passes_for_the_tensor_core_attention_are_always_full():
     assert first == [int(p[-1]) + 1000 for p in prompts]
     assert [len(p[0]) for p in m.passes] == [256, 256, 256, sum(lens) - 3 * 256]
     assert [t for p in m.passes for t in p[0]] == [int(t) for p in prompts for t in p]
+
+
+@pytest.mark.parametrize("prompt", [np.array([5, 2 ** 40 + 5]), np.array([5, 2 ** 32 - 1], dtype=np.uint32), [5, 2 ** 31], np.array(5)])
+def test_ids_that_int32_does_not_hold_are_refused(prompt):
+    m = _Recorder(_cfg())
+    with pytest.raises((OverflowError, TypeError)):   # a number that is no sequence: TypeError
+        m.prefill(0, prompt)
+    assert not m.passes
+
+
+@pytest.mark.parametrize("kind", [np.int32, np.int64, np.uint32, np.uint8, list, iter])
+def test_prompts_of_any_kind_of_ids(kind):
+    ids = [7, 250, 0, 31] * 20
+    m = _Recorder(_cfg())
+    _, first = m.prefill(0, kind(ids) if kind in (list, iter) else np.array(ids, dtype=kind))
+    assert first == ids[-1] + 1000 and [t for p in m.passes for t in p[0]] == ids
