@@ -372,6 +372,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
             r = mega_launch(P, st);
         } else {
             QuantStepParams P = m.qstep;
+            P.cos_table = m.cos_tab.as<float>(); P.sin_table = m.sin_tab.as<float>();   // not kept: a caller may set others
             call(P);
             m.qstep.epoch += (uint32_t)c.n_layers + 1u;
             r = quant_step_launch(c.weight_mode == kModeW4 ? 4 : 8, P, max_ctx, st);
@@ -808,7 +809,7 @@ int setup_quant_step(Model& m) {
     }
     P.n_layers = c.n_layers;
     P.D = c.d_model; P.FF = c.d_mlp; P.Hq = c.n_q_heads; P.Hkv = c.n_kv_heads; P.vocab = c.vocab;
-    P.tok_emb = gain(m.tok_emb); P.final_gain = gain(m.final_g); P.cos_table = m.cos_tab.as<float>(); P.sin_table = m.sin_tab.as<float>();
+    P.tok_emb = gain(m.tok_emb); P.final_gain = gain(m.final_g);
     P.w_head = packed(m.lm_head);
     P.token = m.d_tokens.as<int>(); P.pos = m.d_pos.as<int>(); P.slot = m.d_slot.as<int>(); P.ctx = m.d_ctx.as<int>(); P.page_table = m.d_page_table.as<int>();
     P.history = m.history.as<int>(); P.out = m.step_out(); P.context_length = c.context_length;
@@ -1005,12 +1006,20 @@ int gptrs_cuda_model_set_rope_tables(gptrs_model* h, const float* h_cos, const f
     GPTRS_REQUIRE(h && h_cos && h_sin && n_positions > 0, "null pointer");
     Model& m = *reinterpret_cast<Model*>(h);
     GPTRS_REQUIRE(m.cfg.rotary_dim > 0, "model has no rotary embedding");
-    size_t bytes = (size_t)n_positions * (m.cfg.rotary_dim / 2) * 4;
-    int rc = m.cos_tab.alloc(bytes);
-    if (!rc) rc = m.sin_tab.alloc(bytes);
-    if (rc) return rc;
-    GPTRS_CUDA_OK(cudaMemcpy(m.cos_tab.p, h_cos, bytes, cudaMemcpyHostToDevice));
-    GPTRS_CUDA_OK(cudaMemcpy(m.sin_tab.p, h_sin, bytes, cudaMemcpyHostToDevice));
+    if (m.finalized && !m.layered()) {   // steps may be under way that read the tables, and recorded ones hold their addresses
+        GPTRS_REQUIRE(n_positions >= m.cfg.context_length, "rotary tables shorter than context_length");
+        GPTRS_CUDA_OK(cudaStreamSynchronize(m.stream));
+        m.drop_graphs();
+    }
+    const size_t bytes = (size_t)n_positions * (m.cfg.rotary_dim / 2) * 4;
+    DevBuf cos, sin;
+    int rc;
+    if ((rc = cos.alloc(bytes)) || (rc = sin.alloc(bytes))) return rc;
+    GPTRS_CUDA_OK(cudaMemcpy(cos.p, h_cos, bytes, cudaMemcpyHostToDevice));
+    GPTRS_CUDA_OK(cudaMemcpy(sin.p, h_sin, bytes, cudaMemcpyHostToDevice));
+    GPTRS_CUDA_OK(cudaStreamSynchronize(nullptr));   // the model's stream does not wait for the default one
+    std::swap(m.cos_tab.p, cos.p); std::swap(m.cos_tab.n, cos.n);
+    std::swap(m.sin_tab.p, sin.p); std::swap(m.sin_tab.n, sin.n);
     m.n_rope_pos = (int)n_positions;
     return GPTRS_OK;
 }

@@ -255,8 +255,12 @@ struct Model {
     int max_rows() const { return cfg.max_logit_rows > 0 ? cfg.max_logit_rows : cfg.max_seqs; }
     int stage_stride() const { return std::max(cfg.max_tokens, max_rows()); }
 
-    ~Model() {
+    void drop_graphs() {
         for (auto& g : graphs) cudaGraphExecDestroy(g.second.exec);
+        graphs.clear();
+    }
+    ~Model() {
+        drop_graphs();
         for (auto& r : raw) tensor_release(r.second);
         auto relw = [](Weight& w) { tensor_release(w.f32); tensor_release(w.packed); tensor_release(w.bias); };
         for (auto& l : layers) {

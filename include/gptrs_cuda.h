@@ -936,7 +936,8 @@ int gptrs_cuda_model_load_param(gptrs_model* m, const char* name, uint64_t id_lo
                                 int on_device, int rank, const int64_t* dims);
 /* Optional: the caller's cos/sin tables [n_positions][rotary_dim/2] (the reference builds them on
  * the host and passes them as inputs, model/ministral.rs:253-261); otherwise finalize computes
- * them with the formula of ops/functional/rotary.rs:75-215 (no scaling). */
+ * them with the formula of ops/functional/rotary.rs:75-215 (no scaling). After finalize they hold from the next pass on and
+ * must cover context_length, as there. */
 int gptrs_cuda_model_set_rope_tables(gptrs_model* m, const float* h_cos, const float* h_sin, int64_t n_positions);
 /* Tensor-parallel variant (ministral kind; no counterpart in gpt.rs): w_qkv / w_gate / w_up / lm_head are
  * column-parallel (each rank keeps n_q_heads/tp query heads, n_kv_heads/tp kv heads, d_mlp/tp columns,

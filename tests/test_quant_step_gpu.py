@@ -3,19 +3,22 @@ around the edges of pages and slices of attention, ids from the device and given
 import numpy as np
 import pytest
 
+from gptrs_b200 import BackendError
 from gptrs_b200 import model as gm
 from oracle import models_ref as mr
 
 pytestmark = pytest.mark.gpu
 
 
-def _model(mode, n_q, n_kv, d, mlp, vocab, batch, ctx, params, namespace):
+def _model(mode, n_q, n_kv, d, mlp, vocab, batch, ctx, params, namespace, tables=None):
     pages = (ctx + 15) // 16
     m = gm.LoadedModel(gm.ModelConfig(gm.KIND_MINISTRAL, 2, d, n_q, n_kv, 128, mlp, vocab, ctx, 1e-5, 1e4, 128,
                                       weight_mode=gm.MODE_W4A16 if mode == "w4" else gm.MODE_W8A16, max_seqs=batch, max_tokens=1024, max_logit_rows=batch,
                                       kv_pages=batch * pages + 4, max_pages_per_seq=pages, use_pdl=1), namespace=namespace)
     for name, w in params.items():
         m.load_param(name, w)
+    if tables:
+        m.set_rope_tables(*tables)
     m.finalize()
     return m
 
@@ -78,3 +81,32 @@ def test_window_slide_and_sampling(cuda, mode, monkeypatch):
         _, drawn = m.forward_with_decode_cache([7], [0], [30], [0], temperature=0.8, seed=11)
         out.append((ids, drawn.tolist()))
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("own", ["1", "0"])
+def test_rotary_tables_set_after_finalize(cuda, own, monkeypatch):
+    """Steps read the tables that stand, not those of finalize: the single kernel, and the recorded ones of the kernel-per-projection path."""
+    monkeypatch.setenv("GPTRS_QUANT_STEP", own)
+    d, vocab, ctx = 256, 512, 64
+    cfg = mr.Cfg("ministral", n_layers=2, d_model=d, n_q=4, n_kv=2, hd=128, d_mlp=512, vocab=vocab, ctx=ctx, rot=128, theta=1e4)
+    params = mr.random_params(cfg, seed=4, std=0.05)
+    angle = np.outer(np.arange(ctx), 30.0 ** -(np.arange(64) / 64))
+    tables = np.cos(angle).astype(np.float32), np.sin(angle).astype(np.float32)
+
+    def serve(m):
+        m.prefill_many([0, 1], [np.arange(9), np.arange(20) * 3])
+        gen = gm.Generator(m, [5, 6])
+        for k in range(3):
+            gen.step([k, 7 * k])
+        return m.forward_with_decode_cache([8], [1], [23], [0])[0]
+
+    m = _model("w4", 4, 2, d, 512, vocab, 2, ctx, params, 7720)
+    first = serve(m)
+    with pytest.raises(BackendError):
+        m.set_rope_tables(*(t[:ctx - 1] for t in tables))
+    m.set_rope_tables(*tables)
+    for slot in (0, 1):
+        m.reset_sequence(slot)
+    second = serve(m)
+    fresh = _model("w4", 4, 2, d, 512, vocab, 2, ctx, params, 7721, tables)
+    assert np.array_equal(second, serve(fresh)) and not np.array_equal(first, second)
