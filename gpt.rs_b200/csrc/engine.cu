@@ -1476,7 +1476,7 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
     if (own_step) {   // one launch, which needs no graph
         m.step_tokens = h_tokens_in;
         m.step_advance = true;
-        const int r = enqueue_forward(m, B, bucket, chunk, B, true, 0.f, false, true);
+        const int r = enqueue_forward(m, B, max_ctx, chunk, B, true, 0.f, false, true);   // not recorded: the longest length itself
         m.step_tokens = nullptr;
         m.step_advance = false;
         if (r) return r;

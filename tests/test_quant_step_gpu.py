@@ -26,7 +26,8 @@ def _model(mode, n_q, n_kv, d, mlp, vocab, batch, ctx, params, namespace, tables
 @pytest.mark.parametrize("mode,n_q,n_kv,d,mlp,vocab,lengths", [
     ("w4", 1, 1, 128, 128, 64, [1]),                       # one group of 128 k, eight tiles: most CTAs and warps have nothing
     ("w8", 2, 1, 128, 256, 32, [15, 16, 17]),
-    ("w4", 8, 1, 384, 640, 1616, [223]), ("w4", 8, 1, 384, 640, 1616, [224]), ("w8", 8, 1, 384, 640, 1616, [225, 111]),   # one slice, two slices of pages
+    ("w4", 8, 1, 384, 640, 1616, [111]), ("w4", 8, 1, 384, 640, 1616, [112]),   # a second slice of pages from the third step on, from the first
+    ("w4", 8, 1, 384, 640, 1616, [223]), ("w4", 8, 1, 384, 640, 1616, [224]), ("w8", 8, 1, 384, 640, 1616, [225, 111]),   # a third
     ("w4", 32, 8, 3072, 1152, 256, [40, 350]),             # odd numbers of units per stage; two tiles of the residual stream in some CTAs
     ("w8", 16, 4, 2048, 4864, 256, [100, 7, 64, 65, 31, 1, 200, 90]),
     ("w4", 6, 2, 256, 5120, 512, [129, 128, 127, 30, 2]),  # groups of three query heads
@@ -59,6 +60,27 @@ def test_steps_follow_the_oracle(cuda, mode, n_q, n_kv, d, mlp, vocab, lengths):
     want = np.stack([r.forward([int(t)])[-1] for r, t in zip(refs, given[3])])
     logits, _ = m.forward_with_decode_cache(given[3], list(range(batch)), [n + 4 for n in lengths], list(range(batch)))   # one row: the kernel itself
     assert np.sqrt(np.mean((logits - want) ** 2)) <= 2e-2 * np.sqrt(np.mean(want ** 2))   # bf16 activations through two layers
+
+
+@pytest.mark.parametrize("mode", ["w4", "w8"])
+def test_steps_do_not_depend_on_the_room_of_the_page_table(cuda, mode):
+    """The slices of attention come from the lengths of the step's sequences, so a model with room for more tokens adds up in the same order.
+    Eight rows of 1024 values over 40 steps: some of them lie so close to the middle of two bf16 that another order shows."""
+    d, vocab, rows = 1024, 512, 8
+    cfg = mr.Cfg("ministral", n_layers=2, d_model=d, n_q=8, n_kv=2, hd=128, d_mlp=512, vocab=vocab, ctx=256, rot=128, theta=1e4)
+    params = mr.random_params(cfg, seed=6, std=0.5 * d ** -0.5)
+    params["tok_embeddings.weight"] = np.random.default_rng(0).normal(0, 1, (vocab, d)).astype(np.float32)
+    rng = np.random.default_rng(2)
+    prompts, given = [rng.integers(0, vocab, 95 - 5 * r) for r in range(rows)], rng.integers(0, vocab, (41, rows))
+    out = []
+    for room in (256, 4096):
+        m = _model(mode, 8, 2, d, 512, vocab, rows, room, params, 7740 + room)
+        m.prefill_many(list(range(rows)), prompts)
+        gen = gm.Generator(m, given[0])
+        for ids in given[:40]:   # up to and past 112 tokens, where a second slice begins
+            gen.step(ids)
+        out.append(m.forward_with_decode_cache(given[40], list(range(rows)), [135 - 5 * r for r in range(rows)], list(range(rows)))[0])
+    assert np.array_equal(*out)
 
 
 @pytest.mark.parametrize("mode", ["w4", "w8"])
