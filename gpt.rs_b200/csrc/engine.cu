@@ -343,9 +343,9 @@ size_t sumsq_floats(int d_model, int rows) { return (size_t)rows * (d_model / (r
 
 // Enqueues one forward pass over T tokens whose ids / slots / positions / visible lengths are
 // already in the device arrays. `rows`: number of rows that get logits (row indices in d_rows,
-// or all T rows in order when rows_identity).
+// or all T rows in order when rows_identity). own_step: a token each of T sequences as one cooperative kernel (Model::one_kernel_step).
 int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, bool rows_identity, float temperature,
-                    int prefill_groups = 0, bool skip_logits = false) {
+                    int prefill_groups = 0, bool skip_logits = false, bool own_step = false) {
     if (m.layered()) return layered_forward(m, T, max_ctx, n_rows, rows_identity, temperature, skip_logits);
     m.planes.of = nullptr;
     const auto& c = m.cfg;
@@ -353,8 +353,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
     cudaStream_t st = m.stream;
     float* hidden = m.hidden.as<float>();
     const int act_dt = m.f32() ? GPTRS_F32 : GPTRS_BF16;
-    if (m.one_kernel_step(T) && n_rows == T && (rows_identity || T == 1) && !prefill_groups) {
-        // a token each of a few sequences: the whole step is one cooperative kernel
+    if (own_step) {
         auto call = [&](auto& P) {
             P.rows = T;
             P.advance = m.step_advance ? 1 : 0;
@@ -1341,7 +1340,7 @@ int gptrs_cuda_model_forward_with_decode_cache(gptrs_model* h, const int32_t* h_
     // With the weights' planes, whose first tiles travel while the kernel in front ends, early launches pay at every size: GPT-2 without /
     // with, 300 rows 1602 / 1361, 512 rows 1858 / 1660, 937 rows 3000 / 2753.
     if (c.use_pdl && (m.w_planes.p || T <= (m.layered() ? 128 : 256))) g_use_pdl = 1;
-    rc = enqueue_forward(m, T, max_ctx, chunk, rows, false, temperature, prefill_groups);
+    rc = enqueue_forward(m, T, max_ctx, chunk, rows, false, temperature, prefill_groups, false, T == 1 && m.one_kernel_step(1, max_ctx, max_ctx));
     g_use_pdl = pdl_before;
     if (rc) return rc;
     if (m.layered()) for (size_t r = 0; r < m.lay->runs.size(); r += 2) m.lay->parity[h_slots[m.lay->runs[r]]] ^= 1;
@@ -1440,17 +1439,19 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
         if (any) { int rc = slide_windows(m, h, B, h_tokens_in); if (rc) return rc; }
     }
     int max_ctx = 1;
+    int64_t all_ctx = 0;
     for (int b = 0; b < B; ++b) {
         GPTRS_REQUIRE(m.seq_len[b] < c.context_length, "sequence reached context_length");
         release_passed_pages(m, b, m.seq_len[b]);
         int rc = ensure_pages(m, b, m.seq_len[b]);
         if (rc) return rc;
         max_ctx = std::max(max_ctx, m.seq_len[b] + 1);
+        all_ctx += m.seq_len[b] + 1;
     }
     int rc = sync_page_table(m);
     if (rc) return rc;
     cudaStream_t s = m.stream;
-    const bool own_step = m.one_kernel_step(B);   // takes the ids as parameters and advances its sequences itself
+    const bool own_step = m.one_kernel_step(B, max_ctx, all_ctx);   // takes the ids as parameters and advances its sequences itself
     if (h_tokens_in && !own_step) {
         GPTRS_CUDA_OK(cudaStreamSynchronize(s));  // the staging buffer may still feed an earlier copy
         memcpy(m.h_stage, h_tokens_in, (size_t)B * 4);
@@ -1476,7 +1477,7 @@ int gptrs_cuda_generator_step(gptrs_model* h, const int32_t* h_tokens_in, int32_
     if (own_step) {   // one launch, which needs no graph
         m.step_tokens = h_tokens_in;
         m.step_advance = true;
-        const int r = enqueue_forward(m, B, max_ctx, chunk, B, true, 0.f, false, true);   // not recorded: the longest length itself
+        const int r = enqueue_forward(m, B, max_ctx, chunk, B, true, 0.f, 0, true, true);   // not recorded: the longest length itself
         m.step_tokens = nullptr;
         m.step_advance = false;
         if (r) return r;

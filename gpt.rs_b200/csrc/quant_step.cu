@@ -842,6 +842,19 @@ int quant_step_max_rows(int bits, int n_layers, int D, int FF, int Hq, int Hkv, 
     while (n < kStepMaxRows && (n + 1) * Hkv <= sm_count() && ring_stages(bits, n + 1, D, FF, Hq, Hkv) >= (bits == 4 ? 2 : 3)) ++n;
     return n;
 }
+// Whether a step is faster here than kernel by kernel: what attention takes longer, in us of a layer, against what the rest is faster (the least
+// of widths 1024, 2048 and 3072, 11.5 in W4 and 7.8 in W8). Here it is rounds of pages and slices to add up (see `slices`), and all rows have as
+// many CTAs; there long rows have more splits and two pages per warp under way: at least 0.6 us per 1000 tokens of the longest row, or all
+// pages at 6.1 TB/s. Four layers, us, kernel by kernel / here: W4 of width 3072, 8 rows at 3000 tokens 409 / 330, 8000 511 / 502, 16000
+// 713 / 805; one of 8000 among short ones 364 / 458, of 32000 508 / 1224; 4 rows at 8000 366 / 330, 16000 491 / 496; W4 of width 2048, 8 rows at
+// 16000 424 / 423, 32000 574 / 652; W8 of width 2048, 8 rows at 3000 234 / 229, one of 3000 217 / 224, 4 rows at 16000 340 / 281, one of 16000
+// 255 / 270; one row is faster here at every length up to 32000 (W4 of width 3072 there 445 / 380, W8 of width 1024 at 3000 141 / 140).
+bool quant_step_pays(int bits, int rows, int n_kv_heads, int max_ctx, int64_t all_ctx) {
+    const int s = slices(max_ctx, rows, n_kv_heads);
+    const double here = 1.5 * ceil_div(ceil_div(max_ctx, 16), kPairs * s) + 0.3 * (s - 1);
+    const double there = std::max(1.5 + 0.0006 * max_ctx, (double)all_ctx * n_kv_heads * 512 / 6.1e6);
+    return here - there < (bits == 4 ? 11.5 : 7.8);
+}
 size_t quant_step_exchange_bytes(int D, int FF, int Hq, int Hkv) { return exchange_layout(D, FF, Hq, Hkv).total; }
 
 int quant_step_launch(int bits, QuantStepParams p, int max_ctx, cudaStream_t st) {

@@ -83,6 +83,35 @@ def test_steps_do_not_depend_on_the_room_of_the_page_table(cuda, mode):
     assert np.array_equal(*out)
 
 
+@pytest.mark.parametrize("mode,first", [("w4", 2017), ("w8", 1345)])
+def test_long_rows_among_short_ones_leave_the_kernel(cuda, mode, first):
+    """Eight rows of eight kv heads: a long row has two slices of pages whatever the others have, and from the tenth (W8: the seventh) round of
+    pages on the step goes kernel by kernel, which splits it further; and back when the row has gone. Ids as the oracle's on both sides."""
+    d, vocab, rows = 256, 256, 8
+    cfg = mr.Cfg("ministral", n_layers=2, d_model=d, n_q=8, n_kv=8, hd=128, d_mlp=256, vocab=vocab, ctx=2064, rot=128, theta=1e4)
+    params = mr.random_params(cfg, seed=7, std=0.5 * d ** -0.5)
+    params["tok_embeddings.weight"] = np.random.default_rng(0).normal(0, 1, (vocab, d)).astype(np.float32)
+    params["lm_head"] = (np.roll(params["tok_embeddings.weight"], 1, 0).T * d ** -0.5).astype(np.float32)
+    m = _model(mode, 8, 8, d, 256, vocab, rows, 2064, params, 7760)
+    rng = np.random.default_rng(3)
+    prompts, given = [rng.integers(0, vocab, n) for n in [first - 4] + [9 + r for r in range(rows - 1)]], rng.integers(0, vocab, (6, rows))
+    refs = [mr.RefModel(cfg, mr.quantised_params(cfg, params, mode)) for _ in prompts]
+    for r, p in zip(refs, prompts):
+        r.forward(p)
+    m.prefill_many(list(range(rows)), prompts)
+    gen = gm.Generator(m, given[0])
+    for k, ids in enumerate(given):   # lengths with the new token: first - 3 ... first + 2
+        before = m.stats()["kernel_launches"]
+        want = [int(r.forward([int(t)])[-1].argmax()) for r, t in zip(refs, ids)]
+        assert gen.step(ids).tolist() == want
+        assert (m.stats()["kernel_launches"] - before == 1) == (k < 3)
+    m.reset_sequence(0)
+    m.prefill(0, prompts[1])
+    gen, before = gm.Generator(m, given[0]), m.stats()["kernel_launches"]
+    gen.step(given[0])
+    assert m.stats()["kernel_launches"] - before == 1
+
+
 @pytest.mark.parametrize("mode", ["w4", "w8"])
 def test_window_slide_and_sampling(cuda, mode, monkeypatch):
     """Steps across the end of the context window, and a temperature draw of one row, as the kernel-per-projection path does them."""
