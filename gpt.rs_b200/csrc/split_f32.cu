@@ -329,9 +329,12 @@ int launch(SplitF32Params p, cudaStream_t st) {
 // small K those CTAs are short (K 32, N 4096, 64 and 300 rows 5.0 / 11.1, 13.7 / 12.8; K 64, N 256, 937 rows 11.9 / 13.7; K 64, N 8192,
 // 24 and 64 rows 7.4 / 9.4, 18.6 / 12.3; K 128, N 1024, 64 and 300 rows 6.9 / 10.8, 20.7 / 12.5; K 256, N 1024, 64 rows 16.2 / 10.2): the
 // line is at 16384 CTAs x K.
+bool split_f32_line(int64_t m, int64_t n, int64_t k) {
+    const int64_t few_row_ctas = (int64_t)ceil_div(m, 8) * ceil_div(n, 128);
+    return m >= kSplitF32Rows && few_row_ctas > 48 && few_row_ctas * k >= 16384;
+}
 bool split_f32_takes(const SplitF32Params& p) {
-    const int64_t few_row_ctas = (int64_t)ceil_div(p.M, 8) * ceil_div(p.N, 128);
-    return p.M >= kSplitF32Rows && few_row_ctas > 48 && few_row_ctas * p.K >= 16384 && p.K % kSfBK == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && ((p.ldx | p.x_step) & 3) == 0 &&
+    return split_f32_line(p.M, p.N, p.K) && p.K % kSfBK == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && ((p.ldx | p.x_step) & 3) == 0 &&
            (int64_t)p.K * p.N < (1ll << 30);
 }
 

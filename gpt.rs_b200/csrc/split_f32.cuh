@@ -22,8 +22,9 @@ struct SplitF32Params {
     int debug_starve;       // test switch: the first stage's products are never begun
 };
 
-// Least rows, and whether it takes this shape (the rule stands at its definition).
+// Least rows, the line against the kernel for few rows, and whether it takes this shape (the rule stands at the definitions).
 constexpr int kSplitF32Rows = 24;
+bool split_f32_line(int64_t m, int64_t n, int64_t k);
 bool split_f32_takes(const SplitF32Params& p);
 int split_f32_matmul(SplitF32Params p, cudaStream_t st);
 

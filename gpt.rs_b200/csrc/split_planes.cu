@@ -1,6 +1,6 @@
 // y[M][N] = act(x[M][K] . w[K][N] + bias) + residual in f32 on the tcgen05 tensor cores, as split_f32_kernel does it (three bf16 planes per
-// operand, the six products of at least 2^-18, the leading one summed in tensor memory over 64 k and then in f32 registers, the others in an
-// accumulator of their own; sums that are not finite once more in plain f32), for operands whose planes lie in memory: a model's weights split
+// operand, the six products of at least 2^-18, the leading one summed in tensor memory over 64 k (in tiles of 32 rows over 16) and then in f32
+// registers, the others in an accumulator of their own; sums that are not finite once more in plain f32), for operands whose planes lie in memory: a model's weights split
 // once, and the rows of a pass split once per projection instead of once per column tile.
 //
 // split_f32_kernel splits inside its tiles: 512 threads load, split, store and fence every 32 k, 2900 cycles a stage, of which the MMAs are 770.
@@ -10,10 +10,17 @@
 // stages are under way before the kernel in front has ended, and the norms and the GELU leave the planes of their rows themselves.
 // K is split over a cluster where the output tiles do not fill the SMs, the parts meet in the shared memory of the CTA that owns the row; the
 // epilogue then takes four neighbouring channels per thread (a channel per thread and scalar residuals took 10 to 17 us more at 937 rows).
+// Tensor cores cut their sums where f32 arithmetic rounds them: operands of one sign, leading sums over 64 k, are off by twice what plain f32
+// leaves. With sums of 16 k, one MMA each, nothing is cut but an MMA's own sum, and four of them are added in pairs. Where the kernel for few rows would
+// be taken without planes (split_f32_line), such tiles alone are taken. Error against 64 bits over the sum of magnitudes, that kernel / tiles of
+// 32 rows over 64 k / over 16 k, 64 rows, N 768: one sign, K 768 4.6e-8 / 8.9e-8 / 4.7e-8, K 3072 4.6e-8 / 8.9e-8 / 4.7e-8; either sign 5.8e-9 / 5.1e-9 /
+// 4.3e-9 and 4.2e-9 / - / 2.6e-9. A pass of four layers of width 256, 512, 768 at 24 rows, us, over 64 k / over 16 k: 209 / 214, 237 / 243,
+// 299 / 302; without planes 260, 321, 382.
 // Pieces of a third of a stage, in rings of 6 to 11, bring nothing: what the loads take is hidden with two stages.
 // GPT-2 small, us, split_f32_kernel / this: at 937 rows qkv 47 / 20, attention output 33 / 16, MLP in 96 / 32, MLP out 83 / 32; at 64 rows
 // qkv 11 / 7.5, MLP out 16 / 10.
 #include "matmul_common.cuh"
+#include "split_f32.cuh"
 #include "split_planes.cuh"
 #include "umma_common.cuh"
 
@@ -90,14 +97,16 @@ __device__ __forceinline__ void tmem_ld_16(uint32_t at, float (&v)[16]) {
 }
 
 constexpr int kThreads = 320;   // warps 0-7 sums and epilogue, 8 loader, 9 MMA + tensor memory
-template <int BN> constexpr int kStages = BN >= 128 ? 2 : 3;   // of 64 k, and as many accumulators of leading sums
+template <int BN> constexpr int kStages = BN >= 128 ? 2 : 3;   // of 64 k
+template <int BN> constexpr int kLeads = BN == 32 ? 4 : 1;     // leading sums of a stage (four of 64 rows do not fit beside three stages' others)
 template <int BN> constexpr int kStageBytes = 3 * kBlock + 3 * BN * 128;
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid_constant__ KernelParams kp) {
-    constexpr int S = kStages<BN>, kStage = kStageBytes<BN>, kX = BN * 128, kSumCols = BN >= 64 ? BN / 2 : 32;   // columns of a summing thread
+    constexpr int S = kStages<BN>, L = kLeads<BN>, kStage = kStageBytes<BN>, kX = BN * 128, kSumCols = BN >= 64 ? BN / 2 : 32;   // columns of a summing thread
     constexpr int kSumWarps = 4 * (BN / kSumCols);
-    constexpr uint32_t kCols = BN >= 128 ? 512 : BN == 64 ? 256 : 128;
+    constexpr uint32_t kCols = (S * L + 1) * BN > 256 ? 512 : 256;
+    static_assert((S * L + 1) * BN <= (int)kCols && (L == 1 || (L == 4 && kSumCols == 32)));
     constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | (8u << 24);
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[S], done[S], lead_empty[S];
@@ -172,12 +181,12 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
                 if (!mbar_wait_relaxed(&full[s], phase)) { failed = true; break; }
                 tc_fence_after();
                 const uint32_t at = smem_u32(smem) + (uint32_t)(s * kStage);
-                const uint32_t lead = tmem + (uint32_t)(s * BN), rest = tmem + (uint32_t)(S * BN);
+                const uint32_t lead = tmem + (uint32_t)(s * L * BN), rest = tmem + (uint32_t)(S * L * BN);
                 const uint64_t w3 = make_smem_desc(at + 2 * kBlock), x3 = make_smem_desc(at + 3 * kBlock + 2 * kX);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {   // K steps of 16 are 2 descriptor units apart; plane 2 lies 4 units behind plane 1
                     const uint64_t w = make_smem_desc(at + (k >> 1) * kBlock) + (uint64_t)(2 * (k & 1)), x = make_smem_desc(at + 3 * kBlock + (k >> 1) * kX) + (uint64_t)(2 * (k & 1));
-                    umma_bf16(lead, w, x, kIdesc, k > 0 ? 1u : 0u);
+                    umma_bf16(lead + k * L / 4 * BN, w, x, kIdesc, k % (4 / L) > 0 ? 1u : 0u);
                     umma_bf16(rest, w3 + 2 * k, x, kIdesc, it > 0 || k > 0 ? 1u : 0u);
                     umma_bf16(rest, w, x3 + 2 * k, kIdesc, 1u);
                     umma_bf16(rest, w + 4, x + 4, kIdesc, 1u);
@@ -214,12 +223,20 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
             const int b = it % S;
             if (!wait(&done[b], (uint32_t)(it / S) & 1u)) break;
             tc_fence_after();
-            add((uint32_t)(b * BN));
+            if constexpr (L == 4) {   // in pairs: fewer roundings of the long sum
+                float v[4][32];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) tmem_ld_32(lane_base + (uint32_t)((b * 4 + j) * BN), v[j]);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[i] += (v[0][i] + v[1][i]) + (v[2][i] + v[3][i]);
+            } else {
+                add((uint32_t)(b * BN));
+            }
             tc_fence_before();
             mbar_arrive(&lead_empty[b]);
         }
         tc_fence_after();
-        add((uint32_t)(S * BN));   // complete with the last stage's leading sums
+        add((uint32_t)(S * L * BN));   // complete with the last stage's leading sums
         pdl_wait();     // what the epilogue reads (residual, x of a repeated sum)
     }
     if (failed) atomicExch(p.status, 3);
@@ -443,7 +460,8 @@ int planes_matmul(const PlanesMatmul& q, cudaStream_t st) {
     if (!p.status) p.status = matmul_status_word();
     if (!p.status) return fail(GPTRS_EXECUTION, "no status word");
     Tiling t;
-    consider<32>(p, t); consider<64>(p, t); consider<128>(p, t); consider<160>(p, t);
+    consider<32>(p, t);   // alone where plain f32 is the other choice: see above
+    if (split_f32_line(p.M, p.N, p.K)) { consider<64>(p, t); consider<128>(p, t); consider<160>(p, t); }
     switch (t.rows) {
         case 32: return launch<32>(p, t.split, st);
         case 64: return launch<64>(p, t.split, st);
@@ -453,3 +471,18 @@ int planes_matmul(const PlanesMatmul& q, cudaStream_t st) {
 }
 
 }  // namespace gptrs
+
+extern "C" int gptrs_cuda_debug_planes_matmul(const float* d_x, const float* d_w, const float* d_bias, const float* d_residual, float* d_y, int64_t m, int64_t n,
+                                              int64_t k, int gelu, void* d_planes, size_t planes_bytes, void* stream) {
+    using namespace gptrs;
+    GPTRS_REQUIRE(d_x && d_w && d_y && d_planes, "null pointer");
+    GPTRS_REQUIRE(m > 0 && n > 0 && k > 0 && m <= INT32_MAX && n <= INT32_MAX && k <= INT32_MAX && k % 64 == 0, "planes: K a multiple of 64");
+    const size_t w_bytes = (plane_bytes(n, k) + 255) & ~(size_t)255;
+    GPTRS_REQUIRE(planes_bytes >= w_bytes + plane_bytes(m, k) && (reinterpret_cast<uintptr_t>(d_planes) & 255) == 0, "planes: buffer too small or not aligned to 256 bytes");
+    cudaStream_t st = as_stream(stream);
+    void* const x_planes = static_cast<unsigned char*>(d_planes) + w_bytes;
+    struct PdlGuard { int saved = g_use_pdl; PdlGuard() { g_use_pdl = 0; } ~PdlGuard() { g_use_pdl = saved; } } guard;   // these weights are not constant
+    int rc;
+    if ((rc = split_weight_planes(d_w, d_planes, k, n, st)) || (rc = split_row_planes(d_x, x_planes, m, k, st))) return rc;
+    return planes_matmul({d_planes, x_planes, d_x, d_w, d_bias, d_residual, d_y, nullptr, (int)m, (int)n, (int)k, gelu ? 1 : 0, nullptr}, st);
+}

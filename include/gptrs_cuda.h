@@ -187,6 +187,11 @@ int gptrs_cuda_matmul_status(int32_t* h_status);
  * code 3 in its status word, frees its tensor memory and returns with an unspecified result. Nothing faults
  * and nothing waits without a bound. Process-wide; call with (0, 0) to switch it off again. */
 int gptrs_cuda_debug_matmul_fault(int starve, uint32_t spin_limit);
+/* Debug: y [m][n] = x [m][k] . w [k][n] (+ bias [n]; gelu; + residual [m][n]) in f32 as the engine computes the projections of f32 models in
+ * passes of 24 rows and more, from both operands' bf16 planes, which the call makes itself in d_planes (256-byte aligned, 6 k (m + n) + 256
+ * bytes). k a multiple of 64, n of 4. Reports in gptrs_cuda_matmul_status. */
+int gptrs_cuda_debug_planes_matmul(const float* d_x, const float* d_w, const float* d_bias, const float* d_residual, float* d_y, int64_t m,
+                                   int64_t n, int64_t k, int gelu, void* d_planes, size_t planes_bytes, void* stream);
 
 /* ==============================================================================================
  * Dense (unquantised) linear layers with strided rows and batches, f32 and bf16 (functional::matmul + add_bias,

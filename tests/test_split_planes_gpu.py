@@ -2,7 +2,9 @@
 bf16 terms overflow, against the f32 oracle."""
 import numpy as np
 import pytest
+import torch
 
+from gptrs_b200 import check, lib, ops
 from gptrs_b200 import model as gm
 from oracle import models_ref as mr
 
@@ -52,3 +54,52 @@ def test_terms_that_overflow_bf16(cuda, rows):
         p["blocks.0.feed_forward.w_in"][5, 77] = np.float32(3.4e38)
         p["blocks.0.feed_forward.w_out"][77] *= np.float32(1e-20)
     run(256, 4, 512, rows, edit)
+
+
+def product(x, w):
+    (m, k), n = x.shape, w.shape[1]
+    y, planes = torch.empty(m, n, device=x.device), torch.empty(6 * k * (m + n) + 256, dtype=torch.uint8, device=x.device)
+    check(lib().gptrs_cuda_debug_planes_matmul(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), m, n, k, 0, planes.data_ptr(), planes.numel(),
+                                               torch.cuda.current_stream().cuda_stream))
+    assert ops.matmul_status() == 0
+    return y
+
+
+def rms(y, x, w):
+    """Root of the mean square of the errors over that of the sums of magnitudes."""
+    return float((y.double() - x.double() @ w.double()).norm() / (x.abs().double() @ w.abs().double()).norm())
+
+
+def operands(m, n, k, cuda):
+    g = torch.Generator(cuda).manual_seed(m + n + k)
+    return torch.randn(m, k, device=cuda, generator=g), torch.randn(k, n, device=cuda, generator=g), g
+
+
+@pytest.mark.parametrize("m,n,k", [(24, 768, 768), (64, 768, 3072), (33, 64, 64), (190, 256, 1024), (300, 128, 512), (1001, 132, 64), (64, 516, 2048)])
+def test_error_where_plain_f32_is_the_other_choice(cuda, m, n, k):
+    """Shapes that the f32 matmul leaves to the kernel for few rows, plain f32 arithmetic (rows by eight). Operands of either sign: not above it. Of
+    one sign: an MMA's sum of 16 products is cut by half an ulp on average, 3e-8, beside the 4.6e-8 of plain f32: a quarter more at most (with sums
+    over 64 k it is twice as much)."""
+    x, w, _ = operands(m, n, k, cuda)
+    plain = lambda x, w: torch.cat([ops.matmul_f32(r.contiguous(), w) for r in x.split(8)])  # noqa: E731
+    assert rms(product(x, w), x, w) <= rms(plain(x, w), x, w)
+    x, w = x.abs(), w.abs()
+    assert rms(product(x, w), x, w) <= 1.25 * rms(plain(x, w), x, w)
+
+
+def _three_terms(shape, g):
+    """Positive values whose second and third bf16 terms are positive too, near the largest that such terms can be."""
+    term = lambda low, high, unit: torch.randint(low, high, shape, device=g.device, generator=g).float() * unit  # noqa: E731
+    return 1 + term(0, 128, 2.0 ** -7) + term(64, 127, 2.0 ** -15) + term(64, 127, 2.0 ** -23)
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 2304, 768), (129, 4100, 64), (64, 3072, 768), (300, 768, 3072), (937, 2304, 768), (320, 3072, 768), (30, 128, 128)])
+def test_no_term_of_the_product_is_missing(cuda, m, n, k):
+    """Operands of one sign whose terms all are too: without one of the six products of terms every sum lacks 2^-18 of itself or more (3.7e-6); the
+    tensor core's sums, cut and not rounded, lose up to an ulp of 2^-24 at each of the four steps of 64 k, and the additions in f32 half an ulp
+    each, at random: below 2^-21. Of either sign: not above plain f32 (half as much again allowed, the orders of the sums differ)."""
+    x, w, g = operands(m, n, k, cuda)
+    plain = torch.cat([ops.matmul_f32(r.contiguous(), w) for r in x.split(8)])
+    assert rms(product(x, w), x, w) <= 1.5 * rms(plain, x, w)
+    for a, b in ((x.abs(), w.abs()), (_three_terms((m, k), g), _three_terms((k, n), g))):
+        assert rms(product(a, b), a, b) <= 2.0 ** -21
