@@ -459,7 +459,8 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         if (nr) return fail(GPTRS_EXECUTION, std::string("ncclAllReduce: ") + nccl->GetErrorString(nr));
         return GPTRS_OK;
     };
-    auto norm = [&](const Lane& ln, Tensor* g, Tensor* b) {
+    // behind: the projection that reads the rows next
+    auto norm = [&](const Lane& ln, Tensor* g, Tensor* b, const Weight& behind) {
         ++m.launches;
         const float* delta = pending;
         pending = nullptr;
@@ -470,7 +471,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
             return add_norm_peer(h, delta, m.peer, m.d_status.as<int32_t>(), kPeerSpinLimit, (const float*)g->data,
                                  gpt ? (const float*)b->data : nullptr, c.norm_eps, xn, act_dt, ln.T, D, gpt, ln.st);
         }
-        if (m.x_planes.p && !delta && ln.T >= kSplitF32Rows && ln.st == m.stream && norm_planes_takes(D)) {   // split for the projection behind it
+        if (behind.planes && !delta && ln.T >= kSplitF32Rows && ln.st == m.stream && norm_planes_takes(D)) {   // split for it
             m.planes.leave(xn, ln.T, D);
             return norm_planes(h, (const float*)g->data, gpt && b ? (const float*)b->data : nullptr, c.norm_eps, gpt, static_cast<float*>(xn), m.planes_at(), ln.T, D, ln.st);
         }
@@ -493,7 +494,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
             f = fold32_for(L.ln1_g, L.ln1_b);
             if ((r = linear(m, L.qkv, at(m.hidden, (size_t)D * 4, ln), qkv, ln.T, false, nullptr, false, false, ln.st, &f))) return r;
         } else if (folded && l > 0) f = fold_for(ln, m.layers[l - 1].mlp_out);  // the previous block's last projection left bf16(hidden * gain) and the row sums
-        else if ((r = norm(ln, L.ln1_g, L.ln1_b))) return r;
+        else if ((r = norm(ln, L.ln1_g, L.ln1_b, L.qkv))) return r;
         if (rope_folded) {
             f.rope_positions = ints(m.d_pos, ln);
             f.rope_slot = ints(m.d_slot, ln);
@@ -577,7 +578,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         int r;
         const bool folded = fold;
         if ((r = row_parallel(ln, L.attn_out, at(m.attn, (size_t)m.QD() * act, ln), folded ? L.ln2_g : nullptr))) return r;
-        if (!folded && !fold32 && (r = norm(ln, L.ln2_g, L.ln2_b))) return r;
+        if (!folded && !fold32 && (r = norm(ln, L.ln2_g, L.ln2_b, gpt ? L.mlp_in : m.f32() ? L.mlp_gate : L.mlp_gate_up))) return r;
         void* xn = fold32 ? at(m.hidden, (size_t)D * 4, ln) : at(m.xn, (size_t)D * act, ln);
         void* mlp_h = at(m.mlp_h, (size_t)c.d_mlp * act, ln);
         NormFold f32n;
@@ -636,7 +637,7 @@ int enqueue_forward(Model& m, int T, int max_ctx, int chunk_pages, int n_rows, b
         GPTRS_CUDA_OK(cudaStreamWaitEvent(st, m.ev_join, 0));
     }
     const Lane whole = {st, 0, T, chunk_pages, nullptr, 0};
-    if (!fold32 && (rc = norm(whole, m.final_g, m.final_b))) return rc;
+    if (!fold32 && (rc = norm(whole, m.final_g, m.final_b, m.lm_head))) return rc;
     const void* xr = fold32 ? m.hidden.p : m.xn.p;  // f32: lm_head normalises its rows itself
     if (!rows_identity) {
         ++m.launches;
