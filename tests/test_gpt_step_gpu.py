@@ -37,3 +37,17 @@ def test_contexts_around_chunk_edges(cuda, heads, lengths):
     got, _ = m.forward_with_decode_cache(given[3], list(range(batch)), [n + 3 for n in lengths], list(range(batch)))   # one row: the kernel itself
     # f32 sums of up to 3072 terms in another order, two layers: 3e-7 of the logits, four times that and the oracle's own
     assert np.sqrt(np.mean((got - want) ** 2)) <= 3e-6 * np.sqrt(np.mean(want ** 2))
+
+
+@pytest.mark.parametrize("batch", [1, 8])
+def test_a_step_is_one_launch(cuda, batch):
+    cfg = mr.Cfg("gpt", n_layers=2, d_model=768, n_q=12, n_kv=12, hd=64, d_mlp=3072, vocab=96, ctx=32)
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 768, 12, 12, 64, 3072, 96, 32, cfg.eps, max_seqs=batch, max_tokens=64, max_logit_rows=batch), namespace=8790)
+    for name, w in mr.random_params(cfg, seed=1, std=0.02).items():
+        m.load_param(name, w)
+    m.finalize()
+    m.prefill_many(list(range(batch)), [np.arange(4)] * batch)
+    gen, before = gm.Generator(m, [1] * batch), m.stats()["kernel_launches"]
+    gen.step()
+    gen.step([2] * batch)
+    assert m.stats()["kernel_launches"] == before + 2

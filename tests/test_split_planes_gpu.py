@@ -103,3 +103,24 @@ def test_no_term_of_the_product_is_missing(cuda, m, n, k):
     assert rms(product(x, w), x, w) <= 1.5 * rms(plain, x, w)
     for a, b in ((x.abs(), w.abs()), (_three_terms((m, k), g), _three_terms((k, n), g))):
         assert rms(product(a, b), a, b) <= 2.0 ** -21
+
+
+def launches(kind, d, heads, d_mlp, layers, rows=40):
+    hd, gpt = d // heads, kind == "gpt"
+    cfg = mr.Cfg(kind, n_layers=layers, d_model=d, n_q=heads, n_kv=heads, hd=hd, d_mlp=d_mlp, vocab=32, ctx=64, rot=0 if gpt else hd, theta=1e4)
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT if gpt else gm.KIND_MINISTRAL, layers, d, heads, heads, hd, d_mlp, 32, 64, cfg.eps, cfg.theta, cfg.rot, max_seqs=1,
+                                      max_tokens=64, max_logit_rows=1), namespace=9900 + d)
+    for name, w in mr.random_params(cfg, seed=1, std=0.05).items():
+        m.load_param(name, w)
+    m.finalize()
+    before = m.stats()["kernel_launches"]
+    m.forward_with_decode_cache([1] * rows, [0] * rows, list(range(rows)), [rows - 1])
+    return m.stats()["kernel_launches"] - before
+
+
+# A layer's launches: a norm, qkv, the cache, attention, the output projection, a norm, the MLP in and out (ministral: the rotation, gate and up for MLP in, swiglu),
+# and a split of its rows in front of every projection on planes that no norm of up to 2048 columns, a multiple of 128, and no gelu has split them for.
+@pytest.mark.parametrize("kind,d,heads,d_mlp,splits", [("gpt", 256, 4, 1024, 1), ("gpt", 192, 3, 328, 3), ("gpt", 2176, 34, 192, 3), ("gpt", 40, 1, 80, 0),
+                                                       ("ministral", 256, 4, 512, 3), ("ministral", 320, 5, 328, 4)])
+def test_projections_run_on_planes(cuda, kind, d, heads, d_mlp, splits):
+    assert launches(kind, d, heads, d_mlp, 3) - launches(kind, d, heads, d_mlp, 2) == (8 if kind == "gpt" else 11) + splits
