@@ -221,7 +221,7 @@ struct Model {
     // f32 GPT kind, up to eight sequences: the whole decode step as one cooperative kernel (gpt_decode_mega.cu)
     int mega_rows = 0;   // most sequences of a step that is one kernel (0: none)
     Tensor* wide = nullptr;         // W4 prompts: the widened weights of one projection at a time (a block of the tensor pool: a dropped f32 leaf's)
-    DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors + barrier word
+    DevBuf mega_wt, mega_scratch;   // transposed weights [out][in]; vectors that cross phases, as words
     MegaParams mega = {};
     // quantised Ministral kind, a few sequences: the same (quant_step.cu)
     int qstep_rows = 0;
