@@ -25,7 +25,9 @@
 #include "umma_common.cuh"
 
 namespace gptrs {
-int* matmul_status_word();   // umma_matmul.cu
+// umma_matmul.cu: the library's per-device status word, and the polls of a wait and the test switch of gptrs_cuda_debug_matmul_fault
+int* matmul_status_word();
+void matmul_wait_limits(uint32_t* spin_limit, int* starve);
 namespace {
 
 constexpr int kBlock = 128 * 128;   // bytes of 128 rows of 128
@@ -83,6 +85,8 @@ struct KernelParams {
     CUtensorMap w12, w3, x12, x3;
     PlanesMatmul q;
     int n_split;
+    uint32_t spin_limit;
+    int starve;         // test switch: the products of the first stage are never begun
 };
 
 // 32 lanes x 16 columns of this warp's quarter of the tensor memory
@@ -101,8 +105,10 @@ template <int BN> constexpr int kStages = BN >= 128 ? 2 : 3;   // of 64 k
 template <int BN> constexpr int kLeads = BN == 32 ? 4 : 1;     // leading sums of a stage (four of 64 rows do not fit beside three stages' others)
 template <int BN> constexpr int kStageBytes = 3 * kBlock + 3 * BN * 128;
 
-template <int BN>
+// DEBUG: the wait limits and the test switch of the call
+template <int BN, bool DEBUG = false>
 __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid_constant__ KernelParams kp) {
+    const uint32_t limit = DEBUG ? kp.spin_limit : kSpinLimit;
     constexpr int S = kStages<BN>, L = kLeads<BN>, kStage = kStageBytes<BN>, kX = BN * 128, kSumCols = BN >= 64 ? BN / 2 : 32;   // columns of a summing thread
     constexpr int kSumWarps = 4 * (BN / kSumCols);
     constexpr uint32_t kCols = (S * L + 1) * BN > 256 ? 512 : 256;
@@ -132,7 +138,7 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
     pdl_launch_dependents();
     bool failed = false;
     auto wait = [&](uint64_t* bar, uint32_t parity) {
-        if (!failed && !mbar_wait_relaxed(bar, parity)) failed = true;
+        if (!failed && !mbar_wait_relaxed(bar, parity, limit)) failed = true;
         failed = __any_sync(0xffffffffu, failed);
         return !failed;
     };
@@ -169,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
             __syncwarp();
             last = it + 1;
         }
-        for (int i = max(last - S, 0); i < last; ++i) mbar_wait_relaxed(&full[i % S], (uint32_t)(i / S) & 1u);   // what is in flight writes this CTA's shared memory
+        for (int i = max(last - S, 0); i < last; ++i) mbar_wait_relaxed(&full[i % S], (uint32_t)(i / S) & 1u, limit);   // what is in flight writes this CTA's shared memory
     } else if (warp == 9) {
         // One elected thread waits and issues for the whole loop: with the warp voting at every wait, lane 0 issuing and a commit per consumer, a
         // stage of 128 rows took 1.45 us instead of 0.95, one of 32 rows 1.25 instead of 0.68.
@@ -177,8 +183,9 @@ __global__ void __launch_bounds__(kThreads, 1) planes_matmul_kernel(const __grid
             int s = 0;
             uint32_t phase = 0;
             for (int it = 0; it < n_k; ++it) {
-                if (it >= S && !mbar_wait_relaxed(&lead_empty[s], phase ^ 1u)) { failed = true; break; }
-                if (!mbar_wait_relaxed(&full[s], phase)) { failed = true; break; }
+                if (it >= S && !mbar_wait_relaxed(&lead_empty[s], phase ^ 1u, limit)) { failed = true; break; }
+                if (!mbar_wait_relaxed(&full[s], phase, limit)) { failed = true; break; }
+                if (DEBUG && kp.starve) break;
                 tc_fence_after();
                 const uint32_t at = smem_u32(smem) + (uint32_t)(s * kStage);
                 const uint32_t lead = tmem + (uint32_t)(s * L * BN), rest = tmem + (uint32_t)(S * L * BN);
@@ -373,7 +380,8 @@ template <int BN>
 int allow_smem() {
     static PerDeviceOnce once;
     if (once.first_time())
-        GPTRS_CUDA_OK(cudaFuncSetAttribute(planes_matmul_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem<BN>));
+        for (auto k : {planes_matmul_kernel<BN>, planes_matmul_kernel<BN, true>})
+            GPTRS_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem<BN>));
     return GPTRS_OK;
 }
 
@@ -415,7 +423,8 @@ int launch(const PlanesMatmul& q, int split, cudaStream_t st) {
     if ((rc = make_map(&p.w12, w, 2 * (uint64_t)q.K, (uint64_t)q.N, 128)) || (rc = make_map(&p.w3, w + (size_t)q.N * 2 * q.K, (uint64_t)q.K, (uint64_t)q.N, 128)) ||
         (rc = make_map(&p.x12, x, 2 * (uint64_t)q.K, (uint64_t)q.M, BN)) || (rc = make_map(&p.x3, x + (size_t)q.M * 2 * q.K, (uint64_t)q.K, (uint64_t)q.M, BN))) return rc;
     p.n_split = split;
-    return launch_kernel(planes_matmul_kernel<BN>, dim3((unsigned)ceil_div(q.N, 128), (unsigned)p.n_split, (unsigned)ceil_div(q.M, BN)), dim3(kThreads), kSmem<BN>, st, p.n_split, p);
+    matmul_wait_limits(&p.spin_limit, &p.starve);
+    return launch_kernel(p.starve || p.spin_limit != kSpinLimit ? planes_matmul_kernel<BN, true> : planes_matmul_kernel<BN>, dim3((unsigned)ceil_div(q.N, 128), (unsigned)p.n_split, (unsigned)ceil_div(q.M, BN)), dim3(kThreads), kSmem<BN>, st, p.n_split, p);
 }
 
 // The rows of a tile and the parts of K that make the last CTA end soonest, in hundredths of a microsecond as measured on GPT-2's projections

@@ -182,7 +182,7 @@ int gptrs_cuda_matmul_status(int32_t* h_status);
 
 /* Test switch for the failure path of the tensor-core matmuls (no counterpart in the reference; its GPU backend
  * has no device-side waits). While `starve` is non-zero every decode-sized launch (17..64 rows) withholds the
- * first activation tile, and the f32 matmul on the tensor cores the products of its first stage, so the waits
+ * first activation tile, and the f32 matmuls on the tensor cores the products of their first stage, so the waits
  * that depend on it run out after `spin_limit` polls (0 = the built-in limit of 2^20); the kernel then records
  * code 3 in its status word, frees its tensor memory and returns with an unspecified result. Nothing faults
  * and nothing waits without a bound. Process-wide; call with (0, 0) to switch it off again. */

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from gptrs_b200 import check, lib, ops
+from gptrs_b200 import BackendError, check, lib, ops
 from gptrs_b200 import model as gm
 from oracle import models_ref as mr
 
@@ -56,12 +56,18 @@ def test_terms_that_overflow_bf16(cuda, rows):
     run(256, 4, 512, rows, edit)
 
 
-def product(x, w):
+@pytest.fixture
+def starved():
+    yield lambda limit=2000: check(lib().gptrs_cuda_debug_matmul_fault(1, limit))
+    check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
+
+
+def product(x, w, status=0):
     (m, k), n = x.shape, w.shape[1]
     y, planes = torch.empty(m, n, device=x.device), torch.empty(6 * k * (m + n) + 256, dtype=torch.uint8, device=x.device)
     check(lib().gptrs_cuda_debug_planes_matmul(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), m, n, k, 0, planes.data_ptr(), planes.numel(),
                                                torch.cuda.current_stream().cuda_stream))
-    assert ops.matmul_status() == 0
+    assert ops.matmul_status() == status
     return y
 
 
@@ -124,3 +130,31 @@ def launches(kind, d, heads, d_mlp, layers, rows=40):
                                                        ("ministral", 256, 4, 512, 3), ("ministral", 320, 5, 328, 4)])
 def test_projections_run_on_planes(cuda, kind, d, heads, d_mlp, splits):
     assert launches(kind, d, heads, d_mlp, 3) - launches(kind, d, heads, d_mlp, 2) == (8 if kind == "gpt" else 11) + splits
+
+
+@pytest.mark.parametrize("m,n,k", [(24, 768, 768), (24, 64, 3072), (64, 2304, 768), (100, 3072, 768), (937, 768, 3072), (937, 3072, 768), (2000, 4096, 128)])
+def test_wait_runs_out_sets_status_and_recovers(cuda, starved, m, n, k):
+    """The products of the first stage withheld, K of fewer and of more stages than the ring has: all who wait give up, and the next launch is as before."""
+    x, w, _ = operands(m, n, k, cuda)
+    good = product(x, w)
+    starved()
+    product(x, w, status=3)   # returns; the result is unspecified
+    check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
+    assert torch.equal(product(x, w), good)
+
+
+def test_engine_reports_a_wait_that_ran_out(cuda, starved):
+    cfg = mr.Cfg("gpt", n_layers=2, d_model=256, n_q=4, n_kv=4, hd=64, d_mlp=1024, vocab=96, ctx=64)
+    m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 256, 4, 4, 64, 1024, 96, 64, cfg.eps, max_seqs=1, max_tokens=64, max_logit_rows=1), namespace=9950)
+    for name, w in mr.random_params(cfg, seed=1, std=0.05).items():
+        m.load_param(name, w)
+    m.finalize()
+    good, _ = m.prefill(0, np.arange(40), want_logits=True)
+    m.reset_sequence(0)
+    starved()
+    with pytest.raises(BackendError) as e:
+        m.prefill(0, np.arange(40))
+    assert e.value.kind == "Execution" and "matmul" in str(e.value)
+    check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
+    m.reset_sequence(0)
+    assert np.array_equal(m.prefill(0, np.arange(40), want_logits=True)[0], good)
