@@ -58,5 +58,7 @@ struct FlagWaiter {
     }
 };
 constexpr uint32_t kFlagPolls = 1u << 23;   // of a thread, over the whole step
+// Polls of a wait on a barrier, of a thread's waits for words, and the test switch of gptrs_cuda_debug_matmul_fault (quant_step.cu).
+void step_wait_limits(uint32_t* spin_limit, uint32_t* flag_polls, int* starve);
 
 }  // namespace gptrs

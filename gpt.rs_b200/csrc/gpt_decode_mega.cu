@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
     float* red = big + p.big_floats;   // [64]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rows = p.rows;
     const int H = p.H, hd = p.hd;
-    FlagWaiter wait = {kFlagPolls, p.status};
+    FlagWaiter wait = {p.flag_polls, p.status};
     int n_time = 0;
     auto stamp = [&]() { if (p.timing && blockIdx.x == 0 && tid == 0) p.timing[n_time++] = global_ns(); };
     stamp();
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) gpt_decode_mega_kernel(const 
         const float* w = at_head ? p.lm_head_t : kind == 0 ? L.w_qkv_t : kind == 1 ? L.w_out_t : kind == 2 ? L.w_mlp_in_t : L.w_mlp_out_t;
         const int n_items = at_head ? p.vocab : kind == 0 ? 3 * kD : kind == 1 ? kD : kMlp;   // MLP out: four chunks of 768 rows
         stamp();
-        gemv_items<R>(rnd, w, n_items, xs, kind == 0 ? p.qkv : kind == 1 ? p.pc : kind == 2 ? p.mh : p.pe, flag, at_head ? p.logits : nullptr, rows, best, best_i,
+        gemv_items<R>(rnd, w, n_items, xs, kind == 0 ? p.qkv : kind == 1 ? p.pc : kind == 2 ? p.mh : p.pe, flag - (p.starve && phase == 0 && blockIdx.x == 0 ? 1u : 0u), at_head ? p.logits : nullptr, rows, best, best_i,
                       kind == 2 ? L.b_mlp_in : nullptr);
         stamp();
         if (at_head) break;
@@ -581,6 +581,8 @@ int mega_launch(MegaParams p, cudaStream_t st) {
         for (auto k : kerns) GPTRS_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMegaSmem));
     const int layout = mega_layout(p.rows);
     p.big_floats = (int)mega_big_floats(layout, p.rows, p.H, p.ctx_cap);
+    uint32_t barrier_polls;
+    step_wait_limits(&barrier_polls, &p.flag_polls, &p.starve);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)sm_count());
     cfg.blockDim = dim3(kMegaThreads);

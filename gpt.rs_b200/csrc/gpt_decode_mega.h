@@ -30,6 +30,8 @@ struct MegaParams {
     unsigned long long* timing;   // optional (GPTRS_MEGA_TIMING=1): globaltimer of CTA 0 at kernel start, where its part in attention has ended, and around every projection
     int H, hd, vocab, ctx_cap, n_pos;
     int big_floats;                  // set by the launcher
+    uint32_t flag_polls;             // of a thread, over the whole step; set by the launcher, too
+    int starve;                      // test switch: the first CTA hands its part of the first projection over with an old flag
     float eps;
     int greedy;
 };

@@ -30,6 +30,11 @@
 #include "quant_step.h"
 
 namespace gptrs {
+void matmul_wait_limits(uint32_t* spin_limit, int* starve);   // umma_matmul.cu
+void step_wait_limits(uint32_t* spin_limit, uint32_t* flag_polls, int* starve) {
+    matmul_wait_limits(spin_limit, starve);
+    *flag_polls = *starve ? *spin_limit : kFlagPolls;
+}
 namespace {
 
 // 15 warps that multiply and the producer: 16 warps may have 128 registers a thread. (With 16 + 1 it is 96; what is spilled then does not fit
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_step_kernel(const __grid_co
     const uint32_t ring_bytes = (uint32_t)p.stages * kStageBytes<BITS>;
     if (warp == kWarps) {
         // ---- the producer: lane w keeps the ring of warp w full ----------------------------------------------------------------------
-        const bool mine = lane < kWarps;
+        const bool mine = lane < kWarps && !(p.starve == 2 && lane == kWarps - 1);
         const uint32_t base = smem_u32(sm + S.ring) + min(lane, kWarps - 1) * ring_bytes;
         uint64_t* const full = bars + min(lane, kWarps - 1) * p.stages * 2;
         int layer = 0, kind = -1, left = 0, stage = 0, grp = 0, G = 1;
@@ -320,8 +325,8 @@ __global__ void __launch_bounds__(kThreads, 1) quant_step_kernel(const __grid_co
     }
 
     // ---- the consumers ---------------------------------------------------------------------------------------------------------------
-    Ring ring = {smem_u32(sm + S.ring) + warp * ring_bytes, smem_u32(bars + warp * p.stages * 2), p.stages, 0, 0u, kSpinLimit};
-    FlagWaiter wait = {kFlagPolls, p.status};
+    Ring ring = {smem_u32(sm + S.ring) + warp * ring_bytes, smem_u32(bars + warp * p.stages * 2), p.stages, 0, 0u, p.ring_polls};
+    FlagWaiter wait = {p.flag_polls, p.status};
     const int g = lane >> 2, t = lane & 3;
     float* const slots = reinterpret_cast<float*>(sm + S.slots);
     float* const h_own = reinterpret_cast<float*>(sm + S.h);   // [row][this CTA's columns]
@@ -699,6 +704,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_step_kernel(const __grid_co
         if (kind == kQkv && attends && warp < kPairs && lane == 0 && pg0 + pair < pg1) load_page(l, first_page);
         // ---- the warps' parts in order, and what the projection does with the sums
         const bool sparse = nt * G < kWarps;   // warps without a unit
+        const uint32_t starved = p.starve == 1 && phase == 0 && t0 == 0 ? 1u : 0u;
 #pragma unroll 1
         for (int i = tid; i < ((items + 31) & ~31); i += kConsumers) {
             const bool live = i < items;
@@ -735,7 +741,7 @@ __global__ void __launch_bounds__(kThreads, 1) quant_step_kernel(const __grid_co
                 const float r = inv[m];
                 v.x *= r; v.y *= r; v.z *= r; v.w *= r;
                 if (kind == kQkv) {
-                    if (live) put_words(ex + E.qkv + (uint32_t)(m * QKV + (t0 + tile) * 16 + c) * 4u, pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w), flag);
+                    if (live) put_words(ex + E.qkv + (uint32_t)(m * QKV + (t0 + tile) * 16 + c) * 4u, pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w), flag - starved);
                 } else {   // a tile: 8 gate channels, then the 8 up channels that go with them
                     float4 up;
                     up.x = __shfl_xor_sync(0xffffffffu, v.x, 2); up.y = __shfl_xor_sync(0xffffffffu, v.y, 2);
@@ -869,6 +875,7 @@ int quant_step_launch(int bits, QuantStepParams p, int max_ctx, cudaStream_t st)
     p.ex = exchange_layout(p.D, p.FF, p.Hq, p.Hkv);
     p.sm = smem_of(bits, p.rows, p.D, p.FF, p.Hq, p.Hkv, p.stages);
     p.splits = slices(max_ctx, p.rows, p.Hkv);
+    step_wait_limits(&p.ring_polls, &p.flag_polls, &p.starve);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kThreads);

@@ -37,6 +37,8 @@ struct QuantStepParams {
     float eps, scale_log2;
     // set by the launcher
     int splits, stages;
+    uint32_t ring_polls, flag_polls;   // of a wait for weights; of a thread for words, over the whole step
+    int starve;                        // test switch, 1: the first tile of the first projection is handed over with an old flag; 2: every CTA's last warp, which has a unit if any has, gets no weights
     StepExchange ex;
     StepSmem sm;
 };

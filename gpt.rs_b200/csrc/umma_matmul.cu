@@ -881,7 +881,7 @@ int umma_status(int* out) {
 }
 
 void umma_debug_fault(int starve, uint32_t spin_limit) {
-    g_debug_starve.store(starve ? 1 : 0);
+    g_debug_starve.store(starve);
     g_debug_spin_limit.store(spin_limit);
 }
 

@@ -184,8 +184,10 @@ int gptrs_cuda_matmul_status(int32_t* h_status);
  * has no device-side waits). While `starve` is non-zero every decode-sized launch (17..64 rows) withholds the
  * first activation tile, and the f32 matmuls on the tensor cores the products of their first stage, so the waits
  * that depend on it run out after `spin_limit` polls (0 = the built-in limit of 2^20); the kernel then records
- * code 3 in its status word, frees its tensor memory and returns with an unspecified result. Nothing faults
- * and nothing waits without a bound. Process-wide; call with (0, 0) to switch it off again. */
+ * code 3 in its status word, frees its tensor memory and returns with an unspecified result. A decode step that is
+ * one kernel withholds a part of its first projection's result (code 5); with `starve` 2 the one of quantised models
+ * withholds weights of one warp per CTA instead (code 3). Nothing faults and nothing waits without a bound.
+ * Process-wide; call with (0, 0) to switch it off again. */
 int gptrs_cuda_debug_matmul_fault(int starve, uint32_t spin_limit);
 /* Debug: y [m][n] = x [m][k] . w [k][n] (+ bias [n]; gelu; + residual [m][n]) in f32 as the engine computes the projections of f32 models in
  * passes of 24 rows and more, from both operands' bf16 planes, which the call makes itself in d_planes (256-byte aligned, 6 k (m + n) + 256

@@ -146,3 +146,41 @@ def test_prefill_attention_wait_runs_out_sets_status_and_recovers(cuda):
     assert torch.equal(again, good)
     a, b = again.float().cpu().numpy(), want.float().cpu().numpy()
     assert np.all(np.abs(a - b) <= 8e-3 * np.maximum(1.0, np.abs(b)))
+
+
+@pytest.mark.parametrize("form,starve", [("gpt", 1), ("w4", 1), ("w8", 1), ("w4", 2), ("w8", 2)])
+@pytest.mark.parametrize("batch", [1, 8])
+def test_steps_of_one_kernel_report_a_wait_that_ran_out(cuda, form, starve, batch):
+    """Words that come with an old flag, and weights that never arrive (starve 2): whoever waits gives up, the step ends with an error, and the same step
+    from the same caches is as before."""
+    if form == "gpt":
+        cfg = mr.Cfg("gpt", n_layers=2, d_model=768, n_q=12, n_kv=12, hd=64, d_mlp=3072, vocab=96, ctx=64)
+        m = gm.LoadedModel(gm.ModelConfig(gm.KIND_GPT, 2, 768, 12, 12, 64, 3072, 96, 64, cfg.eps, max_seqs=batch, max_tokens=64, max_logit_rows=batch), namespace=8810)
+    else:
+        cfg = mr.Cfg("ministral", n_layers=2, d_model=256, n_q=4, n_kv=2, hd=128, d_mlp=512, vocab=512, ctx=64, rot=128, theta=1e6)
+        m = gm.LoadedModel(gm.ModelConfig(gm.KIND_MINISTRAL, 2, 256, 4, 2, 128, 512, 512, 64, cfg.eps, cfg.theta, 128, max_seqs=batch, max_tokens=64, max_logit_rows=batch,
+                                          weight_mode=gm.MODE_W4A16 if form == "w4" else gm.MODE_W8A16, kv_pages=batch * 4 + 4, max_pages_per_seq=4), namespace=8811)
+    for name, w in mr.random_params(cfg, seed=5, std=0.05).items():
+        m.load_param(name, w)
+    m.finalize()
+
+    def begin():
+        for s in range(batch):
+            m.reset_sequence(s)
+        m.prefill_many(list(range(batch)), [np.arange(5) + s for s in range(batch)])
+        return gm.Generator(m, list(range(batch)))
+
+    before = m.stats()["kernel_launches"]
+    gen = begin()
+    launched = m.stats()["kernel_launches"]
+    good = gen.step()
+    assert m.stats()["kernel_launches"] == launched + 1 and launched > before
+    gen = begin()
+    check(lib().gptrs_cuda_debug_matmul_fault(starve, 2000))
+    try:
+        with pytest.raises(BackendError) as e:
+            gen.step()
+    finally:
+        check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
+    assert e.value.kind == "Execution" and "gave up" in str(e.value)
+    assert np.array_equal(begin().step(), good)
