@@ -254,7 +254,7 @@ struct Model {
     // a step of these visible lengths (the longest, all together)
     bool one_kernel_step(int rows, int max_ctx, int64_t all_ctx) const {
         if (rows > std::max(mega_rows, qstep_rows) || rows > max_rows()) return false;
-        return f32() || quant_step_pays(cfg.weight_mode == kModeW4 ? 4 : 8, rows, cfg.n_kv_heads, max_ctx, all_ctx);
+        return f32() || quant_step_pays(cfg.weight_mode == kModeW4 ? 4 : 8, rows, cfg.n_q_heads, cfg.n_kv_heads, max_ctx, all_ctx);
     }
     int max_rows() const { return cfg.max_logit_rows > 0 ? cfg.max_logit_rows : cfg.max_seqs; }
     int stage_stride() const { return std::max(cfg.max_tokens, max_rows()); }

@@ -18,12 +18,17 @@
 //   * every projection runs through one copy of the code: with a copy per projection (180 KB of code) the phases ran from a cold instruction
 //     cache and took three times as long.
 // What bounds it: the widening of the weights (a unit of 16 channels x 128 k costs a scheduler 200 to 230 cycles in W4, of which 112 are the shifts and
-// logic operations at half rate; 350 in W8), then 1.6 to 3 us per exchange. A step, kernel per projection / this one, us: W4 of width 3072, six
-// layers, one sequence 304 / 267, three 349 / 261, seven 453 / 321; width 1024, four layers, one 128 / 110, seven 161 / 115; W8 of width 2048, four
-// layers, one 188 / 159, seven 198 / 172; 8000 tokens, W4, width 2048, one sequence 256 / 207.
+// logic operations at half rate; 350 in W8), then 1.6 to 3 us per exchange. A step, kernel per projection / this one, us, 150 tokens: W4 of width
+// 3072, six layers, one sequence 305 / 263, three 346 / 258, seven 451 / 319; width 1024, four layers, one 128 / 109, seven 158 / 112; W8 of width 2048,
+// four layers, one 187 / 159, seven 197 / 173. 3000 tokens, where it gains least, four layers: W4 of width 3072, one 231 / 219, of width 1024 136 / 130; W8
+// of width 1024, eight 164 / 160, of width 2048 232 / 231. 8000 tokens, W4 of width 2048, one 255 / 178. Other lengths and where it is not taken:
+// quant_step_max_rows and quant_step_pays. It has every SM for itself: two models that step on two threads take turns (one sequence each, four
+// layers, us a step, W4 of width 3072 287 / 344, of width 1024 170 / 176; W8 of width 2048 241 / 279); GPTRS_QUANT_STEP=0 at finalize leaves a model with
+// the kernel per projection.
 // Arithmetic of the tiles as in w4_gemv_kernel / quant_matmul_kernel: exact integers in bf16 through mma.sync, group scales on f32 sums.
 // Every wait is bounded: a thread that gives up records a status and stops waiting (code 5; ring or page copies: 3).
 #include <algorithm>
+#include <climits>
 
 #include "flag_words.cuh"
 #include "matmul_common.cuh"
@@ -31,6 +36,7 @@
 
 namespace gptrs {
 void matmul_wait_limits(uint32_t* spin_limit, int* starve);   // umma_matmul.cu
+int attention_step_splits(int64_t max_ctx_len, int64_t n_tokens, int64_t n_q_heads, int64_t n_kv_heads);   // paged_attention.cu
 void step_wait_limits(uint32_t* spin_limit, uint32_t* flag_polls, int* starve) {
     matmul_wait_limits(spin_limit, starve);
     *flag_polls = *starve ? *spin_limit : kFlagPolls;
@@ -843,23 +849,27 @@ int quant_step_max_rows(int bits, int n_layers, int D, int FF, int Hq, int Hkv, 
     if (n_layers < 1 || n_layers > kStepMaxLayers || D % 128 || FF % 128 || vocab % 16 || Hq % Hkv || Hq / Hkv > 8 || sm_count() > 256) return 0;
     if (max_tiles(D, FF, Hq, Hkv) > 32) return 0;
     int n = 0;
-    // W8 rings of two stages lose against a kernel per projection (width 3072, 7 and 8 rows 376 -> 386, 395 -> 439 us a step of six layers;
-    // with three stages, 5 rows, 369 -> 348)
-    while (n < kStepMaxRows && (n + 1) * Hkv <= sm_count() && ring_stages(bits, n + 1, D, FF, Hq, Hkv) >= (bits == 4 ? 2 : 3)) ++n;
+    // W8 rings of two stages lose against a kernel per projection (width 3072, 7 and 8 rows 376 -> 386, 395 -> 439 us a step of six layers).
+    // With three it is the rows of the longest projection that decide, which every CTA reads: 6 x 9216 values lose at every length (four layers,
+    // 20 / 300 / 3000 / 12000 tokens, kernel by kernel / here: 264 / 267, 272 / 281, 314 / 332, 488 / 529), 8 x 6144 (196 / 180, 200 / 189,
+    // 232 / 231) and 5 x 9216 (264 / 245, 270 / 258; 3000 tokens: quant_step_pays) win.
+    const int k_max = std::max({D, FF, Hq * 128}), most_x = bits == 4 ? INT_MAX : 48 * 1024;
+    while (n < kStepMaxRows && (n + 1) * Hkv <= sm_count() && (n + 1) * k_max <= most_x && ring_stages(bits, n + 1, D, FF, Hq, Hkv) >= (bits == 4 ? 2 : 3)) ++n;
     return n;
 }
-// Whether a step is faster here than kernel by kernel: what attention takes longer, in us of a layer, against what the rest is faster (the least
-// of widths 1024, 2048 and 3072, 11.5 in W4 and 7.8 in W8). Here it is rounds of pages and slices to add up (see `slices`), and all rows have as
+// Whether a step is faster here than kernel by kernel: what attention takes longer, in us of a layer, against what the rest is faster (widths 1024,
+// 2048 and 3072, 1 to 8 rows: 11.5 in W4; in W8 5.2 while attention there is one kernel, and 7.8 where it has become three). Here it is rounds of pages and slices to add up (see `slices`), and all rows have as
 // many CTAs; there long rows have more splits and two pages per warp under way: at least 0.6 us per 1000 tokens of the longest row, or all
 // pages at 6.1 TB/s. Four layers, us, kernel by kernel / here: W4 of width 3072, 8 rows at 3000 tokens 409 / 330, 8000 511 / 502, 16000
 // 713 / 805; one of 8000 among short ones 364 / 458, of 32000 508 / 1224; 4 rows at 8000 366 / 330, 16000 491 / 496; W4 of width 2048, 8 rows at
-// 16000 424 / 423, 32000 574 / 652; W8 of width 2048, 8 rows at 3000 234 / 229, one of 3000 217 / 224, 4 rows at 16000 340 / 281, one of 16000
-// 255 / 270; one row is faster here at every length up to 32000 (W4 of width 3072 there 445 / 380, W8 of width 1024 at 3000 141 / 140).
-bool quant_step_pays(int bits, int rows, int n_kv_heads, int max_ctx, int64_t all_ctx) {
+// 16000 424 / 423, 32000 574 / 652; W8 of width 2048, 8 rows at 3000 232 / 231, 6000 298 / 275, one of 2000 210 / 211, one of 3000 217 / 224, 4 rows at
+// 16000 340 / 281, one of 16000 255 / 270; W8 of width 3072, 5 rows at 1000 278 / 273, 3000 307 / 310, 4 rows at 3000 299 / 289; one row is faster
+// here at every length up to 32000 (W4 of width 3072 there 445 / 380, W8 of widths 1024 and 3072 at 3000 146 / 140, 275 / 273).
+bool quant_step_pays(int bits, int rows, int n_q_heads, int n_kv_heads, int max_ctx, int64_t all_ctx) {
     const int s = slices(max_ctx, rows, n_kv_heads);
     const double here = 1.5 * ceil_div(ceil_div(max_ctx, 16), kPairs * s) + 0.3 * (s - 1);
     const double there = std::max(1.5 + 0.0006 * max_ctx, (double)all_ctx * n_kv_heads * 512 / 6.1e6);
-    return here - there < (bits == 4 ? 11.5 : 7.8);
+    return here - there < (bits == 4 ? 11.5 : attention_step_splits(max_ctx, rows, n_q_heads, n_kv_heads) ? 5.2 : 7.8);
 }
 size_t quant_step_exchange_bytes(int D, int FF, int Hq, int Hkv) { return exchange_layout(D, FF, Hq, Hkv).total; }
 

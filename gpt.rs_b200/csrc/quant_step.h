@@ -46,7 +46,7 @@ struct QuantStepParams {
 // Most sequences of a step of this shape on this device, 0: the shape is not taken.
 int quant_step_max_rows(int bits, int n_layers, int D, int FF, int Hq, int Hkv, int vocab);
 // Whether a step of these lengths (the longest, all together) is faster as one kernel.
-bool quant_step_pays(int bits, int rows, int n_kv_heads, int max_ctx, int64_t all_ctx);
+bool quant_step_pays(int bits, int rows, int n_q_heads, int n_kv_heads, int max_ctx, int64_t all_ctx);
 size_t quant_step_exchange_bytes(int D, int FF, int Hq, int Hkv);
 // max_ctx: the longest visible length of the step's sequences (sizes the splits of attention).
 int quant_step_launch(int bits, QuantStepParams p, int max_ctx, cudaStream_t st);
