@@ -760,10 +760,13 @@ int setup_mega(Model& m) {
     return GPTRS_OK;
 }
 
-// bf16 planes of the layers' f32 weights, for passes of many rows: six bytes more per weight, so only for models whose planes take 2 GiB at
-// most and where the memory is there; other models split inside their tiles.
+// bf16 planes of the layers' f32 weights, for passes of many rows: six bytes more per weight, beside four of the leaves and, for the steps of
+// one kernel, four of the transposed copies (GPT-2 small: 510 MB, 340 and 494; splitting takes 1 to 2 ms of finalize), and 12 bytes per value of a pass's widest rows. No
+// measured line: they pay at every size that was looked at, and 2 GiB (358 M weights of the layers) is what they may take of the memory; larger
+// models, and those that it has no room for, split inside their tiles. GPTRS_F32_PLANES=0 at finalize leaves a model without.
 int setup_planes(Model& m) {
     const auto& c = m.cfg;
+    if (const char* e = getenv("GPTRS_F32_PLANES")) if (atoi(e) == 0) return GPTRS_OK;
     if (!m.f32() || c.max_tokens < kSplitF32Rows) return GPTRS_OK;
     std::vector<Weight*> all;
     for (Layer& L : m.layers)

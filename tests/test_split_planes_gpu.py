@@ -158,3 +158,9 @@ def test_engine_reports_a_wait_that_ran_out(cuda, starved):
     check(lib().gptrs_cuda_debug_matmul_fault(0, 0))
     m.reset_sequence(0)
     assert np.array_equal(m.prefill(0, np.arange(40), want_logits=True)[0], good)
+
+
+def test_a_model_without_planes(cuda, monkeypatch):
+    monkeypatch.setenv("GPTRS_F32_PLANES", "0")
+    assert launches("gpt", 256, 4, 1024, 3) - launches("gpt", 256, 4, 1024, 2) == 8   # no splits
+    run(256, 4, 1024, 128)
