@@ -59,3 +59,38 @@ def test_two_threads_two_models(cuda):
     check(lib().gptrs_cuda_destroy(backend))
     bad = ctypes.c_void_p()
     assert lib().gptrs_cuda_create(99, ctypes.byref(bad)) != 0
+
+
+@pytest.mark.parametrize("mode", [gm.MODE_W4A16, gm.MODE_W8A16, None])   # None: GPT-2's widths
+def test_two_threads_whose_steps_take_every_sm(cuda, mode):
+    """Steps of a few sequences are one cooperative kernel with a CTA per SM, whose CTAs wait for each other: two models' take turns."""
+    def model(seed):
+        if mode is None:
+            cfg = mr.Cfg("gpt", n_layers=2, d_model=768, n_q=12, n_kv=12, hd=64, d_mlp=3072, vocab=512, ctx=64)
+            mc = gm.ModelConfig(gm.KIND_GPT, 2, 768, 12, 12, 64, 3072, 512, 64, cfg.eps, max_seqs=3, max_tokens=64, max_logit_rows=3)
+        else:
+            cfg = CFG
+            mc = gm.ModelConfig(gm.KIND_MINISTRAL, CFG.n_layers, CFG.d_model, CFG.n_q, CFG.n_kv, CFG.hd, CFG.d_mlp, CFG.vocab, CFG.ctx, CFG.eps, CFG.theta, CFG.rot,
+                                weight_mode=mode, max_seqs=3, max_tokens=64, max_logit_rows=3, kv_pages=22, max_pages_per_seq=6, use_pdl=1)
+        m = gm.LoadedModel(mc, namespace=9110 + seed)
+        for name, w in mr.random_params(cfg, seed=seed, std=0.05).items():
+            m.load_param(name, w)
+        m.finalize()
+        return m
+
+    def generate(m, out, key):
+        first = m.prefill_many([0, 1, 2], [np.arange(n) * 7 % 512 for n in (3, 9, 14)])
+        gen, before = gm.Generator(m, first), m.stats()["kernel_launches"]
+        out[key] = [gen.step().tolist() for _ in range(40)]
+        out[key, "launches"] = m.stats()["kernel_launches"] - before
+
+    serial, parallel = {}, {}
+    for key in (1, 2):
+        generate(model(key), serial, key)
+    models = [model(key) for key in (1, 2)]
+    threads = [threading.Thread(target=generate, args=(m, parallel, key)) for key, m in zip((1, 2), models)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert parallel == serial and serial[1, "launches"] == 40 and serial[1] != serial[2]
